@@ -368,3 +368,127 @@ def tolerance(case):
         return {"rel": 1.7e-3, "max": 3e-2}
     rows = case["kind"] == "train" or (case["kind"] == "sdpa" and case["seq_q"] > 1)
     return {"rel": 1.2e-2 if case["kind"] == "mha" else 1e-2, "max": 0.45 if rows else 7e-2}
+
+
+# ---- the same in 64 bits ------------------------------------------------------------------------------------------------
+
+def _attend(q, k, v, scale, visible=None, softcap=0.0, bias=None, dout=None):
+    """softmax(scale q k^T) v of one (sequence, head) in float64, some rows at a time: q [Sq, D], k and v [Sk, D],
+    ``visible(rows)`` and ``bias`` of [rows, Sk].  Returns the output and the log-sum-exp, and with ``dout`` the three
+    gradients too."""
+    rows = max(1, (1 << 26) // k.shape[0])
+    out, lse, dq = torch.empty_like(q), torch.empty_like(q[:, 0]), torch.empty_like(q)
+    dk, dv = torch.zeros_like(k), torch.zeros_like(v)
+    for first in range(0, q.shape[0], rows):
+        at = slice(first, min(q.shape[0], first + rows))
+        s = (q[at] @ k.T) * scale
+        if softcap:
+            s = softcap * torch.tanh(s / softcap)
+        if bias is not None:
+            s = s + bias[at].double()
+        if visible is not None:
+            s = s.masked_fill(~visible(torch.arange(at.start, at.stop, device=q.device)), float("-inf"))
+        lse[at] = torch.logsumexp(s, 1)
+        p = torch.exp(s - lse[at, None])
+        out[at] = p @ v
+        if dout is not None:
+            ds = p * (dout[at] @ v.T - (dout[at] * out[at]).sum(1, keepdim=True))
+            dq[at] = scale * (ds @ k)
+            dk += scale * (ds.T @ q[at])
+            dv += p.T @ dout[at]
+    return (out, lse) if dout is None else (out, lse, dq, dk, dv)
+
+
+def _rotated(x, cos, sin, positions):
+    """Interleaved RoPE of x [tokens, heads, D] at the tokens' positions."""
+    half = x.shape[2] // 2
+    c, s = (t.tensor.view(-1, half)[positions].double()[:, None] for t in (cos, sin))
+    even, odd = x[..., 0::2], x[..., 1::2]
+    return torch.stack((even * c - odd * s, even * s + odd * c), -1).flatten(2)
+
+
+def exact(case, seed):
+    """What ``run`` returns, evaluated in float64 with no rounding in between."""
+    st = prepare(case, seed)
+    kind, scale = case["kind"], case.get("dim", 64) ** -0.5
+
+    def wide(name, *shape):
+        return st[name].tensor.double().view(*shape)
+
+    if kind == "sdpa":
+        b, hq, hkv, sq, sk, d = (case[k] for k in ("batch", "heads", "kv_heads", "seq_q", "seq_k", "dim"))
+        q, out = st["q"].tensor.view(b, hq, sq, d), torch.empty(b, hq, sq, d, dtype=torch.float64, device="cuda")
+        k, v = (st[name].tensor.view(b, hkv, sk, d) for name in ("k", "v"))
+        keys = torch.arange(sk, device="cuda")
+        keep = st["mask"].tensor.view(sq, sk) != 0 if st["mask"] is not None else None
+        lens = st["lengths"].tensor.tolist() if st["lengths"] is not None else [sk] * b
+        for i in range(b):
+            def visible(rows):
+                seen = (keys < lens[i])[None, :].expand(len(rows), sk)
+                if case["causal"]:
+                    seen = seen & (keys[None, :] <= rows[:, None] + (sk - sq))
+                return seen if keep is None else seen & keep[rows]
+            for h in range(hq):
+                kv = h // (hq // hkv)
+                out[i, h] = _attend(q[i, h].double(), k[i, kv].double(), v[i, kv].double(), scale, visible,
+                                    case["softcap"])[0]
+        return out.view(-1)
+    if kind == "chunk":
+        t, hq, hkv, d, bs, start = (case[k] for k in ("tokens", "heads", "kv_heads", "dim", "block", "start"))
+        keys = torch.arange(start + t, device="cuda")
+        rows = st["table"].tensor.long()[keys // bs] * bs + keys % bs
+        k, v = wide("k", -1, hkv, d), wide("v", -1, hkv, d)
+        k[rows[start:]], v[rows[start:]] = wide("new_k", t, hkv, d), wide("new_v", t, hkv, d)
+        q, out = wide("q", t, hq, d), torch.empty(t, hq, d, dtype=torch.float64, device="cuda")
+        for h in range(hq):
+            kv = h // (hq // hkv)
+            out[:, h] = _attend(q[:, h], k[rows, kv], v[rows, kv], scale,
+                                lambda r: keys[None, :] <= r[:, None] + start)[0]
+        return {"out": out.view(-1), "keys": k.view(-1), "values": v.view(-1)}
+    if kind in ("step", "token"):
+        if kind == "step":
+            n, hq, hkv, d, bs = (case[k] for k in ("batch", "heads", "kv_heads", "dim", "block"))
+            positions, cache_rows = st["positions"].tensor.long(), st["cache_rows"].tensor.long()
+            table, lens = st["table"].tensor.long().view(n, -1), st["lengths"].tensor.tolist()
+        else:
+            n, hq, hkv, d = 1, case["heads"], case["heads"], 64
+            positions = cache_rows = torch.tensor([case["position"]], device="cuda")
+            lens = [case["position"] + 1]
+        y = wide("x", n, -1) @ wide("w", (hq + 2 * hkv) * d, -1).T + st["bias"].tensor.double()
+        q, new_k, new_v = y.view(n, hq + 2 * hkv, d).split((hq, hkv, hkv), 1)
+        q, k, v = _rotated(q, st["cos"], st["sin"], positions), wide("k", -1, hkv, d), wide("v", -1, hkv, d)
+        k[cache_rows], v[cache_rows] = _rotated(new_k, st["cos"], st["sin"], positions), new_v
+        out = torch.empty(n, hq, d, dtype=torch.float64, device="cuda")
+        for i in range(n):
+            rows = torch.arange(lens[i], device="cuda")
+            if kind == "step":
+                rows = table[i, rows // bs] * bs + rows % bs
+            for h in range(hq):
+                kv = h // (hq // hkv)
+                out[i, h] = _attend(q[i, h:h + 1], k[rows, kv], v[rows, kv], scale)[0][0]
+        return {"out": out.view(-1), "query": q.reshape(-1), "keys": k.view(-1), "values": v.view(-1)}
+    if kind == "train":
+        b, h, s, d = (case[k] for k in ("batch", "heads", "seq", "dim"))
+        got = {name: torch.empty(b, h, s, *size, dtype=torch.float64, device="cuda")
+               for name, size in (("out", (d,)), ("stats", ()), ("dq", (d,)), ("dk", (d,)), ("dv", (d,)))}
+        ins = [st[name].tensor.view(b, h, s, d) for name in ("q", "k", "v", "dout")]
+        bias = st["bias"].tensor.view(h, s, s) if case["bias"] else None
+        keys = torch.arange(s, device="cuda")
+        visible = (lambda r: keys[None, :] <= r[:, None]) if case["causal"] else None
+        for i in range(b):
+            for j in range(h):
+                q, k, v, dout = (t[i, j].double() for t in ins)
+                for name, x in zip(got, _attend(q, k, v, scale, visible, bias=None if bias is None else bias[j],
+                                                dout=dout)):
+                    got[name][i, j] = x
+        return {name: x.view(-1) for name, x in got.items()}
+    b, s, h, d = (case[k] for k in ("batch", "seq", "heads", "dim"))
+    x = wide("x", b * s, h * d)
+    q, k, v = ((x @ w.tensor.double().view(h * d, h * d)).view(b, s, h, d) for w in st["w"][:3])
+    keep = st["mask"].tensor.view(b, s) != 0 if case["mask"] else None
+    out = torch.empty(b, s, h, d, dtype=torch.float64, device="cuda")
+    for i in range(b):
+        for j in range(h):
+            out[i, :, j] = _attend(q[i, :, j], k[i, :, j], v[i, :, j], scale,
+                                   None if keep is None else lambda r: keep[i][None, :].expand(len(r), s))[0]
+    return (out.view(b * s, h * d) @ st["w"][3].tensor.double().view(h * d, h * d)).view(-1)
