@@ -166,6 +166,9 @@ __device__ __forceinline__ void report_bad_block(const SdpaParams& p, bool bad) 
 
 // Host-side launchers (one per kernel family); each returns the CUDA error of its launch.
 cudaError_t launch_generic(const SdpaParams& p, int dtype, cudaStream_t stream);
+// The register-tiled fp32 kernel (csrc/sdpa_f32.cu); launch_generic hands it what it takes.
+bool f32_supported(const SdpaParams& p, int dtype);
+cudaError_t launch_f32(const SdpaParams& p, int dtype, cudaStream_t stream);
 cudaError_t launch_decode(const SdpaParams& p, int dtype, int chunk, int nchunks, float* workspace, cudaStream_t stream,
                           int* launches);
 bool decode_supported(int dtype, int head_dim);

@@ -2,7 +2,8 @@
 //
 // Serves (1) the fp32-input contract (<= 1e-5 relative against the fp32 CPU path), where tensor-core
 // rounding of the inputs is not admissible, and (2) shapes and mask kinds the tcgen05 prefill kernel does
-// not take.  Replaces the one-thread-per-row kernel of the reference
+// not take - what of both csrc/sdpa_f32.cu does not take either: the attention weights on request, paged K / V, head sizes
+// above 128 and rows that are not 16-byte aligned.  Replaces the one-thread-per-row kernel of the reference
 // (src/AiDotNet.Tensors/Engines/DirectGpu/CUDA/Kernels/CudaAttentionKernels.cs:28-112), which recomputes
 // q.k up to D+2 times per key; here K/V tiles are staged once in shared memory per 16 query rows.
 //
@@ -343,6 +344,7 @@ cudaError_t launch_d(const SdpaParams& p, cudaStream_t stream) {
 }  // namespace
 
 cudaError_t launch_generic(const SdpaParams& p, int dtype, cudaStream_t stream) {
+  if (f32_supported(p, dtype)) return launch_f32(p, dtype, stream);
   switch (dtype) {
     case AIDN_F32: return launch_d<float>(p, stream);
     case AIDN_F16: return launch_d<__half>(p, stream);
