@@ -82,3 +82,26 @@ def test_forward_strided_and_unaligned_rows():
         base = flat[shift:]
         out, _, _ = run_gpu(q, base, base[H * D:], dtype="f32", k_stride=stride, v_stride=stride, seq_kv=S, num_kv_heads=H)
         compare(out, ref, "f32", f"shift {shift}")
+
+
+@pytest.mark.parametrize("B,S,H,D", [(1, 5, 3, 4), (1, 63, 2, 10), (2, 64, 5, 36), (3, 43, 4, 32), (1, 2500, 16, 32), (9, 130, 33, 20)])
+def test_projection_f32(B, S, H, D):
+    """The fp32 projections around their 64 / 128-row tiles: one row more or less, widths that end inside a 64-column tile
+    or a 32-deep slice, head sizes that a group of four columns straddles.  A dot product of n terms of unit variance
+    scaled by 1 / sqrt(n) and rounded n times: 4 x 2^-24 x sqrt(n) / 2 on values of magnitude up to 5; two in a row."""
+    from aidotnet.tensors_b200.backend import CudaBackend, GpuBuffer
+    rng = np.random.default_rng(S)
+    dm = H * D
+    x = rng.standard_normal((B, S, dm), dtype=np.float32)
+    ws = [(rng.standard_normal((dm, dm)) / np.sqrt(dm)).astype(np.float32) for _ in range(4)]
+    backend = CudaBackend(0)
+    buf = lambda a: GpuBuffer(torch.from_numpy(a).cuda().reshape(-1))
+    out = backend.AllocateBuffer(B * S * dm)
+    backend.MultiHeadAttentionForward(buf(x), *[buf(w) for w in ws], out, B, S, dm, H, exact=True)
+    xd = torch.from_numpy(x).cuda().double()
+    wd = [torch.from_numpy(w).cuda().double() for w in ws]
+    q, k, v = ((xd @ w).view(B, S, H, D).transpose(1, 2) for w in wd[:3])
+    p = torch.softmax(q @ k.transpose(2, 3) / np.sqrt(D), -1)
+    ref = ((p @ v).transpose(1, 2).reshape(B, S, dm) @ wd[3]).cpu().numpy()
+    err = np.abs(out.tensor.cpu().numpy().reshape(ref.shape) - ref).max()
+    assert err <= 8 * 2.0 ** -24 * np.sqrt(dm) * max(1.0, np.abs(ref).max()), err
