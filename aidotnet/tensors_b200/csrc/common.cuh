@@ -201,6 +201,9 @@ cudaError_t launch_backward(const BwdParams& bp, int dtype, cudaStream_t stream,
 // tcgen05 dQ and dK / dV launches (csrc/sdpa_backward_sm100.cu); delta (and dout_t) must already be on the stream.
 bool backward_sm100_supported(const BwdParams& bp, int dtype);
 cudaError_t launch_backward_sm100(const BwdParams& bp, int dtype, cudaStream_t stream, int* launches, const char** why);
+// fp32 dQ and dK / dV launches on packed multiply-adds (csrc/sdpa_backward_f32.cu); delta must already be on the stream.
+bool backward_f32_supported(const BwdParams& bp, int dtype);
+cudaError_t launch_backward_f32(const BwdParams& bp, cudaStream_t stream);
 
 // Packed Q/K/V projection + RoPE + KV-cache write (csrc/qkv_rope_cache.cu).
 struct QkvRopeParams {

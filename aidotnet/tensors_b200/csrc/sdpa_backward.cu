@@ -780,6 +780,12 @@ cudaError_t launch_bwd_t(const BwdParams& bp, cudaStream_t stream, int* launches
       return launch_backward_sm100(bp, dtype, stream, launches, &why);
     }
   }
+  if constexpr (sizeof(T) == 4) {
+    if (backward_f32_supported(bp, AIDN_F32)) {
+      *launches = 3;
+      return launch_backward_f32(bp, stream);
+    }
+  }
   const size_t smem_q = sizeof(float) * ((2 * kRows + 2 * kKeys) * PITCH + kRows * kKeys);
   const size_t smem_kv = sizeof(float) * ((2 * kRows + 2 * kKeys) * PITCH + 2 * kRows * kKeys);
   auto kq = bwd_dq_kernel<T, DMAX>;

@@ -304,13 +304,14 @@ cudaError_t launch_one(const BwdParams& bp, cudaStream_t stream) {
 
 template <int DP, bool KEYS>
 cudaError_t launch_dir(const BwdParams& bp, cudaStream_t stream) {
-  // Four stationary groups, and as many warps that share them as registers (dQ 128, dK / dV 168 up to head_dim 64, 255
-  // above) and shared memory allow; half the stationary rows when that leaves SMs without a CTA.
+  // Four stationary groups, and as many warps that share them as registers (168 up to head_dim 64, 255 above) and shared
+  // memory allow - sixteen warps of 128 registers spill and are 2 us slower for dQ on B2 H8 S509 D64; half the stationary
+  // rows when four groups leave SMs without a CTA.
   const int64_t rows = KEYS ? bp.p.seq_kv : bp.p.seq_q;
   const int64_t heads = (int64_t)(KEYS ? bp.p.head_count / bp.p.group : bp.p.head_count) * bp.p.batch;
   const bool wide = (rows + 4 * kOwnW - 1) / (4 * kOwnW) * heads >= 112;
   if constexpr (DP <= 64) {
-    if (wide) return launch_one<DP, 4, KEYS ? 3 : 4, KEYS>(bp, stream);
+    if (wide) return launch_one<DP, 4, 3, KEYS>(bp, stream);
     return launch_one<DP, 2, 4, KEYS>(bp, stream);
   } else {
     if (wide) return launch_one<DP, 4, 2, KEYS>(bp, stream);

@@ -105,3 +105,37 @@ def test_projection_f32(B, S, H, D):
     ref = ((p @ v).transpose(1, 2).reshape(B, S, dm) @ wd[3]).cpu().numpy()
     err = np.abs(out.tensor.cpu().numpy().reshape(ref.shape) - ref).max()
     assert err <= 8 * 2.0 ** -24 * np.sqrt(dm) * max(1.0, np.abs(ref).max()), err
+
+
+BWD_SHAPES = [(1, 2, 1, 1, 1, 64), (1, 2, 2, 31, 33, 32), (1, 4, 2, 64, 97, 64), (2, 12, 6, 127, 65, 36), (8, 16, 16, 65, 64, 64),
+              (3, 20, 10, 130, 129, 32), (1, 3, 3, 70, 40, 128), (2, 30, 30, 129, 130, 128), (1, 6, 2, 95, 160, 96)]
+
+
+@pytest.mark.parametrize("shape", BWD_SHAPES)
+@pytest.mark.parametrize("variant", ["plain", "causal", "keep_lengths", "bias"])
+def test_backward_f32(shape, variant):
+    """dQ, dK, dV against float64.  Each is a sum of n <= 160 products of fp32 values, through a probability and a dS that
+    are off by the rounding of two more such sums: 16 x 2^-24 x sqrt(n) of the largest value."""
+    from tests.test_gpu_backward import _fwd_bwd
+    B, Hq, Hkv, Sq, Sk, D = shape
+    ts = [gen(s, "f32", i + 1, 1.0) for i, s in enumerate([(B, Hq, Sq, D), (B, Hkv, Sk, D), (B, Hkv, Sk, D), (B, Hq, Sq, D)])]
+    (q, qf), (k, kf), (v, vf), (g, gf) = ts
+    rng = np.random.default_rng(5)
+    kw, okw = {}, {}
+    if variant == "causal":
+        kw = okw = dict(causal=True, causal_offset=Sk - Sq + 2)
+    elif variant == "keep_lengths":
+        keep = (rng.random((B, 1, Sq, Sk)) < 0.8).astype(np.uint8)
+        lens = rng.integers(1, Sk + 1, B).astype(np.int32)
+        kw, okw = dict(mask=torch.from_numpy(keep).cuda(), mask_kind=N.MASK_KEEP_U8, kv_len=lens), dict(keep=keep, kv_len=lens)
+    elif variant == "bias":
+        bias = rng.standard_normal((1, Hq, Sq, Sk)).astype(np.float32)
+        kw, okw = dict(mask=torch.from_numpy(bias).cuda(), mask_kind=N.MASK_ADD_F32), dict(bias=bias)
+    got = _fwd_bwd(q, k, v, g, dtype="f32", **kw)
+    want = O.sdpa_backward(qf, kf, vf, gf, **okw)[:3]
+    for x, y, name in zip(got, want, ("dQ", "dK", "dV")):
+        x = x.cpu().numpy()
+        assert np.isfinite(x).all(), name
+        assert np.abs(x - y).max() <= 16 * 2.0 ** -24 * np.sqrt(max(Sq, Sk, D)) * max(1.0, np.abs(y).max()), (name, np.abs(x - y).max())
+    again = _fwd_bwd(q, k, v, g, dtype="f32", **kw)
+    assert all(torch.equal(x, y) for x, y in zip(got, again))
