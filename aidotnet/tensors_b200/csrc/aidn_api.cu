@@ -146,6 +146,21 @@ int64_t decode_ws_bytes(const aidn_sdpa* h, int64_t batch, int64_t seq_kv, int* 
   return align_up(batch * h->head_count * nchunks * (h->d.head_dim + 2) * (int64_t)sizeof(float), 256);
 }
 
+// Workspace of the split tcgen05 prefill for these sizes, 0 when it would not be split.
+int64_t prefill_split_need(const aidn_sdpa* h, int64_t batch, int64_t seq_q, int64_t seq_kv) {
+  aidn::SdpaParams p;
+  std::memset(&p, 0, sizeof(p));
+  p.batch = (int)batch;
+  p.num_q_heads = h->d.num_q_heads;
+  p.head_count = h->head_count;
+  p.group = h->group;
+  p.seq_q = seq_q;
+  p.seq_kv = seq_kv;
+  p.head_dim = h->d.head_dim;
+  const int splits = aidn::prefill_splits(p, h->num_sms);
+  return splits > 1 ? align_up(aidn::prefill_split_bytes(p, splits), 256) : 0;
+}
+
 bool aligned16(const void* ptr, const int64_t* stride, size_t esz) {
   if ((uintptr_t)ptr % 16 != 0) return false;
   for (int i = 0; i < 3; ++i)
@@ -260,9 +275,16 @@ int64_t aidn_sdpa_workspace_bytes(aidn_sdpa_t h, int64_t batch, int64_t seq_q, i
     fail(AIDN_EINVAL, "workspace_bytes: bad argument");
     return -1;
   }
-  if (seq_q != 1 || h->d.path == AIDN_PATH_GENERIC || h->d.path == AIDN_PATH_PREFILL_SM100) return 0;
-  if (!aidn::decode_supported(h->d.qkv_dtype, h->d.head_dim)) return 0;
-  return decode_ws_bytes(h, batch, seq_kv, nullptr, nullptr);
+  if (h->d.path == AIDN_PATH_GENERIC) return 0;
+  // the decode kernel's partial results, or those of a tcgen05 prefill with fewer work items than SMs (which runs without
+  // a workspace too, only slower)
+  int64_t need = 0;
+  if (seq_q == 1 && h->d.path != AIDN_PATH_PREFILL_SM100 && aidn::decode_supported(h->d.qkv_dtype, h->d.head_dim))
+    need = decode_ws_bytes(h, batch, seq_kv, nullptr, nullptr);
+  else if (h->d.path != AIDN_PATH_DECODE && h->d.qkv_dtype != AIDN_F32 && (h->d.head_dim == 64 || h->d.head_dim == 128) &&
+           batch <= 65535)
+    need = prefill_split_need(h, batch, seq_q, seq_kv);
+  return need;
 }
 
 int aidn_sdpa_last_path(aidn_sdpa_t h) { return h ? h->last_path : -1; }
@@ -440,9 +462,14 @@ int launch_common(aidn_sdpa_t h, const aidn_sdpa_args* a, const aidn_paged_kv* p
     }
     e = aidn::launch_decode(p, d.qkv_dtype, chunk, nchunks, ws, stream, &launches);
   } else if (path == AIDN_PATH_PREFILL_SM100) {
+    // Keys of few items are split when the caller's workspace holds the partial results; without one they are not.  The
+    // handle's own scratch is not used: it belongs to decode calls, which may be running on another stream.
+    int splits = aidn::prefill_splits(p, h->num_sms);
+    if (!a->workspace || (uintptr_t)a->workspace % 16 != 0 || h->debug || h->debug_mode) splits = 1;
+    if (splits > 1 && a->workspace_bytes < aidn::prefill_split_bytes(p, splits)) splits = 1;
     e = aidn::launch_prefill_sm100(p, d.qkv_dtype, stream, h->status_dev + 1, h->num_sms, h->debug, h->debug_mode,
-                                   &h->prefill_maps, &why);
-    launches = 1;
+                                   &h->prefill_maps, splits, static_cast<float*>(a->workspace), &why);
+    launches = splits > 1 ? 2 : 1;
     if (e != cudaSuccess && why[0]) return fail(AIDN_ECUDA, "launch: %s (%s)", why, cudaGetErrorName(e));
   } else {
     e = aidn::launch_generic(p, d.qkv_dtype, stream);

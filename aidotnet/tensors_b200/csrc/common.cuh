@@ -240,15 +240,20 @@ struct alignas(64) PrefillMapCache {
     const void* q; const void* k; const void* v; const void* out;
     int64_t qs[3], ks[3], vs[3], os[3];
     int64_t seq_q, kv_rows;
-    int32_t batch, kv_batch, num_q_heads, num_kv_heads, head_dim, kv_box, out_f32, dtype;
+    int32_t batch, kv_batch, num_q_heads, num_kv_heads, head_dim, kv_box, out_f32, splits, dtype;
   } key;
   bool valid;
   bool attr_set[16];            // by instantiation: (epilogue warpgroup ? 8 : 0) + (fp16 ? 4 : 0) + (head_dim 128 ? 2 : 0) + (masked ? 1 : 0)
 };
 bool prefill_sm100_supported(const SdpaParams& p, int dtype, const char** why);
-// cache may be null (maps are then encoded on every call).
+// How many parts the keys of every work item should be cut into (1: none), and the workspace (16-byte aligned) that this
+// takes.
+int prefill_splits(const SdpaParams& p, int num_sms);
+int64_t prefill_split_bytes(const SdpaParams& p, int splits);
+// cache may be null (maps are then encoded on every call); workspace is read for splits > 1 only.
 cudaError_t launch_prefill_sm100(const SdpaParams& p, int dtype, cudaStream_t stream, int32_t* sched, int num_sms,
-                                 float* debug, int debug_mode, PrefillMapCache* cache, const char** why);
+                                 float* debug, int debug_mode, PrefillMapCache* cache, int splits, float* workspace,
+                                 const char** why);
 
 // Projection GEMM of the fused multi-head-attention forward (csrc/proj_gemm_sm100.cu):
 // c[i][b, s, n] = sum_k a[b, s, k] * w[i][k, n] for up to three weight matrices that share a; column n lands at

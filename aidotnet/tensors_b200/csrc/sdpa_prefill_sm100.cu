@@ -97,7 +97,7 @@ struct Roles {
                 "setmaxnreg budget exceeds the registers the CTA is launched with");
   static_assert(kStoreWarps * kStageBufs * 4096 == kStageBytes, "staging memory");
 };
-constexpr int kItemWords = 14;   // mailbox entry: item, b, kvh, n_max, (h, t, n, valid) of both tiles, v_tail
+constexpr int kItemWords = 16;   // mailbox entry: item, b, kvh, n_max, (h, t, n, valid) of both tiles, v_tail, k0, out_b
 
 template <int HD>
 struct Cfg {
@@ -128,6 +128,8 @@ struct PrefillParams {
   int32_t items_per_rank;  // batch * work items per rank
   int32_t per_batch;       // work items per rank per batch entry
   int32_t total_items;
+  int32_t splits;          // > 1: each item is cut into this many along its keys; p.out / p.lse are then partial results
+                           // [batch * splits, ...] that sdpa_prefill_merge_kernel puts together
   int32_t* sched;          // [0] next-item counter, [1] finished-CTA counter; both zero between launches
   float* debug;            // trace builds only: tap / timeline buffer
   int32_t debug_mode;      // 3: the producer withholds the Q tiles, so that the bounded waits run out (test hook);
@@ -153,6 +155,8 @@ struct Item {
   TileInfo tile[2];
   int b, kvh;
   int n_max;      // sub-tiles of the longer tile = K and V sub-tiles the item streams
+  int k0;         // first 64-key sub-tile (sub-tiles are counted from it everywhere else)
+  int out_b;      // batch coordinate of the output
   int v_tail;     // > 0: rows of the item's last V sub-tile that hold keys of the sequence; the rows after them are
                   // cleared in shared memory before the P.V product (0 = nothing to clear)
 };
@@ -166,7 +170,7 @@ __device__ __forceinline__ void publish_item(volatile int* box, int item, const 
     box[4 + 4 * i] = it.tile[i].h; box[5 + 4 * i] = it.tile[i].t;
     box[6 + 4 * i] = it.tile[i].n; box[7 + 4 * i] = it.tile[i].valid ? 1 : 0;
   }
-  box[12] = it.v_tail;
+  box[12] = it.v_tail; box[13] = it.k0; box[14] = it.out_b;
   box[0] = item;
 }
 
@@ -178,13 +182,15 @@ __device__ __forceinline__ Item read_item(const volatile int* box) {
     it.tile[i].h = box[4 + 4 * i]; it.tile[i].t = box[5 + 4 * i];
     it.tile[i].n = box[6 + 4 * i]; it.tile[i].valid = box[7 + 4 * i] != 0;
   }
-  it.v_tail = box[12];
+  it.v_tail = box[12]; it.k0 = box[13]; it.out_b = box[14];
   return it;
 }
 
 __device__ __forceinline__ Item decode_item(const PrefillParams& pp, int item) {
   const SdpaParams& p = pp.p;
   Item it;
+  const int split = pp.splits > 1 ? item % pp.splits : 0;
+  if (pp.splits > 1) item /= pp.splits;
   const int rank = item / pp.items_per_rank;
   const int rem = item - rank * pp.items_per_rank;
   it.b = rem / pp.per_batch;
@@ -221,12 +227,25 @@ __device__ __forceinline__ Item decode_item(const PrefillParams& pp, int item) {
     it.tile[i].n = (int)((kend + kBS - 1) / kBS);
   }
   it.n_max = it.tile[0].n > it.tile[1].n ? it.tile[0].n : it.tile[1].n;
+  it.k0 = 0;
+  it.out_b = it.b;
+  if (pp.splits > 1) {   // this split's share of the longer tile's sub-tiles; a tile may end before it begins
+    const int per = (it.n_max + pp.splits - 1) / pp.splits;
+    it.k0 = split * per;
+    it.out_b = it.b * pp.splits + split;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int left = it.tile[i].n - it.k0;
+      it.tile[i].n = left < 0 ? 0 : (left < per ? left : per);
+    }
+    it.n_max = it.tile[0].n > it.tile[1].n ? it.tile[0].n : it.tile[1].n;
+  }
   // Rows of the last V tile past the sequence's last key hold whatever the caller's buffer holds there (padding after
   // kv_len, the unused tail of a pool block).  Their probabilities are 0, but 0 * NaN is NaN in the P.V product, so
   // the UMMA warp clears them.  Rows past seq_kv of a contiguous tensor are zero-filled by TMA itself.
   it.v_tail = 0;
-  if ((p.kv_len || p.block_table) && (int64_t)it.n_max * kBS > kv_limit)
-    it.v_tail = (int)(kv_limit - (int64_t)(it.n_max - 1) * kBS);
+  if ((p.kv_len || p.block_table) && it.n_max > 0 && (int64_t)(it.k0 + it.n_max) * kBS > kv_limit)
+    it.v_tail = (int)(kv_limit - (int64_t)(it.k0 + it.n_max - 1) * kBS);
   return it;
 }
 
@@ -476,7 +495,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
         STEP_STAMP(u, 1);
         float* s = reinterpret_cast<float*>(sr);
 
-        const int64_t col0 = (int64_t)u * kBS;
+        const int64_t col0 = (int64_t)(it.k0 + u) * kBS;
         if constexpr (MASKED) {
           // scale -> softcap -> bias -> keep-mask, the order of the reference (CpuEngine.cs:27807-27816, 29218-29239)
           const float inv_cap = p.softcap > 0.f ? 1.f / p.softcap : 0.f;
@@ -648,7 +667,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_stats_full + 8 * i);
         if (qrow < p.seq_q && p.lse)
-          p.lse[((int64_t)b * p.num_q_heads + ti.h) * p.seq_q + qrow] =
+          p.lse[((int64_t)it.out_b * p.num_q_heads + ti.h) * p.seq_q + qrow] =
               (inv > 0.f) ? m * lse_scale + logf(l) : -INFINITY;
       } else {
         // ---- epilogue: O / l -> swizzled staging (128 B per row) -> TMA stores ------------------------------
@@ -705,15 +724,15 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
               fence_proxy_async_smem();
               __syncwarp();
               if (lane == 0 && box_valid) {
-                tma_store_4d(&tm_o, my_stage, p.out_f32 ? c0 : c0 - 32, row0, ti.h, b);
-                for (int r = 0; r < pm.count; ++r) tma_store_4d(&pm.maps[r], my_stage, p.out_f32 ? c0 : c0 - 32, row0, ti.h, b);
+                tma_store_4d(&tm_o, my_stage, p.out_f32 ? c0 : c0 - 32, row0, ti.h, it.out_b);
+                for (int r = 0; r < pm.count; ++r) tma_store_4d(&pm.maps[r], my_stage, p.out_f32 ? c0 : c0 - 32, row0, ti.h, it.out_b);
                 bulk_commit();
               }
               stores_in_flight = true;
             }
           }
           if (row_valid && p.lse)
-            p.lse[((int64_t)b * p.num_q_heads + ti.h) * p.seq_q + qrow] =
+            p.lse[((int64_t)it.out_b * p.num_q_heads + ti.h) * p.seq_q + qrow] =
                 (inv > 0.f) ? m * lse_scale + logf(l) : -INFINITY;
           if (tracer) trace[5 + 8 * i] = globaltimer_ns();
         }
@@ -788,7 +807,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
         int64_t last_blk = 0;   // the last logical block of the sequence that the item's keys lie in
         if (paged) {
           last_blk = (kv_limit_of(p, it.b) - 1) >> p.block_shift;
-          const int64_t item_last = ((int64_t)it.n_max * kBS - 1) >> p.block_shift;
+          const int64_t item_last = ((int64_t)(it.k0 + it.n_max) * kBS - 1) >> p.block_shift;
           if (item_last < last_blk) last_blk = item_last;
         }
         struct TableWindow { int64_t first; int32_t blk; };
@@ -840,12 +859,12 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
         const int n_sub = it.n_max;
         if (n_sub > 0) {
           load_q(0);
-          if (alive) load_kv(&tm_k, 0, win_k);
+          if (alive) load_kv(&tm_k, it.k0, win_k);
           if (ptrace && leader) ptrace[0] = globaltimer_ns();
           if (alive) load_q(1);
           for (int u = 0; u < n_sub && alive; ++u) {
-            if (u + 1 < n_sub) load_kv(&tm_k, u + 1, win_k);
-            if (alive) load_kv(&tm_v, u, win_v);
+            if (u + 1 < n_sub) load_kv(&tm_k, it.k0 + u + 1, win_k);
+            if (alive) load_kv(&tm_v, it.k0 + u, win_v);
           }
         }
         {
@@ -1121,7 +1140,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
           }
           if (tracer) trace[4 + 8 * i] = globaltimer_ns();
           store_o_tile<HD, kBf16>(p, &tm_o, pm, tmem_base + lane_bits + (uint32_t)(C::kOCol + i * HD), have_o, inv, my_stage,
-                                     n_stores, lane, ti.t * kBM + quarter * 32, ti.h, it.b, bar_o_empty + 8 * i);
+                                     n_stores, lane, ti.t * kBM + quarter * 32, ti.h, it.out_b, bar_o_empty + 8 * i);
           if (tracer) trace[5 + 8 * i] = globaltimer_ns();
         }
       }
@@ -1184,7 +1203,7 @@ bool aligned_bhs(const void* base, const int64_t* stride, int64_t H, int64_t B, 
 
 template <typename T, int HD, bool MASKED, bool EPI>
 cudaError_t launch_e(const SdpaParams& p, cudaStream_t stream, int32_t* sched, int num_sms, float* debug,
-                     int debug_mode, PrefillMapCache* cache, const char** why) {
+                     int debug_mode, PrefillMapCache* cache, int splits, const char** why) {
   using C = Cfg<HD>;
   constexpr bool bf16 = !std::is_same_v<T, __half>;
   // Paged pools are one "sequence" of num_blocks * block_size rows, fetched one block (box of block_size rows) at a time.
@@ -1203,7 +1222,7 @@ cudaError_t launch_e(const SdpaParams& p, cudaStream_t stream, int32_t* sched, i
   for (int i = 0; i < 3; ++i) { key.qs[i] = p.qs[i]; key.ks[i] = p.ks[i]; key.vs[i] = p.vs[i]; key.os[i] = p.os[i]; }
   key.seq_q = p.seq_q; key.kv_rows = kv_rows;
   key.batch = p.batch; key.kv_batch = kv_batch; key.num_q_heads = p.num_q_heads; key.num_kv_heads = p.num_kv_heads;
-  key.head_dim = HD; key.kv_box = kv_box; key.out_f32 = p.out_f32; key.dtype = bf16 ? AIDN_BF16 : AIDN_F16;
+  key.head_dim = HD; key.kv_box = kv_box; key.out_f32 = p.out_f32; key.splits = splits; key.dtype = bf16 ? AIDN_BF16 : AIDN_F16;
   CUtensorMap* tq = reinterpret_cast<CUtensorMap*>(mc->maps[0]);
   CUtensorMap* tk = reinterpret_cast<CUtensorMap*>(mc->maps[1]);
   CUtensorMap* tv = reinterpret_cast<CUtensorMap*>(mc->maps[2]);
@@ -1217,7 +1236,7 @@ cudaError_t launch_e(const SdpaParams& p, cudaStream_t stream, int32_t* sched, i
     const CUtensorMapSwizzle s128 = CU_TENSOR_MAP_SWIZZLE_128B;
     // output boxes are 128 bytes x 32 rows: 32 fp32 or 64 16-bit columns
     const bool ok_o = p.out_f32
-        ? encode_bhsd(to, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, s128, p.out, HD, p.seq_q, p.num_q_heads, p.batch, p.os, 32, 32)
+        ? encode_bhsd(to, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, s128, p.out, HD, p.seq_q, p.num_q_heads, p.batch * splits, p.os, 32, 32)
         : encode_bhsd(to, dt16, 2, s128, p.out, HD, p.seq_q, p.num_q_heads, p.batch, p.os, 64, 32);
     if (!encode_bhsd(tq, dt16, 2, s128, p.q, HD, p.seq_q, p.num_q_heads, p.batch, p.qs, 64, kBM) ||
         !encode_bhsd(tk, dt16, 2, s128, p.k, HD, kv_rows, p.num_kv_heads, kv_batch, p.ks, 64, kv_box) ||
@@ -1269,7 +1288,8 @@ cudaError_t launch_e(const SdpaParams& p, cudaStream_t stream, int32_t* sched, i
     pp.per_batch = p.head_count;
   }
   pp.items_per_rank = p.batch * pp.per_batch;
-  const int64_t total = (int64_t)pp.ranks * pp.items_per_rank;
+  pp.splits = splits;
+  const int64_t total = (int64_t)pp.ranks * pp.items_per_rank * splits;
   if (total <= 0 || total > 0x3fffffff) { *why = "work item count out of range"; return cudaErrorInvalidValue; }
   pp.total_items = (int)total;
   auto kern = sdpa_prefill_sm100_kernel<T, HD, MASKED, EPI>;
@@ -1316,28 +1336,125 @@ bool prefill_sm100_supported(const SdpaParams& p, int dtype, const char** why) {
 // The epilogue warpgroup pays when both tiles of an item end together: head pairs, or row pairs without a causal mask.
 template <typename T, int HD, bool MASKED>
 cudaError_t launch_t(const SdpaParams& p, cudaStream_t stream, int32_t* sched, int num_sms, float* debug,
-                     int debug_mode, PrefillMapCache* cache, const char** why) {
+                     int debug_mode, PrefillMapCache* cache, int splits, const char** why) {
   const bool epi = (p.group % 2 == 0) || !p.causal;
-  if (epi) return launch_e<T, HD, MASKED, true>(p, stream, sched, num_sms, debug, debug_mode, cache, why);
-  return launch_e<T, HD, MASKED, false>(p, stream, sched, num_sms, debug, debug_mode, cache, why);
+  if (epi) return launch_e<T, HD, MASKED, true>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  return launch_e<T, HD, MASKED, false>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
 }
 
 template <typename T, int HD>
 cudaError_t launch_m(const SdpaParams& p, cudaStream_t stream, int32_t* sched, int num_sms, float* debug, int debug_mode,
-                     PrefillMapCache* cache, const char** why) {
+                     PrefillMapCache* cache, int splits, const char** why) {
   if (p.mask_kind != AIDN_MASK_NONE || p.softcap > 0.f)
-    return launch_t<T, HD, true>(p, stream, sched, num_sms, debug, debug_mode, cache, why);
-  return launch_t<T, HD, false>(p, stream, sched, num_sms, debug, debug_mode, cache, why);
+    return launch_t<T, HD, true>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  return launch_t<T, HD, false>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
 }
 
-cudaError_t launch_prefill_sm100(const SdpaParams& p, int dtype, cudaStream_t stream, int32_t* sched, int num_sms,
-                                 float* debug, int debug_mode, PrefillMapCache* cache, const char** why) {
+namespace {
+
+constexpr int kMinSplitSubs = 8;   // sub-tiles per part: below it the item's fixed cost outweighs the keys
+
+cudaError_t launch_type(const SdpaParams& p, int dtype, cudaStream_t stream, int32_t* sched, int num_sms, float* debug,
+                        int debug_mode, PrefillMapCache* cache, int splits, const char** why) {
   if (dtype == AIDN_BF16) {
-    if (p.head_dim == 128) return launch_m<__nv_bfloat16, 128>(p, stream, sched, num_sms, debug, debug_mode, cache, why);
-    return launch_m<__nv_bfloat16, 64>(p, stream, sched, num_sms, debug, debug_mode, cache, why);
+    if (p.head_dim == 128) return launch_m<__nv_bfloat16, 128>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+    return launch_m<__nv_bfloat16, 64>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
   }
-  if (p.head_dim == 128) return launch_m<__half, 128>(p, stream, sched, num_sms, debug, debug_mode, cache, why);
-  return launch_m<__half, 64>(p, stream, sched, num_sms, debug, debug_mode, cache, why);
+  if (p.head_dim == 128) return launch_m<__half, 128>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  return launch_m<__half, 64>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+}
+
+// out = sum_s w_s O_s with w_s = exp(lse_s - lse), lse = log sum_s exp(lse_s): head_dim / 4 lanes per row, one 16-byte
+// load per part and lane.  The partial results were just written and come from L2.
+template <typename T>
+__global__ void __launch_bounds__(256) sdpa_prefill_merge_kernel(const SdpaParams p, const float* __restrict__ parts,
+                                                                 const float* __restrict__ lses, const int splits, const int64_t rows) {
+  const int lanes = p.head_dim / 4;
+  const int64_t row = (int64_t)blockIdx.x * (256 / lanes) + threadIdx.x / lanes;   // over [B, H, Sq]
+  const int d = threadIdx.x % lanes * 4;
+  if (row >= rows) return;
+  const int64_t per_batch = (int64_t)p.num_q_heads * p.seq_q;
+  const int64_t b = row / per_batch, within = row - b * per_batch;
+  const int64_t h = within / p.seq_q, q = within - h * p.seq_q;
+  const int64_t first = b * splits * per_batch + within;
+  float m = -INFINITY;
+  for (int s = 0; s < splits; ++s) m = fmaxf(m, lses[first + s * per_batch]);
+  float l = 0.f;
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (m != -INFINITY) {
+#pragma unroll 4
+    for (int s = 0; s < splits; ++s) {
+      const float w = expf(lses[first + s * per_batch] - m);
+      const float4 x = *reinterpret_cast<const float4*>(parts + (first + s * per_batch) * p.head_dim + d);
+      l += w;
+      o.x = fmaf(w, x.x, o.x); o.y = fmaf(w, x.y, o.y); o.z = fmaf(w, x.z, o.z); o.w = fmaf(w, x.w, o.w);
+    }
+    const float inv = 1.f / l;
+    o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
+  }
+  const int64_t at = b * p.os[0] + h * p.os[1] + q * p.os[2] + d;   // 16-byte aligned rows (prefill_sm100_supported)
+  if (p.out_f32) {
+    *reinterpret_cast<float4*>(static_cast<float*>(p.out) + at) = o;
+  } else {
+    T t[4] = {from_float<T>(o.x), from_float<T>(o.y), from_float<T>(o.z), from_float<T>(o.w)};
+    *reinterpret_cast<uint2*>(static_cast<T*>(p.out) + at) = *reinterpret_cast<const uint2*>(t);
+  }
+  if (p.lse && d == 0) p.lse[row] = m != -INFINITY ? m + logf(l) : -INFINITY;
+}
+
+}  // namespace
+
+int64_t prefill_split_bytes(const SdpaParams& p, int splits) {
+  return (int64_t)p.batch * splits * p.num_q_heads * p.seq_q * (p.head_dim + 1) * (int64_t)sizeof(float);
+}
+
+// Work items are pairs of 128-row tiles; fewer of them than SMs leaves the chip idle however long the keys are (a chunk
+// of 512 queries and 32 heads: 64 items for 148 SMs).  The keys of every item are then cut into the number of parts that
+// ends first by the model below, in units of one 64-key sub-tile: an item costs its sub-tiles plus about four (first
+// scores, last P.V, epilogue), merging costs a launch and the partial results' way through memory.  Measured without and
+// with it (causal, D 128): Hq32 / Hkv8 512 x 8112 132 -> 87 us, Hq8 / Hkv1 1024 x 8192 132 -> 52, Hq2 256 x 16384 248 -> 34,
+// Hq8 256 x 4096 70 -> 27, Hq32 / Hkv8 512 x 1024 28.7 -> 27.7 (the fewest keys that are split).
+int prefill_splits(const SdpaParams& p, int num_sms) {
+  if (p.head_count != p.num_q_heads || p.peer_count > 0) return 1;
+  const int64_t row_tiles = (p.seq_q + kBM - 1) / kBM;
+  const int64_t items = (int64_t)p.batch * (p.group % 2 == 0 ? row_tiles * (p.head_count / 2) : (row_tiles + 1) / 2 * p.head_count);
+  const int64_t n = (p.seq_kv + kBS - 1) / kBS;
+  if (items >= num_sms || n < 2 * kMinSplitSubs) return 1;
+  int best = 1;
+  double best_cost = (double)(n + 4);
+  for (int s = 2; s <= 16 && n / s >= kMinSplitSubs; ++s) {
+    const int64_t waves = (items * s + num_sms - 1) / num_sms;
+    const double merge = 4.0 + (double)prefill_split_bytes(p, s) / 4e6;
+    const double cost = (double)waves * (double)((n + s - 1) / s + 4) + merge;
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return best;
+}
+
+cudaError_t launch_prefill_sm100(const SdpaParams& full, int dtype, cudaStream_t stream, int32_t* sched, int num_sms,
+                                 float* debug, int debug_mode, PrefillMapCache* cache, int splits, float* workspace,
+                                 const char** why) {
+  SdpaParams p = full;
+  if (splits > 1) {   // fp32 partial outputs [batch * splits, H, Sq, D], then their log-sum-exps
+    p.out = workspace;
+    p.out_f32 = 1;
+    p.os[2] = p.head_dim;
+    p.os[1] = p.seq_q * p.head_dim;
+    p.os[0] = p.num_q_heads * p.os[1];
+    p.lse = workspace + (int64_t)p.batch * splits * p.os[0];
+  }
+  const cudaError_t e = launch_type(p, dtype, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  if (e != cudaSuccess || splits <= 1) return e;
+  const int64_t rows = (int64_t)p.batch * p.num_q_heads * p.seq_q;
+  const int rows_per_cta = 256 * 4 / p.head_dim;
+  const unsigned grid = (unsigned)((rows + rows_per_cta - 1) / rows_per_cta);
+  const float* parts = workspace;
+  if (dtype == AIDN_BF16) sdpa_prefill_merge_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(full, parts, p.lse, splits, rows);
+  else sdpa_prefill_merge_kernel<__half><<<grid, 256, 0, stream>>>(full, parts, p.lse, splits, rows);
+  return cudaGetLastError();
 }
 
 }  // namespace aidn

@@ -1,0 +1,80 @@
+"""tcgen05 prefill with the keys of every work item cut into parts (fewer items than SMs): parity where a part can be empty,
+end inside a sub-tile, or see nothing of a row, and what decides whether a launch is split."""
+import numpy as np
+import pytest
+import torch
+
+from aidotnet.tensors_b200 import native as N
+from oracle import sdpa_oracle as O
+
+from tests._harness import compare, compare_lse, gen, run_gpu
+
+pytestmark = pytest.mark.gpu
+
+# (B, Hq, Hkv, Sq, Sk, D): 1024 keys are the fewest that are split; 16 parts at most
+SHAPES = [(1, 2, 1, 128, 1024, 64), (1, 1, 1, 1, 1025, 128), (2, 3, 3, 130, 2113, 64), (1, 4, 2, 257, 3007, 128), (1, 8, 1, 97, 8200, 128)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("dtype,out", [("bf16", "f32"), ("f16", "f16")])
+@pytest.mark.parametrize("variant", ["plain", "causal", "lengths", "keep_softcap"])
+def test_split_prefill(shape, dtype, out, variant):
+    B, Hq, Hkv, Sq, Sk, D = shape
+    q, qf = gen((B, Hq, Sq, D), dtype, 1)
+    k, kf = gen((B, Hkv, Sk, D), dtype, 2)
+    v, vf = gen((B, Hkv, Sk, D), dtype, 3)
+    kw, okw = {}, {}
+    rng = np.random.default_rng(4)
+    if variant == "causal":     # top-left: the first parts hold all that the rows see, the others are empty
+        kw, okw = dict(causal=True, bottom_right=False, causal_offset=70), dict(causal=True, causal_offset=70)
+    elif variant == "lengths":
+        lens = np.array([Sk // 3 + 1, 0][:B], np.int32)
+        for b in range(B):
+            v[b, :, lens[b]:] = float("nan")
+        kw, okw = dict(kv_len=torch.from_numpy(lens).cuda()), dict(kv_len=lens)
+    elif variant == "keep_softcap":
+        keep = (rng.random((1, 1, Sq, Sk)) < 0.5).astype(np.uint8)
+        keep[..., Sq // 2, :] = 0
+        keep[..., 0, : Sk // 2] = 0
+        kw = dict(mask=torch.from_numpy(keep).cuda(), mask_kind=N.MASK_KEEP_U8, softcap=15.0)
+        okw = dict(mask=keep, mask_kind=O.MASK_KEEP_U8, softcap=15.0)
+    got, lse, info = run_gpu(q, k, v, dtype=dtype, out_dtype=out, want_lse=True, path=N.PATH_PREFILL_SM100, **kw)
+    assert info["launches"] == 2
+    ref, ref_lse, _ = O.sdpa(qf, kf, vf, want_lse=True, **({"causal": False} | okw))
+    compare(got, ref, dtype, f"{shape} {variant}")
+    compare_lse(lse, ref_lse, dtype, f"{shape} {variant}")
+
+
+def test_bottom_right_causal_parts_match_one_piece():
+    """A chunk at the end of its keys, with and without a workspace: one is split, the other is not, and they differ by the
+    rounding of P alone.  A weight near 1 / n is off by at most 2^-9 of itself in bf16 on either side, independently, and n
+    of them are averaged over values of standard deviation 0.5: sqrt(2) 2^-9 0.5 / sqrt(n) per output (n >= 3901 visible
+    keys), of which 100 000 outputs stay within six."""
+    q, _ = gen((1, 4, 200, 128), "bf16", 1)
+    k, _ = gen((1, 2, 4100, 128), "bf16", 2)
+    v, _ = gen((1, 2, 4100, 128), "bf16", 3)
+    split, _, info = run_gpu(q, k, v, dtype="bf16", causal=True)
+    assert info["launches"] == 2
+    h = N.Handle(device=0, qkv_dtype=N.BF16, out_dtype=N.F32, head_dim=128, num_q_heads=4, num_kv_heads=2, causal=True)
+    whole = torch.empty(1, 4, 200, 128, device="cuda")
+    args = dict(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), out=whole.data_ptr(), batch=1, seq_q=200, seq_kv=4100,
+                stream=torch.cuda.current_stream().cuda_stream)
+    h.launch(**args)
+    h.poll(args["stream"])
+    assert h.last_launch_count == 1
+    assert (split - whole).abs().max().item() <= 6 * 2 ** 0.5 * 2.0 ** -9 * 0.5 / 3901 ** 0.5
+    small = torch.empty(4096, dtype=torch.uint8, device="cuda")            # too small a workspace: not split either
+    h.launch(workspace=small.data_ptr(), workspace_bytes=4096, **args)
+    assert h.last_launch_count == 1
+    h.close()
+
+
+def test_many_items_or_few_keys_are_not_split():
+    h = N.Handle(device=0, qkv_dtype=N.BF16, out_dtype=N.F32, head_dim=128, num_q_heads=32, num_kv_heads=8)
+    assert h.workspace_bytes(4, 2048, 2048) == 0
+    assert h.workspace_bytes(1, 512, 1023) == 0
+    assert h.workspace_bytes(1, 512, 8112) > 0
+    h.close()
+    shard = N.Handle(device=0, qkv_dtype=N.BF16, out_dtype=N.F32, head_dim=128, num_q_heads=32, num_kv_heads=8, head_begin=8, head_count=8)
+    assert shard.workspace_bytes(1, 512, 8112) == 0
+    shard.close()
