@@ -164,6 +164,28 @@ __device__ __forceinline__ void report_bad_block(const SdpaParams& p, bool bad) 
   if (bad && p.status) atomicOr(p.status, kStatusBadBlock);
 }
 
+// Programmatic dependent launch: a kernel started with launch_dependent may begin while its predecessor on the stream is
+// still running - its launch latency and prologue then cost nothing - and must call pdl_wait before it touches memory that
+// any earlier kernel reads or writes.  pdl_trigger in the predecessor says from when on; a kernel that never calls it is
+// waited for as a whole, which is what the stream order alone would do.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // Host-side launchers (one per kernel family); each returns the CUDA error of its launch.
 cudaError_t launch_generic(const SdpaParams& p, int dtype, cudaStream_t stream);
 // The register-tiled fp32 kernel (csrc/sdpa_f32.cu); launch_generic hands it what it takes.

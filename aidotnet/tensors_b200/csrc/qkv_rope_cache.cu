@@ -67,6 +67,8 @@ __global__ void __launch_bounds__(WARPS * 32) qkv_rope_cache_kernel(const QkvRop
   const int D = p.head_dim;
   const int ntok = min(T, p.tokens - t_base);
 
+  pdl_wait();      // nothing above touches memory that an earlier kernel writes
+  pdl_trigger();   // the attention that follows may be set up while this kernel runs
   extern __shared__ __align__(16) float xs[];   // [T][model] when XS
   if constexpr (XS) {
     constexpr int kStageUnroll = 4;   // independent loads in flight per thread
@@ -97,6 +99,23 @@ __global__ void __launch_bounds__(WARPS * 32) qkv_rope_cache_kernel(const QkvRop
     const int r0 = 2 * pair;
     const WT* w0 = W + (int64_t)r0 * model;
     const WT* w1 = w0 + model;
+    // what lane t needs to finish token t, requested ahead of the weights: after them it was a chain of three loads
+    // (position -> cos, sin) at the end of every pair
+    const bool is_q = r0 < q_rows;
+    const bool is_k = !is_q && r0 < q_rows + kv_rows;
+    const int tok = t_base + lane;
+    int64_t crow = -1;
+    float bias0 = 0.f, bias1 = 0.f, rc = 1.f, rs = 0.f;
+    if (lane < ntok) {
+      const int64_t pos = p.positions ? p.positions[tok] : (int64_t)p.position + tok;
+      crow = p.cache_rows ? p.cache_rows[tok] : pos;
+      if (p.bias) { bias0 = p.bias[r0]; bias1 = p.bias[r0 + 1]; }
+      if ((is_q || is_k) && pos >= 0 && pos < p.max_position) {
+        const int i = ((is_q ? r0 : r0 - q_rows) % D) >> 1;
+        rc = p.cosine[pos * (D / 2) + i];
+        rs = p.sine[pos * (D / 2) + i];
+      }
+    }
     float a0[T], a1[T];
 #pragma unroll
     for (int t = 0; t < T; ++t) a0[t] = a1[t] = 0.f;
@@ -147,21 +166,10 @@ __global__ void __launch_bounds__(WARPS * 32) qkv_rope_cache_kernel(const QkvRop
 #pragma unroll
       for (int t = 0; t < T; ++t)
         if (lane == t) { y0 = a0[t]; y1 = a1[t]; }
-      if (p.bias) { y0 += p.bias[r0]; y1 += p.bias[r0 + 1]; }
-      const int tok = t_base + lane;
-      const int64_t pos = p.positions ? p.positions[tok] : (int64_t)p.position + tok;
-      const int64_t crow = p.cache_rows ? p.cache_rows[tok] : pos;
-      const bool is_q = r0 < q_rows;
-      const bool is_k = !is_q && r0 < q_rows + kv_rows;
+      y0 += bias0;
+      y1 += bias1;
       if (is_q || is_k) {   // interleaved RoPE: (x_even, x_odd) -> (x_even c - x_odd s, x_even s + x_odd c)
-        const int within = is_q ? r0 : r0 - q_rows;
-        const int i = (within % D) >> 1;
-        float c = 1.f, s = 0.f;
-        if (pos >= 0 && pos < p.max_position) {
-          c = p.cosine[pos * (D / 2) + i];
-          s = p.sine[pos * (D / 2) + i];
-        }
-        const float e = y0 * c - y1 * s, o = y0 * s + y1 * c;
+        const float e = y0 * rc - y1 * rs, o = y0 * rs + y1 * rc;
         y0 = e;
         y1 = o;
       }
@@ -219,6 +227,33 @@ __global__ void __launch_bounds__(kMmaThreads) qkv_rope_cache_mma_kernel(const Q
   float* rope = part + 2 * kMmaWarps * 128;                       // [8 tokens][D/2] cos, then [8][D/2] sin
   long long* tokrow = reinterpret_cast<long long*>(rope + 8 * D);   // [8] cache row of each token, -1 = none
 
+  pdl_wait();
+  pdl_trigger();
+  const int q_rows = p.heads * D, kv_rows = p.kv_heads * D;
+  const int tiles = (q_rows + 2 * kv_rows) / 16;
+  const __nv_bfloat16* W = static_cast<const __nv_bfloat16*>(p.weights);
+  const int chunks = model / 8;                     // 16-byte chunks per weight row
+  // This warp's K slice is chunks warp*4 + c, + 64, + 128, ...; a batch is kBatch of them (all loads in flight at once).
+  // The first batch of the next tile is requested before the current tile is handed to the finishing threads, so the
+  // weight stream does not stop at the tile boundary, and that of the first tile before the activations are staged.
+  constexpr int kBatch = 8;
+  constexpr int kChunkStep = 4 * kMmaWarps;
+  uint4 we[kBatch], wo[kBatch];
+  auto load_batch = [&](int tile, int ch0) {
+    // MMA row m < 8 is weight row 16*tile + 2m (the even row of pair m), row m + 8 the odd row of the same pair
+    const __nv_bfloat16* w_even = W + (int64_t)(16 * tile + 2 * g) * model;
+    const __nv_bfloat16* w_odd = w_even + model;
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int ch = ch0 + u * kChunkStep;
+      const bool ok = ch < chunks;
+      we[u] = ok ? ld_stream16(w_even + ch * 8) : make_uint4(0, 0, 0, 0);
+      wo[u] = ok ? ld_stream16(w_odd + ch * 8) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  const int ch_first = warp * 4 + c;
+  if (warp < kMmaWarps && (int)blockIdx.x < tiles) load_batch(blockIdx.x, ch_first);
+
   // stage the activations: four independent 16-byte loads per thread in flight, then split and store
   {
     const int n4 = 8 * model / 4;
@@ -272,37 +307,12 @@ __global__ void __launch_bounds__(kMmaThreads) qkv_rope_cache_mma_kernel(const Q
   }
   __syncthreads();
 
-  const int q_rows = p.heads * D, kv_rows = p.kv_heads * D;
-  const int tiles = (q_rows + 2 * kv_rows) / 16;
-  const __nv_bfloat16* W = static_cast<const __nv_bfloat16*>(p.weights);
-  const int chunks = model / 8;                     // 16-byte chunks per weight row
   const uint32_t hi_s = (uint32_t)__cvta_generic_to_shared(x_hi), lo_s = (uint32_t)__cvta_generic_to_shared(x_lo);
 
-  // This warp's K slice is chunks warp*4 + c, + 64, + 128, ...; a batch is kBatch of them (all loads in flight at once).
-  // The first batch of the next tile is requested before the current tile is handed to the finishing threads, so the
-  // weight stream does not stop at the tile boundary.
-  constexpr int kBatch = 8;
-  constexpr int kChunkStep = 4 * kMmaWarps;
-  uint4 we[kBatch], wo[kBatch];
-  auto load_batch = [&](int tile, int ch0) {
-    // MMA row m < 8 is weight row 16*tile + 2m (the even row of pair m), row m + 8 the odd row of the same pair
-    const __nv_bfloat16* w_even = W + (int64_t)(16 * tile + 2 * g) * model;
-    const __nv_bfloat16* w_odd = w_even + model;
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
-      const int ch = ch0 + u * kChunkStep;
-      const bool ok = ch < chunks;
-      we[u] = ok ? ld_stream16(w_even + ch * 8) : make_uint4(0, 0, 0, 0);
-      wo[u] = ok ? ld_stream16(w_odd + ch * 8) : make_uint4(0, 0, 0, 0);
-    }
-  };
   // Warps 0..15 stream the weights; warps 16..17 finish the tiles.  The partial sums change hands through two buffers
   // and two pairs of named barriers (full: the tile's partials are written; free: they have been read), so the weight
   // stream never waits for a tile to be finished.
   if (warp < kMmaWarps) {
-  const int ch_first = warp * 4 + c;
-  if ((int)blockIdx.x < tiles) load_batch(blockIdx.x, ch_first);
-
   int it = 0;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -394,8 +404,7 @@ cudaError_t launch_qkv_mma(const QkvRopeParams& p, int t_base, int num_sms, cuda
   const int tiles = (p.heads + 2 * p.kv_heads) * p.head_dim / 16;
   const int per_sm = smem <= 100 * 1024 ? 2 : 1;
   int grid = tiles < num_sms * per_sm ? tiles : num_sms * per_sm;
-  qkv_rope_cache_mma_kernel<<<grid, kMmaThreads, smem, stream>>>(p, t_base);
-  return cudaGetLastError();
+  return launch_dependent(qkv_rope_cache_mma_kernel, grid, kMmaThreads, smem, stream, p, t_base);
 }
 
 __global__ void rope_interleaved_kernel(const float* __restrict__ in, const float* __restrict__ cosc,
@@ -434,13 +443,12 @@ cudaError_t launch_qkv_t(const QkvRopeParams& p, int t_base, int num_sms, cudaSt
       if (e != cudaSuccess) return e;
     }
     const int grid = balanced_grid(pairs, kQkvWarps, num_sms);
-    kern<<<grid, kQkvWarps * 32, xbytes, stream>>>(p, t_base);
+    return launch_dependent(kern, grid, kQkvWarps * 32, xbytes, stream, p, t_base);
   } else {
     constexpr int kQkvWarps = 4;
     const int grid = balanced_grid(pairs, kQkvWarps, num_sms);
-    qkv_rope_cache_kernel<WT, T, kQkvWarps, false><<<grid, kQkvWarps * 32, 0, stream>>>(p, t_base);
+    return launch_dependent(qkv_rope_cache_kernel<WT, T, kQkvWarps, false>, grid, kQkvWarps * 32, 0, stream, p, t_base);
   }
-  return cudaGetLastError();
 }
 
 template <typename WT>

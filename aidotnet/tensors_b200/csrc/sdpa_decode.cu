@@ -110,6 +110,8 @@ __global__ void __launch_bounds__(kDecWarps * 32)
   const int nheads = min(GT, p.group - gc * GT);
   const int c = HEAD_FAST ? blockIdx.y : blockIdx.x;
 
+  pdl_wait();      // nothing above touches memory that an earlier kernel writes
+  pdl_trigger();   // the merge may be set up while this kernel runs
   const int64_t L = decode_len(p, b);
   const int64_t start = (int64_t)c * chunk;
   const int Hc = p.head_count;
@@ -354,6 +356,8 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2)
   const int nheads = p.group;
   const int cidx = HEAD_FAST ? blockIdx.y : blockIdx.x;
 
+  pdl_wait();      // nothing above touches memory that an earlier kernel writes
+  pdl_trigger();   // the merge may be set up while this kernel runs
   const int64_t L = decode_len(p, b);
   const int64_t start = (int64_t)cidx * chunk;
   const int Hc = p.head_count;
@@ -641,39 +645,80 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2)
   }
 }
 
+// Merges the splits of one (sequence, head): the weight of every split is formed once, in parallel, and the columns are
+// summed by 16-byte vectors over groups of splits.  Bound by latency - a few KB per CTA - so nothing in it is a serial
+// chain over the splits except the last sum of 128 / (D / 4) partial columns.
+constexpr int kMaxCombine = 1024;   // split weights held in shared memory; more splits are taken in rounds
+
 template <typename T>
 __global__ void __launch_bounds__(128)
     sdpa_decode_combine_kernel(const SdpaParams p, const int chunk, const int nchunks, const float* __restrict__ ws) {
+  __shared__ float weight[kMaxCombine];
+  __shared__ float red[8];
+  __shared__ float4 cols[128];
+  pdl_wait();   // the partial results of the kernel before this one
   const int b = blockIdx.y;
   const int hl = blockIdx.x;
   const int h = p.head_begin + hl;
   const int D = p.head_dim;
   const int Hc = p.head_count;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t L = decode_len(p, b);
   int nvalid = (int)((L + chunk - 1) / chunk);
   if (nvalid > nchunks) nvalid = nchunks;
   const int64_t slot0 = ((int64_t)b * Hc + hl) * nchunks;
-  const float* ml = ws + (int64_t)p.batch * Hc * nchunks * D;
+  const float2* ml = reinterpret_cast<const float2*>(ws + (int64_t)p.batch * Hc * nchunks * D) + slot0;
 
   float M = -INFINITY;
-  for (int c = 0; c < nvalid; ++c) M = fmaxf(M, ml[(slot0 + c) * 2]);
+  for (int c = tid; c < nvalid; c += 128) M = fmaxf(M, ml[c].x);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+  if (lane == 0) red[warp] = M;
+  __syncthreads();
+  M = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+
+  const int vecs = D / 4, groups = 128 / vecs;      // D = 64, 128, 256: 8, 4, 2 groups of splits
+  const int grp = tid / vecs, d4 = tid - grp * vecs;
+  const float4* rows = reinterpret_cast<const float4*>(ws + slot0 * D) + d4;
   float lsum = 0.f;
-  if (M != -INFINITY)
-    for (int c = 0; c < nvalid; ++c) {
-      const float mc = ml[(slot0 + c) * 2];
-      if (mc != -INFINITY) lsum = fmaf(softmax_exp<T>(mc - M), ml[(slot0 + c) * 2 + 1], lsum);
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int c0 = 0; c0 < nvalid; c0 += kMaxCombine) {
+    const int n = min(kMaxCombine, nvalid - c0);
+    if (c0 > 0) __syncthreads();
+    for (int c = tid; c < n; c += 128) {
+      const float2 v = ml[c0 + c];
+      const float w = v.x == -INFINITY ? 0.f : softmax_exp<T>(v.x - M);
+      weight[c] = w;
+      if (w != 0.f) lsum = fmaf(w, v.y, lsum);
     }
-  const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float a = 0.f;
-    if (M != -INFINITY)
-      for (int c = 0; c < nvalid; ++c) {
-        const float mc = ml[(slot0 + c) * 2];
-        if (mc != -INFINITY) a = fmaf(softmax_exp<T>(mc - M), ws[(slot0 + c) * D + d], a);
-      }
-    store_out<T>(p.out, b * p.os[0] + (int64_t)h * p.os[1] + d, a * inv, p.out_f32);
+    __syncthreads();
+#pragma unroll 4
+    for (int c = grp; c < n; c += groups) {
+      const float w = weight[c];
+      if (w == 0.f) continue;   // (a split that saw no key leaves its columns undefined)
+      const float4 x = rows[(int64_t)(c0 + c) * vecs];
+      a.x = fmaf(w, x.x, a.x); a.y = fmaf(w, x.y, a.y); a.z = fmaf(w, x.z, a.z); a.w = fmaf(w, x.w, a.w);
+    }
   }
-  if (p.lse && threadIdx.x == 0)
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+  if (lane == 0) red[4 + warp] = lsum;
+  cols[tid] = a;
+  __syncthreads();
+  lsum = (red[4] + red[5]) + (red[6] + red[7]);
+  if (grp == 0) {
+    for (int g = 1; g < groups; ++g) {
+      const float4 x = cols[g * vecs + d4];
+      a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+    }
+    const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
+    const int64_t at = b * p.os[0] + (int64_t)h * p.os[1] + d4 * 4;
+    store_out<T>(p.out, at, a.x * inv, p.out_f32);
+    store_out<T>(p.out, at + 1, a.y * inv, p.out_f32);
+    store_out<T>(p.out, at + 2, a.z * inv, p.out_f32);
+    store_out<T>(p.out, at + 3, a.w * inv, p.out_f32);
+  }
+  if (p.lse && tid == 0)
     p.lse[((int64_t)b * p.num_q_heads + h) * p.seq_q] = lsum > 0.f ? M + logf(lsum) : -INFINITY;
 }
 
@@ -684,14 +729,15 @@ cudaError_t launch_partial(const SdpaParams& p, int chunk, int nchunks, float* w
   const bool head_fast = p.ks[1] < p.ks[2] && nchunks <= 65535;
   if (head_fast) {
     dim3 grid(heads_y, (unsigned)nchunks, (unsigned)p.batch);
-    if (p.block_table) sdpa_decode_partial_kernel<T, D, GT, true, true><<<grid, kDecWarps * 32, 0, stream>>>(p, chunk, nchunks, ws, direct);
-    else sdpa_decode_partial_kernel<T, D, GT, false, true><<<grid, kDecWarps * 32, 0, stream>>>(p, chunk, nchunks, ws, direct);
+    if (p.block_table)
+      return launch_dependent(sdpa_decode_partial_kernel<T, D, GT, true, true>, grid, kDecWarps * 32, 0, stream, p, chunk, nchunks, ws, direct);
+    return launch_dependent(sdpa_decode_partial_kernel<T, D, GT, false, true>, grid, kDecWarps * 32, 0, stream, p, chunk, nchunks, ws, direct);
   } else {
     dim3 grid((unsigned)nchunks, heads_y, (unsigned)p.batch);
-    if (p.block_table) sdpa_decode_partial_kernel<T, D, GT, true, false><<<grid, kDecWarps * 32, 0, stream>>>(p, chunk, nchunks, ws, direct);
-    else sdpa_decode_partial_kernel<T, D, GT, false, false><<<grid, kDecWarps * 32, 0, stream>>>(p, chunk, nchunks, ws, direct);
+    if (p.block_table)
+      return launch_dependent(sdpa_decode_partial_kernel<T, D, GT, true, false>, grid, kDecWarps * 32, 0, stream, p, chunk, nchunks, ws, direct);
+    return launch_dependent(sdpa_decode_partial_kernel<T, D, GT, false, false>, grid, kDecWarps * 32, 0, stream, p, chunk, nchunks, ws, direct);
   }
-  return cudaGetLastError();
 }
 
 template <typename T, int D, bool NH16>
@@ -707,14 +753,13 @@ cudaError_t launch_gqa(const SdpaParams& p, int chunk, int nchunks, float* ws, i
     auto kern = sdpa_decode_gqa_ring_kernel<T, D, NH16, PG, HF>;                                                \
     cudaError_t ea = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);             \
     if (ea != cudaSuccess) return ea;                                                                           \
-    kern<<<grid, kDecWarps * 32, smem, stream>>>(p, chunk, nchunks, ws, direct);                                \
+    return launch_dependent(kern, grid, kDecWarps * 32, smem, stream, p, chunk, nchunks, ws, direct);           \
   } while (0)
   if (paged && head_fast) AIDN_GQA_LAUNCH(true, true);
   else if (paged) AIDN_GQA_LAUNCH(true, false);
   else if (head_fast) AIDN_GQA_LAUNCH(false, true);
   else AIDN_GQA_LAUNCH(false, false);
 #undef AIDN_GQA_LAUNCH
-  return cudaGetLastError();
 }
 
 template <typename T, int D>
@@ -750,9 +795,8 @@ cudaError_t launch_decode_t(const SdpaParams& p, int chunk, int nchunks, float* 
   *launches = 1;
   if (e != cudaSuccess || direct) return e;
   dim3 grid((unsigned)p.head_count, (unsigned)p.batch);
-  sdpa_decode_combine_kernel<T><<<grid, 128, 0, stream>>>(p, chunk, nchunks, ws);
   *launches = 2;
-  return cudaGetLastError();
+  return launch_dependent(sdpa_decode_combine_kernel<T>, grid, 128, 0, stream, p, chunk, nchunks, static_cast<const float*>(ws));
 }
 
 
