@@ -65,6 +65,7 @@ constexpr int kBS = 64;            // keys per score sub-tile: one softmax step,
 constexpr int kSoftmaxWarps = 8;   // 2 tiles x 4 warps
 constexpr int kProducerWarp = 8;
 constexpr int kMmaWarp = 9;
+constexpr int kVWarp = 11;         // paged K / V: loads V (the producer then loads K only)
 constexpr int kEpilogueWarp = 12;      // warps 12-15: warp 12 + j reads TMEM lanes 32 j .. 32 j + 31, like softmax warp j
 constexpr int kEpilogueWarps = 4;
 constexpr int kStageBytes = 32768;     // epilogue staging: 32-row x 128-byte boxes (128-byte swizzle) of 4 KiB
@@ -91,7 +92,7 @@ struct Roles {
   static constexpr int kOtherWarps = EPI ? 8 : 4;
   static constexpr int kStoreWarps = EPI ? kEpilogueWarps : kSoftmaxWarps;   // warps that stage and store O
   static constexpr int kStageBufs = EPI ? 2 : 1;                             // 4 KiB staging buffers per storing warp
-  // consumers of the item mailbox: softmax warps, the two UMMA issuers, epilogue warps
+  // consumers of the item mailbox: softmax warps, the two UMMA issuers, epilogue warps (and the V loader of paged launches)
   static constexpr int kSchedConsumers = kSoftmaxWarps + 2 + (EPI ? kEpilogueWarps : 0);
   static_assert(kSoftmaxWarps * 32 * kSoftmaxRegs + kOtherWarps * 32 * kOtherRegs <= kThreads * (EPI ? 128 : 168),
                 "setmaxnreg budget exceeds the registers the CTA is launched with");
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
       mbar_init(bar_o_full + 8 * i, 1);
       mbar_init(bar_pv_done + 8 * i, 1);
       mbar_init(bar_sched_full + 8 * i, 1);
-      mbar_init(bar_sched_empty + 8 * i, R::kSchedConsumers);
+      mbar_init(bar_sched_empty + 8 * i, R::kSchedConsumers + (p.block_table ? 1 : 0));
       mbar_init(bar_stats_full + 8 * i, 4);    // one arrival per softmax warp of the tile
       mbar_init(bar_stats_empty + 8 * i, kEpilogueWarps);
       mbar_init(bar_o_empty + 8 * i, kEpilogueWarps);
@@ -747,13 +748,77 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
     setmaxnreg_dec<R::kOtherRegs>();
   }
 
+  // ---- K / V loads: one 64-key sub-tile into ring position t (waits until the position's slot is free) ----
+  // Paged K/V: a sub-tile of 64 keys is 64 / block_size pool blocks, each fetched by its own TMA box (block_size
+  // rows) into its slice of the ring slot - the 128-byte swizzle is a function of the shared-memory address, so
+  // the slices compose into the same image as one 64-row box - or, with 128-token blocks, half of one block.
+  // The table is read 32 entries at a time, lane i holding entry first + i: an entry per slice and sub-tile puts a dependent
+  // global load in front of every one.  Issuing the boxes takes longer still (16 per sub-tile of K and V with 16-token
+  // blocks), so K and V are issued by a warp each, independently: every ring position has one loader, and an item's
+  // positions follow from its number of sub-tiles.  512 queries at 7600 + 512 keys, Hq32 / Hkv8: 16-token blocks 123 us with
+  // one loader, 92 with two (64-token blocks 93 and 92, no table 87).  The loops stay rolled: unrolled, the box loop spilled
+  // registers that the softmax warps' code shares.
+  struct TableWindow { int32_t first, blk; };   // (keys of a paged sequence count in 31 bits)
+  auto last_block = [&](const Item& it) {   // the last logical block of the sequence that the item's keys lie in
+    if (!p.block_table) return 0;
+    const int seq_last = (int)((kv_limit_of(p, it.b) - 1) >> p.block_shift);
+    const int item_last = (int)(((int64_t)(it.k0 + it.n_max) * kBS - 1) >> p.block_shift);
+    return item_last < seq_last ? item_last : seq_last;
+  };
+  auto load_kv = [&](auto paged_kv, const CUtensorMap* tm, const Item& it, int key_sub, uint32_t t, int last_blk, TableWindow& win, bool leader) {
+    const int s = (int)(t % C::kStages);
+    if (!mbar_wait(bar_kv_empty + 8 * s, ((t / C::kStages) & 1u) ^ 1u, abort_flag, wait_ns)) return false;
+    const uint32_t dst = kv_smem + s * C::kSubBytes, bar = bar_kv_full + 8 * s;
+    if (leader) mbar_expect_tx(bar, (uint32_t)C::kSubBytes);
+    if constexpr (!decltype(paged_kv)::value) {
+      if (leader) {
+#pragma unroll
+        for (int hf = 0; hf < C::kHalves; ++hf)
+          tma_load_4d(dst + hf * C::kKvHalfBytes, tm, bar, hf * 64, key_sub * kBS, it.kvh, it.b);
+      }
+    } else {
+      const int rows = p.block_size < kBS ? p.block_size : kBS;   // rows per box
+      const int parts = kBS / rows;
+      // Logical blocks past the last one repeat it: their keys are masked and the table has no entry for them
+      // (the V rows among them are cleared before use, the K rows only feed masked scores).
+      int lb0 = (int)(((int64_t)key_sub * kBS) >> p.block_shift);
+      if (lb0 > last_blk) lb0 = last_blk;
+      if (lb0 < win.first || lb0 + parts > win.first + 32) {
+        win.first = lb0;
+        win.blk = 0;
+        if (lb0 + lane <= last_blk) {
+          win.blk = __ldg(p.block_table + (int64_t)it.b * p.bt_stride + lb0 + lane);
+          if ((win.blk < 0 || win.blk >= p.num_blocks) && p.status) atomicOr(p.status, kStatusBadBlock);
+        }
+      }
+      const int in_block = (key_sub * kBS) & (p.block_size - 1);   // non-zero only for 128-token blocks
+#pragma unroll 1
+      for (int part = 0; part < parts; ++part) {
+        // an entry outside the pool gives an out-of-range coordinate, which TMA fills with zeros
+        const int lb = lb0 + part < last_blk ? lb0 + part : last_blk;
+        const int32_t phys = __shfl_sync(0xffffffffu, win.blk, lb - win.first);
+        if (leader) {
+#pragma unroll
+          for (int hf = 0; hf < C::kHalves; ++hf)
+            tma_load_4d(dst + hf * C::kKvHalfBytes + part * (rows * 128), tm, bar, hf * 64,
+                        phys * p.block_size + (parts == 1 ? in_block : 0), it.kvh, 0);
+        }
+      }
+    }
+    return true;
+  };
+  // ring positions of an item's n sub-tiles: K(0), then K(u+1), V(u) for u = 0 .. n-2, then V(n-1) - the order in which
+  // the issuers need them (the score product runs two sub-tiles ahead of the P.V product)
+  auto ring_k = [](uint32_t t0, int sub) { return t0 + (uint32_t)(sub == 0 ? 0 : 2 * sub - 1); };
+  auto ring_v = [](uint32_t t0, int sub, int n) { return t0 + (uint32_t)(sub + 1 < n ? 2 * sub + 2 : 2 * n - 1); };
+
   if (warp == kProducerWarp) {
     // ==================================== TMA producer + scheduler ====================================
     // warp-uniform like the UMMA issuer: one elected lane issues the TMA loads and barrier operations
     {
       const bool leader = elect_one();
       bool alive = true;
-      uint32_t t_load = 0;          // K/V tiles loaded so far (ring position)
+      uint32_t t_load = 0;          // K/V sub-tiles of earlier items (ring position)
       uint32_t q_uses[2] = {0, 0};  // loads of each Q tile so far
       int item = blockIdx.x;
       for (int seq = 0; alive; ++seq) {
@@ -797,75 +862,26 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
           load_tile(&tm_q, q_smem + i * C::kTileBytes, bar_q_full + 8 * i, it.tile[i].t * kBM, it.tile[i].h);
           ++q_uses[i];
         };
-        // Paged K/V: a sub-tile of 64 keys is 64 / block_size pool blocks, each fetched by its own TMA box (block_size
-        // rows) into its slice of the ring slot - the 128-byte swizzle is a function of the shared-memory address, so
-        // the slices compose into the same image as one 64-row box - or, with 128-token blocks, half of one block.
-        // The table is read 32 entries at a time, lane i holding entry first + i, once for K and once for V (which run a
-        // sub-tile apart): an entry per slice and sub-tile puts a dependent global load in front of every one (512 queries
-        // at 7600 + 512 keys, Hq32 / Hkv8, 16-token blocks: 209.1 us, 205.4 with the windows).
-        const bool paged = p.block_table != nullptr;
-        int64_t last_blk = 0;   // the last logical block of the sequence that the item's keys lie in
-        if (paged) {
-          last_blk = (kv_limit_of(p, it.b) - 1) >> p.block_shift;
-          const int64_t item_last = ((int64_t)(it.k0 + it.n_max) * kBS - 1) >> p.block_shift;
-          if (item_last < last_blk) last_blk = item_last;
-        }
-        struct TableWindow { int64_t first; int32_t blk; };
-        TableWindow win_k = {-64, 0}, win_v = {-64, 0};
-        auto load_kv = [&](const CUtensorMap* tm, int key_sub, TableWindow& win) {
-          const int s = (int)(t_load % C::kStages);
-          const uint32_t phase = (t_load / C::kStages) & 1u;
-          if (!mbar_wait(bar_kv_empty + 8 * s, phase ^ 1u, abort_flag, wait_ns)) { alive = false; return; }
-          const uint32_t dst = kv_smem + s * C::kSubBytes, bar = bar_kv_full + 8 * s;
-          if (leader) mbar_expect_tx(bar, (uint32_t)C::kSubBytes);
-          if (!paged) {
-            if (leader) {
-#pragma unroll
-              for (int hf = 0; hf < C::kHalves; ++hf)
-                tma_load_4d(dst + hf * C::kKvHalfBytes, tm, bar, hf * 64, key_sub * kBS, it.kvh, it.b);
-            }
-          } else {
-            const int rows = p.block_size < kBS ? p.block_size : kBS;   // rows per box
-            const int parts = kBS / rows;
-            // Logical blocks past the last one repeat it: their keys are masked and the table has no entry for them
-            // (the V rows among them are cleared before use, the K rows only feed masked scores).
-            int64_t lb0 = ((int64_t)key_sub * kBS) >> p.block_shift;
-            if (lb0 > last_blk) lb0 = last_blk;
-            if (lb0 < win.first || lb0 + parts > win.first + 32) {
-              win.first = lb0;
-              win.blk = 0;
-              if (lb0 + lane <= last_blk) {
-                win.blk = __ldg(p.block_table + (int64_t)it.b * p.bt_stride + lb0 + lane);
-                if ((win.blk < 0 || win.blk >= p.num_blocks) && p.status) atomicOr(p.status, kStatusBadBlock);
-              }
-            }
-            const int in_block = (int)(((int64_t)key_sub * kBS) & (int64_t)(p.block_size - 1));   // non-zero only for 128-token blocks
-            for (int part = 0; part < parts; ++part) {
-              // an entry outside the pool gives an out-of-range coordinate, which TMA fills with zeros
-              const int64_t lb = lb0 + part < last_blk ? lb0 + part : last_blk;
-              const int32_t phys = __shfl_sync(0xffffffffu, win.blk, (int)(lb - win.first));
-              if (leader) {
-#pragma unroll
-                for (int hf = 0; hf < C::kHalves; ++hf)
-                  tma_load_4d(dst + hf * C::kKvHalfBytes + part * (rows * 128), tm, bar, hf * 64,
-                              phys * p.block_size + (parts == 1 ? in_block : 0), it.kvh, 0);
-              }
-            }
-          }
-          ++t_load;
-        };
-        // Ring order of an item with n sub-tiles: K(0), then K(u+1), V(u) for u = 0 .. n-2, then V(n-1) - the order in
-        // which the issuers need them (the score product runs two sub-tiles ahead of the P.V product).
         const int n_sub = it.n_max;
         if (n_sub > 0) {
+          const int last_blk = last_block(it);
+          TableWindow win = {-64, 0};
           load_q(0);
-          if (alive) load_kv(&tm_k, it.k0, win_k);
+          if (!p.block_table && alive) alive = load_kv(std::false_type{}, &tm_k, it, it.k0, ring_k(t_load, 0), 0, win, leader);
           if (ptrace && leader) ptrace[0] = globaltimer_ns();
           if (alive) load_q(1);
-          for (int u = 0; u < n_sub && alive; ++u) {
-            if (u + 1 < n_sub) load_kv(&tm_k, it.k0 + u + 1, win_k);
-            if (alive) load_kv(&tm_v, it.k0 + u, win_v);
+          if (p.block_table) {
+#pragma unroll 1
+            for (int u = 0; u < n_sub && alive; ++u)
+              alive = load_kv(std::true_type{}, &tm_k, it, it.k0 + u, ring_k(t_load, u), last_blk, win, leader);
+          } else {
+#pragma unroll 1
+            for (int u = 0; u < n_sub && alive; ++u) {
+              if (u + 1 < n_sub) alive = load_kv(std::false_type{}, &tm_k, it, it.k0 + u + 1, ring_k(t_load, u + 1), 0, win, leader);
+              if (alive) alive = load_kv(std::false_type{}, &tm_v, it, it.k0 + u, ring_v(t_load, u, n_sub), 0, win, leader);
+            }
           }
+          t_load += 2 * (uint32_t)n_sub;
         }
         {
           int next = 0;
@@ -873,6 +889,25 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
           item = __shfl_sync(0xffffffffu, next, 0);   // elect.sync picks the lowest lane of the full warp
         }
       }
+    }
+  } else if (warp == kVWarp && p.block_table) {
+    // ======================================= V loads of a paged launch =======================================
+    const bool leader = elect_one();
+    bool alive = true;
+    uint32_t t0 = 0;
+    for (int seq = 0; alive; ++seq) {
+      const int slot = seq & 1;
+      if (!mbar_wait(bar_sched_full + 8 * slot, (uint32_t)((seq >> 1) & 1), abort_flag, wait_ns)) break;
+      const int item = mailbox[slot * kItemWords];
+      if (item >= pp.total_items) break;
+      Item it = read_item(mailbox + slot * kItemWords);
+      __syncwarp();
+      if (leader) mbar_arrive(bar_sched_empty + 8 * slot);
+      const int last_blk = last_block(it);
+      TableWindow win = {-64, 0};
+#pragma unroll 1
+      for (int u = 0; u < it.n_max && alive; ++u) alive = load_kv(std::true_type{}, &tm_v, it, it.k0 + u, ring_v(t0, u, it.n_max), last_blk, win, leader);
+      t0 += 2 * (uint32_t)it.n_max;
     }
   } else if (warp == kMmaWarp || warp == kMmaWarp + 1) {
     // ========================================== UMMA issuers ==========================================
@@ -936,12 +971,11 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
         const int n_max = it.n_max;
         if (n_max == 0) continue;
         const int n0 = it.tile[0].n, n1 = it.tile[1].n;
-        // ring positions of the item's sub-tiles (the producer's order): K(0) at t0, K(s) at t0 + 2s - 1,
-        // V(u) at t0 + 2u + 2 except the last one, which follows K(n_max - 1) directly
+        // ring positions of the item's sub-tiles
         const uint32_t t0 = t_cons;
         t_cons = t0 + 2 * (uint32_t)n_max;
-        auto pos_k = [&](int sub) { return t0 + (uint32_t)(sub == 0 ? 0 : 2 * sub - 1); };
-        auto pos_v = [&](int sub) { return t0 + (uint32_t)(sub + 1 < n_max ? 2 * sub + 2 : 2 * n_max - 1); };
+        auto pos_k = [&](int sub) { return ring_k(t0, sub); };
+        auto pos_v = [&](int sub) { return ring_v(t0, sub, n_max); };
         const int g0 = g;             // turn g0: prologue of issuer 0, g0 + 1: of issuer 1, g0 + 2 + u: sub-tile u
         g = g0 + 2 + n_max;
         auto kv_slot = [&](uint32_t t) { return (int)(t % C::kStages); };

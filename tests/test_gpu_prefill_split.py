@@ -78,3 +78,28 @@ def test_many_items_or_few_keys_are_not_split():
     shard = N.Handle(device=0, qkv_dtype=N.BF16, out_dtype=N.F32, head_dim=128, num_q_heads=32, num_kv_heads=8, head_begin=8, head_count=8)
     assert shard.workspace_bytes(1, 512, 8112) == 0
     shard.close()
+
+
+@pytest.mark.parametrize("block", [8, 16, 32, 64, 128])
+@pytest.mark.parametrize("seq_q,start", [(130, 1000), (300, 2900)])
+def test_paged_split_windows(block, seq_q, start):
+    """Paged K and V, one loader each, over parts that begin anywhere in a 32-entry window of the block table."""
+    from aidotnet.tensors_b200.backend import CudaBackend, GpuBuffer
+    heads, kv_heads, D, keys = 4, 2, 128, start + seq_q
+    blocks = (keys + block - 1) // block
+    pool = blocks + 5
+    q, qf = gen((seq_q, heads, D), "bf16", 1)
+    k, kf = gen((pool * block, kv_heads, D), "bf16", 2)
+    v, vf = gen((pool * block, kv_heads, D), "bf16", 3)
+    table = np.random.default_rng(block).permutation(pool)[:blocks].astype(np.int32)
+    rows = table[np.arange(keys) // block] * block + np.arange(keys) % block
+    unused = np.setdiff1d(np.arange(pool * block), rows)
+    v[torch.from_numpy(unused).cuda()] = float("nan")
+    backend = CudaBackend(0)
+    buf = lambda t: GpuBuffer(t.reshape(-1))
+    out = backend.PagedAttentionPrefillGqa(buf(q), buf(k), buf(v), GpuBuffer(torch.from_numpy(table).cuda()), heads, kv_heads, D, block,
+                                           seq_q, start, D ** -0.5)
+    ref = O.sdpa(qf.transpose(1, 0, 2)[None], kf[rows].transpose(1, 0, 2)[None], vf[rows].transpose(1, 0, 2)[None], causal=True,
+                 causal_offset=start)
+    compare(out.tensor.float().view(seq_q, heads, D), ref[0].transpose(1, 0, 2), "bf16", f"block {block}")
+    backend.Dispose()
