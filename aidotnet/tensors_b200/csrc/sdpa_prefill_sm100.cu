@@ -187,15 +187,48 @@ __device__ __forceinline__ Item read_item(const volatile int* box) {
   return it;
 }
 
-__device__ __forceinline__ Item decode_item(const PrefillParams& pp, int item) {
+// Sequences of a batch in the order of their lengths, longest first: lane r gets the batch index of rank r (warp-uniform
+// call; at most 32 sequences, otherwise - and without lengths - the order they come in).
+constexpr int kMaxSorted = 32;
+
+__device__ __forceinline__ int length_order(const SdpaParams& p, int lane) {
+  if (!p.kv_len || p.batch > kMaxSorted) return lane;
+  const int len = lane < p.batch ? (int)kv_limit_of(p, lane) : -1;
+  int rank = 0;
+#pragma unroll 1
+  for (int s = 0; s < p.batch; ++s) {
+    const int other = __shfl_sync(0xffffffffu, len, s);
+    rank += (other > len || (other == len && s < lane)) ? 1 : 0;
+  }
+  int order = lane;
+#pragma unroll 1
+  for (int s = 0; s < p.batch; ++s)
+    if (__shfl_sync(0xffffffffu, rank, s) == lane) order = s;
+  return order;
+}
+
+// Warp-uniform; `order` is the caller's lane of length_order.
+__device__ __forceinline__ Item decode_item(const PrefillParams& pp, int item, int order) {
   const SdpaParams& p = pp.p;
   Item it;
   const int split = pp.splits > 1 ? item % pp.splits : 0;
   if (pp.splits > 1) item /= pp.splits;
-  const int rank = item / pp.items_per_rank;
-  const int rem = item - rank * pp.items_per_rank;
-  it.b = rem / pp.per_batch;
-  const int w = rem - it.b * pp.per_batch;
+  // Heavy items first, so that the last ones to start are short: by row tile under a causal mask, else by sequence length
+  // (six sequences of 124 to 997 keys, 16 heads of 64, fp16: 44.6 us in the order they come, 40.9 longest first).
+  int rank, w;
+  if (p.kv_len && !p.causal) {
+    const int per_seq = pp.ranks * pp.per_batch;
+    it.b = item / per_seq;
+    const int rem = item - it.b * per_seq;
+    rank = rem / pp.per_batch;
+    w = rem - rank * pp.per_batch;
+  } else {
+    rank = item / pp.items_per_rank;
+    const int rem = item - rank * pp.items_per_rank;
+    it.b = rem / pp.per_batch;
+    w = rem - it.b * pp.per_batch;
+  }
+  if (p.kv_len && p.batch <= kMaxSorted) it.b = __shfl_sync(0xffffffffu, order, it.b);
   if (pp.pair_heads) {
     const int t = pp.row_tiles - 1 - rank;
     it.tile[0].h = p.head_begin + 2 * w;
@@ -820,13 +853,14 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
       bool alive = true;
       uint32_t t_load = 0;          // K/V sub-tiles of earlier items (ring position)
       uint32_t q_uses[2] = {0, 0};  // loads of each Q tile so far
+      const int order = length_order(p, lane);
       int item = blockIdx.x;
       for (int seq = 0; alive; ++seq) {
         const int slot = seq & 1;
         if (!mbar_wait(bar_sched_empty + 8 * slot, (uint32_t)(((seq >> 1) & 1) ^ 1), abort_flag, wait_ns)) break;
         Item it;
         if (item < pp.total_items) {
-          it = decode_item(pp, item);
+          it = decode_item(pp, item, order);
           // Row pairs: the second tile runs two sub-tiles longer.  Alternating which softmax warpgroup gets it keeps
           // that lag from building up on one side from item to item.
           if (!pp.pair_heads && (seq & 1)) {

@@ -80,6 +80,23 @@ def test_many_items_or_few_keys_are_not_split():
     shard.close()
 
 
+@pytest.mark.parametrize("batch", [1, 7, 32, 33])
+@pytest.mark.parametrize("causal", [False, True])
+def test_items_ordered_by_length(batch, causal):
+    """More items than SMs, lengths with ties, zeros and values past the tensor: every sequence is computed once, in whatever
+    order the lengths give (33 sequences are not sorted)."""
+    rng = np.random.default_rng(batch)
+    Hq, Hkv, Sq, Sk, D = 12, 6, 140, 150, 64
+    lens = rng.choice([0, 1, 64, 65, 150, 4000], batch).astype(np.int32)
+    q, qf = gen((batch, Hq, Sq, D), "bf16", 1)
+    k, kf = gen((batch, Hkv, Sk, D), "bf16", 2)
+    v, vf = gen((batch, Hkv, Sk, D), "bf16", 3)
+    got, lse, _ = run_gpu(q, k, v, dtype="bf16", want_lse=True, path=N.PATH_PREFILL_SM100, causal=causal, kv_len=torch.from_numpy(lens).cuda())
+    ref, ref_lse, _ = O.sdpa(qf, kf, vf, want_lse=True, causal=causal, kv_len=np.minimum(lens, Sk))
+    compare(got, ref, "bf16", f"{batch} {causal}")
+    compare_lse(lse, ref_lse, "bf16", f"{batch} {causal}")
+
+
 @pytest.mark.parametrize("block", [8, 16, 32, 64, 128])
 @pytest.mark.parametrize("seq_q,start", [(130, 1000), (300, 2900)])
 def test_paged_split_windows(block, seq_q, start):
