@@ -43,36 +43,95 @@ __global__ void __launch_bounds__(128) bwd_delta_kernel(const BwdParams bp) {
   const int64_t gb = b * bp.dos[0] + (int64_t)h * bp.dos[1] + row * bp.dos[2];
   float acc = 0.f;
   T* gt = bp.dout_t ? static_cast<T*>(bp.dout_t) + (((int64_t)b * p.head_count + hl) * p.seq_q + row) * p.head_dim : nullptr;
-  // fp32 O and dO with 16-byte aligned rows: four elements per lane and load
-  const bool vec = p.out_f32 && p.head_dim % 4 == 0 && ((ob | gb) & 3) == 0 &&
-                   ((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(bp.dout)) & 15) == 0 &&
-                   (!gt || sizeof(T) == 2) && ((reinterpret_cast<uintptr_t>(bp.dout_t) & 7) == 0);
-  if (vec) {
-    const float4* o4 = reinterpret_cast<const float4*>(static_cast<const float*>(p.out) + ob);
-    const float4* g4 = reinterpret_cast<const float4*>(static_cast<const float*>(bp.dout) + gb);
-    for (int d4 = lane; d4 < p.head_dim / 4; d4 += 32) {
-      const float4 o = o4[d4];
-      float4 g = g4[d4];
-      if (gt) {
-        T t4[4] = {from_float<T>(g.x), from_float<T>(g.y), from_float<T>(g.z), from_float<T>(g.w)};
-        *reinterpret_cast<uint2*>(gt + 4 * d4) = *reinterpret_cast<const uint2*>(t4);
-        if (bp.round_dout) g = make_float4(to_float<T>(t4[0]), to_float<T>(t4[1]), to_float<T>(t4[2]), to_float<T>(t4[3]));
-      }
-      acc += g.x * o.x + g.y * o.y + g.z * o.z + g.w * o.w;
+  for (int d = lane; d < p.head_dim; d += 32) {
+    float go = load_o<T>(bp.dout, gb + d, p.out_f32);
+    if (gt) {
+      gt[d] = from_float<T>(go);   // the tensor-core dK / dV kernels stream dO in the input dtype
+      if (bp.round_dout) go = to_float<T>(gt[d]);
     }
-  } else {
-    for (int d = lane; d < p.head_dim; d += 32) {
-      float go = load_o<T>(bp.dout, gb + d, p.out_f32);
-      if (gt) {
-        gt[d] = from_float<T>(go);   // the tensor-core dK / dV kernels stream dO in the input dtype
-        if (bp.round_dout) go = to_float<T>(gt[d]);
-      }
-      acc += go * load_o<T>(p.out, ob + d, p.out_f32);
-    }
+    acc += go * load_o<T>(p.out, ob + d, p.out_f32);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (lane == 0) bp.delta[((int64_t)b * p.head_count + hl) * p.seq_q + row] = acc;
+}
+
+// The same for head_dim 64 / 128 with 16-byte rows of O and dO (TO: their type): a 16-byte vector per lane, D / vector lanes
+// per row, four such steps' loads in flight per warp before the first is used.  HBM-bound (84 MB at
+// B1 H32 S2048 D128 with fp32 O and dO); one row and one load pair per warp in flight made the training step 4.6 us
+// longer (252.6 against 248.0 us).  TT: type of the dO copy.
+template <typename TO, typename TT, int D>
+__global__ void __launch_bounds__(128) bwd_delta_vec_kernel(const BwdParams bp) {
+  const SdpaParams& p = bp.p;
+  constexpr int N = 16 / sizeof(TO), L = D / N, R = 32 / L, kSteps = 4;
+  const int lane = threadIdx.x & 31, d = lane % L * N;
+  const int64_t row0 = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * (R * kSteps) + lane / L;
+  const int hl = blockIdx.y, b = blockIdx.z, h = p.head_begin + hl;
+  const TO* ob = static_cast<const TO*>(p.out) + b * p.os[0] + (int64_t)h * p.os[1] + d;
+  const TO* gb = static_cast<const TO*>(bp.dout) + b * bp.dos[0] + (int64_t)h * bp.dos[1] + d;
+  uint4 o[kSteps], g[kSteps];
+#pragma unroll
+  for (int s = 0; s < kSteps; ++s) {
+    const int64_t row = row0 + s * R;
+    o[s] = g[s] = make_uint4(0, 0, 0, 0);
+    if (row < p.seq_q) {
+      o[s] = *reinterpret_cast<const uint4*>(ob + row * p.os[2]);
+      g[s] = *reinterpret_cast<const uint4*>(gb + row * bp.dos[2]);
+    }
+  }
+  const int64_t first = ((int64_t)b * p.head_count + hl) * p.seq_q;
+#pragma unroll
+  for (int s = 0; s < kSteps; ++s) {
+    const int64_t row = row0 + s * R;
+    TO ov[N], gv[N];
+    *reinterpret_cast<uint4*>(ov) = o[s];
+    *reinterpret_cast<uint4*>(gv) = g[s];
+    float acc = 0.f;
+    TT t[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+      float x = to_float<TO>(gv[e]);
+      t[e] = from_float<TT>(x);
+      if (bp.round_dout) x = to_float<TT>(t[e]);
+      acc = fmaf(x, to_float<TO>(ov[e]), acc);
+    }
+    if (bp.dout_t && row < p.seq_q) {
+      TT* dst = static_cast<TT*>(bp.dout_t) + (first + row) * D + d;
+      if constexpr (N * sizeof(TT) == 16) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(t);
+      else *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(t);
+    }
+#pragma unroll
+    for (int w = L / 2; w > 0; w >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, w);
+    if (lane % L == 0 && row < p.seq_q) bp.delta[first + row] = acc;
+  }
+}
+
+template <typename TO, typename TT>
+cudaError_t launch_delta_vec(const BwdParams& bp, cudaStream_t stream) {
+  const int rows = 4 * 4 * 32 * 16 / (bp.p.head_dim * (int)sizeof(TO));   // rows per CTA
+  const dim3 grid((unsigned)((bp.p.seq_q + rows - 1) / rows), (unsigned)bp.p.head_count, (unsigned)bp.p.batch);
+  if (bp.p.head_dim == 64) bwd_delta_vec_kernel<TO, TT, 64><<<grid, 128, 0, stream>>>(bp);
+  else bwd_delta_vec_kernel<TO, TT, 128><<<grid, 128, 0, stream>>>(bp);
+  return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_delta(const BwdParams& bp, cudaStream_t stream) {
+  const SdpaParams& p = bp.p;
+  const int esz = p.out_f32 ? 4 : 2;
+  auto rows16 = [&](const void* ptr, const int64_t* st) {
+    return reinterpret_cast<uintptr_t>(ptr) % 16 == 0 && st[0] * esz % 16 == 0 && st[1] * esz % 16 == 0 && st[2] * esz % 16 == 0;
+  };
+  if ((p.head_dim == 64 || p.head_dim == 128) && rows16(p.out, p.os) && rows16(bp.dout, bp.dos) &&
+      reinterpret_cast<uintptr_t>(bp.dout_t) % 16 == 0) {
+    if constexpr (sizeof(T) == 2) {
+      if (!p.out_f32) return launch_delta_vec<T, T>(bp, stream);
+    }
+    return launch_delta_vec<float, T>(bp, stream);
+  }
+  const dim3 grid((unsigned)((p.seq_q + 3) / 4), (unsigned)p.head_count, (unsigned)p.batch);
+  bwd_delta_kernel<T><<<grid, 128, 0, stream>>>(bp);
+  return cudaGetLastError();
 }
 
 // Probability and score gradient of (row, key): p = exp(logit - lse), ds = p * (dp - delta).
@@ -758,7 +817,7 @@ template <typename T, int DMAX>
 cudaError_t launch_bwd_t(const BwdParams& bp, cudaStream_t stream, int* launches, int* used_tcgen05) {
   const SdpaParams& p = bp.p;
   constexpr int PITCH = DMAX + 4;
-  dim3 g0((unsigned)((p.seq_q + 3) / 4), (unsigned)p.head_count, (unsigned)p.batch);
+  cudaError_t e;
   {
     // the tensor-core families multiply with dO in the input dtype: sum delta from the same rounded values
     bool tensor_cores = false;
@@ -766,9 +825,8 @@ cudaError_t launch_bwd_t(const BwdParams& bp, cudaStream_t stream, int* launches
       tensor_cores = p.head_dim == DMAX && !p.block_table && mma_aligned(bp) && (bp.dout_t || !p.out_f32);
     BwdParams b0 = bp;
     b0.round_dout = tensor_cores ? 1 : 0;
-    bwd_delta_kernel<T><<<g0, 128, 0, stream>>>(b0);
+    e = launch_delta<T>(b0, stream);
   }
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   *used_tcgen05 = 0;
   if constexpr (sizeof(T) == 2 && (DMAX == 64 || DMAX == 128)) {
