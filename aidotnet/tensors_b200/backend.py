@@ -73,7 +73,7 @@ class CudaBackend:
         self._path = path
         self._decode_chunk = decode_chunk
         self._handles: Dict[Tuple, N.Handle] = {}
-        self._scratch: Optional[torch.Tensor] = None
+        self._scratch: Dict[int, torch.Tensor] = {}   # by stream: calls on different streams may overlap
         self.launch_count = 0  # kernels enqueued by this backend (the reference counts launches in GpuLaunchProbe)
 
     # -- plumbing ---------------------------------------------------------------------------------------
@@ -109,12 +109,20 @@ class CudaBackend:
             self._handles[key] = h
         return h
 
-    def _workspace(self, nbytes: int) -> Tuple[Optional[int], int]:
+    def _workspace(self, nbytes: int, stream: torch.cuda.Stream) -> Tuple[Optional[int], int]:
+        """The scratch buffer of ``stream``, grown on demand.  It is allocated on that stream, so a buffer that is replaced
+        is reused only behind the launches that read it."""
         if nbytes <= 0:
             return None, 0
-        if self._scratch is None or self._scratch.numel() < nbytes:
-            self._scratch = torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{self.device}")
-        return self._scratch.data_ptr(), self._scratch.numel()
+        buf = self._scratch.get(stream.cuda_stream)
+        if buf is None or buf.numel() < nbytes:
+            self._scratch.pop(stream.cuda_stream, None)
+            if len(self._scratch) >= 16:
+                self._scratch.pop(next(iter(self._scratch)))
+            with torch.cuda.stream(stream):
+                buf = torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{self.device}")
+            self._scratch[stream.cuda_stream] = buf
+        return buf.data_ptr(), buf.numel()
 
     @staticmethod
     def _check_dims(batch, numHeads, seqQ, seqK, headDim):
@@ -124,9 +132,10 @@ class CudaBackend:
     def _run(self, h: N.Handle, *, query, key, value, output, batch, seqQ, seqK, scale, lse=None, mask=None,
              mask_stride=(0, 0, 0, 0), kv_len=None, q_stride=None, k_stride=None, v_stride=None, o_stride=None,
              block_table=None, block_table_stride=0, block_size=0, num_blocks=0, weights=None):
-        ws, ws_bytes = self._workspace(h.workspace_bytes(batch, seqQ, seqK))
+        stream = self.stream
+        ws, ws_bytes = self._workspace(h.workspace_bytes(batch, seqQ, seqK), stream)
         h.launch(q=query.Handle, k=key.Handle, v=value.Handle, out=output.Handle, batch=batch, seq_q=seqQ, seq_kv=seqK,
-                 stream=self.stream.cuda_stream, lse=lse.Handle if lse is not None else None,
+                 stream=stream.cuda_stream, lse=lse.Handle if lse is not None else None,
                  mask=mask.Handle if mask is not None else None, mask_stride=mask_stride,
                  kv_len=kv_len.Handle if kv_len is not None else None, q_stride=q_stride, k_stride=k_stride,
                  v_stride=v_stride, o_stride=o_stride, scale=scale, workspace=ws, workspace_bytes=ws_bytes,
@@ -367,10 +376,11 @@ class CudaBackend:
                          causal_offset=0, emit_lse=True,
                          mask_kind=N.MASK_ADD_F32 if attentionBias is not None else N.MASK_NONE)
         nbytes = h.backward_workspace_bytes(batch, seqQ)
-        ws, ws_bytes = self._workspace(nbytes)
+        stream = self.stream
+        ws, ws_bytes = self._workspace(nbytes, stream)
         h.backward(q=query.Handle, k=key.Handle, v=value.Handle, out=output.Handle, lse=softmaxStats.Handle,
                    dout=gradOutput.Handle, dq=gradQuery.Handle, dk=gradKey.Handle, dv=gradValue.Handle, batch=batch,
-                   seq_q=seqQ, seq_kv=seqK, stream=self.stream.cuda_stream, workspace=ws, workspace_bytes=ws_bytes,
+                   seq_q=seqQ, seq_kv=seqK, stream=stream.cuda_stream, workspace=ws, workspace_bytes=ws_bytes,
                    mask=attentionBias.Handle if attentionBias is not None else None,
                    mask_stride=(biasBatchStride, seqQ * seqK, seqK, 1) if attentionBias is not None else (0, 0, 0, 0),
                    scale=float(scale))
@@ -426,13 +436,14 @@ class CudaBackend:
                          num_q_heads=numHeads, num_kv_heads=numHeads,
                          mask_kind=N.MASK_KEEP_U8 if mask is not None else N.MASK_NONE)
         nbytes = h.mha_workspace_bytes(batch, seq, _DTYPE[input.dtype], _DTYPE[qWeight.dtype])
-        ws, ws_bytes = self._workspace(nbytes + 1024)
+        stream = self.stream
+        ws, ws_bytes = self._workspace(nbytes + 1024, stream)
         base = (ws + 1023) // 1024 * 1024
         h.mha_forward(input=input.Handle, q_weight=qWeight.Handle, k_weight=kWeight.Handle, v_weight=vWeight.Handle,
                       out_weight=outWeight.Handle, out=output.Handle, batch=batch, seq=seq,
                       input_dtype=_DTYPE[input.dtype], weight_dtype=_DTYPE[qWeight.dtype],
                       out_dtype=_DTYPE[output.dtype], workspace=base, workspace_bytes=ws_bytes - (base - ws),
-                      stream=self.stream.cuda_stream, mask=mask.Handle if mask is not None else None, mask_stride=ms)
+                      stream=stream.cuda_stream, mask=mask.Handle if mask is not None else None, mask_stride=ms)
         self.launch_count += h.last_launch_count
 
     # -- the decode step in front of attention ----------------------------------------------------------------

@@ -38,8 +38,16 @@ aidn_sdpa_t CudaBackend::Handle(const aidn_sdpa_desc& d) {
 }
 
 void CudaBackend::Run(aidn_sdpa_t h, aidn_sdpa_args& a, const aidn_paged_kv* paged) {
-  const int64_t need = aidn_sdpa_workspace_bytes(h, a.batch, a.seq_q, a.seq_kv);
+  int64_t need = aidn_sdpa_workspace_bytes(h, a.batch, a.seq_q, a.seq_kv);
   if (need < 0) Check(AIDN_EINVAL, "aidn_sdpa_workspace_bytes");
+  if (a.seq_q > 1 && need > workspace_bytes_) {
+    // A prefill runs without its workspace too: it is not grown where that cannot be done (during stream capture).
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream_), &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      need = 0;
+    }
+  }
   if (need > workspace_bytes_) {   // grown outside of launch, like the reference's pooled scratch buffers
     if (workspace_) cudaFree(workspace_);
     workspace_ = nullptr;

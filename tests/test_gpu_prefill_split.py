@@ -120,3 +120,55 @@ def test_paged_split_windows(block, seq_q, start):
                  causal_offset=start)
     compare(out.tensor.float().view(seq_q, heads, D), ref[0].transpose(1, 0, 2), "bf16", f"block {block}")
     backend.Dispose()
+
+
+def _chunk(backend, case):
+    q, k, v, out, heads, kv_heads, sq, sk, D = case
+    backend.ScaledDotProductAttention(q, k, v, out, None, None, 1, heads, sq, sk, D, D ** -0.5, True, 0.0, kv_heads)
+
+
+def _chunk_case(D, seed):
+    from aidotnet.tensors_b200.backend import GpuBuffer
+    heads, kv_heads, sq, sk = 4, 2, 200, 4100
+    q, k, v = (gen(s, "bf16", seed + i)[0].reshape(-1) for i, s in
+               enumerate([(1, heads, sq, D), (1, kv_heads, sk, D), (1, kv_heads, sk, D)]))
+    return (GpuBuffer(q), GpuBuffer(k), GpuBuffer(v), GpuBuffer(torch.zeros(heads * sq * D, device="cuda")), heads, kv_heads, sq, sk, D)
+
+
+def test_overlapping_streams_do_not_share_a_workspace():
+    from aidotnet.tensors_b200.backend import CudaBackend
+    backend = CudaBackend(0)
+    cases = [_chunk_case(64, 1), _chunk_case(128, 5)]           # two handles: a handle's launches do not overlap
+    for c in cases:
+        _chunk(backend, c)
+    torch.cuda.synchronize()
+    want = [c[3].tensor.clone() for c in cases]
+    streams = [torch.cuda.Stream() for _ in cases]
+    for c in cases:
+        c[3].tensor.zero_()
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for c, s in zip(cases, streams):
+            with torch.cuda.stream(s):
+                _chunk(backend, c)
+    torch.cuda.synchronize()
+    assert all(torch.equal(c[3].tensor, w) for c, w in zip(cases, want))
+    assert len({backend._scratch[s.cuda_stream].data_ptr() for s in streams}) == 2
+    backend.Dispose()
+
+
+def test_split_prefill_in_a_graph():
+    from aidotnet.tensors_b200.backend import CudaBackend
+    backend, case = CudaBackend(0), _chunk_case(128, 9)
+    _chunk(backend, case)
+    torch.cuda.synchronize()
+    want = case[3].tensor.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        _chunk(backend, case)
+    case[3].tensor.zero_()
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(case[3].tensor, want)
+    backend.Dispose()
