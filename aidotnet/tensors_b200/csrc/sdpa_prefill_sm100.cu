@@ -909,7 +909,6 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
             for (int u = 0; u < n_sub && alive; ++u)
               alive = load_kv(std::true_type{}, &tm_k, it, it.k0 + u, ring_k(t_load, u), last_blk, win, leader);
           } else {
-#pragma unroll 1
             for (int u = 0; u < n_sub && alive; ++u) {
               if (u + 1 < n_sub) alive = load_kv(std::false_type{}, &tm_k, it, it.k0 + u + 1, ring_k(t_load, u + 1), 0, win, leader);
               if (alive) alive = load_kv(std::false_type{}, &tm_v, it, it.k0 + u, ring_v(t_load, u, n_sub), 0, win, leader);
