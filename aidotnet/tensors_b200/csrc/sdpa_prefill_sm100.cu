@@ -129,7 +129,7 @@ struct PrefillParams {
   int32_t items_per_rank;  // batch * work items per rank
   int32_t per_batch;       // work items per rank per batch entry
   int32_t total_items;
-  int32_t splits;          // > 1: each item is cut into this many along its keys; p.out / p.lse are then partial results
+  int32_t splits;          // > 1: each item is cut into this many along its keys; p.out and p.lse (pairs) are then partial results
                            // [batch * splits, ...] that sdpa_prefill_merge_kernel puts together
   int32_t* sched;          // [0] next-item counter, [1] finished-CTA counter; both zero between launches
   float* debug;            // trace builds only: tap / timeline buffer
@@ -281,6 +281,13 @@ __device__ __forceinline__ Item decode_item(const PrefillParams& pp, int item, i
   if ((p.kv_len || p.block_table) && it.n_max > 0 && (int64_t)(it.k0 + it.n_max) * kBS > kv_limit)
     it.v_tail = (int)(kv_limit - (int64_t)(it.k0 + it.n_max - 1) * kBS);
   return it;
+}
+
+// The log-sum-exp of a row or, in a split launch, the maximum (natural-log units) and the row sum of this part: as one
+// rounded number they would lose the sum as soon as the maximum is large - at a bias of -1e9 an ulp is 64.
+__device__ __forceinline__ void put_row_stats(const PrefillParams& pp, int64_t row, float m, float l, float inv) {
+  if (pp.splits > 1) reinterpret_cast<float2*>(pp.p.lse)[row] = make_float2(m, l);
+  else pp.p.lse[row] = inv > 0.f ? m + logf(l) : -INFINITY;
 }
 
 // Epilogue warps: O_i / l of one tile, 32 rows per warp: TMEM -> registers -> swizzled staging (128 bytes per row) -> TMA
@@ -701,8 +708,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_stats_full + 8 * i);
         if (qrow < p.seq_q && p.lse)
-          p.lse[((int64_t)it.out_b * p.num_q_heads + ti.h) * p.seq_q + qrow] =
-              (inv > 0.f) ? m * lse_scale + logf(l) : -INFINITY;
+          put_row_stats(pp, ((int64_t)it.out_b * p.num_q_heads + ti.h) * p.seq_q + qrow, m * lse_scale, l, inv);
       } else {
         // ---- epilogue: O / l -> swizzled staging (128 B per row) -> TMA stores ------------------------------
         {
@@ -766,8 +772,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
             }
           }
           if (row_valid && p.lse)
-            p.lse[((int64_t)it.out_b * p.num_q_heads + ti.h) * p.seq_q + qrow] =
-                (inv > 0.f) ? m * lse_scale + logf(l) : -INFINITY;
+            put_row_stats(pp, ((int64_t)it.out_b * p.num_q_heads + ti.h) * p.seq_q + qrow, m * lse_scale, l, inv);
           if (tracer) trace[5 + 8 * i] = globaltimer_ns();
         }
       }
@@ -1431,11 +1436,11 @@ cudaError_t launch_type(const SdpaParams& p, int dtype, cudaStream_t stream, int
   return launch_m<__half, 64>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
 }
 
-// out = sum_s w_s O_s with w_s = exp(lse_s - lse), lse = log sum_s exp(lse_s): head_dim / 4 lanes per row, one 16-byte
-// load per part and lane.  The partial results were just written and come from L2.
+// out = sum_s w_s O_s / sum_s w_s with w_s = exp(m_s - M) l_s, M = max_s m_s; lse = M + log sum_s w_s: head_dim / 4 lanes per
+// row, one 16-byte load per part and lane.  The partial results were just written and come from L2.
 template <typename T>
 __global__ void __launch_bounds__(256) sdpa_prefill_merge_kernel(const SdpaParams p, const float* __restrict__ parts,
-                                                                 const float* __restrict__ lses, const int splits, const int64_t rows) {
+                                                                 const float2* __restrict__ stats, const int splits, const int64_t rows) {
   const int lanes = p.head_dim / 4;
   const int64_t row = (int64_t)blockIdx.x * (256 / lanes) + threadIdx.x / lanes;   // over [B, H, Sq]
   const int d = threadIdx.x % lanes * 4;
@@ -1445,13 +1450,14 @@ __global__ void __launch_bounds__(256) sdpa_prefill_merge_kernel(const SdpaParam
   const int64_t h = within / p.seq_q, q = within - h * p.seq_q;
   const int64_t first = b * splits * per_batch + within;
   float m = -INFINITY;
-  for (int s = 0; s < splits; ++s) m = fmaxf(m, lses[first + s * per_batch]);
+  for (int s = 0; s < splits; ++s) m = fmaxf(m, stats[first + s * per_batch].x);
   float l = 0.f;
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
   if (m != -INFINITY) {
 #pragma unroll 4
     for (int s = 0; s < splits; ++s) {
-      const float w = expf(lses[first + s * per_batch] - m);
+      const float2 ml = stats[first + s * per_batch];
+      const float w = expf(ml.x - m) * ml.y;
       const float4 x = *reinterpret_cast<const float4*>(parts + (first + s * per_batch) * p.head_dim + d);
       l += w;
       o.x = fmaf(w, x.x, o.x); o.y = fmaf(w, x.y, o.y); o.z = fmaf(w, x.z, o.z); o.w = fmaf(w, x.w, o.w);
@@ -1466,13 +1472,13 @@ __global__ void __launch_bounds__(256) sdpa_prefill_merge_kernel(const SdpaParam
     T t[4] = {from_float<T>(o.x), from_float<T>(o.y), from_float<T>(o.z), from_float<T>(o.w)};
     *reinterpret_cast<uint2*>(static_cast<T*>(p.out) + at) = *reinterpret_cast<const uint2*>(t);
   }
-  if (p.lse && d == 0) p.lse[row] = m != -INFINITY ? m + logf(l) : -INFINITY;
+  if (p.lse && d == 0) p.lse[row] = l > 0.f ? m + logf(l) : -INFINITY;
 }
 
 }  // namespace
 
 int64_t prefill_split_bytes(const SdpaParams& p, int splits) {
-  return (int64_t)p.batch * splits * p.num_q_heads * p.seq_q * (p.head_dim + 1) * (int64_t)sizeof(float);
+  return (int64_t)p.batch * splits * p.num_q_heads * p.seq_q * (p.head_dim + 2) * (int64_t)sizeof(float);
 }
 
 // Work items are pairs of 128-row tiles; fewer of them than SMs leaves the chip idle however long the keys are (a chunk
@@ -1505,7 +1511,7 @@ cudaError_t launch_prefill_sm100(const SdpaParams& full, int dtype, cudaStream_t
                                  float* debug, int debug_mode, PrefillMapCache* cache, int splits, float* workspace,
                                  const char** why) {
   SdpaParams p = full;
-  if (splits > 1) {   // fp32 partial outputs [batch * splits, H, Sq, D], then their log-sum-exps
+  if (splits > 1) {   // fp32 partial outputs [batch * splits, H, Sq, D], then the (maximum, sum) of their rows
     p.out = workspace;
     p.out_f32 = 1;
     p.os[2] = p.head_dim;
@@ -1519,8 +1525,9 @@ cudaError_t launch_prefill_sm100(const SdpaParams& full, int dtype, cudaStream_t
   const int rows_per_cta = 256 * 4 / p.head_dim;
   const unsigned grid = (unsigned)((rows + rows_per_cta - 1) / rows_per_cta);
   const float* parts = workspace;
-  if (dtype == AIDN_BF16) sdpa_prefill_merge_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(full, parts, p.lse, splits, rows);
-  else sdpa_prefill_merge_kernel<__half><<<grid, 256, 0, stream>>>(full, parts, p.lse, splits, rows);
+  const float2* stats = reinterpret_cast<const float2*>(p.lse);
+  if (dtype == AIDN_BF16) sdpa_prefill_merge_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(full, parts, stats, splits, rows);
+  else sdpa_prefill_merge_kernel<__half><<<grid, 256, 0, stream>>>(full, parts, stats, splits, rows);
   return cudaGetLastError();
 }
 

@@ -172,3 +172,27 @@ def test_split_prefill_in_a_graph():
     torch.cuda.synchronize()
     assert torch.equal(case[3].tensor, want)
     backend.Dispose()
+
+
+@pytest.mark.parametrize("group", [1, 2])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("bias", [-1e9, -1e6, 1e9])
+def test_merge_of_parts_with_large_logits(bias, D, group):
+    """An additive bias whose ulp is as large as the row sums' logarithm (64 at 1e9): every visible key of the even rows
+    carries it and those rows are the plain mean over their keys, however the keys fall into parts - 129 keys put a single one into
+    the second part.  The odd rows hide half of their keys behind it."""
+    lens = np.array([129, 1, 193, 2113], np.int32)
+    B, H, Sq, Sk = 4, 2, 130, 2113
+    q, qf = gen((B, H, Sq, D), "bf16", 1)
+    k, kf = gen((B, H // group, Sk, D), "bf16", 2)
+    v, vf = gen((B, H // group, Sk, D), "bf16", 3)
+    mask = np.full((1, 1, Sq, Sk), bias, np.float32)
+    mask[..., 1::2, :] = np.where(np.random.default_rng(5).random((Sq // 2, Sk)) < 0.5, 0.0, -abs(bias))
+    got, lse, info = run_gpu(q, k, v, dtype="bf16", want_lse=True, path=N.PATH_PREFILL_SM100, mask=torch.from_numpy(mask).cuda(),
+                             mask_kind=N.MASK_ADD_F32, kv_len=torch.from_numpy(lens).cuda())
+    assert info["launches"] == 2
+    ref, ref_lse, _ = O.sdpa(qf, kf, vf, want_lse=True, causal=False, mask=mask, mask_kind=O.MASK_ADD_F32, kv_len=lens)
+    compare(got, ref, "bf16", f"{bias} {D}")
+    # both round m + log(l) once: an ulp of the bias on top of the contract's 2e-2
+    got, ref = lse.cpu().numpy(), ref_lse
+    assert (np.abs(got - ref) <= 2e-2 + np.spacing(np.abs(ref))).all()
