@@ -1451,20 +1451,20 @@ __global__ void __launch_bounds__(256) sdpa_prefill_merge_kernel(const SdpaParam
   const int64_t first = b * splits * per_batch + within;
   float m = -INFINITY;
   for (int s = 0; s < splits; ++s) m = fmaxf(m, stats[first + s * per_batch].x);
+  // No part saw a finite logit: the row sees no key (sums and outputs are 0) or its logits are NaN (both are NaN).
+  const float base = m == -INFINITY ? 0.f : m;
   float l = 0.f;
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (m != -INFINITY) {
 #pragma unroll 4
-    for (int s = 0; s < splits; ++s) {
-      const float2 ml = stats[first + s * per_batch];
-      const float w = expf(ml.x - m) * ml.y;
-      const float4 x = *reinterpret_cast<const float4*>(parts + (first + s * per_batch) * p.head_dim + d);
-      l += w;
-      o.x = fmaf(w, x.x, o.x); o.y = fmaf(w, x.y, o.y); o.z = fmaf(w, x.z, o.z); o.w = fmaf(w, x.w, o.w);
-    }
-    const float inv = 1.f / l;
-    o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
+  for (int s = 0; s < splits; ++s) {
+    const float2 ml = stats[first + s * per_batch];
+    const float w = expf(ml.x - base) * ml.y;
+    const float4 x = *reinterpret_cast<const float4*>(parts + (first + s * per_batch) * p.head_dim + d);
+    l += w;
+    o.x = fmaf(w, x.x, o.x); o.y = fmaf(w, x.y, o.y); o.z = fmaf(w, x.z, o.z); o.w = fmaf(w, x.w, o.w);
   }
+  const float inv = l == 0.f ? 0.f : 1.f / l;
+  o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
   const int64_t at = b * p.os[0] + h * p.os[1] + q * p.os[2] + d;   // 16-byte aligned rows (prefill_sm100_supported)
   if (p.out_f32) {
     *reinterpret_cast<float4*>(static_cast<float*>(p.out) + at) = o;

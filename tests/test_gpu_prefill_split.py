@@ -196,3 +196,40 @@ def test_merge_of_parts_with_large_logits(bias, D, group):
     # both round m + log(l) once: an ulp of the bias on top of the contract's 2e-2
     got, ref = lse.cpu().numpy(), ref_lse
     assert (np.abs(got - ref) <= 2e-2 + np.spacing(np.abs(ref))).all()
+
+
+def _unsplit(q, k, v, **kw):
+    """The same launch without a workspace: one part."""
+    B, Hq, Sq, D = q.shape
+    out = torch.empty(B, Hq, Sq, D, device="cuda")
+    lse = torch.empty(B, Hq, Sq, device="cuda")
+    h = N.Handle(device=0, qkv_dtype=N.F16 if q.dtype == torch.float16 else N.BF16, out_dtype=N.F32, head_dim=D, num_q_heads=Hq,
+                 num_kv_heads=k.shape[1], emit_lse=True, **kw)
+    stream = torch.cuda.current_stream().cuda_stream
+    h.launch(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), out=out.data_ptr(), lse=lse.data_ptr(), batch=B, seq_q=Sq,
+             seq_kv=k.shape[2], stream=stream)
+    h.poll(stream)
+    assert h.last_launch_count == 1
+    h.close()
+    return out, lse
+
+
+@pytest.mark.parametrize("group", [1, 2])
+@pytest.mark.parametrize("causal", [False, True])
+def test_rows_of_nan_stay_nan(causal, group):
+    """A NaN in a query row, an infinity in another, and one in a key and in a value of the second part: NaN comes out wherever it
+    does without the split, and nowhere else."""
+    H, Sq, Sk, D = 2, 130, 2113, 128
+    q, _ = gen((1, H, Sq, D), "f16", 1)
+    k, _ = gen((1, H // group, Sk, D), "f16", 2)
+    v, _ = gen((1, H // group, Sk, D), "f16", 3)
+    q[0, 1, 5] = float("nan")
+    q[0, 0, 77, 3] = float("inf")
+    for change in (lambda: None, lambda: v[0, 0, 1500, 9].fill_(float("nan")), lambda: k[0, 0, 1400].fill_(float("inf"))):
+        change()
+        got, lse, info = run_gpu(q, k, v, dtype="f16", want_lse=True, path=N.PATH_PREFILL_SM100, causal=causal)
+        assert info["launches"] == 2
+        whole, whole_lse = _unsplit(q, k, v, causal=causal)
+        assert torch.isnan(whole[0, 1, 5]).all() and torch.isnan(whole[0, 0, 77]).all()
+        assert torch.equal(torch.isnan(got), torch.isnan(whole))
+        assert torch.equal(torch.isneginf(lse), torch.isneginf(whole_lse))
