@@ -71,6 +71,7 @@ constexpr int kEpilogueWarps = 4;
 constexpr int kStageBytes = 32768;     // epilogue staging: 32-row x 128-byte boxes (128-byte swizzle) of 4 KiB
 constexpr int kTmemCols = 512;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units: P stays below 2^8 between rescales
+constexpr float kHugeLogit = 2e38f;        // anything below FLT_MAX / log2(e)
 
 // Two role layouts, chosen by the host per launch.
 //   EPI = false: 3 warpgroups (384 threads); the softmax warps run the epilogue of their own tile (one 4 KiB staging
@@ -661,7 +662,10 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
           }
         }
 
-        const float neg_ms = (m == -INFINITY) ? 0.f : -m * sl2;
+        // A bias of the lowest float is a mask too, and log2(e) times it is an infinity.  Logits of that size are equal or
+        // more than 2^100 apart, so any factor gives their exponentials: one that does not overflow.
+        const float mul = MASKED && fabsf(m) > kHugeLogit ? 0.5f : sl2;
+        const float neg_ms = (m == -INFINITY) ? 0.f : -m * mul;
         float ls0 = 0.f, ls1 = 0.f, ls2 = 0.f, ls3 = 0.f;
         // (Computing one exponential in 2, 4 or 8 on the FMA pipe instead - a cubic after the 1.5 * 2^23 rounding trick -
         // was measured and is slower here, 6-10 %: with two softmax warps per scheduler the loop is bound by their
@@ -671,10 +675,10 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
           uint32_t pk[16];
 #pragma unroll
           for (int c = 0; c < 32; c += 4) {
-            const float p0 = ex2_approx(fmaf(s[c0 + c], sl2, neg_ms));
-            const float p1 = ex2_approx(fmaf(s[c0 + c + 1], sl2, neg_ms));
-            const float p2 = ex2_approx(fmaf(s[c0 + c + 2], sl2, neg_ms));
-            const float p3 = ex2_approx(fmaf(s[c0 + c + 3], sl2, neg_ms));
+            const float p0 = ex2_approx(fmaf(s[c0 + c], mul, neg_ms));
+            const float p1 = ex2_approx(fmaf(s[c0 + c + 1], mul, neg_ms));
+            const float p2 = ex2_approx(fmaf(s[c0 + c + 2], mul, neg_ms));
+            const float p3 = ex2_approx(fmaf(s[c0 + c + 3], mul, neg_ms));
             ls0 += p0;
             ls1 += p1;
             ls2 += p2;

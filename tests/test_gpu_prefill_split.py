@@ -233,3 +233,37 @@ def test_rows_of_nan_stay_nan(causal, group):
         assert torch.isnan(whole[0, 1, 5]).all() and torch.isnan(whole[0, 0, 77]).all()
         assert torch.equal(torch.isnan(got), torch.isnan(whole))
         assert torch.equal(torch.isneginf(lse), torch.isneginf(whole_lse))
+
+
+@pytest.mark.parametrize("group", [1, 2])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("how", ["right", "left", "causal", "rows"])
+def test_bias_of_the_lowest_float(how, D, group):
+    """Masks written as an additive bias of the lowest float: hidden keys get weight 0 wherever they stand - a whole part or the
+    first sub-tiles of a row can consist of them - and a row of nothing else is the mean over its keys."""
+    low = np.finfo(np.float32).min
+    H, Sq, Sk = 2, 130, 2113
+    q, qf = gen((1, H, Sq, D), "bf16", 1)
+    k, kf = gen((1, H // group, Sk, D), "bf16", 2)
+    v, vf = gen((1, H // group, Sk, D), "bf16", 3)
+    mask = np.zeros((1, 1, Sq, Sk), np.float32)
+    if how == "right":
+        mask[..., 300:] = low
+    elif how == "left":
+        mask[..., :1500] = low
+    elif how == "causal":
+        mask[0, 0] = np.where(np.arange(Sk)[None] > np.arange(Sq)[:, None], low, 0)
+    else:
+        mask[0, 0, ::3] = low
+    tmask = torch.from_numpy(mask).cuda()
+    got, lse, info = run_gpu(q, k, v, dtype="bf16", want_lse=True, path=N.PATH_PREFILL_SM100, mask=tmask, mask_kind=N.MASK_ADD_F32)
+    assert info["launches"] == 2
+    ref, ref_lse, _ = O.sdpa(qf, kf, vf, want_lse=True, causal=False, mask=mask, mask_kind=O.MASK_ADD_F32)
+    compare(got, ref, "bf16", f"{how} {D}")
+    compare_lse(lse, ref_lse, "bf16", f"{how} {D}")
+    few, _, info = run_gpu(q, k[:, :, :900].contiguous(), v[:, :, :900].contiguous(), dtype="bf16", path=N.PATH_PREFILL_SM100,
+                           mask=tmask[..., -900:].contiguous(), mask_kind=N.MASK_ADD_F32)
+    assert info["launches"] == 1
+    ref = O.sdpa(qf, np.ascontiguousarray(kf[:, :, :900]), np.ascontiguousarray(vf[:, :, :900]), causal=False,
+                 mask=np.ascontiguousarray(mask[..., -900:]), mask_kind=O.MASK_ADD_F32)
+    compare(few, ref, "bf16", f"{how} {D} in one part")
