@@ -687,15 +687,15 @@ __global__ void __launch_bounds__(128)
     if (c0 > 0) __syncthreads();
     for (int c = tid; c < n; c += 128) {
       const float2 v = ml[c0 + c];
-      const float w = v.x == -INFINITY ? 0.f : softmax_exp<T>(v.x - M);
+      const float w = v.x == -INFINITY ? -1.f : softmax_exp<T>(v.x - M);   // -1: a split that saw no key
       weight[c] = w;
-      if (w != 0.f) lsum = fmaf(w, v.y, lsum);
+      if (v.x != -INFINITY) lsum = fmaf(w, v.y, lsum);
     }
     __syncthreads();
 #pragma unroll 4
     for (int c = grp; c < n; c += groups) {
       const float w = weight[c];
-      if (w == 0.f) continue;   // (a split that saw no key leaves its columns undefined)
+      if (w < 0.f) continue;   // its columns are undefined; a weight that underflows to 0 still carries their NaN and Inf
       const float4 x = rows[(int64_t)(c0 + c) * vecs];
       a.x = fmaf(w, x.x, a.x); a.y = fmaf(w, x.y, a.y); a.z = fmaf(w, x.z, a.z); a.w = fmaf(w, x.w, a.w);
     }

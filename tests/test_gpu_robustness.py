@@ -181,3 +181,22 @@ print("launch check ok")
     env = dict(os.environ, AIDOTNET_KERNEL_LAUNCH_CHECK="1", PYTHONPATH=root)
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, env=env, cwd=root)
     assert r.returncode == 0 and "launch check ok" in r.stdout, f"stdout:\n{r.stdout}\nstderr:\n{r.stderr[-2000:]}"
+
+
+@pytest.mark.parametrize("dtype,D,Hq,Hkv", [("f32", 64, 4, 4), ("bf16", 64, 4, 2), ("bf16", 128, 4, 4), ("f16", 256, 2, 2)])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_decode_splits_keep_non_finite_values(dtype, D, Hq, Hkv, value):
+    """A visible NaN or infinity in V behind a weight that underflows to 0 (the largest logit, in another split, is 400 above
+    it): 0 * NaN is NaN, in a launch of eight splits as in one of one."""
+    B, Sk = 2, 2048
+    q, _ = gen((B, Hq, 1, D), dtype, 1)
+    k, _ = gen((B, Hkv, Sk, D), dtype, 2, 0.01)
+    v, _ = gen((B, Hkv, Sk, D), dtype, 3)
+    q[...] = 1.0
+    k[:, :, 700] = 400.0 / D
+    v[1, Hkv - 1, 1500, 7] = value
+    split, _, info = run_gpu(q, k, v, dtype=dtype, path=N.PATH_DECODE, scale=1.0, decode_chunk=256)
+    one, _, info1 = run_gpu(q, k, v, dtype=dtype, path=N.PATH_DECODE, scale=1.0, decode_chunk=2048)
+    assert info["launches"] == 2 and info1["launches"] == 1
+    assert torch.isnan(one[1, Hq - 1, 0, 7])
+    assert torch.equal(torch.isnan(split), torch.isnan(one))
