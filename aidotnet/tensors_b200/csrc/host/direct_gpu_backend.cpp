@@ -2,8 +2,11 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <iterator>
+#include <vector>
 
 namespace aidn {
 namespace host {
@@ -15,6 +18,35 @@ void CudaBackend::Check(int status, const char* where) {
   throw std::runtime_error(msg);
 }
 
+// The buffers that a graph was recorded with.  The graph owns a user object whose destructor (run by CUDA on a thread of
+// its own) says that it and every executable made from it have gone; the note belongs to both sides, as either may go first.
+struct CudaBackend::GraphScratch {
+  struct Note {
+    std::atomic<int> owners{2};
+    std::atomic<bool> gone{false};
+    void Drop() {
+      if (owners.fetch_sub(1) == 1) delete this;
+    }
+  };
+  std::vector<Scratch> buffers;
+  Note* note = new Note;
+
+  explicit GraphScratch(cudaGraph_t graph) {
+    auto on_gone = [](void* p) {
+      static_cast<Note*>(p)->gone = true;
+      static_cast<Note*>(p)->Drop();
+    };
+    cudaUserObject_t object = nullptr;
+    if (cudaUserObjectCreate(&object, note, on_gone, 1, cudaUserObjectNoDestructorSync) != cudaSuccess ||
+        cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove) != cudaSuccess)
+      cudaGetLastError();   // nobody will tell: the buffers stay as long as the backend
+  }
+  ~GraphScratch() {
+    for (const Scratch& s : buffers) cudaFree(s.ptr);
+    note->Drop();
+  }
+};
+
 CudaBackend::CudaBackend(int device, void* stream) : device_(device), stream_(stream) {
   if (cudaSetDevice(device) != cudaSuccess) throw std::runtime_error("CudaBackend: cannot select the device");
   if (!aidn_sdpa_device_supported(device))
@@ -23,7 +55,57 @@ CudaBackend::CudaBackend(int device, void* stream) : device_(device), stream_(st
 
 CudaBackend::~CudaBackend() {
   for (auto& kv : handles_) aidn_sdpa_destroy(kv.second);
-  if (workspace_) cudaFree(workspace_);
+  if (scratch_.ptr) cudaFree(scratch_.ptr);
+}
+
+// A scratch buffer of at least `need` bytes.  Calls that run when they are made share one, which is grown - outside of
+// launch, like the reference's pooled scratch buffers.  A call that is being captured gets the buffer of its capture: a
+// graph keeps the address and may be replayed beside anything, another graph of this stream included, so such a buffer
+// is not shared with any other call, and given back when the graph (or the backend) has gone.
+CudaBackend::Scratch CudaBackend::Workspace(int64_t need, bool optional) {
+  if (need <= 0) return {};
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream_), &status, &id, &graph) != cudaSuccess) {
+    cudaGetLastError();   // the launch will report it
+    status = cudaStreamCaptureStatusNone;
+  }
+  if (status == cudaStreamCaptureStatusActive) {
+    std::unique_ptr<GraphScratch>& held = captured_[id];
+    if (!held) held.reset(new GraphScratch(graph));
+    if (!held->buffers.empty() && held->buffers.back().bytes >= need) return held->buffers.back();
+    Scratch s;
+    for (auto& kv : captured_) {
+      std::vector<Scratch>& old = kv.second->buffers;
+      if (kv.second->note->gone && !old.empty() && old.back().bytes >= need) {
+        s = old.back();
+        old.pop_back();
+        break;
+      }
+    }
+    if (!s.ptr) {
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // allows cudaMalloc, which enqueues nothing
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      const cudaError_t e = cudaMalloc(&s.ptr, (size_t)need);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        if (optional) return {};
+        throw std::runtime_error("CudaBackend: out of device memory");
+      }
+      s.bytes = need;
+    }
+    held->buffers.push_back(s);
+    return s;
+  }
+  for (auto it = captured_.begin(); it != captured_.end();) it = it->second->note->gone ? captured_.erase(it) : std::next(it);
+  if (scratch_.bytes >= need) return scratch_;
+  if (scratch_.ptr) cudaFree(scratch_.ptr);
+  scratch_ = {};
+  if (cudaMalloc(&scratch_.ptr, (size_t)need) != cudaSuccess) throw std::runtime_error("CudaBackend: out of device memory");
+  scratch_.bytes = need;
+  return scratch_;
 }
 
 aidn_sdpa_t CudaBackend::Handle(const aidn_sdpa_desc& d) {
@@ -38,25 +120,11 @@ aidn_sdpa_t CudaBackend::Handle(const aidn_sdpa_desc& d) {
 }
 
 void CudaBackend::Run(aidn_sdpa_t h, aidn_sdpa_args& a, const aidn_paged_kv* paged) {
-  int64_t need = aidn_sdpa_workspace_bytes(h, a.batch, a.seq_q, a.seq_kv);
+  const int64_t need = aidn_sdpa_workspace_bytes(h, a.batch, a.seq_q, a.seq_kv);
   if (need < 0) Check(AIDN_EINVAL, "aidn_sdpa_workspace_bytes");
-  if (a.seq_q > 1 && need > workspace_bytes_) {
-    // A prefill runs without its workspace too: it is not grown where that cannot be done (during stream capture).
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream_), &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-      cudaGetLastError();
-      need = 0;
-    }
-  }
-  if (need > workspace_bytes_) {   // grown outside of launch, like the reference's pooled scratch buffers
-    if (workspace_) cudaFree(workspace_);
-    workspace_ = nullptr;
-    workspace_bytes_ = 0;
-    if (cudaMalloc(&workspace_, (size_t)need) != cudaSuccess) throw std::runtime_error("CudaBackend: out of device memory");
-    workspace_bytes_ = need;
-  }
-  a.workspace = need > 0 ? workspace_ : nullptr;
-  a.workspace_bytes = need > 0 ? workspace_bytes_ : 0;
+  const Scratch ws = Workspace(need, a.seq_q > 1);   // a prefill runs without its workspace too
+  a.workspace = ws.ptr;
+  a.workspace_bytes = ws.bytes;
   if (paged) Check(aidn_sdpa_launch_paged(h, &a, paged, stream_), "aidn_sdpa_launch_paged");
   else Check(aidn_sdpa_launch(h, &a, stream_), "aidn_sdpa_launch");
   launch_count_ += aidn_sdpa_last_launch_count(h);
@@ -306,19 +374,13 @@ void CudaBackend::FlashAttentionBackward(const GpuBuffer& gradOutput, const GpuB
   aidn_sdpa_t h = Handle(d);
   const int64_t need = aidn_sdpa_backward_workspace_bytes(h, batch, seqQ);
   if (need < 0) Check(AIDN_EINVAL, "aidn_sdpa_backward_workspace_bytes");
-  if (need > workspace_bytes_) {
-    if (workspace_) cudaFree(workspace_);
-    workspace_ = nullptr;
-    workspace_bytes_ = 0;
-    if (cudaMalloc(&workspace_, (size_t)need) != cudaSuccess) throw std::runtime_error("CudaBackend: out of device memory");
-    workspace_bytes_ = need;
-  }
+  const Scratch ws = Workspace(need);
   aidn_sdpa_bwd_args a;
   std::memset(&a, 0, sizeof(a));
   a.fwd.q = query.Handle; a.fwd.k = key.Handle; a.fwd.v = value.Handle; a.fwd.out = output.Handle;
   a.fwd.lse = static_cast<float*>(softmaxStats.Handle);
   a.fwd.batch = batch; a.fwd.seq_q = seqQ; a.fwd.seq_kv = seqK; a.fwd.scale = scale;
-  a.fwd.workspace = workspace_; a.fwd.workspace_bytes = workspace_bytes_;
+  a.fwd.workspace = ws.ptr; a.fwd.workspace_bytes = ws.bytes;
   if (attentionBias) {
     a.fwd.mask = attentionBias->Handle;
     a.fwd.mask_stride[0] = biasBatchStride; a.fwd.mask_stride[1] = (int64_t)seqQ * seqK;
@@ -382,20 +444,14 @@ void CudaBackend::MultiHeadAttentionForward(const GpuBuffer& input, const GpuBuf
   aidn_sdpa_t h = Handle(d);
   const int64_t need = aidn_mha_workspace_bytes(h, batch, seq, input.Dtype, qWeight.Dtype);
   if (need < 0) Check(AIDN_EUNSUPPORTED, "aidn_mha_workspace_bytes");
-  if (need > workspace_bytes_) {
-    if (workspace_) cudaFree(workspace_);
-    workspace_ = nullptr;
-    workspace_bytes_ = 0;
-    if (cudaMalloc(&workspace_, (size_t)need) != cudaSuccess) throw std::runtime_error("CudaBackend: out of device memory");
-    workspace_bytes_ = need;
-  }
+  const Scratch ws = Workspace(need);
   a.input = input.Handle;
   a.q_weight = qWeight.Handle; a.k_weight = kWeight.Handle; a.v_weight = vWeight.Handle; a.out_weight = outWeight.Handle;
   a.out = output.Handle;
   a.batch = batch; a.seq = seq;
   a.input_dtype = input.Dtype; a.weight_dtype = qWeight.Dtype; a.out_dtype = output.Dtype;
-  a.workspace = workspace_;            // cudaMalloc memory is at least 256-byte aligned, which is what the call asks for
-  a.workspace_bytes = workspace_bytes_;
+  a.workspace = ws.ptr;                // cudaMalloc memory is at least 256-byte aligned, which is what the call asks for
+  a.workspace_bytes = ws.bytes;
   Check(aidn_mha_forward(h, &a, stream_), "aidn_mha_forward");
   launch_count_ += aidn_sdpa_last_launch_count(h);
 }

@@ -15,6 +15,7 @@
 
 #include <cstdint>
 #include <map>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <tuple>
@@ -109,12 +110,18 @@ class CudaBackend {
              const GpuBuffer& blockTable, const GpuBuffer& output, int heads, int kvHeads, int headDim, int blockSize,
              int numQueries, int64_t keyLen, int startPos, float scale);
   static void Check(int status, const char* where);
+  struct Scratch {
+    void* ptr = nullptr;
+    int64_t bytes = 0;
+  };
+  Scratch Workspace(int64_t need, bool optional = false);
 
   int device_;
   void* stream_;
   std::map<Key, aidn_sdpa_t> handles_;
-  void* workspace_ = nullptr;
-  int64_t workspace_bytes_ = 0;
+  Scratch scratch_;                                                       // of the calls that run when they are made
+  struct GraphScratch;
+  std::map<unsigned long long, std::unique_ptr<GraphScratch>> captured_;  // by capture: what a graph was recorded with
   int64_t launch_count_ = 0;
   int last_path_ = 0;
 };

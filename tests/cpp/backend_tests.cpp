@@ -489,6 +489,39 @@ int main() {
     try { backend.ScaledDotProductAttention(a.buf, a.buf, a.buf, out.buf, nullptr, nullptr, 4, 4, 4, 4, 8, 1.f, false); } catch (const std::invalid_argument&) { threw = true; }
     EXPECT(threw, "undersized buffers must throw");
   }
+  {  // a captured decode keeps its scratch whatever later calls need, and memory comes back with the graph
+    std::printf("captured decode, larger calls after it, replay\n");
+    const int H = 4, D = 64, Sk = 2048, Sq = 200;
+    std::vector<float> hq((size_t)H * Sq * D), hk((size_t)H * Sk * D), hv(hk.size());
+    for (size_t i = 0; i < hq.size(); ++i) hq[i] = 0.5f * std::sin(0.37f * (float)i);
+    for (size_t i = 0; i < hk.size(); ++i) { hk[i] = 0.5f * std::cos(0.11f * (float)i); hv[i] = std::sin(0.05f * (float)i); }
+    DeviceArray q(hq, AIDN_BF16), k(hk, AIDN_BF16), v(hv, AIDN_BF16), out((int64_t)H * D), big((int64_t)H * Sq * D);
+    CudaBackend be(0, stream);
+    auto decode = [&] { be.ScaledDotProductAttention(q.buf, k.buf, v.buf, out.buf, nullptr, nullptr, 1, H, 1, Sk, D, 0.125f, false); };
+    auto prefill = [&] { be.ScaledDotProductAttention(q.buf, k.buf, v.buf, big.buf, nullptr, nullptr, 1, H, Sq, Sk, D, 0.125f, false); };
+    decode();
+    be.Synchronize();
+    const auto want = out.download();
+    for (int round = 0; round < 3; ++round) {
+      cudaGraph_t graph = nullptr;
+      cudaGraphExec_t exec = nullptr;
+      cudaStreamBeginCapture((cudaStream_t)stream, cudaStreamCaptureModeThreadLocal);
+      decode();
+      prefill();
+      EXPECT(cudaStreamEndCapture((cudaStream_t)stream, &graph) == cudaSuccess && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess,
+             "capture failed");
+      prefill();   // eager, in the buffer of the eager calls
+      be.Synchronize();
+      const auto whole = big.download();
+      cudaMemset(out.buf.Handle, 0, (size_t)H * D * 4);
+      cudaMemset(big.buf.Handle, 0, (size_t)H * Sq * D * 4);
+      EXPECT(cudaGraphLaunch(exec, (cudaStream_t)stream) == cudaSuccess, "replay failed");
+      be.Synchronize();
+      EXPECT(out.download() == want && big.download() == whole, "a replay differs from the calls it recorded");
+      cudaGraphExecDestroy(exec);
+      cudaGraphDestroy(graph);
+    }
+  }
   std::printf(g_failed ? "%d case(s) FAILED\n" : "all cases passed (%d failures)\n", g_failed);
   cudaStreamDestroy(stream);
   return g_failed ? 1 : 0;
