@@ -23,7 +23,7 @@ Differences from the reference methods, all deliberate:
 from __future__ import annotations
 
 import math
-from typing import Dict, Optional, Tuple
+from typing import Dict, List, Optional, Tuple
 
 import torch
 
@@ -74,6 +74,8 @@ class CudaBackend:
         self._decode_chunk = decode_chunk
         self._handles: Dict[Tuple, N.Handle] = {}
         self._scratch: Dict[int, torch.Tensor] = {}   # by stream: calls on different streams may overlap
+        # by stream and capture: what a graph was recorded with
+        self._captured: Dict[Tuple[int, int], Tuple[N.Capture, List[torch.Tensor]]] = {}
         self.launch_count = 0  # kernels enqueued by this backend (the reference counts launches in GpuLaunchProbe)
 
     # -- plumbing ---------------------------------------------------------------------------------------
@@ -111,18 +113,39 @@ class CudaBackend:
 
     def _workspace(self, nbytes: int, stream: torch.cuda.Stream) -> Tuple[Optional[int], int]:
         """The scratch buffer of ``stream``, grown on demand.  It is allocated on that stream, so a buffer that is replaced
-        is reused only behind the launches that read it."""
+        is reused only behind the launches that read it.  A call that is being captured gets the buffer of its capture: a
+        graph keeps the address and may be replayed beside anything, another graph captured on this stream included, so such
+        a buffer is not shared with any other call, and given back when the graph (or the backend) has gone."""
         if nbytes <= 0:
             return None, 0
-        buf = self._scratch.get(stream.cuda_stream)
+        handle = stream.cuda_stream
+        if self._stream is not None or torch.cuda.is_current_stream_capturing():
+            capture = N.Capture.of(handle)
+            if capture is not None:
+                key = (handle, capture[0])
+                if key not in self._captured:
+                    self._give_back()
+                    self._captured[key] = (N.Capture(*capture), [])
+                held = self._captured[key][1]
+                if not held or held[-1].numel() < nbytes:
+                    held.append(self._scratch_tensor(nbytes, stream))
+                return held[-1].data_ptr(), held[-1].numel()
+        buf = self._scratch.get(handle)
         if buf is None or buf.numel() < nbytes:
-            self._scratch.pop(stream.cuda_stream, None)
+            self._give_back()
+            self._scratch.pop(handle, None)
             if len(self._scratch) >= 16:
                 self._scratch.pop(next(iter(self._scratch)))
-            with torch.cuda.stream(stream):
-                buf = torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{self.device}")
-            self._scratch[stream.cuda_stream] = buf
+            buf = self._scratch[handle] = self._scratch_tensor(nbytes, stream)
         return buf.data_ptr(), buf.numel()
+
+    def _give_back(self) -> None:
+        for key in [key for key, (capture, _) in list(self._captured.items()) if capture.gone]:
+            self._captured.pop(key, None)
+
+    def _scratch_tensor(self, nbytes: int, stream: torch.cuda.Stream) -> torch.Tensor:
+        with torch.cuda.stream(stream):
+            return torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{self.device}")
 
     @staticmethod
     def _check_dims(batch, numHeads, seqQ, seqK, headDim):

@@ -8,7 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from typing import Optional, Sequence
+from typing import Optional, Sequence, Tuple
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # AIDN_SDPA_LIB selects a development variant of the library (see build.build_variant); unset = the shipped one.
@@ -181,6 +181,47 @@ def check(status: int) -> None:
 
 def _arr3(values: Optional[Sequence[int]]):
     return (ctypes.c_int64 * 3)(*(values if values is not None else (0, 0, 0)))
+
+
+class Capture:
+    """The graph that a stream is being captured into: ``id`` (unique in the process), and whether it and every executable
+    made from it have ``gone``.  A user object of the graph tells: its destructor, which CUDA runs on a thread of its own
+    where no Python code could, is the C library's ``sem_post``."""
+
+    _driver: Optional[ctypes.CDLL] = None
+    _libc: Optional[ctypes.CDLL] = None
+
+    def __init__(self, ident: int, graph: int):
+        self.id = ident
+        self._gone = False
+        libc, obj = Capture._libc, ctypes.c_void_p()
+        self._sem = libc.malloc(64)   # never given back: the graph may outlive this object, and the interpreter
+        libc.sem_init(self._sem, 0, 0)
+        post = ctypes.cast(libc.sem_post, ctypes.c_void_p)
+        if Capture._driver.cuUserObjectCreate(ctypes.byref(obj), self._sem, post, 1, 1) == 0:   # no destructor sync
+            Capture._driver.cuGraphRetainUserObject(graph, obj, 1, 1)                           # the graph owns it now
+
+    @property
+    def gone(self) -> bool:
+        if not self._gone and Capture._libc.sem_trywait(self._sem) == 0:
+            self._gone = True
+        return self._gone
+
+    @staticmethod
+    def of(stream: int) -> Optional[Tuple[int, int]]:
+        """(id, graph) of the capture that ``stream`` takes part in, or None."""
+        if Capture._driver is None:
+            libc, driver = ctypes.CDLL(None), ctypes.CDLL("libcuda.so.1")
+            libc.malloc.argtypes, libc.malloc.restype = [ctypes.c_size_t], ctypes.c_void_p
+            libc.sem_init.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_uint]
+            libc.sem_trywait.argtypes = [ctypes.c_void_p]
+            driver.cuStreamGetCaptureInfo_v2.argtypes = [ctypes.c_void_p] * 6
+            driver.cuUserObjectCreate.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_uint] * 2
+            driver.cuGraphRetainUserObject.argtypes = [ctypes.c_void_p] * 2 + [ctypes.c_uint] * 2
+            Capture._libc, Capture._driver = libc, driver
+        status, ident, graph = ctypes.c_int(0), ctypes.c_uint64(0), ctypes.c_void_p()
+        rc = Capture._driver.cuStreamGetCaptureInfo_v2(stream, ctypes.byref(status), ctypes.byref(ident), ctypes.byref(graph), None, None)
+        return (ident.value, graph.value) if rc == 0 and status.value == 1 else None   # 1: active
 
 
 class Handle:

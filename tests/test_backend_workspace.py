@@ -18,3 +18,90 @@ def test_cpp_mirror(tmp_path):
                     os.path.join(build.CSRC, "host", "direct_gpu_backend.cpp"), "-Wl,--unresolved-symbols=ignore-in-object-files"], check=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0 and "all cases passed" in r.stdout, r.stdout + r.stderr
+
+
+class _Stream:
+    def __init__(self, handle):
+        self.cuda_stream = handle
+
+
+class _Memory:
+    """Stands in for torch: hands out numbered buffers, knows which the backend still holds and can run out of memory."""
+
+    def __init__(self, monkeypatch):
+        import contextlib
+        import torch
+        from aidotnet.tensors_b200 import backend, native
+        self.capture, self.left, self.live, self.count, self.gone = None, 1 << 40, {}, 0, set()
+        memory = self
+
+        class Tensor:
+            def __init__(self, n):
+                memory.count += 1
+                self.n, self.address = n, memory.count
+                memory.live[self.address] = n
+
+            def numel(self):
+                return self.n
+
+            def data_ptr(self):
+                return self.address
+
+            def __del__(self):
+                memory.live.pop(self.address, None)
+
+        def empty(n, **_):
+            if n > memory.left:
+                raise torch.OutOfMemoryError("fake")
+            return Tensor(n)
+
+        class Capture:
+            def __init__(self, ident, graph):
+                self.id = ident
+
+            @property
+            def gone(self):
+                return self.id in memory.gone
+
+            @staticmethod
+            def of(stream):
+                return (memory.capture, 1) if memory.capture else None
+
+        monkeypatch.setattr(torch, "empty", empty)
+        monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+        monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: memory.capture is not None)
+        monkeypatch.setattr(native, "Capture", Capture, raising=False)
+        self.backend = object.__new__(backend.CudaBackend)
+        self.backend.device, self.backend._stream, self.backend._scratch, self.backend._captured = 0, None, {}, {}
+
+
+def test_python_mirror_keeps_what_graphs_were_recorded_with(monkeypatch):
+    memory = _Memory(monkeypatch)
+    stream = _Stream(100)
+    ws = lambda n, s=stream: memory.backend._workspace(n, s)[0]
+    eager = ws(100)
+    memory.capture = 7
+    first = ws(100)
+    assert ws(50) == first                  # the layers of one graph take turns with one buffer
+    grown = ws(300)
+    memory.capture = 8                      # a second graph on the same stream: may be replayed beside the first
+    second = ws(100)
+    memory.capture = None
+    recorded = {first, grown, second}
+    assert len(recorded) == 3 and eager not in recorded
+    assert ws(5000) not in recorded
+    for handle in range(200, 220):          # more streams than the backend keeps a buffer for
+        assert ws(100, _Stream(handle)) not in recorded
+    assert recorded <= set(memory.live) and eager not in memory.live
+    memory.gone = {7}
+    ws(6000)
+    assert second in memory.live and not {first, grown} & set(memory.live)
+
+
+def test_python_mirror_gives_back(monkeypatch):
+    memory = _Memory(monkeypatch)
+    for ident in range(1, 51):              # a program that captures again and again
+        memory.capture = ident
+        memory.backend._workspace(100, _Stream(100))
+        memory.gone.add(ident - 1)
+    assert len(memory.live) <= 2

@@ -267,3 +267,56 @@ def test_bias_of_the_lowest_float(how, D, group):
     ref = O.sdpa(qf, np.ascontiguousarray(kf[:, :, :900]), np.ascontiguousarray(vf[:, :, :900]), causal=False,
                  mask=np.ascontiguousarray(mask[..., -900:]), mask_kind=O.MASK_ADD_F32)
     compare(few, ref, "bf16", f"{how} {D} in one part")
+
+
+def test_graphs_own_their_workspaces():
+    """Two graphs captured on one stream and replayed on two, after a larger call and more streams than the backend keeps a
+    buffer for; new tensors take whatever memory the backend let go.  The graphs' memory comes back with them."""
+    from aidotnet.tensors_b200.backend import CudaBackend
+    backend = CudaBackend(0)
+    cases = [_chunk_case(64, 1), _chunk_case(128, 5)]           # two handles: a handle's launches do not overlap
+    stream = torch.cuda.Stream()
+    graphs = []
+    with torch.cuda.stream(stream):
+        for c in cases:
+            _chunk(backend, c)
+    torch.cuda.synchronize()
+    want = [c[3].tensor.clone() for c in cases]
+    for c in cases:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            _chunk(backend, c)
+        graphs.append(graph)
+    assert len(backend._captured) == 2
+    from aidotnet.tensors_b200.backend import GpuBuffer
+    q, k, v = (GpuBuffer(gen(s, "bf16", 20)[0].reshape(-1)) for s in ((1, 8, 1024, 64), (1, 8, 4096, 64), (1, 8, 4096, 64)))
+    larger = (q, k, v, GpuBuffer(torch.zeros(8 * 1024 * 64, device="cuda")), 8, 8, 1024, 4096, 64)
+    torch.cuda.synchronize()
+    for s in [stream] + [torch.cuda.Stream() for _ in range(20)]:
+        with torch.cuda.stream(s):
+            _chunk(backend, larger)
+            _chunk(backend, cases[0])
+    torch.cuda.synchronize()
+    taken = [torch.full((n,), 7, dtype=torch.uint8, device="cuda") for n in (1 << 20, 1 << 22, 1 << 24) for _ in range(8)]
+    for c in cases:
+        c[3].tensor.zero_()
+    torch.cuda.synchronize()
+    sides = [torch.cuda.Stream() for _ in graphs]
+    for _ in range(20):
+        for graph, s in zip(graphs, sides):
+            with torch.cuda.stream(s):
+                graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(c[3].tensor, w) for c, w in zip(cases, want))
+    assert all((t == 7).all() for t in taken)
+    import time
+    graphs.clear()
+    graph = None
+    torch.cuda.synchronize()
+    for _ in range(100):                                        # the note comes from a thread of CUDA's
+        backend._give_back()
+        if not backend._captured:
+            break
+        time.sleep(0.05)
+    assert not backend._captured
+    backend.Dispose()
