@@ -111,11 +111,12 @@ class CudaBackend:
             self._handles[key] = h
         return h
 
-    def _workspace(self, nbytes: int, stream: torch.cuda.Stream) -> Tuple[Optional[int], int]:
+    def _workspace(self, nbytes: int, stream: torch.cuda.Stream, optional: bool = False) -> Tuple[Optional[int], int]:
         """The scratch buffer of ``stream``, grown on demand.  It is allocated on that stream, so a buffer that is replaced
         is reused only behind the launches that read it.  A call that is being captured gets the buffer of its capture: a
         graph keeps the address and may be replayed beside anything, another graph captured on this stream included, so such
-        a buffer is not shared with any other call, and given back when the graph (or the backend) has gone."""
+        a buffer is not shared with any other call, and given back when the graph (or the backend) has gone.  Without the
+        memory for it an ``optional`` buffer is None, and the one that the stream has stays."""
         if nbytes <= 0:
             return None, 0
         handle = stream.cuda_stream
@@ -128,24 +129,37 @@ class CudaBackend:
                     self._captured[key] = (N.Capture(*capture), [])
                 held = self._captured[key][1]
                 if not held or held[-1].numel() < nbytes:
-                    held.append(self._scratch_tensor(nbytes, stream))
+                    new = self._scratch_tensor(nbytes, stream, optional)
+                    if new is None:
+                        return None, 0
+                    held.append(new)
                 return held[-1].data_ptr(), held[-1].numel()
         buf = self._scratch.get(handle)
         if buf is None or buf.numel() < nbytes:
             self._give_back()
+            if not optional:   # make room first
+                self._scratch.pop(handle, None)
+            buf = self._scratch_tensor(nbytes, stream, optional)
+            if buf is None:
+                return None, 0
             self._scratch.pop(handle, None)
             if len(self._scratch) >= 16:
                 self._scratch.pop(next(iter(self._scratch)))
-            buf = self._scratch[handle] = self._scratch_tensor(nbytes, stream)
+            self._scratch[handle] = buf
         return buf.data_ptr(), buf.numel()
 
     def _give_back(self) -> None:
         for key in [key for key, (capture, _) in list(self._captured.items()) if capture.gone]:
             self._captured.pop(key, None)
 
-    def _scratch_tensor(self, nbytes: int, stream: torch.cuda.Stream) -> torch.Tensor:
-        with torch.cuda.stream(stream):
-            return torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{self.device}")
+    def _scratch_tensor(self, nbytes: int, stream: torch.cuda.Stream, optional: bool) -> Optional[torch.Tensor]:
+        try:
+            with torch.cuda.stream(stream):
+                return torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{self.device}")
+        except torch.OutOfMemoryError:
+            if not optional:
+                raise
+            return None
 
     @staticmethod
     def _check_dims(batch, numHeads, seqQ, seqK, headDim):
@@ -156,7 +170,8 @@ class CudaBackend:
              mask_stride=(0, 0, 0, 0), kv_len=None, q_stride=None, k_stride=None, v_stride=None, o_stride=None,
              block_table=None, block_table_stride=0, block_size=0, num_blocks=0, weights=None):
         stream = self.stream
-        ws, ws_bytes = self._workspace(h.workspace_bytes(batch, seqQ, seqK), stream)
+        # a prefill runs without its workspace too
+        ws, ws_bytes = self._workspace(h.workspace_bytes(batch, seqQ, seqK), stream, optional=seqQ > 1)
         h.launch(q=query.Handle, k=key.Handle, v=value.Handle, out=output.Handle, batch=batch, seq_q=seqQ, seq_kv=seqK,
                  stream=stream.cuda_stream, lse=lse.Handle if lse is not None else None,
                  mask=mask.Handle if mask is not None else None, mask_stride=mask_stride,

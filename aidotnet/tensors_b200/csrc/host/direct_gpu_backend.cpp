@@ -61,7 +61,8 @@ CudaBackend::~CudaBackend() {
 // A scratch buffer of at least `need` bytes.  Calls that run when they are made share one, which is grown - outside of
 // launch, like the reference's pooled scratch buffers.  A call that is being captured gets the buffer of its capture: a
 // graph keeps the address and may be replayed beside anything, another graph of this stream included, so such a buffer
-// is not shared with any other call, and given back when the graph (or the backend) has gone.
+// is not shared with any other call, and given back when the graph (or the backend) has gone.  Without the memory for
+// it an `optional` buffer is null, and the one that is there stays.
 CudaBackend::Scratch CudaBackend::Workspace(int64_t need, bool optional) {
   if (need <= 0) return {};
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
@@ -101,11 +102,23 @@ CudaBackend::Scratch CudaBackend::Workspace(int64_t need, bool optional) {
   }
   for (auto it = captured_.begin(); it != captured_.end();) it = it->second->note->gone ? captured_.erase(it) : std::next(it);
   if (scratch_.bytes >= need) return scratch_;
-  if (scratch_.ptr) cudaFree(scratch_.ptr);
-  scratch_ = {};
-  if (cudaMalloc(&scratch_.ptr, (size_t)need) != cudaSuccess) throw std::runtime_error("CudaBackend: out of device memory");
-  scratch_.bytes = need;
-  return scratch_;
+  Scratch grown;
+  if (optional) {
+    if (cudaMalloc(&grown.ptr, (size_t)need) != cudaSuccess) {
+      cudaGetLastError();
+      return {};
+    }
+    if (scratch_.ptr) cudaFree(scratch_.ptr);
+  } else {   // make room first
+    if (scratch_.ptr) cudaFree(scratch_.ptr);
+    scratch_ = {};
+    if (cudaMalloc(&grown.ptr, (size_t)need) != cudaSuccess) {
+      cudaGetLastError();
+      throw std::runtime_error("CudaBackend: out of device memory");
+    }
+  }
+  grown.bytes = need;
+  return scratch_ = grown;
 }
 
 aidn_sdpa_t CudaBackend::Handle(const aidn_sdpa_desc& d) {

@@ -175,7 +175,26 @@ static void graphs_give_back() {
   destroy_graph(50);                                    // the graph may outlive the backend
 }
 
+// A prefill that finds no memory for its optional buffer runs without one; the buffer that is there stays for decode calls.
+static void optional_buffers() {
+  CudaBackend be(0, nullptr);
+  void* eager = attention(be, 100, 1);
+  g_limit = 1000;
+  EXPECT(attention(be, 2000, 4) == nullptr && live(eager) && attention(be, 100, 1) == eager);
+  g_capture = 9;
+  EXPECT(attention(be, 2000, 4) == nullptr);
+  EXPECT(live(attention(be, 100, 1)));
+  g_capture = 0;
+  bool threw = false;
+  try { attention(be, 2000, 1); } catch (const std::runtime_error&) { threw = true; }
+  EXPECT(threw);
+  EXPECT(live(attention(be, 500, 1)));
+  g_limit = ~(size_t)0;
+}
+
 int main() {
+  optional_buffers();
+  EXPECT(g_live.empty());
   graphs_keep_their_buffers();
   EXPECT(g_live.empty());
   destroy_graph(8);

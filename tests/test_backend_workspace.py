@@ -105,3 +105,43 @@ def test_python_mirror_gives_back(monkeypatch):
         memory.backend._workspace(100, _Stream(100))
         memory.gone.add(ident - 1)
     assert len(memory.live) <= 2
+
+
+def test_python_mirror_runs_a_prefill_without_memory_for_its_workspace(monkeypatch):
+    import torch
+    memory = _Memory(monkeypatch)
+    ws = lambda n, optional=False: memory.backend._workspace(n, _Stream(100), optional)[0]
+    eager = ws(100)
+    memory.left = 1000
+    assert ws(2000, optional=True) is None and ws(100) == eager
+    memory.capture = 9
+    assert ws(2000, optional=True) is None and ws(100) in memory.live
+    memory.capture = None
+    with pytest.raises(torch.OutOfMemoryError):
+        ws(2000)
+    assert ws(500) in memory.live
+
+
+def test_only_a_prefill_does_without(monkeypatch):
+    """What the mirror's calls pass on: a decode asks, a prefill may."""
+    from aidotnet.tensors_b200.backend import CudaBackend
+
+    class Handle:
+        last_launch_count = last_path = 0
+
+        def workspace_bytes(self, *_):
+            return 100
+
+        def launch(self, **kw):
+            self.kw = kw
+
+    class Buffer:
+        Handle = 1
+
+    asked = []
+    backend = object.__new__(CudaBackend)
+    backend._stream, backend.launch_count = _Stream(100), 0
+    backend._workspace = lambda n, stream, optional=False: asked.append(optional) or (None, 0)
+    for rows in (1, 2):
+        backend._run(Handle(), query=Buffer, key=Buffer, value=Buffer, output=Buffer, batch=1, seqQ=rows, seqK=9, scale=1.0)
+    assert asked == [False, True]
