@@ -183,7 +183,9 @@ inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, unsigned thre
   cfg.stream = stream;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();   // reported here: the next launch must not find it as its own
+  return e;
 }
 
 // Host-side launchers (one per kernel family); each returns the CUDA error of its launch.

@@ -200,3 +200,45 @@ def test_decode_splits_keep_non_finite_values(dtype, D, Hq, Hkv, value):
     assert info["launches"] == 2 and info1["launches"] == 1
     assert torch.isnan(one[1, Hq - 1, 0, 7])
     assert torch.equal(torch.isnan(split), torch.isnan(one))
+
+
+@pytest.mark.parametrize("call", ["decode", "projection"])
+def test_a_refused_launch_is_not_reported_by_the_next(call):
+    """The runtime refuses a launch on the legacy stream while a blocking stream is being captured (on the host; nothing is
+    enqueued).  That call fails, and the one after it does not."""
+    import ctypes
+    cu = ctypes.CDLL("libcuda.so.1")
+    q, _ = gen((1, 2, 1, 64), "bf16", 1)
+    k, _ = gen((1, 2, 512, 64), "bf16", 2)
+    out = torch.empty(1, 2, 1, 64, device="cuda")
+    ws = torch.empty(1 << 16, dtype=torch.uint8, device="cuda")
+    h = N.Handle(device=0, qkv_dtype=N.BF16, out_dtype=N.F32, head_dim=64, num_q_heads=2, num_kv_heads=2, decode_chunk=512)
+    x, w = torch.zeros(128, device="cuda"), torch.zeros(384, 128, device="cuda")
+
+    def go():
+        if call == "projection":
+            N.qkv_rope_cache(input=x.data_ptr(), weights=w.data_ptr(), bias=w.data_ptr(), cosine=w.data_ptr(), sine=w.data_ptr(),
+                             query=out.data_ptr(), key_cache=ws.data_ptr(), value_cache=ws.data_ptr(), tokens=1, heads=2, kv_heads=2,
+                             head_dim=64, position=0, weight_dtype=N.F32, query_dtype=N.F32, cache_dtype=N.F32, cache_capacity=4,
+                             max_position=4, stream=0)
+        else:
+            h.launch(q=q.data_ptr(), k=k.data_ptr(), v=k.data_ptr(), out=out.data_ptr(), batch=1, seq_q=1, seq_kv=512, stream=0,
+                     workspace=ws.data_ptr(), workspace_bytes=ws.numel())
+
+    go()
+    torch.cuda.synchronize()
+    stream, graph = ctypes.c_void_p(), ctypes.c_void_p()
+    assert cu.cuStreamCreate(ctypes.byref(stream), 0) == 0
+    assert cu.cuStreamBeginCapture_v2(stream, 1) == 0          # thread-local mode
+    try:
+        with pytest.raises(N.AidnError):
+            go()
+    finally:
+        cu.cuStreamEndCapture(stream, ctypes.byref(graph))
+        cu.cuStreamDestroy_v2(stream)
+    src, dst = torch.full((64,), 3.0, device="cuda"), torch.zeros(64, device="cuda", dtype=torch.bfloat16)
+    N.cast("f32_to_bf16", src.data_ptr(), dst.data_ptr(), 64, 0)
+    go()
+    torch.cuda.synchronize()
+    assert (dst == 3).all()
+    h.close()
