@@ -141,7 +141,7 @@ __device__ __forceinline__ int32_t kv_block_read(const SdpaParams& p, int b, int
   const uint32_t k32 = (uint32_t)key;
   const uint32_t blk = p.block_shift >= 0 ? (k32 >> p.block_shift) : (k32 / (uint32_t)p.block_size);
   int32_t phys;
-  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(phys) : "l"(p.block_table + (int64_t)b * p.bt_stride + blk));
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(phys) : "l"(p.block_table + (int64_t)b * p.bt_stride + blk));
   return phys;
 }
 
@@ -166,10 +166,21 @@ __device__ __forceinline__ void report_bad_block(const SdpaParams& p, bool bad) 
 
 // Programmatic dependent launch: a kernel started with launch_dependent may begin while its predecessor on the stream is
 // still running - its launch latency and prologue then cost nothing - and must call pdl_wait before it touches memory that
-// any earlier kernel reads or writes.  pdl_trigger in the predecessor says from when on; a kernel that never calls it is
-// waited for as a whole, which is what the stream order alone would do.
+// any earlier kernel reads or writes.  What an earlier kernel may write is not read-only for the whole of its life, so it
+// must not go through the non-coherent path (ld.global.nc, __ldg, const __restrict__) either.  pdl_trigger in the
+// predecessor says from when on; a kernel that never calls it is waited for as a whole, which is what the stream order
+// alone would do.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// 16 bytes that are read once.
+__device__ __forceinline__ uint4 ld_stream16(const void* ptr) {
+  uint4 r;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+               : "l"(ptr));
+  return r;
+}
 
 template <typename... P, typename... A>
 inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A... args) {

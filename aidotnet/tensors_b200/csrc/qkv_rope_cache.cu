@@ -18,14 +18,6 @@ namespace aidn {
 namespace {
 
 
-__device__ __forceinline__ uint4 ld_stream16(const void* ptr) {
-  uint4 r;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-               : "l"(ptr));
-  return r;
-}
-
 template <typename WT>
 struct WVec;
 template <>
@@ -143,7 +135,7 @@ __global__ void __launch_bounds__(WARPS * 32) qkv_rope_cache_kernel(const QkvRop
           const float* x = XS ? xs + t * model + k : p.input + (int64_t)(t_base + t) * model + k;
 #pragma unroll
           for (int e = 0; e < N; e += 4) {
-            const float4 xv = XS ? *reinterpret_cast<const float4*>(x + e) : __ldg(reinterpret_cast<const float4*>(x + e));
+            const float4 xv = *reinterpret_cast<const float4*>(x + e);
             a0[t] = fmaf(f0[e], xv.x, a0[t]); a0[t] = fmaf(f0[e + 1], xv.y, a0[t]);
             a0[t] = fmaf(f0[e + 2], xv.z, a0[t]); a0[t] = fmaf(f0[e + 3], xv.w, a0[t]);
             a1[t] = fmaf(f1[e], xv.x, a1[t]); a1[t] = fmaf(f1[e + 1], xv.y, a1[t]);

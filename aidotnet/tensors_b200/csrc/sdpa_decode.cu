@@ -64,14 +64,6 @@ __device__ __forceinline__ void unpack16<__half>(const uint4& u, float* f) {
   }
 }
 
-__device__ __forceinline__ uint4 ld_stream16(const void* ptr) {
-  uint4 r;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-               : "l"(ptr));
-  return r;
-}
-
 // Visible key count of a decode query of batch entry b: padding limit, then the causal limit of query 0.
 __device__ __forceinline__ int64_t decode_len(const SdpaParams& p, int b) {
   int64_t L = kv_limit_of(p, b);
@@ -652,7 +644,7 @@ constexpr int kMaxCombine = 1024;   // split weights held in shared memory; more
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-    sdpa_decode_combine_kernel(const SdpaParams p, const int chunk, const int nchunks, const float* __restrict__ ws) {
+    sdpa_decode_combine_kernel(const SdpaParams p, const int chunk, const int nchunks, const float* ws) {
   __shared__ float weight[kMaxCombine];
   __shared__ float red[8];
   __shared__ float4 cols[128];

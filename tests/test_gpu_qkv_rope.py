@@ -228,3 +228,54 @@ def test_backend_mirror_methods():
     with pytest.raises(ValueError):
         be.RopeInterleaved(buf(xin), buf(c2), buf(s2), out, 18, 8, 6, 30)
     be.Dispose()
+
+
+@pytest.mark.parametrize("weights,cache,D,heads,kv_heads,chunk", [("f32", "f32", 64, 8, 8, 64), ("bf16", "bf16", 64, 8, 8, 64),
+                                                                  ("bf16", "bf16", 128, 8, 2, 1024), ("bf16", "bf16", 64, 40, 2, 128),
+                                                                  ("f32", "f32", 128, 6, 6, 1024)])
+@pytest.mark.parametrize("tokens", [1, 2])
+def test_steps_follow_each_other_without_synchronisation(weights, cache, D, heads, kv_heads, chunk, tokens):
+    """Projection, attention, projection of what the attention wrote, ...: the kernels of a step start before the ones in front
+    of them have ended, and each reads what those write (cache rows, partial results, activations).  The chain gives the bits
+    that it gives with a synchronisation after every call."""
+    types = {"f32": (torch.float32, N.F32), "bf16": (torch.bfloat16, N.BF16)}
+    model, capacity, start, steps = heads * D, 1024, 700, 60
+    rng = torch.Generator(device="cuda").manual_seed(7)
+    rnd = lambda *shape: torch.randn(*shape, generator=rng, device="cuda")
+    x0 = rnd(tokens, model)
+    w = (rnd((heads + 2 * kv_heads) * D, model) * (2.0 / model ** 0.5)).to(types[weights][0])
+    bias, cos, sin = rnd((heads + 2 * kv_heads) * D), torch.cos(rnd(capacity, D // 2)), torch.sin(rnd(capacity, D // 2))
+    k0, v0 = (rnd(tokens, capacity, kv_heads, D).to(types[cache][0]) for _ in range(2))
+    q = torch.empty(tokens, model, device="cuda", dtype=types[cache][0])
+    positions = [torch.arange(tokens, device="cuda", dtype=torch.int32) * 0 + start + i for i in range(steps)]
+    rows = [torch.arange(tokens, device="cuda", dtype=torch.int32) * capacity + start + i for i in range(steps)]
+    h = N.Handle(device=0, qkv_dtype=types[cache][1], out_dtype=N.F32, head_dim=D, num_q_heads=heads, num_kv_heads=kv_heads,
+                 decode_chunk=chunk)
+    ws = torch.empty(max(16, h.workspace_bytes(tokens, 1, capacity)), dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def chain(synchronise):
+        x, k, v = x0.clone(), k0.clone(), v0.clone()
+        torch.cuda.synchronize()
+        for i in range(steps):
+            N.qkv_rope_cache(input=x.data_ptr(), weights=w.data_ptr(), bias=bias.data_ptr(), cosine=cos.data_ptr(), sine=sin.data_ptr(),
+                             query=q.data_ptr(), key_cache=k.data_ptr(), value_cache=v.data_ptr(), tokens=tokens, heads=heads,
+                             kv_heads=kv_heads, head_dim=D, positions=positions[i].data_ptr(), cache_rows=rows[i].data_ptr(),
+                             weight_dtype=types[weights][1], query_dtype=types[cache][1], cache_dtype=types[cache][1],
+                             cache_capacity=tokens * capacity, max_position=capacity, stream=stream)
+            if synchronise:
+                torch.cuda.synchronize()
+            # the new key is the last one that the query sees; the output is the next step's input
+            h.launch(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), out=x.data_ptr(), batch=tokens, seq_q=1, seq_kv=start + i + 1,
+                     k_stride=(capacity * kv_heads * D, D, kv_heads * D), v_stride=(capacity * kv_heads * D, D, kv_heads * D),
+                     stream=stream, workspace=ws.data_ptr(), workspace_bytes=ws.numel())
+            if synchronise:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return x, k, v
+
+    want = chain(True)
+    assert torch.isfinite(want[0]).all() and not torch.equal(want[0], x0)
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(chain(False), want))
+    h.close()
