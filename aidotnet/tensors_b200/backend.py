@@ -120,7 +120,7 @@ class CudaBackend:
         if nbytes <= 0:
             return None, 0
         handle = stream.cuda_stream
-        if self._stream is not None or torch.cuda.is_current_stream_capturing():
+        if handle and (self._stream is not None or torch.cuda.is_current_stream_capturing()):   # (stream 0 is never captured)
             capture = N.Capture.of(handle)
             if capture is not None:
                 key = (handle, capture[0])
