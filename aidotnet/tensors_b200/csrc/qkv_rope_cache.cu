@@ -227,7 +227,8 @@ __global__ void __launch_bounds__(kMmaThreads) qkv_rope_cache_mma_kernel(const Q
   const int chunks = model / 8;                     // 16-byte chunks per weight row
   // This warp's K slice is chunks warp*4 + c, + 64, + 128, ...; a batch is kBatch of them (all loads in flight at once).
   // The first batch of the next tile is requested before the current tile is handed to the finishing threads, so the
-  // weight stream does not stop at the tile boundary, and that of the first tile before the activations are staged.
+  // weight stream does not stop at the tile boundary, and that of the first tile before the activations are staged
+  // (56 bytes spilled meanwhile, 44 without).
   constexpr int kBatch = 8;
   constexpr int kChunkStep = 4 * kMmaWarps;
   uint4 we[kBatch], wo[kBatch];

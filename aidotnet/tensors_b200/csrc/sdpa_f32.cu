@@ -7,7 +7,8 @@
 // cycle to the registers whether lanes read the same words or not.  Each warp owns 16 query rows and walks tiles of 32
 // keys on its own; lane (ty, tx) of the 4 x 8 lanes holds a 4 x 4 block of logits and a 4 x (head_dim / 8) block of the
 // output.  8-row blocks would halve the shared-memory reads, but take 255 registers and with them half of the warps:
-// B1 H8 S512 D64 took 42 us that way against 27 (62 for the kernel of sdpa_generic.cu).
+// B1 H8 S512 D64 took 42 us that way against 27 (62 for the kernel of sdpa_generic.cu).  Sixteen warps leave 128 registers:
+// at head_dim 64 the fp32 instantiations spill up to 56 bytes (mask values), the 16-bit ones, with a tile in registers, 172.
 //   S = Q K^T   both operands have d contiguous, so the two halves of `fma.rn.f32x2` sum the even and the odd d of one
 //               logit: no operand has to be duplicated
 //   O += P V    the pair runs along d; P goes through shared memory transposed (rows contiguous) and is duplicated in

@@ -1,10 +1,8 @@
 // Generic attention forward: fp32 FFMA arithmetic, online softmax, any head_dim <= 256, every mask kind.
 //
-// Serves (1) the fp32-input contract (<= 1e-5 relative against the fp32 CPU path), where tensor-core
-// rounding of the inputs is not admissible, and (2) shapes and mask kinds the tcgen05 prefill kernel does
-// not take - what of both csrc/sdpa_f32.cu does not take either: the attention weights on request, paged K / V, head sizes
-// above 128 and rows that are not 16-byte aligned.  Replaces the one-thread-per-row kernel of the reference
-// (src/AiDotNet.Tensors/Engines/DirectGpu/CUDA/Kernels/CudaAttentionKernels.cs:28-112), which recomputes
+// Serves what neither the tcgen05 prefill kernel nor csrc/sdpa_f32.cu takes: the attention weights on request, paged K / V in
+// fp32 or odd head sizes, head sizes above 128 and rows that are not 16-byte aligned.  Replaces the one-thread-per-row kernel
+// of the reference (src/AiDotNet.Tensors/Engines/DirectGpu/CUDA/Kernels/CudaAttentionKernels.cs:28-112), which recomputes
 // q.k up to D+2 times per key; here K/V tiles are staged once in shared memory per 16 query rows.
 //
 // A group of 4 warps takes 16 query rows (4 per warp) over key tiles of 32.  In the score phase lane j owns key j of
@@ -12,8 +10,8 @@
 // g takes the key tiles g, g + KS, ..., keeps its own running max / sum / accumulator, and the groups' results are
 // merged through shared memory at the end (the rescaling rule of the online softmax, applied once more).  KS = 4 is
 // used when the launch has few CTAs: a small problem is one wave of CTAs whose length is the number of key tiles a
-// group walks through, each with a lone warp per scheduler and nothing to hide its latencies behind
-// (B1 H8 S512 D64: 72 us with KS = 1).
+// group walks through, each with a lone warp per scheduler and nothing to hide its latencies behind (B1 H8 S512 D64, which
+// comes here with unaligned rows or for its weights: 72 us with KS = 1, 62 with KS = 4).
 #include "common.cuh"
 
 namespace aidn {
@@ -87,8 +85,8 @@ __global__ void __launch_bounds__(KS * kWarps * 32) sdpa_generic_kernel(const Sd
   }
 
   // Contiguous K / V with head_dim <= 128: the next tile's elements are fetched into registers before the current
-  // tile is multiplied, so the loads run under the arithmetic.  (Without it every tile paid a full memory latency,
-  // which is what small problems - few CTAs, a handful of warps per SM - consist of: B1 H8 S512 D64 took 79 us.)
+  // tile is multiplied, so the loads run under the arithmetic.  (Without it every tile paid a full memory latency, which is
+  // what small problems - few CTAs, a handful of warps per SM - consist of: B1 H8 S512 D64 took 79 us, KS = 1 both times.)
   constexpr int kPre = DMAX <= 128 ? (kBN * DMAX) / (kWarps * 32) : 1;
   const bool prefetch = DMAX <= 128 && !paged;
   T kreg[kPre], vreg[kPre];

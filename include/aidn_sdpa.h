@@ -171,7 +171,8 @@ typedef struct {
 AIDN_API int aidn_sdpa_create(const aidn_sdpa_desc* desc, aidn_sdpa_t* out);
 /* Bytes of caller workspace for a launch of this shape; < 0 on error.  A decode launch needs them (or the handle's scratch);
  * a tcgen05 prefill with fewer work items than SMs uses them for the partial results of its split keys, and runs unsplit
- * when the workspace is NULL or smaller.  Launches that overlap on the GPU must not share a workspace. */
+ * when the workspace is NULL or smaller.  Launches that overlap on the GPU must not share a workspace, and a launch that
+ * was captured into a graph uses the same one at every replay. */
 AIDN_API int64_t aidn_sdpa_workspace_bytes(aidn_sdpa_t h, int64_t batch, int64_t seq_q, int64_t seq_kv);
 /* Enqueues the attention forward on `cu_stream` (a CUstream / cudaStream_t).  No allocation, no synchronisation; safe
  * under stream capture once the handle has launched that kernel once outside capture (the first launch raises the
