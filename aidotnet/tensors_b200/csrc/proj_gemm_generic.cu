@@ -227,28 +227,34 @@ __global__ void __launch_bounds__(WM* KG * 32, 2) proj_gemm_f32_kernel(const Gen
     }
   }
 
+  // Divisions in 32 bits (rows fit: at most 65535 tiles), and those of the columns ahead of the rows: 64-bit ones at every
+  // stored element made the attention layer of B2 S33 H6 D6 take 41 us instead of 29.
   float* c = static_cast<float*>(mat == 0 ? g.c[0] : (mat == 1 ? g.c[1] : g.c[2]));
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
-    const int64_t col = col0 + half * 32 + tx * 4;
+    const int col = (int)col0 + half * 32 + tx * 4;
     if (col >= g.n) continue;   // n is a multiple of 4: the group of four columns is inside or outside as a whole
-    const int h = (int)(col / g.head_dim), within = (int)(col - (int64_t)h * g.head_dim);
+    int64_t at[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (e > 0 && vec_out) break;   // head_dim % 4 == 0: the four columns belong to one head
+      const int h = (col + e) / g.head_dim;
+      at[e] = (int64_t)h * g.cs[1] + (col + e - h * g.head_dim);
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int64_t row = row0 + wm * 32 + ty + 4 * i;
+      const int row = (int)row0 + wm * 32 + ty + 4 * i;
       if (row >= g.rows) continue;
-      const int64_t b = row / g.seq, s = row - b * g.seq;
+      const int b = row / g.seq, s = row - b * g.seq;
       const float2 lo = unpack2(acc[i][2 * half]), hi = unpack2(acc[i][2 * half + 1]);
-      const int64_t base = b * g.cs[0] + s * g.cs[2];
-      if (vec_out) {   // head_dim % 4 == 0: the four columns belong to one head
-        *reinterpret_cast<float4*>(c + base + (int64_t)h * g.cs[1] + within) = make_float4(lo.x, lo.y, hi.x, hi.y);
+      float* dst = c + b * g.cs[0] + s * g.cs[2];
+      if (vec_out) {
+        *reinterpret_cast<float4*>(dst + at[0]) = make_float4(lo.x, lo.y, hi.x, hi.y);
       } else {
-        const float v[4] = {lo.x, lo.y, hi.x, hi.y};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int64_t hc = (col + e) / g.head_dim;
-          c[base + hc * g.cs[1] + (col + e - hc * g.head_dim)] = v[e];
-        }
+        dst[at[0]] = lo.x;
+        dst[at[1]] = lo.y;
+        dst[at[2]] = hi.x;
+        dst[at[3]] = hi.y;
       }
     }
   }
