@@ -439,6 +439,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  if (pp.splits > 1) pdl_trigger();   // the merge may be set up while this kernel runs
 #if AIDN_PREFILL_TRACE
   // mode 7: SM clock and wall-clock time at the start and end of every CTA (4 x u64 per CTA): the effective SM clock
   if (pp.debug_mode == 7 && threadIdx.x == 0) {
@@ -1441,39 +1442,45 @@ cudaError_t launch_type(const SdpaParams& p, int dtype, cudaStream_t stream, int
 }
 
 // out = sum_s w_s O_s / sum_s w_s with w_s = exp(m_s - M) l_s, M = max_s m_s; lse = M + log sum_s w_s: head_dim / 4 lanes per
-// row, one 16-byte load per part and lane.  The partial results were just written and come from L2.
+// row, of which lane s forms w_s; one 16-byte load per part and lane.  The partial results were just written and come from
+// L2.  The launch is a dependent one: set up while the parts are being computed.
+constexpr int kMaxSplits = 16;   // lanes of a row at head_dim 64
+
 template <typename T>
-__global__ void __launch_bounds__(256) sdpa_prefill_merge_kernel(const SdpaParams p, const float* __restrict__ parts,
-                                                                 const float2* __restrict__ stats, const int splits, const int64_t rows) {
-  const int lanes = p.head_dim / 4;
-  const int64_t row = (int64_t)blockIdx.x * (256 / lanes) + threadIdx.x / lanes;   // over [B, H, Sq]
-  const int d = threadIdx.x % lanes * 4;
-  if (row >= rows) return;
+__global__ void __launch_bounds__(256) sdpa_prefill_merge_kernel(const SdpaParams p, const float* parts, const float2* stats,
+                                                                 const int splits, const int64_t rows) {
+  const int lanes = p.head_dim / 4, lane = threadIdx.x % lanes;
+  int64_t row = (int64_t)blockIdx.x * (256 / lanes) + threadIdx.x / lanes;   // over [B, H, Sq]
+  const bool live = row < rows;
+  if (!live) row = rows - 1;
+  const int d = lane * 4;
   const int64_t per_batch = (int64_t)p.num_q_heads * p.seq_q;
   const int64_t b = row / per_batch, within = row - b * per_batch;
   const int64_t h = within / p.seq_q, q = within - h * p.seq_q;
   const int64_t first = b * splits * per_batch + within;
-  float m = -INFINITY;
-  for (int s = 0; s < splits; ++s) m = fmaxf(m, stats[first + s * per_batch].x);
+  pdl_wait();
+  const float2 ml = lane < splits ? stats[first + lane * per_batch] : make_float2(-INFINITY, 0.f);
+  float m = ml.x;
+  for (int o = lanes / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   // No part saw a finite logit: the row sees no key (sums and outputs are 0) or its logits are NaN (both are NaN).
-  const float base = m == -INFINITY ? 0.f : m;
+  const float w = expf(ml.x - (m == -INFINITY ? 0.f : m)) * ml.y;
   float l = 0.f;
-  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
+  float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
   for (int s = 0; s < splits; ++s) {
-    const float2 ml = stats[first + s * per_batch];
-    const float w = expf(ml.x - base) * ml.y;
+    const float ws = __shfl_sync(0xffffffffu, w, s, lanes);
     const float4 x = *reinterpret_cast<const float4*>(parts + (first + s * per_batch) * p.head_dim + d);
-    l += w;
-    o.x = fmaf(w, x.x, o.x); o.y = fmaf(w, x.y, o.y); o.z = fmaf(w, x.z, o.z); o.w = fmaf(w, x.w, o.w);
+    l += ws;
+    o4.x = fmaf(ws, x.x, o4.x); o4.y = fmaf(ws, x.y, o4.y); o4.z = fmaf(ws, x.z, o4.z); o4.w = fmaf(ws, x.w, o4.w);
   }
+  if (!live) return;
   const float inv = l == 0.f ? 0.f : 1.f / l;
-  o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
+  o4.x *= inv; o4.y *= inv; o4.z *= inv; o4.w *= inv;
   const int64_t at = b * p.os[0] + h * p.os[1] + q * p.os[2] + d;   // 16-byte aligned rows (prefill_sm100_supported)
   if (p.out_f32) {
-    *reinterpret_cast<float4*>(static_cast<float*>(p.out) + at) = o;
+    *reinterpret_cast<float4*>(static_cast<float*>(p.out) + at) = o4;
   } else {
-    T t[4] = {from_float<T>(o.x), from_float<T>(o.y), from_float<T>(o.z), from_float<T>(o.w)};
+    T t[4] = {from_float<T>(o4.x), from_float<T>(o4.y), from_float<T>(o4.z), from_float<T>(o4.w)};
     *reinterpret_cast<uint2*>(static_cast<T*>(p.out) + at) = *reinterpret_cast<const uint2*>(t);
   }
   if (p.lse && d == 0) p.lse[row] = l > 0.f ? m + logf(l) : -INFINITY;
@@ -1488,9 +1495,13 @@ int64_t prefill_split_bytes(const SdpaParams& p, int splits) {
 // Work items are pairs of 128-row tiles; fewer of them than SMs leaves the chip idle however long the keys are (a chunk
 // of 512 queries and 32 heads: 64 items for 148 SMs).  The keys of every item are then cut into the number of parts that
 // ends first by the model below, in units of one 64-key sub-tile: an item costs its sub-tiles plus about four (first
-// scores, last P.V, epilogue), merging costs a launch and the partial results' way through memory.  Measured without and
-// with it (causal, D 128): Hq32 / Hkv8 512 x 8112 132 -> 87 us, Hq8 / Hkv1 1024 x 8192 132 -> 52, Hq2 256 x 16384 248 -> 34,
-// Hq8 256 x 4096 70 -> 27, Hq32 / Hkv8 512 x 1024 28.7 -> 27.7 (the fewest keys that are split).
+// scores, last P.V, epilogue), merging costs a launch and the partial results' way through memory.  The model takes every
+// item for a full one: that half of a causal square's items end early, and what kv_len holds, it does not see.  Measured
+// without and with the split: D 128 Hq32 / Hkv8 512 x 8112 132 -> 87 us, Hq8 / Hkv1 1024 x 8192 132 -> 52, Hq2 256 x 16384
+// 248 -> 34, Hq8 256 x 4096 70 -> 26 (causal or not within 3 %); at the fewest keys that are split, D 64 H16 1024 x 1024
+// 24.7 -> 22.7 (causal 22.7 -> 22.1), 8 sequences H8 128 x 1024 18.6 -> 17.9, D 128 Hq28 / Hkv4 384 x 1100 29.8 -> 26.8.  It loses
+// where the sequences are far shorter than the tensor: H8 128 x 16384 with ten keys 10.4 -> 18, Hq32 / Hkv8 512 x 8192 with 600
+// keys 22.7 -> 26.6, while from 1000 keys of 16384 on it gains.
 int prefill_splits(const SdpaParams& p, int num_sms) {
   if (p.head_count != p.num_q_heads || p.peer_count > 0) return 1;
   const int64_t row_tiles = (p.seq_q + kBM - 1) / kBM;
@@ -1499,7 +1510,7 @@ int prefill_splits(const SdpaParams& p, int num_sms) {
   if (items >= num_sms || n < 2 * kMinSplitSubs) return 1;
   int best = 1;
   double best_cost = (double)(n + 4);
-  for (int s = 2; s <= 16 && n / s >= kMinSplitSubs; ++s) {
+  for (int s = 2; s <= kMaxSplits && n / s >= kMinSplitSubs; ++s) {
     const int64_t waves = (items * s + num_sms - 1) / num_sms;
     const double merge = 4.0 + (double)prefill_split_bytes(p, s) / 4e6;
     const double cost = (double)waves * (double)((n + s - 1) / s + 4) + merge;
@@ -1528,11 +1539,9 @@ cudaError_t launch_prefill_sm100(const SdpaParams& full, int dtype, cudaStream_t
   const int64_t rows = (int64_t)p.batch * p.num_q_heads * p.seq_q;
   const int rows_per_cta = 256 * 4 / p.head_dim;
   const unsigned grid = (unsigned)((rows + rows_per_cta - 1) / rows_per_cta);
-  const float* parts = workspace;
-  const float2* stats = reinterpret_cast<const float2*>(p.lse);
-  if (dtype == AIDN_BF16) sdpa_prefill_merge_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(full, parts, stats, splits, rows);
-  else sdpa_prefill_merge_kernel<__half><<<grid, 256, 0, stream>>>(full, parts, stats, splits, rows);
-  return cudaGetLastError();
+  const auto merge = dtype == AIDN_BF16 ? sdpa_prefill_merge_kernel<__nv_bfloat16> : sdpa_prefill_merge_kernel<__half>;
+  return launch_dependent(merge, grid, 256, 0, stream, full, static_cast<const float*>(workspace),
+                          reinterpret_cast<const float2*>(p.lse), splits, rows);
 }
 
 }  // namespace aidn
