@@ -99,6 +99,7 @@ struct Roles {
                 "setmaxnreg budget exceeds the registers the CTA is launched with");
   static_assert(kStoreWarps * kStageBufs * 4096 == kStageBytes, "staging memory");
 };
+constexpr int kMaxSorted = 32;   // sequences that are started in the order of their lengths
 constexpr int kItemWords = 16;   // mailbox entry: item, b, kvh, n_max, (h, t, n, valid) of both tiles, v_tail, k0, out_b
 
 template <int HD>
@@ -117,7 +118,8 @@ struct Cfg {
   static constexpr int kMiscOff = kBarOff + kNumBars * 8;  // issue lock, tmem ptr, abort flag, then the 2-slot item mailbox
   static constexpr int kMailOff = kMiscOff + 16;
   static constexpr int kStatsOff = kMailOff + 2 * kItemWords * 4;   // 1 / row sum of both tiles: [2][128] floats
-  static constexpr int kSmemBytes = kStatsOff + 2 * kBM * 4 + 1024 /*align slack*/;
+  static constexpr int kOrderOff = kStatsOff + 2 * kBM * 4;         // sequences by length: [kMaxSorted]
+  static constexpr int kSmemBytes = kOrderOff + kMaxSorted * 4 + 1024 /*align slack*/;
   static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
   static constexpr int kOCol = 256;
 };
@@ -188,34 +190,29 @@ __device__ __forceinline__ Item read_item(const volatile int* box) {
   return it;
 }
 
-// Sequences of a batch in the order of their lengths, longest first: lane r gets the batch index of rank r (warp-uniform
-// call; at most 32 sequences, otherwise - and without lengths - the order they come in).
-constexpr int kMaxSorted = 32;
+// Sequences of a batch in the order of their lengths, longest first (at most 32 sequences; otherwise, and without lengths,
+// they are taken as they come).  Called by one warp while the CTA is being set up: in the producer, ahead of its first item,
+// it cost a short launch 1 to 1.5 us (32 sequences H16 128 x 128 D 64, kernel alone: 22.0 us there, 20.7 here, 18.9 unsorted).
+__device__ __forceinline__ bool by_length(const SdpaParams& p) { return p.kv_len && p.batch <= kMaxSorted; }
 
-__device__ __forceinline__ int length_order(const SdpaParams& p, int lane) {
-  if (!p.kv_len || p.batch > kMaxSorted) return lane;
+__device__ __forceinline__ void length_order(const SdpaParams& p, int lane, volatile int* order) {
   const int len = lane < p.batch ? (int)kv_limit_of(p, lane) : -1;
   int rank = 0;
-#pragma unroll 1
+#pragma unroll 2
   for (int s = 0; s < p.batch; ++s) {
     const int other = __shfl_sync(0xffffffffu, len, s);
     rank += (other > len || (other == len && s < lane)) ? 1 : 0;
   }
-  int order = lane;
-#pragma unroll 1
-  for (int s = 0; s < p.batch; ++s)
-    if (__shfl_sync(0xffffffffu, rank, s) == lane) order = s;
-  return order;
+  if (lane < p.batch) order[rank] = lane;
 }
 
-// Warp-uniform; `order` is the caller's lane of length_order.
-__device__ __forceinline__ Item decode_item(const PrefillParams& pp, int item, int order) {
+__device__ __forceinline__ Item decode_item(const PrefillParams& pp, int item, const volatile int* order) {
   const SdpaParams& p = pp.p;
   Item it;
   const int split = pp.splits > 1 ? item % pp.splits : 0;
   if (pp.splits > 1) item /= pp.splits;
   // Heavy items first, so that the last ones to start are short: by row tile under a causal mask, else by sequence length
-  // (six sequences of 124 to 997 keys, 16 heads of 64, fp16: 44.6 us in the order they come, 40.9 longest first).
+  // (six sequences of 166 to 997 keys, 16 heads of 64, fp16, kernel alone: 45.0 us in the order they come, 40.9 longest first).
   int rank, w;
   if (p.kv_len && !p.causal) {
     const int per_seq = pp.ranks * pp.per_batch;
@@ -229,7 +226,7 @@ __device__ __forceinline__ Item decode_item(const PrefillParams& pp, int item, i
     it.b = rem / pp.per_batch;
     w = rem - it.b * pp.per_batch;
   }
-  if (p.kv_len && p.batch <= kMaxSorted) it.b = __shfl_sync(0xffffffffu, order, it.b);
+  if (by_length(p)) it.b = order[it.b];
   if (pp.pair_heads) {
     const int t = pp.row_tiles - 1 - rank;
     it.tile[0].h = p.head_begin + 2 * w;
@@ -397,6 +394,8 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem_gen + C::kMiscOff + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + C::kMiscOff + 12);
 
+  volatile int* order = reinterpret_cast<volatile int*>(smem_gen + C::kOrderOff);
+
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint64_t wait_ns = pp.wait_budget_ns;
 
@@ -431,6 +430,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
     prefetch_tensormap(&tm_v);
     prefetch_tensormap(&tm_o);
   }
+  if (warp == 1 && by_length(p)) length_order(p, lane, order);
   if (warp == kMmaWarp) {
     tmem_alloc(smem_u32(tmem_ptr_smem), kTmemCols);
     tmem_relinquish();
@@ -863,7 +863,6 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
       bool alive = true;
       uint32_t t_load = 0;          // K/V sub-tiles of earlier items (ring position)
       uint32_t q_uses[2] = {0, 0};  // loads of each Q tile so far
-      const int order = length_order(p, lane);
       int item = blockIdx.x;
       for (int seq = 0; alive; ++seq) {
         const int slot = seq & 1;
