@@ -338,10 +338,16 @@ cudaError_t launch_dp(const SdpaParams& p, cudaStream_t stream) {
   for (int i = 0; i < 3; ++i) vec = vec && p.os[i] % 4 == 0;
   // Row warps against key warps.  An SM's time is its share of the row tiles (the busiest SM counts) times the key tiles,
   // rounded up to what its key warps take at once; the most row warps of equal cost share each K / V tile best.
+  // With lengths the CTAs are unequal, half of a full one on average for the host that cannot see them: what counts is the
+  // average SM and the tail of one CTA, with the merge of its key warps on top, and smaller CTAs win.  34 shapes with lengths
+  // spread from 1 / 8 of the keys: at most 15 % from the best of the three, the rule above up to 2.8 times (B2 H4 S2048 D64 337 us
+  // with 8 x 1, 154 with 4 x 4, 176 with 2 x 8, causal 331, 150 and 118; B8 H16 S197 D32 35, 35 and 56).
   const int64_t heads = (int64_t)p.head_count * p.batch, key_tiles = (p.seq_kv + kKeysW - 1) / kKeysW;
   auto cost = [&](int wr, int wk) {
     const int64_t ctas = (p.seq_q + wr * kRowsW - 1) / (wr * kRowsW) * heads;
-    return (ctas + 147) / 148 * wr * ((key_tiles + wk - 1) / wk * wk);
+    const int64_t steps = (key_tiles + wk - 1) / wk * wk;
+    if (p.kv_len) return (ctas * 10 + 4 * 148) * (wr * steps + wk);   // (ctas / 148 + 0.4) CTAs, in whole numbers
+    return (ctas + 147) / 148 * wr * steps;
   };
   if constexpr (DP <= 64) {
     const int64_t c8 = cost(8, 1), c4 = cost(4, 4), c2 = cost(2, 8);
