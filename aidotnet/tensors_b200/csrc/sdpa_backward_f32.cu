@@ -304,9 +304,11 @@ cudaError_t launch_one(const BwdParams& bp, cudaStream_t stream) {
 
 template <int DP, bool KEYS>
 cudaError_t launch_dir(const BwdParams& bp, cudaStream_t stream) {
-  // Four stationary groups, and as many warps that share them as registers (168 up to head_dim 64, 255 above) and shared
-  // memory allow - sixteen warps of 128 registers spill and are 2 us slower for dQ on B2 H8 S509 D64; half the stationary
-  // rows when four groups leave SMs without a CTA.
+  // Four stationary groups, and as many warps that share them as registers (168 up to head_dim 64, with 4 to 24 bytes
+  // spilled; 255 above) and shared memory allow - sixteen warps of 128 registers spill more and are 2 us slower for dQ on
+  // B2 H8 S509 D64; half the stationary rows when four groups leave a good part of the SMs without a CTA.  Both sides
+  // measured (whole backward, CTAs of 64 rows, four groups / two, us): D 64 S 512: 48 CTAs 141 / 84, 112 143 / 156, 128 144 / 156,
+  // 144 145 / 156; D 128 104 CTAs 245 / 322, 128 246 / 323.  Above one wave two groups can be ahead again: D 64 160 CTAs 241 / 219.
   const int64_t rows = KEYS ? bp.p.seq_kv : bp.p.seq_q;
   const int64_t heads = (int64_t)(KEYS ? bp.p.head_count / bp.p.group : bp.p.head_count) * bp.p.batch;
   const bool wide = (rows + 4 * kOwnW - 1) / (4 * kOwnW) * heads >= 112;

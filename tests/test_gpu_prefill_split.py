@@ -320,3 +320,20 @@ def test_graphs_own_their_workspaces():
         time.sleep(0.05)
     assert not backend._captured
     backend.Dispose()
+
+
+def test_head_shards_give_the_rows_of_the_call_in_one_piece():
+    """A head shard is never split, whatever workspace it is given, so its bits are those of the same rows of the full call
+    without a workspace; with one the full call is split here and differs by the rounding of P."""
+    q, _ = gen((1, 8, 200, 128), "bf16", 1)
+    k, _ = gen((1, 4, 2100, 128), "bf16", 2)
+    v, _ = gen((1, 4, 2100, 128), "bf16", 3)
+    split, _, info = run_gpu(q, k, v, dtype="bf16", causal=True)
+    assert info["launches"] == 2
+    whole, _ = _unsplit(q, k, v, causal=True)
+    for begin in (0, 4):
+        out = torch.zeros(1, 8, 200, 128, device="cuda")
+        _, _, info = run_gpu(q, k, v, dtype="bf16", causal=True, head_begin=begin, head_count=4, out=out)
+        assert info["launches"] == 1
+        assert torch.equal(out[:, begin:begin + 4], whole[:, begin:begin + 4])
+    assert not torch.equal(split, whole)
