@@ -17,6 +17,8 @@
 //   warp  8     TMA producer + scheduler: Q tiles, then K and V sub-tiles of 64 keys through a ring of 8 slots, in the
 //               order the issuers need them (K(0), K(1), V(0), K(2), V(1), ...): three sub-tiles of look-ahead, which
 //               a TMA load under full load needs (2700 cycles from a slot's release to its data, measured)
+//               (paged K / V: Q and K only)
+//   warp  11    paged K / V: TMA producer of V; otherwise idle
 //   warps 9,10  UMMA issuers (one lane each): S = Q K^T (smem x smem), O += P V (TMEM x smem); issuer b handles the
 //               sub-tiles of parity b of both query tiles, the two take turns; warp 9 owns TMEM
 //
