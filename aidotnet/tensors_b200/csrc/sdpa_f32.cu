@@ -355,7 +355,9 @@ cudaError_t launch_dp(const SdpaParams& p, cudaStream_t stream) {
     if (c4 <= c2) return launch_cfg<T, DP, 4, 4>(p, vec, stream);
     return launch_cfg<T, DP, 2, 8>(p, vec, stream);
   } else {
-    if (cost(8, 1) <= cost(2, 4)) return launch_cfg<T, DP, 8, 1>(p, vec, stream);
+    // Above head_dim 64 one CTA fills an SM and 2 x 4 reads every K / V tile four times as often: with lengths it needs a margin
+    // (B3 H16 S700 D80, costs 1.06 to 1: 177 us with 8 x 1, 221 with 2 x 4; B16 H8 100 x 1500 D128, 1.24 to 1: 387 and 257).
+    if (cost(8, 1) * 20 <= cost(2, 4) * (p.kv_len ? 23 : 20)) return launch_cfg<T, DP, 8, 1>(p, vec, stream);
     return launch_cfg<T, DP, 2, 4>(p, vec, stream);
   }
 }
