@@ -711,7 +711,7 @@ int aidn_qkv_rope_cache(const aidn_qkv_rope_args* a, void* cu_stream) {
   int launches = 0;
   e = aidn::launch_qkv_rope_cache(p, a->weight_dtype, sms, (cudaStream_t)cu_stream, &launches);
   if (e != cudaSuccess) return fail_cuda(e, "qkv_rope_cache");
-  return post_launch_check((cudaStream_t)cu_stream, "aidn_qkv_rope_cache", nullptr);
+  return post_launch_check((cudaStream_t)cu_stream, "aidn_qkv_rope_cache", launch_check_enabled() ? aidn::qkv_rope_sm100_status() : nullptr);
 }
 
 int aidn_rope_interleaved(const float* input, const float* cosine, const float* sine, float* output, int64_t rows,

@@ -182,21 +182,51 @@ __device__ __forceinline__ uint4 ld_stream16(const void* ptr) {
   return r;
 }
 
+// Launched as thread-block clusters of `cluster` CTAs (1 x 1 x 1: none).
 template <typename... P, typename... A>
-inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A... args) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+inline cudaError_t launch_dependent_cluster(void (*kern)(P...), dim3 grid, unsigned threads, dim3 cluster, size_t smem,
+                                            cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster.x;
+  attr[1].val.clusterDim.y = cluster.y;
+  attr[1].val.clusterDim.z = cluster.z;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster.x * cluster.y * cluster.z > 1 ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
   if (e != cudaSuccess) cudaGetLastError();   // reported here: the next launch must not find it as its own
   return e;
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A... args) {
+  return launch_dependent_cluster(kern, grid, threads, dim3(1), smem, stream, args...);
+}
+
+// Thread-block clusters: the barrier of all their threads (release / acquire), and reads of another CTA's shared memory.
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t rank) {
+  uint32_t remote;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr, uint32_t rank) {
+  uint32_t remote;
+  float2 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(remote) : "memory");
+  return v;
 }
 
 // Host-side launchers (one per kernel family); each returns the CUDA error of its launch.
@@ -262,6 +292,10 @@ struct QkvRopeParams {
 int64_t qkv_rope_max_model();
 cudaError_t launch_qkv_rope_cache(const QkvRopeParams& p, int weight_dtype, int num_sms, cudaStream_t stream,
                                   int* launches);
+// Several tokens with bf16 weights on tcgen05 (csrc/qkv_rope_sm100.cu); launch_qkv_rope_cache hands it what it takes.
+bool qkv_rope_sm100_supported(const QkvRopeParams& p, int weight_dtype);
+cudaError_t launch_qkv_rope_sm100(const QkvRopeParams& p, int num_sms, cudaStream_t stream, int* launches);
+int32_t* qkv_rope_sm100_status();   // address of its status word in the current context, or null
 cudaError_t launch_rope_interleaved(const float* in, const float* cosc, const float* sinc, float* out, int64_t rows,
                                     int head_dim, int seq_len, int start_position, cudaStream_t stream);
 

@@ -279,3 +279,57 @@ def test_steps_follow_each_other_without_synchronisation(weights, cache, D, head
     for _ in range(5):
         assert all(torch.equal(a, b) for a, b in zip(chain(False), want))
     h.close()
+
+
+@pytest.mark.parametrize("tokens", [2, 15, 16, 17, 33, 64, 65, 130])
+@pytest.mark.parametrize("heads,kv_heads,D", [(4, 4, 64), (5, 1, 72), (6, 3, 20), (40, 8, 128)])
+def test_several_tokens_bf16_weights(tokens, heads, kv_heads, D):
+    """The tensor-core projection at its edges: passes of up to 64 tokens padded to 16, row tiles of 128, K blocks of 64 and
+    splits of K that do not divide.  An element is a sum of `model` products with exact bf16 weights; the accumulation truncates
+    (2^-23 of a partial sum) over chains of at most model / 96 + 8 additions per split: 2^-23 x (model / 96 + 16) of the sum of magnitudes,
+    twice for the rotation."""
+    rng = np.random.default_rng(300 + tokens)
+    model, rows, capacity, max_pos = heads * D, (heads + 2 * kv_heads) * D, 200, 96
+    x = rng.standard_normal((tokens, model)).astype(np.float32)
+    w = torch.from_numpy((rng.standard_normal((rows, model)) / np.sqrt(model)).astype(np.float32)).to(torch.bfloat16).float().numpy()
+    b = rng.uniform(-0.1, 0.1, rows).astype(np.float32)
+    cos, sin = _rope_tables(max_pos, D, rng)
+    positions = rng.integers(0, max_pos, tokens).astype(np.int32)
+    cache_rows = rng.permutation(capacity)[:tokens].astype(np.int32)
+    q, kc, vc = _run(x, w, b, cos, sin, heads=heads, kv_heads=kv_heads, head_dim=D, capacity=capacity, positions=positions,
+                     cache_rows=cache_rows, weight_dtype="bf16")
+    y = x.astype(np.float64) @ w.T.astype(np.float64) + b
+    y = y.reshape(tokens, -1, D)
+    c, s = cos[positions].astype(np.float64)[:, None], sin[positions].astype(np.float64)[:, None]
+    even, odd = y[:, :heads + kv_heads, 0::2].copy(), y[:, :heads + kv_heads, 1::2].copy()
+    y[:, :heads + kv_heads, 0::2], y[:, :heads + kv_heads, 1::2] = even * c - odd * s, even * s + odd * c
+    want = y.reshape(tokens, rows)
+    got = torch.cat([q, kc[torch.from_numpy(cache_rows).long()], vc[torch.from_numpy(cache_rows).long()]], 1).cpu().numpy()
+    bound = 2 * 2.0 ** -23 * (model / 96 + 16) * (np.abs(x) @ np.abs(w).T).max()
+    assert np.abs(got - want).max() <= bound, (np.abs(got - want).max(), bound)
+    unused = np.setdiff1d(np.arange(capacity), cache_rows)
+    assert torch.count_nonzero(kc[torch.from_numpy(unused).long()]) == 0
+
+
+def test_infinite_activations_and_weights_of_several_tokens():
+    """An infinity or a NaN stays in its token or its row, and an infinite sum is an infinity, as with fp32 multiply-adds."""
+    rng = np.random.default_rng(6)
+    heads, D, tokens = 2, 64, 3
+    model = heads * D
+    x = rng.uniform(0.5, 1, (tokens, model)).astype(np.float32)
+    w = rng.uniform(0.5, 1, (3 * model, model)).astype(np.float32)
+    x[0, 5] = np.inf
+    x[1, 7] = 1.0                      # mid and lo of it are 0
+    w[9, 7] = -np.inf
+    w[300, 3] = np.nan
+    w = torch.from_numpy(w).to(torch.bfloat16).float().numpy()
+    cos, sin = np.ones((4, D // 2), np.float32), np.zeros((4, D // 2), np.float32)
+    q, kc, vc = _run(x, w, None, cos, sin, heads=heads, kv_heads=heads, head_dim=D, capacity=4, positions=[0, 1, 2],
+                     cache_rows=[0, 1, 2], weight_dtype="bf16")
+    v = vc.cpu().numpy()[:tokens]      # no rotation, which would mix the elements of a pair
+    want = x @ w[2 * model:].T
+    assert np.array_equal(np.isnan(v), np.isnan(want)) and np.array_equal(np.isinf(v), np.isinf(want))
+    assert np.array_equal(v[np.isinf(v)], want[np.isinf(want)])
+    got = q.cpu().numpy()
+    assert np.isneginf(got[1, 9]) or np.isnan(got[1, 9])     # -inf through the rotation's 0 * x of the pair
+    assert np.isfinite(np.delete(got[1:], [8, 9], axis=1)).all()
