@@ -460,7 +460,9 @@ int launch_common(aidn_sdpa_t h, const aidn_sdpa_args* a, const aidn_paged_kv* p
                     (long long)need, (long long)h->scratch_bytes);
       }
     }
-    e = aidn::launch_decode(p, d.qkv_dtype, chunk, nchunks, ws, stream, &launches);
+    aidn::DecodePlan plan = {chunk, nchunks, 1};
+    if (d.decode_chunk == 0 && nchunks > 1) aidn::decode_plan_clusters(p, d.qkv_dtype, h->num_sms, &plan);
+    e = aidn::launch_decode(p, d.qkv_dtype, plan, ws, stream, &launches);
   } else if (path == AIDN_PATH_PREFILL_SM100) {
     // Keys of few items are split when the caller's workspace holds the partial results; without one they are not.  The
     // handle's own scratch is not used: it belongs to decode calls, which may be running on another stream.
@@ -653,7 +655,7 @@ int aidn_sdpa_decode_noalloc(const aidn_sdpa_desc* desc, const aidn_sdpa_args* a
                 "lower batch*heads*ceil(seq_kv/chunk) (a larger decode_chunk helps) or use aidn_sdpa_launch with a workspace",
                 (long long)need, (long long)have);
   int launches = 0;
-  cudaError_t e = aidn::launch_decode_static(p, d.qkv_dtype, chunk, nchunks, (cudaStream_t)cu_stream, &launches);
+  cudaError_t e = aidn::launch_decode_static(p, d.qkv_dtype, {chunk, nchunks, 1}, (cudaStream_t)cu_stream, &launches);
   if (e != cudaSuccess) return fail_cuda(e, "decode_noalloc");
   return post_launch_check((cudaStream_t)cu_stream, "aidn_sdpa_decode_noalloc", nullptr);
 }

@@ -234,12 +234,17 @@ cudaError_t launch_generic(const SdpaParams& p, int dtype, cudaStream_t stream);
 // The register-tiled fp32 kernel (csrc/sdpa_f32.cu); launch_generic hands it what it takes.
 bool f32_supported(const SdpaParams& p, int dtype);
 cudaError_t launch_f32(const SdpaParams& p, int dtype, cudaStream_t stream);
-cudaError_t launch_decode(const SdpaParams& p, int dtype, int chunk, int nchunks, float* workspace, cudaStream_t stream,
-                          int* launches);
+// How the keys of a decode are cut: `nchunks` parts, of `chunk` keys each where cluster is 1; else `nchunks` clusters of
+// `cluster` CTAs per (sequence, KV head), which share the sequence's keys evenly.  nchunks > 1 takes the workspace.
+struct DecodePlan {
+  int chunk, nchunks, cluster;
+};
+// Turns a plan of several chunks into one with clusters where that is faster; never one that needs more workspace.
+void decode_plan_clusters(const SdpaParams& p, int dtype, int num_sms, DecodePlan* plan);
+cudaError_t launch_decode(const SdpaParams& p, int dtype, const DecodePlan& plan, float* workspace, cudaStream_t stream, int* launches);
 bool decode_supported(int dtype, int head_dim);
 int64_t decode_static_scratch_bytes();
-cudaError_t launch_decode_static(const SdpaParams& p, int dtype, int chunk, int nchunks, cudaStream_t stream,
-                                 int* launches);
+cudaError_t launch_decode_static(const SdpaParams& p, int dtype, const DecodePlan& plan, cudaStream_t stream, int* launches);
 cudaError_t launch_cast(int kind, const void* src, void* dst, int64_t n, cudaStream_t stream);
 cudaError_t launch_paged_append(const void* src_k, const void* src_v, void* pool_k, void* pool_v,
                                 const int32_t* block_table, int64_t start, int64_t tokens, int block_size, int num_blocks,

@@ -1,8 +1,9 @@
 // Split-KV decode (seq_q == 1): the HBM-bound half of the attention path.
 //
 // One CTA streams one chunk of one (batch, kv head)'s keys and values exactly once, serves all query heads of that
-// kv head, and writes an un-normalised partial (max, sum, acc[D]); a second kernel merges the partials of a
-// (batch, head) by log-sum-exp.  Only keys below kv_len[b] (and the causal limit) are touched, so padding costs no
+// kv head, and forms an un-normalised partial (max, sum, acc[D]).  The partials of a (batch, head) are merged by
+// log-sum-exp: among the CTAs of a cluster through distributed shared memory where few enough CTAs run at once, by a
+// second kernel through a workspace otherwise (decode_plan_clusters).  Only keys below kv_len[b] (and the causal limit) are touched, so padding costs no
 // bandwidth.  Two partial kernels:
 //   * sdpa_decode_gqa_ring_kernel - fp16 / bf16, head_dim 64 or 128, up to 16 query heads per kv head (plain
 //     multi-head attention included): K/V go through a per-warp cp.async shared-memory ring and both products run
@@ -75,10 +76,75 @@ __device__ __forceinline__ int64_t decode_len(const SdpaParams& p, int b) {
   return L;
 }
 
+// What a CTA does with the merged partial of its keys.
+enum DecodeMerge : int {
+  kMergeWorkspace = 0,   // write it to the workspace; sdpa_decode_combine_kernel merges the splits
+  kMergeDirect = 1,      // there is one split: it is the result
+  kMergeCluster = 2,     // the splits are the CTAs of one cluster, which merge through distributed shared memory
+  kMergeBoth = 3,        // `nchunks` clusters per item: each merges its CTAs' partials and writes the result to the workspace
+};
+
+// Keys [start, end) of CTA c of `parts`.  With clusters every sequence is cut evenly by its own length (in steps of 16 keys),
+// so that the CTAs that wait for one another end together; otherwise by `chunk`.
+__device__ __forceinline__ void split_range(int64_t L, int chunk, int parts, int c, int merge, int64_t& start, int64_t& end) {
+  const int64_t step = merge >= kMergeCluster ? ((L + parts - 1) / parts + 15) / 16 * 16 : chunk;
+  start = c * step;
+  end = start + step < L ? start + step : L;
+}
+
+// Merge of a cluster's partials: each CTA holds ROWS heads as acc[ROWS][D], m[ROWS], l[ROWS] from shared address `part` on
+// (m = -inf: it saw no key), and forms one share of the (head, column) pairs, the splits in rank order.
+template <typename T, int D, int ROWS>
+__device__ __forceinline__ void merge_cluster(const SdpaParams& p, int b, int h0, int nheads, int rank, int splits, uint32_t part,
+                                              float* ws, int slot, int nslots) {
+  constexpr int kMaxSplits = 8;
+  cluster_sync_all();   // every CTA's partial is written
+  const int stride = splits * (int)blockDim.x;
+  for (int idx = rank * (int)blockDim.x + (int)threadIdx.x; idx < nheads * D; idx += stride) {
+    const int hh = idx / D, d = idx - hh * D, h = h0 + hh;
+    float m[kMaxSplits], l[kMaxSplits], a[kMaxSplits];
+#pragma unroll
+    for (int r = 0; r < kMaxSplits; ++r) {
+      m[r] = -INFINITY;
+      l[r] = a[r] = 0.f;
+      if (r < splits) {
+        m[r] = ld_cluster_f32(part + (uint32_t)((ROWS * D + hh) * 4), r);
+        l[r] = ld_cluster_f32(part + (uint32_t)((ROWS * (D + 1) + hh) * 4), r);
+        a[r] = ld_cluster_f32(part + (uint32_t)((hh * D + d) * 4), r);
+      }
+    }
+    float M = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < kMaxSplits; ++r) M = fmaxf(M, m[r]);
+    float acc = 0.f, lsum = 0.f;
+#pragma unroll
+    for (int r = 0; r < kMaxSplits; ++r) {
+      if (m[r] == -INFINITY) continue;   // a weight that underflows to 0 still carries the split's NaN and Inf
+      const float w = softmax_exp<T>(m[r] - M);
+      acc = fmaf(w, a[r], acc);
+      lsum = fmaf(w, l[r], lsum);
+    }
+    if (nslots > 1) {
+      const int64_t at = ((int64_t)b * p.head_count + (h - p.head_begin)) * nslots + slot;
+      ws[at * D + d] = acc;
+      if (d == 0) {
+        float* ml = ws + (int64_t)p.batch * p.head_count * nslots * D;
+        ml[at * 2] = M;
+        ml[at * 2 + 1] = lsum;
+      }
+      continue;
+    }
+    store_out<T>(p.out, b * p.os[0] + (int64_t)h * p.os[1] + d, acc * (lsum > 0.f ? 1.f / lsum : 0.f), p.out_f32);
+    if (p.lse && d == 0) p.lse[((int64_t)b * p.num_q_heads + h) * p.seq_q] = lsum > 0.f ? M + logf(lsum) : -INFINITY;
+  }
+  __syncwarp();
+  cluster_sync_all();   // nobody reads this CTA's shared memory any more
+}
+
 template <typename T, int D, int GT, bool PAGED, bool HEAD_FAST>
 __global__ void __launch_bounds__(kDecWarps * 32)
     sdpa_decode_partial_kernel(const SdpaParams p, const int chunk, const int nchunks, float* __restrict__ ws,
-                               const int direct) {
+                               const int merge, const int cluster) {
   constexpr int EPL = Vec16<T>::EPL;
   constexpr int LPK = D / EPL;    // lanes per key row
   constexpr int KPI = 32 / LPK;   // keys per warp-wide load
@@ -88,6 +154,7 @@ __global__ void __launch_bounds__(kDecWarps * 32)
   __shared__ float sm_m[NG][GT];
   __shared__ float sm_l[NG][GT];
   __shared__ __align__(16) float sm_acc[NG][GT][D];
+  __shared__ float sm_part[GT * (D + 2)];   // for the cluster: acc[GT][D], m[GT], l[GT]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int grp = lane / LPK, gl = lane % LPK, d0 = gl * EPL;
@@ -105,11 +172,12 @@ __global__ void __launch_bounds__(kDecWarps * 32)
   pdl_wait();      // nothing above touches memory that an earlier kernel writes
   pdl_trigger();   // the merge may be set up while this kernel runs
   const int64_t L = decode_len(p, b);
-  const int64_t start = (int64_t)c * chunk;
+  int64_t start, end;
+  split_range(L, chunk, nchunks * cluster, c, merge, start, end);
   const int Hc = p.head_count;
 
-  if (start >= L) {
-    if (direct && c == 0) {  // nothing visible: zero output, -inf LSE
+  if (start >= L && merge < kMergeCluster) {
+    if (merge == kMergeDirect && c == 0) {  // nothing visible: zero output, -inf LSE
       for (int idx = tid; idx < nheads * D; idx += kDecWarps * 32) {
         const int g = idx / D, d = idx - g * D;
         store_out<T>(p.out, b * p.os[0] + (int64_t)(h0 + g) * p.os[1] + d, 0.f, p.out_f32);
@@ -118,7 +186,6 @@ __global__ void __launch_bounds__(kDecWarps * 32)
     }
     return;
   }
-  const int64_t end = (start + chunk < L) ? start + chunk : L;
 
   float qf[GT][EPL];
 #pragma unroll
@@ -268,7 +335,13 @@ __global__ void __launch_bounds__(kDecWarps * 32)
       }
     }
     const int h = h0 + g;
-    if (direct) {
+    if (merge >= kMergeCluster) {
+      sm_part[g * D + d] = a;
+      if (d == 0) {
+        sm_part[GT * D + g] = M;
+        sm_part[GT * (D + 1) + g] = lsum;
+      }
+    } else if (merge == kMergeDirect) {
       store_out<T>(p.out, b * p.os[0] + (int64_t)h * p.os[1] + d, lsum > 0.f ? a / lsum : 0.f, p.out_f32);
       if (p.lse && d == 0)
         p.lse[((int64_t)b * p.num_q_heads + h) * p.seq_q] = lsum > 0.f ? M + logf(lsum) : -INFINITY;
@@ -282,6 +355,8 @@ __global__ void __launch_bounds__(kDecWarps * 32)
       }
     }
   }
+  __syncwarp();
+  if (merge >= kMergeCluster) merge_cluster<T, D, GT>(p, b, h0, nheads, c % cluster, cluster, ptx::smem_u32(sm_part), ws, c / cluster, nchunks);
 }
 
 // ---- grouped-query decode on the warp-level tensor-core path ---------------------------------------------------
@@ -329,7 +404,7 @@ struct RingCfg {
 template <typename T, int D, bool NH16, bool PAGED, bool HEAD_FAST>
 __global__ void __launch_bounds__(kDecWarps * 32, 2)
     sdpa_decode_gqa_ring_kernel(const SdpaParams p, const int chunk, const int nchunks, float* __restrict__ ws,
-                                const int direct) {
+                                const int merge, const int cluster) {
   static_assert(sizeof(T) == 2 && (D == 64 || D == 128), "16-bit inputs, head_dim 64 or 128");
   using R = RingCfg<D>;
   constexpr int KI = D / 32, VX = D / 64, MT = D / 16;
@@ -351,11 +426,12 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2)
   pdl_wait();      // nothing above touches memory that an earlier kernel writes
   pdl_trigger();   // the merge may be set up while this kernel runs
   const int64_t L = decode_len(p, b);
-  const int64_t start = (int64_t)cidx * chunk;
+  int64_t start, end;
+  split_range(L, chunk, nchunks * cluster, cidx, merge, start, end);
   const int Hc = p.head_count;
 
-  if (start >= L) {
-    if (direct && cidx == 0) {
+  if (start >= L && merge < kMergeCluster) {
+    if (merge == kMergeDirect && cidx == 0) {
       for (int idx = tid; idx < nheads * D; idx += kDecWarps * 32) {
         const int hh = idx / D, d = idx - hh * D;
         store_out<T>(p.out, b * p.os[0] + (int64_t)(h0 + hh) * p.os[1] + d, 0.f, p.out_f32);
@@ -364,7 +440,6 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2)
     }
     return;
   }
-  const int64_t end = (start + chunk < L) ? start + chunk : L;
 
   const uint32_t my_ring = smem0 + warp * R::kWarpBytes;
   const T* kbase = static_cast<const T*>(p.k) + (PAGED ? 0 : b * p.ks[0]) + (int64_t)kvh * p.ks[1];
@@ -605,6 +680,8 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2)
   __syncthreads();
 
   const float* all = reinterpret_cast<const float*>(ring_smem);   // warp n's partials start at n * kWarpFloats
+  float* part = reinterpret_cast<float*>(ring_smem) + ROWS * (D + 2);   // for the cluster: acc[ROWS][D], m[ROWS], l[ROWS], behind warp 0's
+  static_assert(2 * ROWS * (D + 2) <= kWarpFloats, "the CTA's partials must fit behind warp 0's");
   for (int idx = tid; idx < nheads * D; idx += kDecWarps * 32) {
     const int hh = idx / D, d = idx - hh * D;
     float M = -INFINITY;
@@ -621,7 +698,13 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2)
       }
     }
     const int h = h0 + hh;
-    if (direct) {
+    if (merge >= kMergeCluster) {
+      part[hh * D + d] = a;
+      if (d == 0) {
+        part[ROWS * D + hh] = M;
+        part[ROWS * (D + 1) + hh] = lsum;
+      }
+    } else if (merge == kMergeDirect) {
       store_out<T>(p.out, b * p.os[0] + (int64_t)h * p.os[1] + d, lsum > 0.f ? a / lsum : 0.f, p.out_f32);
       if (p.lse && d == 0)
         p.lse[((int64_t)b * p.num_q_heads + h) * p.seq_q] = lsum > 0.f ? M + logf(lsum) : -INFINITY;
@@ -635,6 +718,8 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2)
       }
     }
   }
+  __syncwarp();
+  if (merge >= kMergeCluster) merge_cluster<T, D, ROWS>(p, b, h0, nheads, cidx % cluster, cluster, ptx::smem_u32(part), ws, cidx / cluster, nchunks);
 }
 
 // Merges the splits of one (sequence, head): the weight of every split is formed once, in parallel, and the columns are
@@ -715,80 +800,70 @@ __global__ void __launch_bounds__(128)
 }
 
 template <typename T, int D, int GT>
-cudaError_t launch_partial(const SdpaParams& p, int chunk, int nchunks, float* ws, int direct, cudaStream_t stream) {
-  const int gchunks = (p.group + GT - 1) / GT;
-  const unsigned heads_y = (unsigned)((p.head_count / p.group) * gchunks);
-  const bool head_fast = p.ks[1] < p.ks[2] && nchunks <= 65535;
-  if (head_fast) {
-    dim3 grid(heads_y, (unsigned)nchunks, (unsigned)p.batch);
-    if (p.block_table)
-      return launch_dependent(sdpa_decode_partial_kernel<T, D, GT, true, true>, grid, kDecWarps * 32, 0, stream, p, chunk, nchunks, ws, direct);
-    return launch_dependent(sdpa_decode_partial_kernel<T, D, GT, false, true>, grid, kDecWarps * 32, 0, stream, p, chunk, nchunks, ws, direct);
-  } else {
-    dim3 grid((unsigned)nchunks, heads_y, (unsigned)p.batch);
-    if (p.block_table)
-      return launch_dependent(sdpa_decode_partial_kernel<T, D, GT, true, false>, grid, kDecWarps * 32, 0, stream, p, chunk, nchunks, ws, direct);
-    return launch_dependent(sdpa_decode_partial_kernel<T, D, GT, false, false>, grid, kDecWarps * 32, 0, stream, p, chunk, nchunks, ws, direct);
-  }
+cudaError_t launch_partial(const SdpaParams& p, const DecodePlan& plan, float* ws, int merge, cudaStream_t stream) {
+  const unsigned heads_y = (unsigned)((p.head_count / p.group) * ((p.group + GT - 1) / GT)), parts = (unsigned)(plan.nchunks * plan.cluster);
+  const bool head_fast = p.ks[1] < p.ks[2] && parts <= 65535;
+  const dim3 grid = head_fast ? dim3(heads_y, parts, (unsigned)p.batch) : dim3(parts, heads_y, (unsigned)p.batch);
+  const dim3 shape = head_fast ? dim3(1, (unsigned)plan.cluster) : dim3((unsigned)plan.cluster);
+  auto kern = head_fast ? (p.block_table ? sdpa_decode_partial_kernel<T, D, GT, true, true> : sdpa_decode_partial_kernel<T, D, GT, false, true>)
+                        : (p.block_table ? sdpa_decode_partial_kernel<T, D, GT, true, false> : sdpa_decode_partial_kernel<T, D, GT, false, false>);
+  return launch_dependent_cluster(kern, grid, kDecWarps * 32, shape, 0, stream, p, plan.chunk, plan.nchunks, ws, merge, plan.cluster);
 }
 
 template <typename T, int D, bool NH16>
-cudaError_t launch_gqa(const SdpaParams& p, int chunk, int nchunks, float* ws, int direct, cudaStream_t stream) {
-  const unsigned kvheads = (unsigned)(p.head_count / p.group);
-  const bool head_fast = p.ks[1] < p.ks[2] && nchunks <= 65535;
-  const dim3 grid = head_fast ? dim3(kvheads, (unsigned)nchunks, (unsigned)p.batch)
-                              : dim3((unsigned)nchunks, kvheads, (unsigned)p.batch);
-  const bool paged = p.block_table != nullptr;
+cudaError_t launch_gqa(const SdpaParams& p, const DecodePlan& plan, float* ws, int merge, cudaStream_t stream) {
+  const unsigned kvheads = (unsigned)(p.head_count / p.group), parts = (unsigned)(plan.nchunks * plan.cluster);
+  const bool head_fast = p.ks[1] < p.ks[2] && parts <= 65535;
+  const dim3 grid = head_fast ? dim3(kvheads, parts, (unsigned)p.batch) : dim3(parts, kvheads, (unsigned)p.batch);
+  const dim3 shape = head_fast ? dim3(1, (unsigned)plan.cluster) : dim3((unsigned)plan.cluster);
+  auto kern = head_fast ? (p.block_table ? sdpa_decode_gqa_ring_kernel<T, D, NH16, true, true> : sdpa_decode_gqa_ring_kernel<T, D, NH16, false, true>)
+                        : (p.block_table ? sdpa_decode_gqa_ring_kernel<T, D, NH16, true, false> : sdpa_decode_gqa_ring_kernel<T, D, NH16, false, false>);
   constexpr int smem = RingCfg<D>::kSmemBytes;
-#define AIDN_GQA_LAUNCH(PG, HF)                                                                                 \
-  do {                                                                                                          \
-    auto kern = sdpa_decode_gqa_ring_kernel<T, D, NH16, PG, HF>;                                                \
-    cudaError_t ea = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);             \
-    if (ea != cudaSuccess) return ea;                                                                           \
-    return launch_dependent(kern, grid, kDecWarps * 32, smem, stream, p, chunk, nchunks, ws, direct);           \
-  } while (0)
-  if (paged && head_fast) AIDN_GQA_LAUNCH(true, true);
-  else if (paged) AIDN_GQA_LAUNCH(true, false);
-  else if (head_fast) AIDN_GQA_LAUNCH(false, true);
-  else AIDN_GQA_LAUNCH(false, false);
-#undef AIDN_GQA_LAUNCH
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  return launch_dependent_cluster(kern, grid, kDecWarps * 32, shape, smem, stream, p, plan.chunk, plan.nchunks, ws, merge, plan.cluster);
+}
+
+// 16-bit inputs with up to 16 query heads per KV head (plain multi-head attention included: the padding rows of the MMA
+// tile cost nothing on an HBM-bound kernel): the tensor-core kernel with the cp.async ring.
+bool takes_ring(const SdpaParams& p, int dtype) {
+  return dtype != AIDN_F32 && (p.head_dim == 64 || p.head_dim == 128) && p.group <= 16;
 }
 
 template <typename T, int D>
-cudaError_t launch_partial_g(const SdpaParams& p, int chunk, int nchunks, float* ws, int direct, cudaStream_t stream) {
+cudaError_t launch_partial_g(const SdpaParams& p, const DecodePlan& plan, float* ws, int merge, cudaStream_t stream) {
   if constexpr (sizeof(T) == 2 && (D == 64 || D == 128)) {
-    // 16-bit inputs with up to 16 query heads per KV head (plain multi-head attention included: the padding rows
-    // of the MMA tile cost nothing on an HBM-bound kernel): the tensor-core kernel with the cp.async ring
-    if (p.group <= 8) return launch_gqa<T, D, false>(p, chunk, nchunks, ws, direct, stream);
-    if (p.group > 8 && p.group <= 16) return launch_gqa<T, D, true>(p, chunk, nchunks, ws, direct, stream);
+    if (p.group <= 8) return launch_gqa<T, D, false>(p, plan, ws, merge, stream);
+    if (p.group <= 16) return launch_gqa<T, D, true>(p, plan, ws, merge, stream);
   }
-  if (p.group == 1) return launch_partial<T, D, 1>(p, chunk, nchunks, ws, direct, stream);
-  if (p.group == 2) return launch_partial<T, D, 2>(p, chunk, nchunks, ws, direct, stream);
-  if (p.group <= 4) return launch_partial<T, D, 4>(p, chunk, nchunks, ws, direct, stream);
-  return launch_partial<T, D, 8>(p, chunk, nchunks, ws, direct, stream);
+  if (p.group == 1) return launch_partial<T, D, 1>(p, plan, ws, merge, stream);
+  if (p.group == 2) return launch_partial<T, D, 2>(p, plan, ws, merge, stream);
+  if (p.group <= 4) return launch_partial<T, D, 4>(p, plan, ws, merge, stream);
+  return launch_partial<T, D, 8>(p, plan, ws, merge, stream);
 }
 
 template <typename T>
-cudaError_t launch_decode_t(const SdpaParams& p, int chunk, int nchunks, float* ws, cudaStream_t stream,
-                            int* launches) {
-  const int direct = nchunks == 1 ? 1 : 0;
+cudaError_t launch_decode_t(const SdpaParams& p, const DecodePlan& plan, float* ws, cudaStream_t stream, int* launches) {
+  const int nchunks = plan.nchunks;
+  const int merge = plan.cluster > 1 ? (nchunks == 1 ? kMergeCluster : kMergeBoth) : (nchunks == 1 ? kMergeDirect : kMergeWorkspace);
   cudaError_t e;
   switch (p.head_dim) {
-    case 64: e = launch_partial_g<T, 64>(p, chunk, nchunks, ws, direct, stream); break;
-    case 128: e = launch_partial_g<T, 128>(p, chunk, nchunks, ws, direct, stream); break;
+    case 64: e = launch_partial_g<T, 64>(p, plan, ws, merge, stream); break;
+    case 128: e = launch_partial_g<T, 128>(p, plan, ws, merge, stream); break;
     case 256:
       if constexpr (sizeof(T) == 2) {
-        e = launch_partial_g<T, 256>(p, chunk, nchunks, ws, direct, stream);
+        e = launch_partial_g<T, 256>(p, plan, ws, merge, stream);
         break;
       }
       return cudaErrorInvalidValue;
     default: return cudaErrorInvalidValue;
   }
   *launches = 1;
-  if (e != cudaSuccess || direct) return e;
+  if (e != cudaSuccess || nchunks == 1) return e;
   dim3 grid((unsigned)p.head_count, (unsigned)p.batch);
   *launches = 2;
-  return launch_dependent(sdpa_decode_combine_kernel<T>, grid, 128, 0, stream, p, chunk, nchunks, static_cast<const float*>(ws));
+  // chunk 1: with clusters every slot is written (m = -inf where there was no key)
+  return launch_dependent(sdpa_decode_combine_kernel<T>, grid, 128, 0, stream, p, plan.cluster > 1 ? 1 : plan.chunk, nchunks, static_cast<const float*>(ws));
 }
 
 
@@ -859,12 +934,48 @@ bool decode_supported(int dtype, int head_dim) {
   return head_dim == 256 && dtype != AIDN_F32;
 }
 
-cudaError_t launch_decode(const SdpaParams& p, int dtype, int chunk, int nchunks, float* workspace, cudaStream_t stream,
-                          int* launches) {
+// Clusters save the merge kernel and its trip through L2, and cut each sequence by its own length; but CTAs that wait for one
+// another hold their place, so they pay only while all of a launch's CTAs are resident at once.  Measured, us, chunks with a
+// merge kernel / clusters of (n), bf16 unless stated: 32 heads of 64, 1237 keys 9.8 / 6.5 (8), 8192 keys 22 / 19 (8);
+// 32/8 heads of 128, 1000 keys 7.8 / 6.1 (8); B8 8/8 x 1024 13.6 / 9.0 (4), 12.7 (8); B20 4/2 x 700 8.9 / 7.2 (4), 10.4 (8);
+// B12 8/8 x 2000 19.0 / 20.2 (2), B3 32/32 x 900 13.0 / 12.5 (2); B16 32/8 x 2048 27.5 / 26.4 (2); B8 32/32 x 300 15.6 / 12.8 (2);
+// B40 32/8 x 1000 30.7 / 32.0 (2).  Where eight CTAs would walk many keys each, several clusters and the merge kernel: 64/8
+// heads of 128, 16384 keys 35 / 29 (8) / 20.8 (4 x 8); 8/2 30 / 12.7 (8 x 8).  fp32 on the FP32 units needs more CTAs:
+// 32 heads of 64, 1237 keys 13.8 / 11.4 (8), 6000 keys 29.6 / 38.7 (8) / 27.1 (2 x 8); 128 wide 3000 keys 21.6 / 22.1 (4 x 8).
+void decode_plan_clusters(const SdpaParams& p, int dtype, int num_sms, DecodePlan* plan) {
+  const bool ring = takes_ring(p, dtype);
+  if (!ring && (dtype != AIDN_F32 || p.group > 8)) return;
+  const int64_t items = (int64_t)p.batch * (p.head_count / p.group), keys = p.seq_kv;
+  const int64_t room = (ring ? (p.head_dim == 128 ? 2 : 3) : 4) * (int64_t)num_sms;   // CTAs that are resident at once
+  const int64_t parts = room / items;
+  int cluster = 1;
+  int64_t clusters = 1;
+  if (parts >= 8) {
+    if (!ring && p.head_dim == 128 && keys > 512) return;
+    cluster = 8;
+    clusters = keys / 8 / (ring ? 256 : 80);
+    if (clusters > parts / 8) clusters = parts / 8;
+    if (clusters > plan->nchunks) clusters = plan->nchunks;
+    if (clusters < 1) clusters = 1;
+  } else if (!ring) {
+    return;
+  } else if (parts >= 4) {
+    cluster = 4;
+  } else if (parts == 3) {
+    cluster = keys <= 1024 ? 2 : 1;
+  } else if (parts >= 1) {
+    cluster = keys <= 2048 ? 2 : 1;
+  }
+  if (cluster == 1) return;
+  plan->cluster = cluster;
+  plan->nchunks = (int)clusters;
+}
+
+cudaError_t launch_decode(const SdpaParams& p, int dtype, const DecodePlan& plan, float* workspace, cudaStream_t stream, int* launches) {
   switch (dtype) {
-    case AIDN_F32: return launch_decode_t<float>(p, chunk, nchunks, workspace, stream, launches);
-    case AIDN_F16: return launch_decode_t<__half>(p, chunk, nchunks, workspace, stream, launches);
-    default: return launch_decode_t<__nv_bfloat16>(p, chunk, nchunks, workspace, stream, launches);
+    case AIDN_F32: return launch_decode_t<float>(p, plan, workspace, stream, launches);
+    case AIDN_F16: return launch_decode_t<__half>(p, plan, workspace, stream, launches);
+    default: return launch_decode_t<__nv_bfloat16>(p, plan, workspace, stream, launches);
   }
 }
 
@@ -876,12 +987,11 @@ int64_t decode_static_scratch_bytes() { return kStaticScratchFloats * (int64_t)s
 
 // Same two kernels as launch_decode, with the partials in the library's static array.  `need_bytes` is what the
 // shape requires; the caller has already checked it against decode_static_scratch_bytes().
-cudaError_t launch_decode_static(const SdpaParams& p, int dtype, int chunk, int nchunks, cudaStream_t stream,
-                                 int* launches) {
+cudaError_t launch_decode_static(const SdpaParams& p, int dtype, const DecodePlan& plan, cudaStream_t stream, int* launches) {
   float* scratch = nullptr;
   cudaError_t e = static_scratch_address(&scratch);
   if (e != cudaSuccess) return e;
-  return launch_decode(p, dtype, chunk, nchunks, scratch, stream, launches);
+  return launch_decode(p, dtype, plan, scratch, stream, launches);
 }
 
 }  // namespace aidn
