@@ -860,7 +860,10 @@ int aidn_mha_forward(aidn_sdpa_t h, const aidn_mha_args* a, void* cu_stream) {
       e = aidn::launch_proj_gemm_sm100(g, stream, h->num_sms, h->status_dev, &why, h->debug_mode == 3);
     } else {
       if (!aidn::proj_gemm_generic_supported(g, &why)) return fail(AIDN_EUNSUPPORTED, "mha: %s", why);
-      e = aidn::launch_proj_gemm_generic(g, d.qkv_dtype, stream);
+      if (d.qkv_dtype == AIDN_F32 && aidn::proj_gemm_f32_sm100_supported(g))
+        e = aidn::launch_proj_gemm_f32_sm100(g, stream, h->num_sms, h->status_dev, h->debug_mode == 3);
+      else
+        e = aidn::launch_proj_gemm_generic(g, d.qkv_dtype, stream);
     }
     if (e != cudaSuccess) return why[0] ? fail(AIDN_ECUDA, "mha: %s (%s)", why, cudaGetErrorName(e)) : fail_cuda(e, what);
     ++launches;

@@ -347,6 +347,9 @@ bool proj_gemm_sm100_supported(const ProjGemm& g, const char** why);
 // expire: test hook - the producer withholds its loads and every bounded wait gives up after 20 ms.
 cudaError_t launch_proj_gemm_sm100(const ProjGemm& g, cudaStream_t stream, int num_sms, int32_t* status,
                                    const char** why, bool expire = false);
+// fp32 operands with 16-byte rows, every one as three bf16 terms on tcgen05 (csrc/proj_gemm_f32_sm100.cu).
+bool proj_gemm_f32_sm100_supported(const ProjGemm& g);
+cudaError_t launch_proj_gemm_f32_sm100(const ProjGemm& g, cudaStream_t stream, int num_sms, int32_t* status, bool expire = false);
 // The same contract in fp32 FFMA arithmetic for any sizes and for a / w of `dtype` (csrc/proj_gemm_generic.cu).
 bool proj_gemm_generic_supported(const ProjGemm& g, const char** why);
 cudaError_t launch_proj_gemm_generic(const ProjGemm& g, int dtype, cudaStream_t stream);

@@ -954,6 +954,7 @@ void decode_plan_clusters(const SdpaParams& p, int dtype, int num_sms, DecodePla
     if (!ring && p.head_dim == 128 && keys > 512) return;
     cluster = 8;
     clusters = keys / 8 / (ring ? 256 : 80);
+    if (!ring && clusters >= 5) clusters = 8;   // 4 heads of 64, 4000 keys: 10.2 us with six clusters, 9.0 with eight
     if (clusters > parts / 8) clusters = parts / 8;
     if (clusters > plan->nchunks) clusters = plan->nchunks;
     if (clusters < 1) clusters = 1;
