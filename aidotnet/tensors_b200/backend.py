@@ -68,6 +68,7 @@ class CudaBackend:
             raise RuntimeError("no CUDA device: this backend has no CPU path")
         N.load()
         self.device = device
+        self._torch_device = torch.device("cuda", device)
         torch.cuda.set_device(device)
         self._stream = stream
         self._path = path
@@ -83,8 +84,13 @@ class CudaBackend:
     def stream(self) -> torch.cuda.Stream:
         return self._stream if self._stream is not None else torch.cuda.current_stream(self.device)
 
+    @property
+    def _raw_stream(self) -> int:
+        """``stream.cuda_stream`` without the stream object."""
+        return self._stream.cuda_stream if self._stream is not None else torch._C._cuda_getCurrentRawStream(self.device)
+
     def AllocateBuffer(self, size: int, dtype: torch.dtype = torch.float32) -> GpuBuffer:
-        return GpuBuffer(torch.empty(int(size), dtype=dtype, device=f"cuda:{self.device}"))
+        return GpuBuffer(torch.empty(int(size), dtype=dtype, device=self._torch_device))
 
     def AllocateByteBuffer(self, size: int) -> GpuBuffer:
         return GpuBuffer(torch.empty(int(size), dtype=torch.uint8, device=f"cuda:{self.device}"))
@@ -102,7 +108,7 @@ class CudaBackend:
         self.stream.synchronize()
 
     def _handle(self, **kw) -> N.Handle:
-        key = tuple(sorted(kw.items()))
+        key = frozenset(kw.items())   # (field, value) pairs, in whatever order the caller names them
         h = self._handles.get(key)
         if h is None:
             if len(self._handles) >= 128:  # e.g. one handle per startPos of a long chunked prefill: drop the oldest
@@ -169,11 +175,18 @@ class CudaBackend:
     def _run(self, h: N.Handle, *, query, key, value, output, batch, seqQ, seqK, scale, lse=None, mask=None,
              mask_stride=(0, 0, 0, 0), kv_len=None, q_stride=None, k_stride=None, v_stride=None, o_stride=None,
              block_table=None, block_table_stride=0, block_size=0, num_blocks=0, weights=None):
-        stream = self.stream
-        # a prefill runs without its workspace too
-        ws, ws_bytes = self._workspace(h.workspace_bytes(batch, seqQ, seqK), stream, optional=seqQ > 1)
+        need = h.workspace_bytes(batch, seqQ, seqK)
+        stream = self._raw_stream
+        ws, ws_bytes = None, 0
+        if need > 0:
+            held = self._scratch.get(0) if stream == 0 else None   # (stream 0 is never captured)
+            if held is not None and held.numel() >= need:
+                ws, ws_bytes = held.data_ptr(), held.numel()
+            else:
+                # a prefill runs without its workspace too
+                ws, ws_bytes = self._workspace(need, self.stream, optional=seqQ > 1)
         h.launch(q=query.Handle, k=key.Handle, v=value.Handle, out=output.Handle, batch=batch, seq_q=seqQ, seq_kv=seqK,
-                 stream=stream.cuda_stream, lse=lse.Handle if lse is not None else None,
+                 stream=stream, lse=lse.Handle if lse is not None else None,
                  mask=mask.Handle if mask is not None else None, mask_stride=mask_stride,
                  kv_len=kv_len.Handle if kv_len is not None else None, q_stride=q_stride, k_stride=k_stride,
                  v_stride=v_stride, o_stride=o_stride, scale=scale, workspace=ws, workspace_bytes=ws_bytes,
@@ -289,7 +302,7 @@ class CudaBackend:
             chunk = max(8, (math.ceil(seqLen / min(splits, seqLen)) + 7) // 8 * 8)
         key = dict(qkv_dtype=_DTYPE[q.dtype], out_dtype=N.F32, head_dim=headDim, num_q_heads=heads,
                    num_kv_heads=kvHeads, causal=False)
-        hkey = tuple(sorted(key.items())) + (("chunk", chunk),)
+        hkey = frozenset(key.items()) | {("chunk", chunk)}
         h = self._handles.get(hkey)
         if h is None:
             h = N.Handle(device=self.device, path=self._path, decode_chunk=chunk or self._decode_chunk, **key)
@@ -514,7 +527,7 @@ class CudaBackend:
                          tokens=1, heads=heads, kv_heads=heads, head_dim=dimension, position=position,
                          weight_dtype=_DTYPE[packedWeights.dtype], query_dtype=_DTYPE[query.dtype],
                          cache_dtype=_DTYPE[keyCache.dtype], cache_capacity=cacheCapacity, max_position=cacheCapacity,
-                         stream=self.stream.cuda_stream)
+                         stream=self._raw_stream)
         self.launch_count += 1
 
     def RopeInterleaved(self, input: GpuBuffer, cos: GpuBuffer, sin: GpuBuffer, output: GpuBuffer, rows: int,

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 from typing import Optional, Sequence, Tuple
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -95,6 +96,16 @@ class MhaArgs(ctypes.Structure):
     ]
 
 
+# The argument blocks of the calls that a decode step makes, packed in one go: filling a ctypes structure field by field took
+# longer than the kernels of a small step.
+_SDPA_ARGS = struct.Struct("@6P4qP3q12qfPqiPi8P")
+_PAGED_KV = struct.Struct("@Pqii")
+_QKV_ROPE_ARGS = struct.Struct("@10P8i2q")
+assert (_SDPA_ARGS.size, _PAGED_KV.size, _QKV_ROPE_ARGS.size) == tuple(
+    ctypes.sizeof(t) for t in (SdpaArgs, PagedKv, QkvRopeArgs))
+_NO_STRIDE, _NO_PEERS = (0, 0, 0), (0,) * 8
+
+
 class AidnError(RuntimeError):
     def __init__(self, status: int, message: str):
         super().__init__(f"aidn_sdpa status {status}: {message}")
@@ -103,11 +114,13 @@ class AidnError(RuntimeError):
 
 
 _lib: Optional[ctypes.CDLL] = None
+# the entry points that take packed argument blocks (bytes)
+_launch_packed = _launch_paged_packed = _qkv_rope_packed = None
 
 
 def load() -> ctypes.CDLL:
     """Loads the CUDA library.  Raises if it has not been built: there is no CPU path behind this API."""
-    global _lib
+    global _lib, _launch_packed, _launch_paged_packed, _qkv_rope_packed
     if _lib is not None:
         return _lib
     if not os.path.exists(LIB_PATH):
@@ -166,6 +179,10 @@ def load() -> ctypes.CDLL:
     lib.aidn_rope_interleaved.restype = ctypes.c_int
     lib.aidn_sdpa_debug_set.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int]
     lib.aidn_sdpa_debug_set.restype = ctypes.c_int
+    pointer, block = ctypes.c_void_p, ctypes.c_char_p
+    _launch_packed = ctypes.CFUNCTYPE(ctypes.c_int, pointer, block, pointer)(("aidn_sdpa_launch", lib))
+    _launch_paged_packed = ctypes.CFUNCTYPE(ctypes.c_int, pointer, block, block, pointer)(("aidn_sdpa_launch_paged", lib))
+    _qkv_rope_packed = ctypes.CFUNCTYPE(ctypes.c_int, block, pointer)(("aidn_qkv_rope_cache", lib))
     _lib = lib
     return lib
 
@@ -181,6 +198,10 @@ def check(status: int) -> None:
 
 def _arr3(values: Optional[Sequence[int]]):
     return (ctypes.c_int64 * 3)(*(values if values is not None else (0, 0, 0)))
+
+
+def _strides(values: Optional[Sequence[int]]) -> Sequence[int]:
+    return _NO_STRIDE if values is None else values
 
 
 class Capture:
@@ -262,23 +283,18 @@ class Handle:
                peer_out: Sequence[int] = ()) -> None:
         """Enqueues one forward.  With ``block_table`` (a device int32 array) ``k`` / ``v`` are the paged pools
         ``[num_blocks, block_size, Hkv, D]`` and the call goes through ``aidn_sdpa_launch_paged``."""
-        a = SdpaArgs()
-        a.q, a.k, a.v, a.out, a.lse, a.mask, a.kv_len = q, k, v, out, lse, mask, kv_len
-        a.mask_stride = (ctypes.c_int64 * 4)(*mask_stride)
-        a.batch, a.seq_q, a.seq_kv = batch, seq_q, seq_kv
-        a.q_stride, a.k_stride, a.v_stride, a.o_stride = _arr3(q_stride), _arr3(k_stride), _arr3(v_stride), _arr3(o_stride)
-        a.scale, a.workspace, a.workspace_bytes, a.gather_output = scale, workspace, workspace_bytes, int(gather_output)
-        a.weights = weights
-        a.peer_count = len(peer_out)
-        for i, ptr in enumerate(peer_out):
-            a.peer_out[i] = ptr
+        peers = tuple(peer_out)
+        block = _SDPA_ARGS.pack(
+            q or 0, k or 0, v or 0, out or 0, lse or 0, mask or 0, *mask_stride, kv_len or 0, batch, seq_q, seq_kv,
+            *_strides(q_stride), *_strides(k_stride), *_strides(v_stride), *_strides(o_stride), scale,
+            workspace or 0, workspace_bytes, bool(gather_output), weights or 0, len(peers), *(peers + _NO_PEERS)[:8])
         if block_table is not None:
-            pg = PagedKv()
-            pg.block_table, pg.block_table_stride = block_table, block_table_stride
-            pg.block_size, pg.num_blocks = block_size, num_blocks
-            check(self._lib.aidn_sdpa_launch_paged(self._h, ctypes.byref(a), ctypes.byref(pg), ctypes.c_void_p(stream)))
-            return
-        check(self._lib.aidn_sdpa_launch(self._h, ctypes.byref(a), ctypes.c_void_p(stream)))
+            paged = _PAGED_KV.pack(block_table, block_table_stride, block_size, num_blocks)
+            status = _launch_paged_packed(self._h, block, paged, stream)
+        else:
+            status = _launch_packed(self._h, block, stream)
+        if status != OK:
+            raise AidnError(status, last_error())
 
     def backward_workspace_bytes(self, batch: int, seq_q: int) -> int:
         n = self._lib.aidn_sdpa_backward_workspace_bytes(self._h, batch, seq_q)
@@ -370,13 +386,14 @@ def qkv_rope_cache(*, input: int, weights: int, bias: Optional[int], cosine: int
                    query_dtype: int = F32, cache_dtype: int = F32, cache_capacity: int, max_position: int,
                    stream: int) -> None:
     """Packed Q/K/V projection + bias + interleaved RoPE + KV-cache write for ``tokens`` resident tokens."""
-    a = QkvRopeArgs()
-    a.input, a.weights, a.bias, a.cosine, a.sine = input, weights, bias, cosine, sine
-    a.query, a.key_cache, a.value_cache, a.positions, a.cache_rows = query, key_cache, value_cache, positions, cache_rows
-    a.tokens, a.heads, a.kv_heads, a.head_dim, a.position = tokens, heads, kv_heads, head_dim, position
-    a.weight_dtype, a.query_dtype, a.cache_dtype = weight_dtype, query_dtype, cache_dtype
-    a.cache_capacity, a.max_position = cache_capacity, max_position
-    check(load().aidn_qkv_rope_cache(ctypes.byref(a), ctypes.c_void_p(stream)))
+    if _lib is None:
+        load()
+    status = _qkv_rope_packed(_QKV_ROPE_ARGS.pack(
+        input or 0, weights or 0, bias or 0, cosine or 0, sine or 0, query or 0, key_cache or 0, value_cache or 0,
+        positions or 0, cache_rows or 0, tokens, heads, kv_heads, head_dim, position, weight_dtype, query_dtype, cache_dtype,
+        cache_capacity, max_position), stream)
+    if status != OK:
+        raise AidnError(status, last_error())
 
 
 def rope_interleaved(input: int, cosine: int, sine: int, output: int, rows: int, head_dim: int, seq_len: int,
