@@ -365,6 +365,7 @@ int build_params(aidn_sdpa_t h, const aidn_sdpa_args* a, const aidn_paged_kv* pg
   p.scale = a->scale > 0.f ? a->scale : 1.0f / std::sqrt((float)d.head_dim);
   p.softcap = d.softcap;
   p.status = h->status_dev;
+  p.no_tcgen05 = d.path == AIDN_PATH_GENERIC ? 1 : 0;
   const int64_t D = d.head_dim;
   if (all_zero(a->q_stride)) dense_strides(p.qs, d.num_q_heads, a->seq_q, D);
   else std::memcpy(p.qs, a->q_stride, sizeof(p.qs));

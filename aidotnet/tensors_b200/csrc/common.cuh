@@ -51,6 +51,7 @@ struct SdpaParams {
   int32_t block_size;
   int32_t block_shift;  // log2(block_size) when it is a power of two, else -1
   int32_t num_blocks;   // > 0: entries are range-checked against it
+  int32_t no_tcgen05;   // 1: stay on the FP32 units (desc.path == AIDN_PATH_GENERIC); fp32 attention only
 };
 
 template <typename T>
@@ -81,6 +82,13 @@ __device__ __forceinline__ void store_out(void* base, int64_t idx, float x, int 
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// The largest of three (a NaN counts only where all are), one instruction.
+__device__ __forceinline__ float fmax3(float a, float b, float c) {
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
   return y;
 }
 
@@ -234,6 +242,9 @@ cudaError_t launch_generic(const SdpaParams& p, int dtype, cudaStream_t stream);
 // The register-tiled fp32 kernel (csrc/sdpa_f32.cu); launch_generic hands it what it takes.
 bool f32_supported(const SdpaParams& p, int dtype);
 cudaError_t launch_f32(const SdpaParams& p, int dtype, cudaStream_t stream);
+// fp32 tensors as three bf16 terms on tcgen05 (csrc/sdpa_f32_sm100.cu), of the calls that f32_supported accepts.
+bool f32_sm100_supported(const SdpaParams& p, int dtype);
+cudaError_t launch_f32_sm100(const SdpaParams& p, cudaStream_t stream);
 // How the keys of a decode are cut: `nchunks` parts, of `chunk` keys each where cluster is 1; else `nchunks` clusters of
 // `cluster` CTAs per (sequence, KV head), which share the sequence's keys evenly.  nchunks > 1 takes the workspace.
 struct DecodePlan {
@@ -274,6 +285,9 @@ cudaError_t launch_backward_sm100(const BwdParams& bp, int dtype, cudaStream_t s
 // fp32 dQ and dK / dV launches on packed multiply-adds (csrc/sdpa_backward_f32.cu); delta must already be on the stream.
 bool backward_f32_supported(const BwdParams& bp, int dtype);
 cudaError_t launch_backward_f32(const BwdParams& bp, cudaStream_t stream);
+// The same as three bf16 terms on tcgen05 (csrc/sdpa_backward_f32_sm100.cu), of the calls that backward_f32_supported accepts.
+bool backward_f32_sm100_supported(const BwdParams& bp);
+cudaError_t launch_backward_f32_sm100(const BwdParams& bp, cudaStream_t stream);
 
 // Packed Q/K/V projection + RoPE + KV-cache write (csrc/qkv_rope_cache.cu).
 struct QkvRopeParams {

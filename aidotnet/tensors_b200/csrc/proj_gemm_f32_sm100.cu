@@ -93,24 +93,23 @@ __global__ void __launch_bounds__(kThreads, 1) proj_gemm_f32_sm100_kernel(const 
   if (warp < kWorkers / 32) {
     setmaxnreg_inc<208>();
     constexpr int kAChunks = kBM * 8 / kWorkers, kWChunks = kBK * (BN / 8) / kWorkers, kChunks = kAChunks + kWChunks;
-    float4 next[kChunks][2];
+    ulonglong2 next[kChunks][2];
     auto request = [&](int kb) {
-      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int e = 0; e < kAChunks; ++e) {
         const int idx = tid + e * kWorkers, r = idx >> 3, k = kb * kBK + (idx & 7) * 8;
         const float* src = g.a + (row0 + r) * g.k + k;
         const bool ok = row0 + r < g.rows;
-        next[e][0] = ok && k < g.k ? *reinterpret_cast<const float4*>(src) : zero;
-        next[e][1] = ok && k + 4 < g.k ? *reinterpret_cast<const float4*>(src + 4) : zero;
+        next[e][0] = split3::load4(src, ok && k < g.k);
+        next[e][1] = split3::load4(src + 4, ok && k + 4 < g.k);
       }
 #pragma unroll
       for (int e = 0; e < kWChunks; ++e) {
         const int idx = tid + e * kWorkers, r = idx / (BN / 8), n = col0 + (idx % (BN / 8)) * 8, k = kb * kBK + r;
         const float* src = w + (int64_t)k * g.n + n;
         const bool ok = k < g.k;
-        next[kAChunks + e][0] = ok && n < g.n ? *reinterpret_cast<const float4*>(src) : zero;
-        next[kAChunks + e][1] = ok && n + 4 < g.n ? *reinterpret_cast<const float4*>(src + 4) : zero;
+        next[kAChunks + e][0] = split3::load4(src, ok && n < g.n);
+        next[kAChunks + e][1] = split3::load4(src + 4, ok && n + 4 < g.n);
       }
     };
     const int quarter = warp & 3;   // the TMEM lanes a warp may read: 32 * (warp % 4) ...
@@ -198,12 +197,14 @@ __global__ void __launch_bounds__(kThreads, 1) proj_gemm_f32_sm100_kernel(const 
         if (!mbar_wait(bar_full + 8 * buf, (uint32_t)((kb / kBufs) & 1), abort_flag, g.wait_budget_ns)) break;
         tc_fence_after();
         const uint32_t a_s = smem_base + buf * C::kBuf, w_s = a_s + split3::kTerms * C::kAPlane;
+        // (a descriptor is its base plus a constant: one warp issues 24 products a block)
+        const uint64_t ad = make_smem_desc(a_s, 16, 1024), wd = make_smem_desc(w_s, C::kWBlock, 1024);
         auto product = [&](uint32_t d, int ta, int tb, bool fresh) {
 #pragma unroll
-          for (int kk = 0; kk < kBK / 16; ++kk)
-            if (leader)
-              mma_ss(d, make_smem_desc(a_s + (uint32_t)(ta * C::kAPlane + kk * 32), 16, 1024),
-                     make_smem_desc(w_s + (uint32_t)(tb * C::kWPlane + kk * 2048), C::kWBlock, 1024), idesc, !fresh || kk > 0 ? 1u : 0u);
+          for (int kk = 0; kk < kBK / 16; ++kk) {
+            const uint64_t x = ad + (uint64_t)((ta * C::kAPlane + kk * 32) >> 4), y = wd + (uint64_t)((tb * C::kWPlane + kk * 2048) >> 4);
+            if (leader) mma_ss(d, x, y, idesc, !fresh || kk > 0 ? 1u : 0u);
+          }
         };
         product(tmem_base + (uint32_t)((kb & 1) * BN), 0, 0, true);
 #pragma unroll
@@ -238,10 +239,9 @@ cudaError_t launch_t(F32GemmParams& f, int mats, cudaStream_t stream) {
 
 }  // namespace
 
-// 8 x 197 rows x 512 x 512: three projections 82 -> 21 us, one 37 -> 9; layers of 64 x 3072 and 1024 x 1024 211 -> 138 and
-// 336 -> 130 us.  Error of a whole layer against 64 bits 7.2e-7 -> 4.0e-7 at K = 768, 5.4e-7 -> 3.8e-7 at 512; below K = 256
-// the truncation of four additions weighs more than the rounding of K (2.5e-7 -> 3.4e-7 at 64) and the times are equal: there
-// the multiply-adds stay.
+// Whole layers, the attention unchanged: 64 rows x 3072 and 1024 x 1024 211 -> 138 and 336 -> 181 us.  Error of a whole layer against
+// 64 bits 7.2e-7 -> 4.0e-7 at K = 768, 5.4e-7 -> 3.8e-7 at 512; below K = 256 the truncation of four additions weighs more than the
+// rounding of K (2.5e-7 -> 3.4e-7 at 64) and the times are equal: there the multiply-adds stay.
 bool proj_gemm_f32_sm100_supported(const ProjGemm& g) {
   bool ok = g.k >= 256 && g.k % 4 == 0 && g.n % 4 == 0 && reinterpret_cast<uintptr_t>(g.a) % 16 == 0;
   for (int i = 0; i < g.num_mats; ++i) ok = ok && reinterpret_cast<uintptr_t>(g.w[i]) % 16 == 0;

@@ -158,14 +158,12 @@ __global__ void __launch_bounds__(kThreads) qkv_rope_cache_sm100_kernel(const __
       }
       tc_fence_after();
       const uint32_t d = tmem_base + (uint32_t)((2 + i % kAccs) * tpad);   // behind the columns of mid and lo
-      const uint32_t w_addr = smem_base + s * kWBytes, b_addr = smem_base + b_off + bs * b_bytes;
+      const uint64_t wd = make_smem_desc(smem_base + s * kWBytes, 16, 1024), hd = make_smem_desc(smem_base + b_off + bs * b_bytes, 16, 1024);
+      const uint64_t ld = hd + (uint64_t)(tpad * 128 >> 4);
 #pragma unroll
       for (int kk = 0; kk < kBK / 16; ++kk) {
-        const uint64_t wd = make_smem_desc(w_addr + kk * 32, 16, 1024);
-        if (leader) {
-          mma_ss(d, wd, make_smem_desc(b_addr + kk * 32, 16, 1024), idesc_hi, (i >= kAccs || kk > 0) ? 1u : 0u);
-          mma_ss(tmem_base, wd, make_smem_desc(b_addr + (uint32_t)(tpad * 128) + kk * 32, 16, 1024), idesc_low, (i > 0 || kk > 0) ? 1u : 0u);
-        }
+        if (leader) mma_ss(d, wd + 2 * kk, hd + 2 * kk, idesc_hi, (i >= kAccs || kk > 0) ? 1u : 0u);
+        if (leader) mma_ss(tmem_base, wd + 2 * kk, ld + 2 * kk, idesc_low, (i > 0 || kk > 0) ? 1u : 0u);
       }
       if (leader) {
         tc_commit(bar_empty + 8 * s);

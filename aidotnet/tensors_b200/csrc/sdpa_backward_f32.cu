@@ -1,5 +1,6 @@
 // Attention backward of fp32 tensors on register-tiled packed multiply-adds: dQ and dK / dV as two launches of one kernel
-// (head_dim <= 128, contiguous K / V, 16-byte rows; the formulas and the mask rules are those of sdpa_backward.cu).
+// (head_dim <= 128, contiguous K / V, 16-byte rows; the formulas and the mask rules are those of sdpa_backward.cu).  Head sizes up
+// to 64 go to the three-term products of csrc/sdpa_backward_f32_sm100.cu where the sequences are long enough for them.
 //
 // A warp keeps 16 rows of one sequence ("stationary") and walks 32-row tiles of the other past them:
 //   KEYS = true  (dK, dV): X = its K rows, Y = its V rows; a tile is U = Q rows, W = dO rows of one query head of the group.
@@ -338,6 +339,7 @@ bool backward_f32_supported(const BwdParams& bp, int dtype) {
 }
 
 cudaError_t launch_backward_f32(const BwdParams& bp, cudaStream_t stream) {
+  if (backward_f32_sm100_supported(bp)) return launch_backward_f32_sm100(bp, stream);
   if (bp.p.head_dim <= 32) return launch_dp<32>(bp, stream);
   if (bp.p.head_dim <= 64) return launch_dp<64>(bp, stream);
   if (bp.p.head_dim <= 96) return launch_dp<96>(bp, stream);

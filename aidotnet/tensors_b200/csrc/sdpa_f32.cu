@@ -1,7 +1,6 @@
-// Attention forward in fp32 arithmetic on register-tiled packed multiply-adds: the exact path for fp32 tensors and for
-// the 16-bit head sizes that the tcgen05 kernel does not take (head_dim <= 128, contiguous K / V, 16-byte rows).
-// Tensor cores are no option here: fp32 products formed from tf32 parts were measured at 2e-6 .. 5e-6 relative, this
-// kernel at 3e-7.
+// Attention forward in fp32 arithmetic on register-tiled packed multiply-adds: the path for the 16-bit head sizes that the tcgen05
+// kernel does not take and for fp32 tensors whose calls are too small for the three-term products of csrc/sdpa_f32_sm100.cu
+// (head_dim <= 128, contiguous K / V, 16-byte rows).
 //
 // Two things bound it: the FP32 pipe (128 multiply-adds per SM and cycle) and shared memory, which hands 128 bytes per
 // cycle to the registers whether lanes read the same words or not.  Each warp owns 16 query rows and walks tiles of 32
@@ -381,6 +380,7 @@ bool f32_supported(const SdpaParams& p, int dtype) {
 }
 
 cudaError_t launch_f32(const SdpaParams& p, int dtype, cudaStream_t stream) {
+  if (f32_sm100_supported(p, dtype)) return launch_f32_sm100(p, stream);
   switch (dtype) {
     case AIDN_F32: return launch_type<float>(p, stream);
     case AIDN_F16: return launch_type<__half>(p, stream);

@@ -6,6 +6,7 @@
 
 #include <stdint.h>
 
+#include "ffma2.cuh"
 #include "sm100_ptx.cuh"
 
 namespace aidn {
@@ -16,22 +17,28 @@ constexpr int kSmall = 5;   // products besides t0 * t0
 __host__ __device__ constexpr int small_a(int i) { return i == 0 ? 0 : (i == 1 ? 1 : (i == 2 ? 0 : (i == 3 ? 2 : 1))); }
 __host__ __device__ constexpr int small_b(int i) { return i == 0 ? 1 : (i == 1 ? 0 : (i == 2 ? 2 : (i == 3 ? 0 : 1))); }
 
-// The next term of a pair, packed (lo in bits 0-15), which is taken off the pair.
-__device__ __forceinline__ uint32_t take_term(float& lo, float& hi) {
-  const uint32_t w = ptx::pack2<true>(lo, hi);
-  lo -= __uint_as_float(w << 16);
-  hi -= __uint_as_float(w & 0xffff0000u);
+// The next term of a pair of floats (packed, lo in bits 0-15), which is taken off the pair.
+__device__ __forceinline__ uint32_t take_term(uint64_t& pair) {
+  const float2 x = unpack2(pair);
+  const uint32_t w = ptx::pack2<true>(x.x, x.y);
+  pair = fma2(pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)), 0xbf800000bf800000ull, pair);   // - 1 * term: exact
   return w;
 }
 
 // Eight neighbouring elements -> one 16-byte chunk of each term's image (128-byte swizzled rows of 64 elements); `addr` is the
 // chunk in the image of the first term, the others lie `plane` bytes apart.
-__device__ __forceinline__ void store_split8(uint32_t addr, uint32_t plane, float4 a, float4 b) {
+__device__ __forceinline__ void store_split8(uint32_t addr, uint32_t plane, ulonglong2 a, ulonglong2 b) {
+  uint64_t x[4] = {a.x, a.y, b.x, b.y};
 #pragma unroll
   for (int t = 0; t < kTerms; ++t) {
-    const uint32_t w0 = take_term(a.x, a.y), w1 = take_term(a.z, a.w), w2 = take_term(b.x, b.y), w3 = take_term(b.z, b.w);
+    const uint32_t w0 = take_term(x[0]), w1 = take_term(x[1]), w2 = take_term(x[2]), w3 = take_term(x[3]);
     ptx::st_shared_v4(addr + (uint32_t)t * plane, w0, w1, w2, w3);
   }
+}
+
+// Four floats in global memory, or zeros.
+__device__ __forceinline__ ulonglong2 load4(const float* src, bool valid) {
+  return valid ? *reinterpret_cast<const ulonglong2*>(src) : make_ulonglong2(0, 0);
 }
 
 // Offset of chunk c (eight elements) of row r in an image of 64-element rows.

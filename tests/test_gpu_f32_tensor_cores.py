@@ -1,0 +1,115 @@
+"""fp32 attention from three bf16 terms (csrc/sdpa_f32_sm100.cu, sdpa_backward_f32_sm100.cu) where it can go wrong: one row or key
+more or less than a tile, every number of k steps, one to eight CTAs per tile, every mask kind, values that are not finite, and
+the line between these kernels and the register-tiled ones."""
+import numpy as np
+import pytest
+import torch
+
+from aidotnet.tensors_b200 import native as N
+from oracle import sdpa_oracle as O
+
+from tests._harness import compare, compare_lse, gen, run_gpu
+
+pytestmark = pytest.mark.gpu
+
+# (B, Hq, Hkv, Sq, Sk, D): many heads keep a tile in one CTA, few cut its keys over up to eight
+SHAPES = [(2, 40, 40, 129, 257, 64), (1, 2, 1, 128, 520, 64), (1, 2, 2, 127, 449, 20), (2, 80, 20, 130, 321, 32), (1, 4, 2, 257, 511, 80),
+          (3, 30, 30, 100, 385, 96), (1, 8, 4, 16, 1025, 128), (2, 40, 40, 200, 330, 100), (1, 3, 3, 320, 64, 64)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("variant", ["plain", "causal", "lengths", "keep", "keep_f32", "bias", "softcap", "bias_softcap"])
+def test_forward(shape, variant):
+    B, Hq, Hkv, Sq, Sk, D = shape
+    q, qf = gen((B, Hq, Sq, D), "f32", 1, 1.0)
+    k, kf = gen((B, Hkv, Sk, D), "f32", 2, 1.0)
+    v, vf = gen((B, Hkv, Sk, D), "f32", 3, 1.0)
+    kw, okw = {}, {}
+    rng = np.random.default_rng(4)
+    if variant == "causal":
+        kw, okw = dict(causal=True, bottom_right=False, causal_offset=Sk - Sq - 3), dict(causal=True, causal_offset=Sk - Sq - 3)
+    elif variant == "lengths":
+        lens = rng.integers(0, Sk + 1, B).astype(np.int32)
+        lens[0] = Sk - 1
+        for b in range(B):                                    # what lies beyond a sequence's keys must never matter
+            k[b, :, lens[b]:], v[b, :, lens[b]:] = float("nan"), float("inf")
+        kw, okw = dict(kv_len=torch.from_numpy(lens).cuda()), dict(kv_len=lens)
+    elif variant in ("keep", "keep_f32"):
+        keep = (rng.random((1, Hq, Sq, Sk)) < 0.7).astype(np.uint8)
+        keep[:, :, Sq // 2] = 0                               # a row that sees nothing
+        keep[:, 0, :, : Sk // 2] = 0                          # a head whose first blocks hold nothing
+        kind = N.MASK_KEEP_U8 if variant == "keep" else N.MASK_KEEP_F32
+        dev = torch.from_numpy(keep).cuda()
+        kw, okw = dict(mask=dev if variant == "keep" else dev.float(), mask_kind=kind), dict(mask=keep, mask_kind=O.MASK_KEEP_U8)
+    elif variant == "bias" or variant == "bias_softcap":
+        bias = rng.standard_normal((B, 1, Sq, Sk)).astype(np.float32)
+        bias[..., ::7] = -np.inf
+        bias[..., 1] = np.finfo(np.float32).min
+        kw, okw = dict(mask=torch.from_numpy(bias).cuda(), mask_kind=N.MASK_ADD_F32), dict(mask=bias, mask_kind=O.MASK_ADD_F32)
+    if "softcap" in variant:
+        kw["softcap"] = okw["softcap"] = 20.0
+    out, lse, _ = run_gpu(q, k, v, dtype="f32", want_lse=True, **kw)
+    ref, ref_lse, _ = O.sdpa(qf, kf, vf, want_lse=True, **okw)
+    compare(out, ref, "f32", f"{shape} {variant}")
+    compare_lse(lse, ref_lse, "f32", f"{shape} {variant}")
+    again, _, _ = run_gpu(q, k, v, dtype="f32", want_lse=True, **kw)
+    assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("where", ["q", "k", "v", "v_masked", "k_masked"])
+@pytest.mark.parametrize("heads", [2, 80])
+def test_forward_non_finite(value, where, heads):
+    """What is not a number or infinite in one row comes out where the fp32 kernels (path generic) bring it out."""
+    B, S, D = 2, 300, 64
+    q, _ = gen((B, heads, S, D), "f32", 1, 1.0)
+    k, _ = gen((B, heads, S, D), "f32", 2, 1.0)
+    v, _ = gen((B, heads, S, D), "f32", 3, 1.0)
+    kw = {}
+    if "masked" in where:
+        keep = torch.ones((1, 1, S, S), dtype=torch.uint8, device="cuda")
+        keep[..., 7] = 0
+        kw = dict(mask=keep, mask_kind=N.MASK_KEEP_U8)
+    {"q": q, "k": k, "v": v}[where[0]][1, 1, 7, 5] = value
+    got, _, _ = run_gpu(q, k, v, dtype="f32", **kw)
+    want, _, _ = run_gpu(q, k, v, dtype="f32", path=N.PATH_GENERIC, **kw)
+    for test in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(test(got), test(want))
+    fin = torch.isfinite(want)
+    assert (got - want)[fin].abs().max() <= 1e-5
+
+
+BWD_SHAPES = [(1, 4, 4, 384, 384, 64), (1, 4, 2, 385, 449, 64), (2, 30, 30, 400, 385, 64), (1, 2, 2, 513, 640, 32), (2, 12, 6, 511, 450, 36),
+              (1, 8, 4, 390, 700, 20)]
+
+
+@pytest.mark.parametrize("shape", BWD_SHAPES)
+@pytest.mark.parametrize("variant", ["plain", "causal", "keep_lengths", "keep_f32", "bias"])
+def test_backward(shape, variant):
+    """dQ, dK, dV against float64: 16 x 2^-24 x sqrt(n) of the largest value, as for the register-tiled kernels."""
+    from tests.test_gpu_backward import _fwd_bwd
+    B, Hq, Hkv, Sq, Sk, D = shape
+    ts = [gen(s, "f32", i + 1, 1.0) for i, s in enumerate([(B, Hq, Sq, D), (B, Hkv, Sk, D), (B, Hkv, Sk, D), (B, Hq, Sq, D)])]
+    (q, qf), (k, kf), (v, vf), (g, gf) = ts
+    rng = np.random.default_rng(5)
+    kw, okw = {}, {}
+    if variant == "causal":
+        kw = okw = dict(causal=True, causal_offset=Sk - Sq + 2)
+    elif variant == "keep_lengths":
+        keep = (rng.random((B, 1, Sq, Sk)) < 0.8).astype(np.uint8)
+        lens = rng.integers(1, Sk + 1, B).astype(np.int32)
+        kw, okw = dict(mask=torch.from_numpy(keep).cuda(), mask_kind=N.MASK_KEEP_U8, kv_len=lens), dict(keep=keep, kv_len=lens)
+    elif variant == "keep_f32":
+        keep = (rng.random((B, 1, Sq, Sk)) < 0.8).astype(np.uint8)
+        kw, okw = dict(mask=torch.from_numpy(keep).cuda().float(), mask_kind=N.MASK_KEEP_F32), dict(keep=keep)
+    elif variant == "bias":
+        bias = rng.standard_normal((1, Hq, Sq, Sk)).astype(np.float32)
+        kw, okw = dict(mask=torch.from_numpy(bias).cuda(), mask_kind=N.MASK_ADD_F32), dict(bias=bias)
+    got = _fwd_bwd(q, k, v, g, dtype="f32", **kw)
+    want = O.sdpa_backward(qf, kf, vf, gf, **okw)[:3]
+    for x, y, name in zip(got, want, ("dQ", "dK", "dV")):
+        x = x.cpu().numpy()
+        assert np.isfinite(x).all(), name
+        assert np.abs(x - y).max() <= 16 * 2.0 ** -24 * np.sqrt(max(Sq, Sk, D)) * max(1.0, np.abs(y).max()), (name, np.abs(x - y).max())
+    again = _fwd_bwd(q, k, v, g, dtype="f32", **kw)
+    assert all(torch.equal(x, y) for x, y in zip(got, again))
