@@ -287,6 +287,7 @@ bool backward_f32_supported(const BwdParams& bp, int dtype);
 cudaError_t launch_backward_f32(const BwdParams& bp, cudaStream_t stream);
 // The same as three bf16 terms on tcgen05 (csrc/sdpa_backward_f32_sm100.cu), of the calls that backward_f32_supported accepts.
 bool backward_f32_sm100_supported(const BwdParams& bp);
+inline bool backward_f32_sm100_fits(const SdpaParams& p) { return p.head_dim <= 64 && p.seq_q >= 320 && p.seq_kv >= 320; }
 cudaError_t launch_backward_f32_sm100(const BwdParams& bp, cudaStream_t stream);
 
 // Packed Q/K/V projection + RoPE + KV-cache write (csrc/qkv_rope_cache.cu).

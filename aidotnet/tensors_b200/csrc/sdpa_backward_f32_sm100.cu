@@ -90,12 +90,6 @@ __device__ __forceinline__ void add_gradient(uint32_t t_acc, uint64_t (&acc)[N])
   }
 }
 
-__device__ __forceinline__ float max_nan(float a, float b) {   // not a number where a or b is not
-  float d;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
-  return d;
-}
-
 // KS: k steps of 16 columns (2: head sizes up to 32).
 template <int KS, bool KEYS, bool PLAIN>
 __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const BwdParams bp, const BwdTcParams tp) {
@@ -250,9 +244,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const BwdPar
         nl_own = lse == -INFINITY ? -INFINITY : -lse;
         nd_own = -bp.delta[((int64_t)b * p.head_count + hl0) * p.seq_q + own];
       }
-      const uint64_t scale2 = pack2(p.scale, p.scale), log2e2 = pack2(kLog2e, kLog2e), nlog2e2 = pack2(-kLog2e, -kLog2e);
-      constexpr float kLow = (float)(1.4426950408889634 - (double)kLog2e), kLn2 = 0.69314718f;
-      const uint64_t log2e_low2 = pack2(kLow, kLow), ln2_2 = pack2(kLn2, kLn2);
+      const uint64_t scale2 = pack2(p.scale, p.scale), log2e2 = pack2(kLog2e, kLog2e);
 
       auto add_block = [&](int j) {
         wait(bar_g + 8 * (j & 1), j >> 1);
@@ -341,13 +333,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const BwdPar
               const float2 x = unpack2(pr[k]), q = unpack2(nlk);
               t = add2(pack2(q.x == -INFINITY ? -INFINITY : x.x, q.y == -INFINITY ? -INFINITY : x.y), nlk);
             }
-            {   // e^t = 2^y (1 + ln(2) r), r what the product y = t log2(e) has lost
-              const float2 u = unpack2(t);
-              t = pack2(max_nan(u.x, -1000.f), max_nan(u.y, -1000.f));   // (no infinity: its r is not a number)
-            }
             const float2 y = unpack2(mul2(t, log2e2));
-            const uint64_t r = fma2(t, log2e_low2, fma2(t, log2e2, mul2(t, nlog2e2))), pw = pack2(ex2_approx(y.x), ex2_approx(y.y));
-            pr[k] = fma2(pw, mul2(r, ln2_2), pw);
+            pr[k] = pack2(ex2_approx(y.x), ex2_approx(y.y));
             if (!whole) {
               const float2 x = unpack2(pr[k]);
               pr[k] = pack2(2 * k >= lo && 2 * k < hi ? x.x : 0.f, 2 * k + 1 >= lo && 2 * k + 1 < hi ? x.y : 0.f);
@@ -594,11 +581,13 @@ cudaError_t launch_both(const BwdParams& bp, cudaStream_t stream) {
 // and dV: B1 H4 S333 D64 64 -> 44 us, B4 H8 S333 189 -> 64, B2 H8 S509 with a bias 151 -> 72, B4 H16 S1024 causal 1092 -> 332.
 // Shorter sequences would often gain as well (8 x 16 heads of 100 rows 88 -> 39 us, 2 heads of 64 rows 27 -> 32), but there the
 // multiply-adds' sums are as short as a block's and the truncation of four additions weighs more than their rounding: error
-// against 64 bits 2.7e-7 -> 2.9e-7 at 8 x 4 heads of 64 rows, 3.0e-7 -> 3.2e-7 at 197, 3.9e-7 -> 3.6e-7 at 509.
+// against 64 bits 2.9e-7 -> 3.2e-7 at 8 x 4 heads of 64 rows, 3.3e-7 -> 3.5e-7 at 197, 3.6e-7 -> 3.5e-7 at 333, 3.9e-7 -> 3.6e-7
+// at 509.  (With the roundings of t log2(e) made up for, here or in the forward kernel too, none of these is smaller: the
+// log-sum-exp carries the same ones, and they cancel.)
 bool backward_f32_sm100_supported(const BwdParams& bp) {
   const SdpaParams& p = bp.p;
-  const int64_t longer = p.seq_q > p.seq_kv ? p.seq_q : p.seq_kv, shorter = p.seq_q > p.seq_kv ? p.seq_kv : p.seq_q;
-  return !bp.no_tcgen05 && p.head_dim <= kDP && shorter >= 384 && (longer + kOwn) / kStr * 8 * (int64_t)p.group <= 0x7fffffff;
+  const int64_t longer = p.seq_q > p.seq_kv ? p.seq_q : p.seq_kv;
+  return !bp.no_tcgen05 && backward_f32_sm100_fits(p) && (longer + kOwn) / kStr * 8 * (int64_t)p.group <= 0x7fffffff;
 }
 
 cudaError_t launch_backward_f32_sm100(const BwdParams& bp, cudaStream_t stream) {

@@ -620,10 +620,12 @@ cudaError_t launch_mode(const SdpaParams& p, const F32TcParams& tp, Mode mode, c
 //                        8 heads 100 x 100: D 64 15.2 -> 12.7, D 128 16.8 -> 18.8; 2 heads 100 x 300: D 80 27 -> 19
 //   softcap              a tanh per score, the same on both sides: 16 x 32 heads 64 x 64: D 64 37 -> 54, D 128 84 -> 68; 8 x 16 heads
 //                        197 x 197, causal: D 64 74 -> 80; 2 x 8 heads 333 x 333: D 64 39 -> 35; 8 heads 100 x 100: D 128 19 -> 25
-// The error against 64 bits is below that of the multiply-adds in all of them (by a fifth to a half).
+// The error against 64 bits is below that of the multiply-adds in all of them (by a fifth to a half).  But where a log-sum-exp is
+// asked for and its backward pass stays on the multiply-adds, so does the forward pass: the roundings of the one cancel against
+// those of the other only in the same arithmetic (gradients of 4 x 8 heads of 333 rows: 3.9e-7 mixed, 3.6e-7 not).
 bool f32_sm100_supported(const SdpaParams& p, int dtype) {
   const int64_t tiles = (p.seq_q + kRows - 1) / kRows;
-  if (dtype != AIDN_F32 || p.no_tcgen05 || tiles == 0 || tiles * 8 > 0x7fffffff) return false;
+  if (dtype != AIDN_F32 || p.no_tcgen05 || (p.lse && !backward_f32_sm100_fits(p)) || tiles == 0 || tiles * 8 > 0x7fffffff) return false;
   const bool many = tiles * p.head_count * p.batch > 148, wide = p.head_dim > 64;
   const int64_t pairs = p.seq_q / tiles * p.seq_kv;   // of a tile
   if (wide) return many ? pairs >= (p.softcap > 0.f ? 4096 : 2048) : p.seq_kv > (p.softcap > 0.f ? 256 : 128);

@@ -14,12 +14,14 @@ pytestmark = pytest.mark.gpu
 
 # (B, Hq, Hkv, Sq, Sk, D): many heads keep a tile in one CTA, few cut its keys over up to eight
 SHAPES = [(2, 40, 40, 129, 257, 64), (1, 2, 1, 128, 520, 64), (1, 2, 2, 127, 449, 20), (2, 80, 20, 130, 321, 32), (1, 4, 2, 257, 511, 80),
-          (3, 30, 30, 100, 385, 96), (1, 8, 4, 16, 1025, 128), (2, 40, 40, 200, 330, 100), (1, 3, 3, 320, 64, 64)]
+          (3, 30, 30, 100, 385, 96), (1, 8, 4, 16, 1025, 128), (2, 40, 40, 200, 330, 100), (1, 3, 3, 320, 64, 64), (2, 4, 2, 330, 515, 64)]
 
 
 @pytest.mark.parametrize("shape", SHAPES)
 @pytest.mark.parametrize("variant", ["plain", "causal", "lengths", "keep", "keep_f32", "bias", "softcap", "bias_softcap"])
 def test_forward(shape, variant):
+    """Within the contract's tolerance of float64.  The log-sum-exp, which only long sequences get from these kernels, is that of
+    the same call; the output without it is the kernels' own for every shape."""
     B, Hq, Hkv, Sq, Sk, D = shape
     q, qf = gen((B, Hq, Sq, D), "f32", 1, 1.0)
     k, kf = gen((B, Hkv, Sk, D), "f32", 2, 1.0)
@@ -48,11 +50,13 @@ def test_forward(shape, variant):
         kw, okw = dict(mask=torch.from_numpy(bias).cuda(), mask_kind=N.MASK_ADD_F32), dict(mask=bias, mask_kind=O.MASK_ADD_F32)
     if "softcap" in variant:
         kw["softcap"] = okw["softcap"] = 20.0
-    out, lse, _ = run_gpu(q, k, v, dtype="f32", want_lse=True, **kw)
+    out, _, _ = run_gpu(q, k, v, dtype="f32", **kw)
+    with_lse, lse, _ = run_gpu(q, k, v, dtype="f32", want_lse=True, **kw)
     ref, ref_lse, _ = O.sdpa(qf, kf, vf, want_lse=True, **okw)
     compare(out, ref, "f32", f"{shape} {variant}")
+    compare(with_lse, ref, "f32", f"{shape} {variant}")
     compare_lse(lse, ref_lse, "f32", f"{shape} {variant}")
-    again, _, _ = run_gpu(q, k, v, dtype="f32", want_lse=True, **kw)
+    again, _, _ = run_gpu(q, k, v, dtype="f32", **kw)
     assert torch.equal(out, again)
 
 
@@ -79,7 +83,7 @@ def test_forward_non_finite(value, where, heads):
     assert (got - want)[fin].abs().max() <= 1e-5
 
 
-BWD_SHAPES = [(1, 4, 4, 384, 384, 64), (1, 4, 2, 385, 449, 64), (2, 30, 30, 400, 385, 64), (1, 2, 2, 513, 640, 32), (2, 12, 6, 511, 450, 36),
+BWD_SHAPES = [(1, 4, 4, 320, 320, 64), (1, 4, 2, 321, 449, 64), (2, 30, 30, 400, 385, 64), (1, 2, 2, 513, 640, 32), (2, 12, 6, 511, 450, 36),
               (1, 8, 4, 390, 700, 20)]
 
 
