@@ -10,7 +10,9 @@
 // S(j + 1) and P(j - 1) V are formed while the softmax of block j runs.  TMEM: two score buffers (leading products, small ones;
 // P over them) and one pair of output accumulators that start afresh with every block, so that the tensor cores, which
 // truncate when they accumulate, never add more than head_dim / 16 or four times into one cell.
-// An infinity times a term that is 0 is not a number: where a block holds one, the leading products alone say what the sum is.
+// An infinity times a term that is 0 is not a number, and a value above the largest bf16 rounds to an infinity: a score that does
+// not come out finite is formed again with multiply-adds, before the two threads of its row exchange their maxima (once they have,
+// either may store P over the scores of both).  In an output block the leading products alone say what such a sum is.
 //
 // A block is 48 products (24 at head sizes up to 32), so their issue counts: every number of k steps has its own instantiation,
 // descriptors are a base plus a constant, and scores and P V have a warp each (with one warp that formed every descriptor anew
@@ -70,8 +72,30 @@ struct F32TcParams {
   uint64_t wait_budget_ns;
 };
 
+// The largest of three; a NaN where any of them is one.
+__device__ __forceinline__ float fmax3_nan(float a, float b, float c) {
+  float y;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+
+// A score that the tensor cores could not form, as the row loop holds them: raw, or the finished logit with a bias or a softcap.
+// (Called, not inlined, and two chains of maxima: either costs the row loop registers otherwise, 14.35 -> 14.8 us for B1 H8 S512 D64.)
+__device__ __noinline__ float exact_score(const SdpaParams& p, int b, int h, int64_t row, int64_t key) {
+  const float* q = static_cast<const float*>(p.q) + b * p.qs[0] + h * p.qs[1] + row * p.qs[2];
+  const float* k = static_cast<const float*>(p.k) + b * p.ks[0] + (h / p.group) * p.ks[1] + key * p.ks[2];
+  float s = 0.f;
+#pragma unroll 1
+  for (int d = 0; d < p.head_dim; d += 4) {   // head sizes are multiples of 4, rows are 16-byte aligned
+    const float4 x = *reinterpret_cast<const float4*>(q + d), y = *reinterpret_cast<const float4*>(k + d);
+    s = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, s))));
+  }
+  if (!(p.softcap > 0.f) && p.mask_kind != AIDN_MASK_ADD_F32) return s;
+  return finish_logit(p, s * p.scale, b, h, row, key, key + 1);
+}
+
 template <int DP, int KS, Mode MODE>
-__global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const SdpaParams p, const F32TcParams tp) {
+__global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __grid_constant__ SdpaParams p, const F32TcParams tp) {
   using C = TCfg<DP, KS, MODE>;
   constexpr bool PLAIN = C::PLAIN;
   extern __shared__ uint8_t smem_raw[];
@@ -306,12 +330,38 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const SdpaP
             }
           }
         }
-        float mt = -INFINITY;
+        float mt = -INFINITY, mt1 = -INFINITY;
 #pragma unroll
-        for (int k = 0; k < kHalf / 2; ++k) {
-          const float2 x = unpack2(s[k]);
-          mt = fmaxf(mt, fmaxf(x.x, x.y));
+        for (int k = 0; k < kHalf / 2; k += 2) {
+          const float2 x = unpack2(s[k]), y = unpack2(s[k + 1]);
+          mt = fmax3_nan(mt, x.x, x.y);
+          mt1 = fmax3_nan(mt1, y.x, y.y);
         }
+        mt = fmax3_nan(mt, mt1, mt1);
+        if (!(mt < INFINITY) && row < p.seq_q) {
+          uint32_t bad = 0;
+#pragma unroll
+          for (int k = 0; k < kHalf / 2; ++k) {
+            const float2 x = unpack2(s[k]);
+            bad |= (fabsf(x.x) < INFINITY ? 0u : 1u << (2 * k)) | (fabsf(x.y) < INFINITY ? 0u : 2u << (2 * k));
+          }
+          for (bad &= keep; bad; bad &= bad - 1) {
+            const int at = __ffs(bad) - 1;
+            const float v = exact_score(p, b, h, row, (blk0 + j) * kKeys + half * kHalf + at);
+#pragma unroll
+            for (int k = 0; k < kHalf / 2; ++k) {
+              const float2 x = unpack2(s[k]);
+              s[k] = pack2(2 * k == at ? v : x.x, 2 * k + 1 == at ? v : x.y);
+            }
+          }
+          mt = -INFINITY;   // (what is not a number does not count: its weight is not a number either way)
+#pragma unroll
+          for (int k = 0; k < kHalf / 2; ++k) {
+            const float2 x = unpack2(s[k]);
+            mt = fmaxf(mt, fmaxf(x.x, x.y));
+          }
+        }
+        __syncwarp();
         x_of(j, half) = mt;
         pair_sync();   // the row's other thread has left its maximum, and has read its scores
         const float m_new = fmaxf(m, fmaxf(mt, x_of(j, 1 - half)));
@@ -321,36 +371,11 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const SdpaP
         m = m_new;
         uint64_t sums = 0;
         const uint64_t neg = pack2(-m_use, -m_use);
-        auto weights = [&] {
-          sums = 0;
 #pragma unroll
-          for (int k = 0; k < kHalf / 2; ++k) {
-            const float2 x = unpack2(mul2(add2(s[k], neg), c2));
-            s[k] = pack2(ex2_approx(x.x), ex2_approx(x.y));
-            sums = add2(sums, s[k]);
-          }
-        };
-        weights();
-        if (__any_sync(0xffffffffu, !(sum2(sums) < INFINITY))) {
-          // something is not a number: take the leading products alone where they are not finite (-inf is a weight of 0)
-          uint32_t hi[kHalf];
-          tmem_ld32(t_s, hi);
-          ptx::tc_wait_ld();
-          sums = 0;
-#pragma unroll
-          for (int k = 0; k < kHalf; ++k) {
-            const float2 pw = unpack2(s[k / 2]);
-            float w = k & 1 ? pw.y : pw.x;
-            const float x = __uint_as_float(hi[k]);
-            if (!(w < INFINITY) && !(fabsf(x) < INFINITY)) {
-              float f = x;
-              if (MODE == kSoftcap && x == x) f = copysignf(p.softcap, x);
-              if (add) f = (MODE == kSoftcap ? f : f * p.scale) + mine[k];
-              w = keep & (1u << k) ? ex2_approx((f - m_use) * c) : 0.f;
-            }
-            s[k / 2] = k & 1 ? pack2(pw.x, w) : pack2(w, pw.y);
-            if (k & 1) sums = add2(sums, s[k / 2]);
-          }
+        for (int k = 0; k < kHalf / 2; ++k) {
+          const float2 x = unpack2(mul2(add2(s[k], neg), c2));
+          s[k] = pack2(ex2_approx(x.x), ex2_approx(x.y));
+          sums = add2(sums, s[k]);
         }
         l = fmaf(l, corr, sum2(sums));
         if (masked && j + 1 < n) {

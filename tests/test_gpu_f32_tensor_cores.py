@@ -83,6 +83,51 @@ def test_forward_non_finite(value, where, heads):
     assert (got - want)[fin].abs().max() <= 1e-5
 
 
+@pytest.mark.parametrize("D", [32, 64, 80, 128])
+@pytest.mark.parametrize("heads", [2, 80])
+@pytest.mark.parametrize("variant", ["plain", "bias", "softcap"])
+def test_forward_keys_of_weight_zero(D, heads, variant):
+    """Infinite keys whose logits are -infinity for every row, in either half of a block or in both: their weight is 0, and no row may
+    become NaN, whichever of the two warps of a row is first.  (With a softcap tanh makes them -20, an ordinary logit.)"""
+    B, Sq, Sk = 2, 200, 330
+    q, _ = gen((B, heads, Sq, D), "f32", 1, 1.0)
+    k, _ = gen((B, heads, Sk, D), "f32", 2, 1.0)
+    v, vf = gen((B, heads, Sk, D), "f32", 3, 1.0)
+    q[..., 0] = -q[..., 0].abs() - 0.1
+    for key in (7, 8, 40, 100, 200, 205, 250, 329):
+        k[..., key, 0] = float("inf")
+    kw = dict(softcap=20.0) if variant == "softcap" else {}
+    s = (q.double() @ k.double().transpose(-1, -2)) / np.sqrt(D)
+    if variant == "bias":
+        bias = torch.randn((1, 1, Sq, Sk), device="cuda", generator=torch.Generator("cuda").manual_seed(4))
+        kw, s = dict(mask=bias, mask_kind=N.MASK_ADD_F32), s + bias
+    if variant == "softcap":
+        s = 20 * torch.tanh(s / 20)
+    want = torch.softmax(s, -1) @ v.double()
+    first = None
+    for _ in range(20):
+        got, _, _ = run_gpu(q, k, v, dtype="f32", **kw)
+        assert (got - want).abs().max() <= 1e-5 * want.abs().max()
+        first = got if first is None else first
+        assert torch.equal(got, first)
+
+
+@pytest.mark.parametrize("D", [32, 64, 80, 128])
+@pytest.mark.parametrize("heads", [2, 80])
+def test_forward_logits_from_the_largest_floats(D, heads):
+    """Finite elements above the largest bf16 (3.39e38) against queries that make ordinary logits of them."""
+    B, Sq, Sk = 2, 200, 330
+    q, _ = gen((B, heads, Sq, D), "f32", 1, 1.0)
+    k, _ = gen((B, heads, Sk, D), "f32", 2, 1.0)
+    v, _ = gen((B, heads, Sk, D), "f32", 3, 1.0)
+    q[..., 3] = q[..., 3] * 2e-38
+    k[..., ::5, 3] = torch.finfo(torch.float32).max
+    k[..., 1::7, 3] = torch.finfo(torch.float32).min
+    want = torch.softmax((q.double() @ k.double().transpose(-1, -2)) / np.sqrt(D), -1) @ v.double()
+    got, _, _ = run_gpu(q, k, v, dtype="f32")
+    assert (got - want).abs().max() <= 1e-5 * want.abs().max()
+
+
 BWD_SHAPES = [(1, 4, 4, 320, 320, 64), (1, 4, 2, 321, 449, 64), (2, 30, 30, 400, 385, 64), (1, 2, 2, 513, 640, 32), (2, 12, 6, 511, 450, 36),
               (1, 8, 4, 390, 700, 20)]
 
