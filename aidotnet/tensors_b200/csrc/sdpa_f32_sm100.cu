@@ -12,7 +12,8 @@
 // truncate when they accumulate, never add more than head_dim / 16 or four times into one cell.
 // An infinity times a term that is 0 is not a number, and a value above the largest bf16 rounds to an infinity: a score that does
 // not come out finite is formed again with multiply-adds, before the two threads of its row exchange their maxima (once they have,
-// either may store P over the scores of both).  In an output block the leading products alone say what such a sum is.
+// either may store P over the scores of both).  So is an output that is not finite in the end, from the keys that its row sees: the
+// tensor cores multiply every key of a block with all 128 rows, and 0 times an infinity reaches rows that do not see it.
 //
 // A block is 48 products (24 at head sizes up to 32), so their issue counts: every number of k steps has its own instantiation,
 // descriptors are a base plus a constant, and scores and P V have a warp each (with one warp that formed every descriptor anew
@@ -79,6 +80,29 @@ __device__ __forceinline__ float fmax3_nan(float a, float b, float c) {
   return y;
 }
 
+// What a CTA works on: 128 query rows of a head from row0 on, and n blocks of keys from blk0 on.
+struct Place {
+  int b, h, n;
+  int64_t row0, kv_limit, blk0;
+};
+__device__ __forceinline__ int64_t visible_end(const SdpaParams& p, int64_t kv_limit, int64_t row) {   // keys [0, end) are visible to the row
+  return p.causal && row + p.causal_offset + 1 < kv_limit ? row + p.causal_offset + 1 : kv_limit;
+}
+__device__ __forceinline__ Place place_of(const SdpaParams& p, int splits) {
+  Place at;
+  at.b = blockIdx.z;
+  at.h = p.head_begin + blockIdx.y;
+  const int rank = (int)blockIdx.x % splits, tiles = (int)gridDim.x / splits, at_x = (int)blockIdx.x / splits;
+  // under a causal mask the last rows see the most keys: start them first
+  at.row0 = (int64_t)(p.causal ? tiles - 1 - at_x : at_x) * kRows;
+  at.kv_limit = kv_limit_of(p, at.b);
+  const int64_t kend = visible_end(p, at.kv_limit, at.row0 + kRows < p.seq_q ? at.row0 + kRows - 1 : p.seq_q - 1);
+  const int64_t blocks = kend > 0 ? (kend + kKeys - 1) / kKeys : 0;
+  at.blk0 = rank * blocks / splits;
+  at.n = (int)((rank + 1) * blocks / splits - at.blk0);
+  return at;
+}
+
 // A score that the tensor cores could not form, as the row loop holds them: raw, or the finished logit with a bias or a softcap.
 // (Called, not inlined, and two chains of maxima: either costs the row loop registers otherwise, 14.35 -> 14.8 us for B1 H8 S512 D64.)
 __device__ __noinline__ float exact_score(const SdpaParams& p, int b, int h, int64_t row, int64_t key) {
@@ -92,6 +116,43 @@ __device__ __noinline__ float exact_score(const SdpaParams& p, int b, int h, int
   }
   if (!(p.softcap > 0.f) && p.mask_kind != AIDN_MASK_ADD_F32) return s;
   return finish_logit(p, s * p.scale, b, h, row, key, key + 1);
+}
+
+// Columns col .. col + cols - 1 of `factor` times the output that the CTA's keys add to its row `lrow`, in y where that is not finite
+// (m: the maximum that the weights are relative to).
+__device__ __noinline__ void exact_output(const SdpaParams& p, int splits, int lrow, float m, float factor, int col, int cols, float* y) {
+  const Place at = place_of(p, splits);   // (not handed over: the row loop would hold it in registers)
+  const int b = at.b, h = at.h;
+  const int64_t row = at.row0 + lrow, key0 = at.blk0 * kKeys, seen = visible_end(p, at.kv_limit, row);
+  const int64_t end = (at.blk0 + at.n) * kKeys < seen ? (at.blk0 + at.n) * kKeys : seen;
+  const bool raw = !(p.softcap > 0.f) && p.mask_kind != AIDN_MASK_ADD_F32;   // as in the row loop
+  const float c = raw ? p.scale * kLog2e : kLog2e;
+  if (m == -INFINITY) m = 0.f;
+  for (int c0 = 0; c0 < cols; c0 += 16) {
+    uint32_t bad = 0;
+    for (int e = 0; e < 16; ++e)
+      if (col + c0 + e < p.head_dim && !(fabsf(y[c0 + e]) < INFINITY)) bad |= 1u << e;
+    if (!bad) continue;
+    float s[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) s[e] = 0.f;
+    const float* v = static_cast<const float*>(p.v) + b * p.vs[0] + (h / p.group) * p.vs[1] + key0 * p.vs[2] + col + c0;
+    uint32_t open = bad;   // columns that are not NaN yet
+    for (int64_t key = key0; key < end && open; ++key, v += p.vs[2]) {
+      float x = exact_score(p, b, h, row, key);
+      if (raw && p.mask_kind != AIDN_MASK_NONE && finish_logit(p, 0.f, b, h, row, key, end) == -INFINITY) x = -INFINITY;
+      const float w = x == -INFINITY ? 0.f : ex2_approx((x - m) * c);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        if (!(open & (1u << e))) continue;
+        s[e] = fmaf(w, v[e], s[e]);
+        if (s[e] != s[e]) open &= ~(1u << e);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 16; ++e)
+      if (bad & (1u << e)) y[c0 + e] = s[e] * factor;
+  }
 }
 
 template <int DP, int KS, Mode MODE>
@@ -108,21 +169,10 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int D = p.head_dim;
 
-  const int b = blockIdx.z, h = p.head_begin + blockIdx.y, kvh = h / p.group;
-  const int rank = (int)blockIdx.x % tp.splits, tiles = (int)gridDim.x / tp.splits, at_x = (int)blockIdx.x / tp.splits;
-  // under a causal mask the last rows see the most keys: start them first
-  const int64_t row0 = (int64_t)(p.causal ? tiles - 1 - at_x : at_x) * kRows;
-  const int64_t kv_limit = kv_limit_of(p, b);
-  auto visible_end = [&](int64_t row) {   // keys [0, end) are visible to the row
-    int64_t end = kv_limit;
-    if (p.causal && row + p.causal_offset + 1 < end) end = row + p.causal_offset + 1;
-    return end;
-  };
-  const int64_t last_row = row0 + kRows < p.seq_q ? row0 + kRows - 1 : p.seq_q - 1;
-  const int64_t kend = visible_end(last_row);
-  const int64_t blocks = kend > 0 ? (kend + kKeys - 1) / kKeys : 0;
-  const int64_t blk0 = rank * blocks / tp.splits;
-  const int n = (int)((rank + 1) * blocks / tp.splits - blk0);
+  const Place at = place_of(p, tp.splits);
+  const int b = at.b, h = at.h, kvh = h / p.group, rank = (int)blockIdx.x % tp.splits, n = at.n;
+  const int64_t row0 = at.row0, kv_limit = at.kv_limit, blk0 = at.blk0;
+  const int64_t kend = visible_end(p, kv_limit, row0 + kRows < p.seq_q ? row0 + kRows - 1 : p.seq_q - 1);
 
   if (tid == 0) {
     *abort_flag = 0;
@@ -164,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
     const int quarter = warp & 3, half = warp >> 2, lrow = quarter * 32 + lane;
     const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const int64_t row = row0 + lrow;
-    const int64_t row_end = row < p.seq_q ? visible_end(row) : kend;
+    const int64_t row_end = row < p.seq_q ? visible_end(p, kv_limit, row) : kend;
     constexpr int kCols = C::kOut / 2;                           // output columns of a half
     int pair_phase = 0;
     auto pair_sync = [&] {   // the two warps of the same rows
@@ -250,22 +300,8 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
           tmem_ld16(t_o + (uint32_t)c0, reinterpret_cast<uint32_t*>(hi));
           tmem_ld16(t_o + (uint32_t)(C::kOut + c0), reinterpret_cast<uint32_t*>(lo));
           ptx::tc_wait_ld();
-          uint64_t chk = 0;
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            lo[e] = add2(hi[e], lo[e]);
-            chk = add2(chk, lo[e]);
-          }
-          if (!(fabsf(sum2(chk)) < INFINITY)) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const float2 x = unpack2(hi[e]), y = unpack2(lo[e]);
-              lo[e] = pack2(fabsf(x.x) < INFINITY ? y.x : x.x, fabsf(x.y) < INFINITY ? y.y : x.y);
-            }
-          }
-          __syncwarp();
-#pragma unroll
-          for (int e = 0; e < 8; ++e) acc[c0 / 2 + e] = add2(acc[c0 / 2 + e], lo[e]);
+          for (int e = 0; e < 8; ++e) acc[c0 / 2 + e] = add2(acc[c0 / 2 + e], add2(hi[e], lo[e]));
         }
       };
 
@@ -346,12 +382,12 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
             bad |= (fabsf(x.x) < INFINITY ? 0u : 1u << (2 * k)) | (fabsf(x.y) < INFINITY ? 0u : 2u << (2 * k));
           }
           for (bad &= keep; bad; bad &= bad - 1) {
-            const int at = __ffs(bad) - 1;
-            const float v = exact_score(p, b, h, row, (blk0 + j) * kKeys + half * kHalf + at);
+            const int i = __ffs(bad) - 1;
+            const float v = exact_score(p, b, h, row, (blk0 + j) * kKeys + half * kHalf + i);
 #pragma unroll
             for (int k = 0; k < kHalf / 2; ++k) {
               const float2 x = unpack2(s[k]);
-              s[k] = pack2(2 * k == at ? v : x.x, 2 * k + 1 == at ? v : x.y);
+              s[k] = pack2(2 * k == i ? v : x.x, 2 * k + 1 == i ? v : x.y);
             }
           }
           mt = -INFINITY;   // (what is not a number does not count: its weight is not a number either way)
@@ -408,40 +444,46 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
         pair_sync();
         l = half == 0 ? l + x_of(n, 1) : x_of(n, 0) + l;
       }
-      if (raw) m *= p.scale;
     }
 
+    float inv = 1.f;
+    float* dst;
     if (tp.splits > 1) {   // this CTA's partial, over the images (every product has read them)
       if (n > 0) asm volatile("bar.sync 1, 256;" ::: "memory");
       float* part = reinterpret_cast<float*>(smem_gen);
-      float* mine = part + lrow * C::kPartPitch + half * kCols;
+      dst = part + lrow * C::kPartPitch + half * kCols;
 #pragma unroll
       for (int i = 0; i < kCols; i += 4)
-        *reinterpret_cast<ulonglong2*>(mine + i) = make_ulonglong2(acc[i / 2], acc[i / 2 + 1]);
+        *reinterpret_cast<ulonglong2*>(dst + i) = make_ulonglong2(acc[i / 2], acc[i / 2 + 1]);
       if (half == 0) {
-        part[kRows * C::kPartPitch + lrow] = m;
+        part[kRows * C::kPartPitch + lrow] = raw ? m * p.scale : m;
         part[kRows * (C::kPartPitch + 1) + lrow] = l;
       }
     } else if (alive && row < p.seq_q) {
-      const float inv = l > 0.f ? 1.f / l : 0.f;
+      inv = l > 0.f ? 1.f / l : 0.f;
       const uint64_t inv2 = pack2(inv, inv);
-      float* o = static_cast<float*>(p.out) + b * p.os[0] + h * p.os[1] + row * p.os[2] + half * kCols;
+      dst = static_cast<float*>(p.out) + b * p.os[0] + h * p.os[1] + row * p.os[2] + half * kCols;
 #pragma unroll
       for (int i = 0; i < kCols; i += 4) {
         if (half * kCols + i >= D) continue;   // D is a multiple of 4
         const uint64_t x = mul2(acc[i / 2], inv2), y = mul2(acc[i / 2 + 1], inv2);
         if (tp.vec_out) {
-          *reinterpret_cast<ulonglong2*>(o + i) = make_ulonglong2(x, y);
+          *reinterpret_cast<ulonglong2*>(dst + i) = make_ulonglong2(x, y);
         } else {
           const float2 f = unpack2(x), g = unpack2(y);
-          o[i] = f.x;
-          o[i + 1] = f.y;
-          o[i + 2] = g.x;
-          o[i + 3] = g.y;
+          dst[i] = f.x;
+          dst[i + 1] = f.y;
+          dst[i + 2] = g.x;
+          dst[i + 3] = g.y;
         }
       }
-      if (p.lse && half == 0) p.lse[((int64_t)b * p.num_q_heads + h) * p.seq_q + row] = l > 0.f ? m + logf(l) : -INFINITY;
+      if (p.lse && half == 0) p.lse[((int64_t)b * p.num_q_heads + h) * p.seq_q + row] = l > 0.f ? (raw ? m * p.scale : m) + logf(l) : -INFINITY;
     }
+    uint64_t chk = 0;
+#pragma unroll
+    for (int i = 0; i < kCols / 2; ++i) chk = add2(chk, acc[i]);
+    // (a sum of weights that is not a number leaves nothing to save)
+    if (!(fabsf(sum2(chk)) < INFINITY) && l == l && alive && row < p.seq_q) exact_output(p, tp.splits, lrow, m, inv, half * kCols, kCols, dst);
   } else if (warp < (kWorkers + kLoaders) / 32) {
     ptx::setmaxnreg_dec<C::kRegRest>();
     // Blocks go in pieces of up to four chunks a thread, in the order K(0), V(0), K(1), ..., the next piece requested before the

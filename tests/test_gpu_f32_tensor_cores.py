@@ -128,6 +128,44 @@ def test_forward_logits_from_the_largest_floats(D, heads):
     assert (got - want).abs().max() <= 1e-5 * want.abs().max()
 
 
+@pytest.mark.parametrize("D", [32, 64, 80, 128])
+@pytest.mark.parametrize("heads", [2, 80])
+@pytest.mark.parametrize("variant", ["plain", "keep", "bias_softcap"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf"), 3.4e38])
+def test_forward_values_reach_the_rows_that_see_them(D, heads, variant, value):
+    """Under a causal mask with lengths, a value that is not finite, or above the largest bf16, in some columns of V: rows before
+    the key come out as if it were not there, and those that see it as float64 has them."""
+    B, Sq, Sk, offset = 2, 300, 330, 20
+    q, _ = gen((B, heads, Sq, D), "f32", 1, 1.0)
+    k, _ = gen((B, heads, Sk, D), "f32", 2, 1.0)
+    v, _ = gen((B, heads, Sk, D), "f32", 3, 1.0)
+    lens = torch.tensor([Sk, 290], dtype=torch.int32, device="cuda")
+    s = (q.double() @ k.double().transpose(-1, -2)) / np.sqrt(D)
+    key, row = torch.arange(Sk, device="cuda"), torch.arange(Sq, device="cuda")
+    seen = (key[None, None, None] <= row[None, None, :, None] + offset) & (key[None, None, None] < lens[:, None, None, None])
+    kw = {}
+    if variant == "keep":
+        keep = (torch.rand((1, 1, Sq, Sk), device="cuda", generator=torch.Generator("cuda").manual_seed(4)) < 0.9).to(torch.uint8)
+        keep[..., [5, 77, 190, 299]] = 1
+        kw, seen = dict(mask=keep, mask_kind=N.MASK_KEEP_U8), seen & (keep != 0)
+    elif variant == "bias_softcap":
+        bias = torch.randn((1, 1, Sq, Sk), device="cuda", generator=torch.Generator("cuda").manual_seed(4))
+        kw, s = dict(mask=bias, mask_kind=N.MASK_ADD_F32, softcap=20.0), 20 * torch.tanh(s / 20) + bias
+    w = torch.softmax(s.masked_fill(~seen, -torch.inf), -1)
+    clean = w @ v.double()
+    places = [(5, 0), (77, D - 1), (190, 9), (299, 17)]
+    for j, c in places:
+        v[:, :, j, c] = value
+    want = clean.clone()
+    for j, c in places:   # what the key adds (beside which its old value does not count), to the rows that see it
+        want[..., c] = torch.where(seen[..., j].expand(B, heads, Sq), clean[..., c] + w[..., j] * value, clean[..., c])
+    got, _, _ = run_gpu(q, k, v, dtype="f32", causal=True, bottom_right=False, causal_offset=offset, kv_len=lens, **kw)
+    for test in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(test(got), test(want.float()))
+    fin = torch.isfinite(want.float())
+    assert ((got - want).abs()[fin] <= 1e-5 * want.abs()[fin].clamp(min=2.0)).all()
+
+
 BWD_SHAPES = [(1, 4, 4, 320, 320, 64), (1, 4, 2, 321, 449, 64), (2, 30, 30, 400, 385, 64), (1, 2, 2, 513, 640, 32), (2, 12, 6, 511, 450, 36),
               (1, 8, 4, 390, 700, 20)]
 
