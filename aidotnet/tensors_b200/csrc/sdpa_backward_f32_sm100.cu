@@ -12,6 +12,9 @@
 //   warps 12-13 UMMA issuers (one elected lane each) of the scores and of the gradients; the first one owns TMEM
 // The scores of block j + 1 are formed while the row threads work on block j.  The gradient accumulators start afresh with every
 // block, so that the tensor cores, which truncate when they accumulate, never add more than four times into one cell.
+// An infinity times a term that is 0 is not a number, a value above the largest bf16 rounds to an infinity, and a block is multiplied
+// with rows that take no part with one another: a score that does not come out finite is formed again with multiply-adds, and so
+// is an element of a gradient that is not finite in the end.
 //
 // Launches with few tiles cut the walk over the CTAs of a cluster, which add their gradients in rank order through distributed
 // shared memory: every gradient is summed in a fixed order (deterministic, no atomics).
@@ -45,7 +48,7 @@ static_assert(smem_bytes(false) <= 227 * 1024, "shared memory");
 constexpr int kPartPitch = kDP + 4;   // floats per row of a CTA's partial gradient, over the images
 static_assert(2 * kOwn * kPartPitch * 4 <= kRowOff, "the partial gradients reuse the images");
 // TMEM columns: S, dP | terms of P | terms of dS | acc0 | acc1 (dV).  dQ and dV keep leading and small products apart; for dK
-// there are no columns left (its infinities come with an infinite Q, which makes S and with it dS not a number anyway).
+// there are no columns left.
 constexpr int kTS = 0, kTdP = 64, kTP = 128, kTdS = 224, kTAcc0 = 320, kTAcc1 = 384;
 
 struct BwdTcParams {
@@ -60,6 +63,88 @@ __device__ __noinline__ float dot_rows(const float* x, const float* u, int n) {
   return s;
 }
 
+// What a CTA works on: 128 own rows from own0 on, of which those before own_end take part, and n steps from s_begin on: blocks of
+// streamed rows [first, last), per_head of them for each query head from h0 on (hl0 within the shard).
+struct Place {
+  int b, hl0, h0, per_head, s_begin, n;
+  int64_t own0, own_end, kv_limit, first, last;
+};
+template <bool KEYS>
+__device__ __forceinline__ Place place_of(const SdpaParams& p, int splits) {
+  Place at;
+  at.b = blockIdx.z;
+  at.hl0 = KEYS ? blockIdx.y * p.group : blockIdx.y;
+  at.h0 = p.head_begin + at.hl0;
+  const int rank = (int)blockIdx.x % splits, tiles = (int)gridDim.x / splits, at_x = (int)blockIdx.x / splits;
+  // under a causal mask the last query rows and the first keys have the most to do: start them first
+  at.own0 = (int64_t)(!KEYS && p.causal ? tiles - 1 - at_x : at_x) * kOwn;
+  at.kv_limit = kv_limit_of(p, at.b);
+  // streamed rows [first, last) of one head that any of the CTA's own rows takes part with
+  at.first = 0;
+  at.last = KEYS ? p.seq_q : at.kv_limit;
+  if (p.causal) {
+    if constexpr (KEYS) {
+      at.first = at.own0 - p.causal_offset;              // query rows that see the CTA's first key
+      at.first = at.first > 0 ? at.first / kStr * kStr : 0;
+    } else {
+      int64_t last_row = at.own0 + kOwn - 1;
+      if (last_row > p.seq_q - 1) last_row = p.seq_q - 1;
+      if (last_row + p.causal_offset + 1 < at.last) at.last = last_row + p.causal_offset + 1;
+    }
+  }
+  if (KEYS && at.own0 >= at.kv_limit) at.last = 0;
+  at.own_end = KEYS ? at.kv_limit : p.seq_q;
+  at.per_head = at.last > at.first ? (int)((at.last - at.first + kStr - 1) / kStr) : 0;
+  const int64_t steps = (int64_t)at.per_head * (KEYS ? p.group : 1);
+  at.s_begin = (int)(rank * steps / splits);
+  at.n = (int)((rank + 1) * steps / splits) - at.s_begin;
+  return at;
+}
+
+// Columns col .. col + cols - 1 (at most 32) of `factor` times what the CTA's blocks add to the gradient of its own row `lrow` - dQ
+// or dK, or with of_v dV - in y where that is not finite: from the rows that take part with it.
+template <bool KEYS>
+__device__ __noinline__ void exact_gradient(const BwdParams& bp, int splits, int lrow, bool of_v, float factor, int col, int cols, float* y) {
+  const SdpaParams& p = bp.p;
+  const Place at = place_of<KEYS>(p, splits);   // (not handed over: the row loop would hold it in registers)
+  const int D = p.head_dim, kvh = at.h0 / p.group;
+  const int64_t own = at.own0 + lrow;
+  uint32_t bad = 0;
+  for (int e = 0; e < cols; ++e)
+    if (col + e < D && !(fabsf(y[e]) < INFINITY)) bad |= 1u << e;
+  float s[32];
+#pragma unroll
+  for (int e = 0; e < 32; ++e) s[e] = 0.f;
+  uint32_t open = own < at.own_end ? bad : 0;   // columns that are not NaN yet
+  for (int j = 0; j < at.n && open; ++j) {
+    const int g = KEYS ? (at.s_begin + j) / at.per_head : 0, h = at.h0 + g;
+    const int64_t base = at.first + (int64_t)(at.s_begin + j - g * at.per_head) * kStr;
+    const float* qb = static_cast<const float*>(p.q) + at.b * p.qs[0] + h * p.qs[1];
+    const float* gb = static_cast<const float*>(bp.dout) + at.b * bp.dos[0] + h * bp.dos[1];
+    const float* kb = static_cast<const float*>(p.k) + at.b * p.ks[0] + kvh * p.ks[1];
+    const float* vb = static_cast<const float*>(p.v) + at.b * p.vs[0] + kvh * p.vs[1];
+    for (int64_t r = base; r < base + kStr && r < at.last && open; ++r) {
+      const int64_t query = KEYS ? r : own, key = KEYS ? own : r;
+      if (p.causal && key > query + p.causal_offset) continue;
+      const float val = finish_logit(p, dot_rows(qb + query * p.qs[2], kb + key * p.ks[2], D) * p.scale, at.b, h, query, key, at.kv_limit);
+      const float lse = p.lse[((int64_t)at.b * p.num_q_heads + h) * p.seq_q + query];
+      float w = val == -INFINITY || lse == -INFINITY ? 0.f : ex2_approx((val - lse) * kLog2e);
+      if (!of_v)
+        w *= dot_rows(gb + query * bp.dos[2], vb + key * p.vs[2], D) - bp.delta[((int64_t)at.b * p.head_count + at.hl0 + g) * p.seq_q + query];
+      const float* u = (of_v ? gb + query * bp.dos[2] : (KEYS ? qb + query * p.qs[2] : kb + key * p.ks[2])) + col;
+#pragma unroll
+      for (int e = 0; e < 32; ++e) {
+        if (!(open & (1u << e))) continue;
+        s[e] = fmaf(w, u[e], s[e]);
+        if (s[e] != s[e]) open &= ~(1u << e);
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 32; ++e)
+    if (bad & (1u << e)) y[e] = s[e] * factor;
+}
+
 // One block's gradient (N column pairs of the thread's row) onto the registers; APART: small products kDP columns on.
 template <bool APART, int N>
 __device__ __forceinline__ void add_gradient(uint32_t t_acc, uint64_t (&acc)[N]) {
@@ -69,30 +154,21 @@ __device__ __forceinline__ void add_gradient(uint32_t t_acc, uint64_t (&acc)[N])
     tmem_ld16(t_acc + (uint32_t)c0, reinterpret_cast<uint32_t*>(hi));
     if (APART) tmem_ld16(t_acc + (uint32_t)(kDP + c0), reinterpret_cast<uint32_t*>(lo));
     ptx::tc_wait_ld();
-    if (APART) {
-      uint64_t chk = 0;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        lo[e] = add2(hi[e], lo[e]);
-        chk = add2(chk, lo[e]);
-      }
-      if (!(fabsf(sum2(chk)) < INFINITY)) {   // then the leading products alone say what the sum is
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float2 x = unpack2(hi[e]), y = unpack2(lo[e]);
-          lo[e] = pack2(fabsf(x.x) < INFINITY ? y.x : x.x, fabsf(x.y) < INFINITY ? y.y : x.y);
-        }
-      }
-      __syncwarp();
-    }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[c0 / 2 + e] = add2(acc[c0 / 2 + e], APART ? lo[e] : hi[e]);
+    for (int e = 0; e < 8; ++e) acc[c0 / 2 + e] = add2(acc[c0 / 2 + e], APART ? add2(hi[e], lo[e]) : hi[e]);
   }
+}
+template <int N>
+__device__ __forceinline__ bool all_finite(const uint64_t (&acc)[N]) {   // (or their sum is not)
+  uint64_t chk = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) chk = add2(chk, acc[i]);
+  return fabsf(sum2(chk)) < INFINITY;
 }
 
 // KS: k steps of 16 columns (2: head sizes up to 32).
 template <int KS, bool KEYS, bool PLAIN>
-__global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const BwdParams bp, const BwdTcParams tp) {
+__global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid_constant__ BwdParams bp, const BwdTcParams tp) {
   const SdpaParams& p = bp.p;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -103,32 +179,10 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const BwdPar
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int D = p.head_dim;
 
-  const int b = blockIdx.z;
-  const int kv_heads = p.head_count / p.group;
-  const int hl0 = KEYS ? blockIdx.y * p.group : blockIdx.y;    // (first) query head within the shard
-  const int h0 = p.head_begin + hl0, kvh = h0 / p.group;
-  const int rank = (int)blockIdx.x % tp.splits, tiles = (int)gridDim.x / tp.splits, at_x = (int)blockIdx.x / tp.splits;
-  // under a causal mask the last query rows and the first keys have the most to do: start them first
-  const int64_t own0 = (int64_t)(!KEYS && p.causal ? tiles - 1 - at_x : at_x) * kOwn;
-  const int64_t kv_limit = kv_limit_of(p, b);
-
-  // streamed rows [first, last) of one head that any of the CTA's own rows takes part with
-  int64_t first = 0, last = KEYS ? p.seq_q : kv_limit;
-  if (p.causal) {
-    if constexpr (KEYS) {
-      first = own0 - p.causal_offset;              // query rows that see the CTA's first key
-      first = first > 0 ? first / kStr * kStr : 0;
-    } else {
-      int64_t last_row = own0 + kOwn - 1;
-      if (last_row > p.seq_q - 1) last_row = p.seq_q - 1;
-      if (last_row + p.causal_offset + 1 < last) last = last_row + p.causal_offset + 1;
-    }
-  }
-  if (KEYS && own0 >= kv_limit) last = 0;
-  const int64_t own_end = KEYS ? kv_limit : p.seq_q;    // own rows past it take no part
-  const int per_head = last > first ? (int)((last - first + kStr - 1) / kStr) : 0;
-  const int64_t steps = (int64_t)per_head * (KEYS ? p.group : 1);
-  const int s_begin = (int)(rank * steps / tp.splits), n = (int)((rank + 1) * steps / tp.splits) - s_begin;
+  const Place at = place_of<KEYS>(p, tp.splits);
+  const int b = at.b, hl0 = at.hl0, h0 = at.h0, kvh = h0 / p.group, kv_heads = p.head_count / p.group, rank = (int)blockIdx.x % tp.splits;
+  const int per_head = at.per_head, s_begin = at.s_begin, n = at.n;
+  const int64_t own0 = at.own0, own_end = at.own_end, kv_limit = at.kv_limit, first = at.first, last = at.last;
 
   if (tid == 0) {
     *abort_flag = 0;
@@ -375,25 +429,33 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const BwdPar
     }
 
     const int64_t out_rows = KEYS ? p.seq_kv : p.seq_q;
+    const bool out_of_range = !all_finite(acc0) || (KEYS && !all_finite(acc1));
+    float *dst0, *dst1 = nullptr;
     if (tp.splits > 1) {   // this CTA's partial gradients, over the images (every product has read them)
       if (n > 0) asm volatile("bar.sync 1, 256;" ::: "memory");
-      float* mine = reinterpret_cast<float*>(smem_gen) + lrow * kPartPitch + half * kCols;
+      dst0 = reinterpret_cast<float*>(smem_gen) + lrow * kPartPitch + half * kCols;
+      dst1 = dst0 + kOwn * kPartPitch;
 #pragma unroll
       for (int c = 0; c < kCols; c += 4) {
-        *reinterpret_cast<ulonglong2*>(mine + c) = make_ulonglong2(acc0[c / 2], acc0[c / 2 + 1]);
-        if constexpr (KEYS) *reinterpret_cast<ulonglong2*>(mine + kOwn * kPartPitch + c) = make_ulonglong2(acc1[c / 2], acc1[c / 2 + 1]);
+        *reinterpret_cast<ulonglong2*>(dst0 + c) = make_ulonglong2(acc0[c / 2], acc0[c / 2 + 1]);
+        if constexpr (KEYS) *reinterpret_cast<ulonglong2*>(dst1 + c) = make_ulonglong2(acc1[c / 2], acc1[c / 2 + 1]);
       }
     } else if (alive && own < out_rows) {
       const int64_t base = KEYS ? ((int64_t)b * kv_heads + blockIdx.y) * out_rows : ((int64_t)b * p.head_count + hl0) * out_rows;
-      const int64_t at = (base + own) * D + half * kCols;
+      const int64_t to = (base + own) * D + half * kCols;
       const uint64_t scale2 = pack2(p.scale, p.scale);
-      float* out0 = (KEYS ? bp.dk : bp.dq) + at;
+      dst0 = (KEYS ? bp.dk : bp.dq) + to;
+      if constexpr (KEYS) dst1 = bp.dv + to;
 #pragma unroll
       for (int c = 0; c < kCols; c += 4) {
         if (half * kCols + c >= D) continue;   // D is a multiple of 4
-        *reinterpret_cast<ulonglong2*>(out0 + c) = make_ulonglong2(mul2(acc0[c / 2], scale2), mul2(acc0[c / 2 + 1], scale2));
-        if constexpr (KEYS) *reinterpret_cast<ulonglong2*>(bp.dv + at + c) = make_ulonglong2(acc1[c / 2], acc1[c / 2 + 1]);
+        *reinterpret_cast<ulonglong2*>(dst0 + c) = make_ulonglong2(mul2(acc0[c / 2], scale2), mul2(acc0[c / 2 + 1], scale2));
+        if constexpr (KEYS) *reinterpret_cast<ulonglong2*>(dst1 + c) = make_ulonglong2(acc1[c / 2], acc1[c / 2 + 1]);
       }
+    }
+    if (out_of_range && alive && own < out_rows) {
+      exact_gradient<KEYS>(bp, tp.splits, lrow, false, tp.splits > 1 ? 1.f : p.scale, half * kCols, kCols, dst0);
+      if constexpr (KEYS) exact_gradient<KEYS>(bp, tp.splits, lrow, true, 1.f, half * kCols, kCols, dst1);
     }
   } else if (warp < (kWorkers + kLoaders) / 32) {
     ptx::setmaxnreg_dec<104>();

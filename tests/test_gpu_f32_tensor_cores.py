@@ -200,3 +200,55 @@ def test_backward(shape, variant):
         assert np.abs(x - y).max() <= 16 * 2.0 ** -24 * np.sqrt(max(Sq, Sk, D)) * max(1.0, np.abs(y).max()), (name, np.abs(x - y).max())
     again = _fwd_bwd(q, k, v, g, dtype="f32", **kw)
     assert all(torch.equal(x, y) for x, y in zip(got, again))
+
+
+@pytest.mark.parametrize("D", [32, 64])
+@pytest.mark.parametrize("heads", [2, 30])
+@pytest.mark.parametrize("where", ["q", "k", "v", "dout"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf"), 3.4e38])
+def test_backward_values_reach_the_pairs_that_take_part(D, heads, where, value):
+    """Under a causal mask with lengths: the gradients of rows and keys that take no part with a row (of Q, dO) or a key (of K, V)
+    that holds something that is not finite, or above the largest bf16, are those without it."""
+    from tests.test_gpu_backward import _fwd_bwd
+    B, Sq, Sk, offset, row, key, col = 2, 400, 420, 10, 150, 160, 9
+    (q, qf), (k, kf), (v, vf), (g, gf) = [gen((B, heads, S, D), "f32", i + 1, 1.0) for i, S in enumerate([Sq, Sk, Sk, Sq])]
+    lens = np.array([Sk, 330], np.int32)
+    if where in ("q", "dout"):
+        gf = gf.copy()
+        gf[:, :, row] = 0                       # the row adds nothing
+    want = [x.astype(np.float64) for x in O.sdpa_backward(qf, kf, vf, gf, causal=True, causal_offset=offset, kv_len=lens)[:3]]
+    {"q": q, "k": k, "v": v, "dout": g}[where][:, :, row if where in ("q", "dout") else key, col] = value
+    got = [x.cpu().numpy() for x in _fwd_bwd(q, k, v, g, dtype="f32", causal=True, causal_offset=offset, kv_len=lens)]
+    if where in ("q", "dout"):
+        rows, keys = np.arange(Sq) != row, np.arange(Sk) > row + offset
+    else:
+        rows, keys = np.arange(Sq) + offset < key, np.arange(Sk) < 0
+    for x, y, name, part in zip(got, want, ("dQ", "dK", "dV"), (rows, keys, keys)):
+        x, y = x[:, :, part], y[:, :, part]
+        assert np.isfinite(x).all(), name
+        assert np.abs(x - y).max(initial=0) <= 16 * 2.0 ** -24 * np.sqrt(Sk) * max(1.0, np.abs(y).max(initial=0)), name
+    if where == "dout":                         # and in dV nothing but the value's column changes
+        dv, seen = got[2], np.arange(Sk) <= row + offset
+        other = np.delete(dv, col, axis=3)
+        assert np.isfinite(other).all()
+        if np.isfinite(value):
+            assert (dv[:, :, seen, col] > 1e30).all()
+        else:
+            assert (np.isnan(dv[:, :, seen, col]) if np.isnan(value) else dv[:, :, seen, col] == value).all()
+
+
+@pytest.mark.parametrize("D", [32, 64])
+@pytest.mark.parametrize("heads", [2, 30])
+def test_backward_infinite_value_in_v(D, heads):
+    """One infinity in V makes the row sums of dO * O infinite and with them dS of every other key: with positive Q and dO its dK is
+    -infinity, not NaN; dV does not know of it."""
+    from tests.test_gpu_backward import _fwd_bwd
+    B, S, key = 1, 350, 200
+    (q, qf), (k, kf), (v, vf), (g, gf) = [gen((B, heads, S, D), "f32", i + 1, 1.0) for i in range(4)]
+    q, g, qf, gf = q.abs(), g.abs(), np.abs(qf), np.abs(gf)
+    v[:, :, key, 5] = float("inf")
+    dq, dk, dv = _fwd_bwd(q, k, v, g, dtype="f32")
+    others = torch.arange(S, device="cuda") != key
+    assert torch.isneginf(dk[:, :, others]).all() and torch.isnan(dk[:, :, key]).all() and torch.isnan(dq).all()
+    want = O.sdpa_backward(qf, kf, vf, gf)[2]
+    assert np.abs(dv.cpu().numpy() - want).max() <= 16 * 2.0 ** -24 * np.sqrt(S) * np.abs(want).max()
