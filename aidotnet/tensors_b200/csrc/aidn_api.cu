@@ -819,7 +819,8 @@ int aidn_mha_forward(aidn_sdpa_t h, const aidn_mha_args* a, void* cu_stream) {
   const int64_t H = d.num_q_heads, D = d.head_dim, dm = H * D, S = a->seq, B = a->batch;
   const int cast_kind = d.qkv_dtype == AIDN_BF16 ? 0 : 1;
   const int64_t esz = (int64_t)elem_size(d.qkv_dtype);
-  // tcgen05 GEMMs for 16-bit arithmetic on head sizes 64 / 128; the fp32 FFMA GEMM for everything else
+  // tcgen05 GEMMs for 16-bit arithmetic on head sizes 64 / 128, and for fp32 from three bf16 terms where the width allows; the fp32
+  // FFMA GEMM for everything else
   const bool tensor_route = d.qkv_dtype != AIDN_F32 && (D == 64 || D == 128) && dm % 128 == 0 && d.path != AIDN_PATH_GENERIC;
   int launches = 0;
   cudaError_t e = cudaSuccess;
@@ -861,7 +862,7 @@ int aidn_mha_forward(aidn_sdpa_t h, const aidn_mha_args* a, void* cu_stream) {
       e = aidn::launch_proj_gemm_sm100(g, stream, h->num_sms, h->status_dev, &why, h->debug_mode == 3);
     } else {
       if (!aidn::proj_gemm_generic_supported(g, &why)) return fail(AIDN_EUNSUPPORTED, "mha: %s", why);
-      if (d.qkv_dtype == AIDN_F32 && aidn::proj_gemm_f32_sm100_supported(g))
+      if (d.qkv_dtype == AIDN_F32 && d.path != AIDN_PATH_GENERIC && aidn::proj_gemm_f32_sm100_supported(g))
         e = aidn::launch_proj_gemm_f32_sm100(g, stream, h->num_sms, h->status_dev, h->debug_mode == 3);
       else
         e = aidn::launch_proj_gemm_generic(g, d.qkv_dtype, stream);

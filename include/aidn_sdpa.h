@@ -81,7 +81,9 @@ typedef enum {
 } aidn_mask_kind;
 
 /* Kernel selection.  AUTO picks: split-KV decode when seq_q == 1, the tcgen05 prefill kernel for 16-bit
- * inputs with head_dim 64 or 128, the generic FFMA kernel otherwise.  The others force one kernel (tests). */
+ * inputs with head_dim 64 or 128, otherwise the fp32 kernels: products on the tensor cores from three bf16 terms per operand
+ * (fp32 inputs, calls that are large enough) or FFMA.  aidn_sdpa_last_path reports both as GENERIC.  The others force one
+ * kernel (tests); GENERIC keeps everything, backward and projections included, on FFMA. */
 typedef enum {
   AIDN_PATH_AUTO = 0,
   AIDN_PATH_GENERIC = 1,
@@ -289,9 +291,10 @@ AIDN_API int aidn_rope_interleaved(const float* input, const float* cosine, cons
  *   - 16-bit qkv_dtype, head_dim 64 or 128, heads*head_dim a multiple of 128: tcgen05 GEMMs and the tcgen05 attention
  *     kernel, fp32 accumulation.  fp32 inputs or weights are first rounded to the 16-bit type inside the workspace
  *     (pass 16-bit weights, converted once with aidn_cast_*, to skip that per call).
- *   - anything else (fp32 qkv_dtype, other head sizes or widths, desc.path == AIDN_PATH_GENERIC): FFMA GEMMs and the
- *     generic attention kernel in fp32 arithmetic; with an fp32 handle this meets the 1e-4 bound of the reference's own
- *     tests of the fused call (tests/AiDotNet.Tensors.Tests/Engines/MultiHeadAttentionForwardTests.cs:123).
+ *   - anything else (fp32 qkv_dtype, other head sizes or widths, desc.path == AIDN_PATH_GENERIC): GEMMs and attention to
+ *     fp32 accuracy, for an fp32 handle on the tensor cores from three bf16 terms per operand where the width is at least
+ *     256 (FFMA below that, and for desc.path == AIDN_PATH_GENERIC); with an fp32 handle this meets the 1e-4 bound of the reference's
+ *     own tests of the fused call (tests/AiDotNet.Tensors.Tests/Engines/MultiHeadAttentionForwardTests.cs:123).
  * The handle gives heads, head_dim and the mask kind (none or a keep-mask broadcastable to [B, H, S, S]; a fully masked
  * row gives zeros, CpuEngine.MultiHeadAttention.cs:481-485; a handle created with desc.causal = 1 additionally applies
  * the causal rule without a materialised mask - an extension, the reference expresses causality through the mask); it

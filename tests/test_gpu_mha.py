@@ -312,3 +312,32 @@ def test_mha_forward_bounded_waits_expire_cleanly():
     h.poll(stream)
     _check(out, O.mha_forward(xf, *wfs, heads), "call after a timed-out call")
     h.close()
+
+
+def test_mha_forward_fp32_path_generic_stays_on_multiply_adds():
+    """Two ways to an fp32 layer of width 256: by default the projections run on the tensor cores, with path GENERIC on multiply-adds.
+    The time-out hook tells them apart, for only the former have bounded waits that can run out."""
+    B, S, heads, d = 2, 300, 4, 64
+    Dm = heads * d
+    x, xf, ws, wfs = _inputs(B, S, heads, d, "f32", 5200)
+    want = O.mha_forward(xf, *wfs, heads)
+    stream = torch.cuda.current_stream().cuda_stream
+    for path in (N.PATH_AUTO, N.PATH_GENERIC):
+        out = torch.zeros((B, S, Dm), device="cuda")
+        h = N.Handle(device=0, qkv_dtype=N.F32, out_dtype=N.F32, head_dim=d, num_q_heads=heads, num_kv_heads=heads, path=path)
+        nb = h.mha_workspace_bytes(B, S, N.F32, N.F32)
+        wsb = torch.zeros(nb + 1024, dtype=torch.uint8, device="cuda")
+        call = lambda: h.mha_forward(input=x.data_ptr(), q_weight=ws[0].data_ptr(), k_weight=ws[1].data_ptr(), v_weight=ws[2].data_ptr(),
+                                     out_weight=ws[3].data_ptr(), out=out.data_ptr(), batch=B, seq=S, input_dtype=N.F32, weight_dtype=N.F32,
+                                     out_dtype=N.F32, workspace=_align(wsb.data_ptr()), workspace_bytes=nb, stream=stream)
+        h.debug_set(None, 3)
+        call()
+        if path == N.PATH_AUTO:
+            with pytest.raises(N.AidnError) as e:
+                h.poll(stream)
+            assert e.value.status == N.ETIMEOUT
+            h.debug_set(None, 0)
+            call()
+        h.poll(stream)
+        assert np.abs(out.cpu().numpy() - want).max() <= 1e-5 * np.abs(want).max(), path
+        h.close()
