@@ -123,6 +123,7 @@ namespace AiDotNet.Tensors.Engines.DirectGpu.CUDA
         [DllImport(Lib)] public static extern long aidn_mha_workspace_bytes(IntPtr handle, long batch, long seq, int inputDtype, int weightDtype);
         [DllImport(Lib)] public static extern int aidn_mha_forward(IntPtr handle, ref AidnMhaArgs args, IntPtr cuStream);
         [DllImport(Lib)] public static extern int aidn_qkv_rope_cache(ref AidnQkvRopeArgs args, IntPtr cuStream);
+        [DllImport(Lib)] public static extern int aidn_qkv_rope_poll(IntPtr cuStream);
         [DllImport(Lib)] public static extern int aidn_rope_interleaved(IntPtr input, IntPtr cosine, IntPtr sine, IntPtr output, long rows, int headDim, int seqLen, int startPosition, IntPtr cuStream);
         [DllImport(Lib)] public static extern int aidn_sdpa_poll(IntPtr handle, IntPtr cuStream);
         [DllImport(Lib)] public static extern int aidn_sdpa_last_path(IntPtr handle);

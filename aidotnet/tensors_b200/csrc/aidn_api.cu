@@ -17,6 +17,7 @@
 namespace {
 
 thread_local char g_err[512] = "";
+thread_local bool g_expire_qkv = false;   // test hook: this thread's next aidn_qkv_rope_cache lets its bounded waits run out
 
 int fail(int code, const char* fmt, ...) {
   va_list ap;
@@ -43,7 +44,8 @@ bool launch_check_enabled() {
   return on;
 }
 
-int post_launch_check(cudaStream_t stream, const char* what, int32_t* status_dev) {
+// `reset`: the status word has no handle whose poll would clear it, so that reporting it does.
+int post_launch_check(cudaStream_t stream, const char* what, int32_t* status_dev, bool reset = false) {
   if (!launch_check_enabled()) return AIDN_OK;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
@@ -56,6 +58,7 @@ int post_launch_check(cudaStream_t stream, const char* what, int32_t* status_dev
     int32_t st = 0;
     e = cudaMemcpy(&st, status_dev, sizeof(st), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return fail_cuda(e, "launch check: status read");
+    if (st && reset) cudaMemset(status_dev, 0, sizeof(st));
     if (st & aidn::kStatusTimeout) return fail(AIDN_ETIMEOUT, "[LAUNCH-FAULT] %s: a kernel gave up a bounded wait (status word 0x%x)", what, st);
   }
   return AIDN_OK;
@@ -292,7 +295,10 @@ int aidn_sdpa_last_launch_count(aidn_sdpa_t h) { return h ? h->last_launches : -
 
 // Test and development hook, declared in include/aidn_sdpa_debug.h.
 int aidn_sdpa_debug_set(aidn_sdpa_t h, float* buf, int mode) {
-  if (!h) return AIDN_EINVAL;
+  if (!h) {
+    g_expire_qkv = mode == 3;
+    return mode == 0 || mode == 3 ? AIDN_OK : AIDN_EINVAL;
+  }
   h->debug = buf;
   h->debug_mode = (buf || mode == 3) ? mode : 0;
   return AIDN_OK;
@@ -663,6 +669,8 @@ int aidn_sdpa_decode_noalloc(const aidn_sdpa_desc* desc, const aidn_sdpa_args* a
 
 int aidn_qkv_rope_cache(const aidn_qkv_rope_args* a, void* cu_stream) {
   g_err[0] = 0;
+  const bool expire = g_expire_qkv;
+  g_expire_qkv = false;
   if (!a) return fail(AIDN_EINVAL, "qkv_rope_cache: null argument");
   if (!a->input || !a->weights || !a->cosine || !a->sine || !a->query || !a->key_cache || !a->value_cache)
     return fail(AIDN_EINVAL, "qkv_rope_cache: null buffer");
@@ -712,9 +720,24 @@ int aidn_qkv_rope_cache(const aidn_qkv_rope_args* a, void* cu_stream) {
   p.position = a->position; p.query_dtype = a->query_dtype; p.cache_dtype = a->cache_dtype;
   p.cache_capacity = a->cache_capacity; p.max_position = a->max_position; p.model = (int32_t)model;
   int launches = 0;
-  e = aidn::launch_qkv_rope_cache(p, a->weight_dtype, sms, (cudaStream_t)cu_stream, &launches);
+  e = aidn::launch_qkv_rope_cache(p, a->weight_dtype, sms, (cudaStream_t)cu_stream, &launches, expire);
   if (e != cudaSuccess) return fail_cuda(e, "qkv_rope_cache");
-  return post_launch_check((cudaStream_t)cu_stream, "aidn_qkv_rope_cache", launch_check_enabled() ? aidn::qkv_rope_sm100_status() : nullptr);
+  const bool waits = launch_check_enabled() && aidn::qkv_rope_sm100_supported(p, a->weight_dtype);   // the kernel with bounded waits
+  return post_launch_check((cudaStream_t)cu_stream, "aidn_qkv_rope_cache", waits ? aidn::qkv_rope_sm100_status() : nullptr, true);
+}
+
+int aidn_qkv_rope_poll(void* cu_stream) {
+  g_err[0] = 0;
+  cudaError_t e = cudaStreamSynchronize((cudaStream_t)cu_stream);
+  if (e != cudaSuccess) return fail_cuda(e, "qkv_rope_poll: stream");
+  int32_t* status = aidn::qkv_rope_sm100_status();
+  if (!status) return fail(AIDN_ECUDA, "qkv_rope_poll: no status word in the current context");
+  int32_t st = 0;
+  e = cudaMemcpy(&st, status, sizeof(st), cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) return fail_cuda(e, "qkv_rope_poll: status read");
+  if (st == 0) return AIDN_OK;
+  cudaMemset(status, 0, sizeof(st));
+  return fail(AIDN_ETIMEOUT, "qkv_rope_poll: a kernel gave up a bounded wait (status word 0x%x)", st);
 }
 
 int aidn_rope_interleaved(const float* input, const float* cosine, const float* sine, float* output, int64_t rows,

@@ -310,11 +310,12 @@ struct QkvRopeParams {
 };
 
 int64_t qkv_rope_max_model();
+// expire: test hook - the tcgen05 kernel withholds its loads and its bounded waits give up after 20 ms.
 cudaError_t launch_qkv_rope_cache(const QkvRopeParams& p, int weight_dtype, int num_sms, cudaStream_t stream,
-                                  int* launches);
+                                  int* launches, bool expire = false);
 // Several tokens with bf16 weights on tcgen05 (csrc/qkv_rope_sm100.cu); launch_qkv_rope_cache hands it what it takes.
 bool qkv_rope_sm100_supported(const QkvRopeParams& p, int weight_dtype);
-cudaError_t launch_qkv_rope_sm100(const QkvRopeParams& p, int num_sms, cudaStream_t stream, int* launches);
+cudaError_t launch_qkv_rope_sm100(const QkvRopeParams& p, int num_sms, cudaStream_t stream, int* launches, bool expire);
 int32_t* qkv_rope_sm100_status();   // address of its status word in the current context, or null
 cudaError_t launch_rope_interleaved(const float* in, const float* cosc, const float* sinc, float* out, int64_t rows,
                                     int head_dim, int seq_len, int start_position, cudaStream_t stream);

@@ -256,8 +256,8 @@ cudaError_t launch_qkv_w(const QkvRopeParams& p, int num_sms, cudaStream_t strea
 int64_t qkv_rope_max_model() { return 1 << 20; }
 
 cudaError_t launch_qkv_rope_cache(const QkvRopeParams& p, int weight_dtype, int num_sms, cudaStream_t stream,
-                                  int* launches) {
-  if (qkv_rope_sm100_supported(p, weight_dtype)) return launch_qkv_rope_sm100(p, num_sms, stream, launches);
+                                  int* launches, bool expire) {
+  if (qkv_rope_sm100_supported(p, weight_dtype)) return launch_qkv_rope_sm100(p, num_sms, stream, launches, expire);
   if (weight_dtype == AIDN_F32) return launch_qkv_w<float>(p, num_sms, stream, launches);
   return launch_qkv_w<__nv_bfloat16>(p, num_sms, stream, launches);
 }

@@ -28,7 +28,7 @@ EXPORTS = (
     "aidn_sdpa_create", "aidn_sdpa_workspace_bytes", "aidn_sdpa_launch", "aidn_sdpa_poll", "aidn_sdpa_last_path",
     "aidn_sdpa_last_launch_count", "aidn_sdpa_destroy", "aidn_sdpa_last_error", "aidn_sdpa_device_supported",
     "aidn_cast_f32_to_bf16", "aidn_cast_f32_to_f16", "aidn_cast_bf16_to_f32", "aidn_cast_f16_to_f32",
-    "aidn_sdpa_decode_noalloc", "aidn_sdpa_launch_paged", "aidn_qkv_rope_cache", "aidn_rope_interleaved",
+    "aidn_sdpa_decode_noalloc", "aidn_sdpa_launch_paged", "aidn_qkv_rope_cache", "aidn_qkv_rope_poll", "aidn_rope_interleaved",
     "aidn_sdpa_backward", "aidn_sdpa_backward_workspace_bytes", "aidn_paged_kv_append", "aidn_mha_forward",
     "aidn_mha_workspace_bytes", "aidn_peer_export", "aidn_peer_open", "aidn_peer_close",
     "aidn_sdpa_debug_set",   # include/aidn_sdpa_debug.h
@@ -174,6 +174,8 @@ def load() -> ctypes.CDLL:
     lib.aidn_mha_forward.restype = ctypes.c_int
     lib.aidn_qkv_rope_cache.argtypes = [ctypes.POINTER(QkvRopeArgs), ctypes.c_void_p]
     lib.aidn_qkv_rope_cache.restype = ctypes.c_int
+    lib.aidn_qkv_rope_poll.argtypes = [ctypes.c_void_p]
+    lib.aidn_qkv_rope_poll.restype = ctypes.c_int
     lib.aidn_rope_interleaved.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64,
                                           ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p]
     lib.aidn_rope_interleaved.restype = ctypes.c_int
@@ -394,6 +396,11 @@ def qkv_rope_cache(*, input: int, weights: int, bias: Optional[int], cosine: int
         cache_capacity, max_position), stream)
     if status != OK:
         raise AidnError(status, last_error())
+
+
+def qkv_rope_poll(stream: int) -> None:
+    """Synchronises ``stream`` and raises if a projection of several tokens gave up a bounded wait since the last report."""
+    check(load().aidn_qkv_rope_poll(ctypes.c_void_p(stream)))
 
 
 def rope_interleaved(input: int, cosine: int, sine: int, output: int, rows: int, head_dim: int, seq_len: int,

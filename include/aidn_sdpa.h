@@ -64,7 +64,8 @@ typedef enum {
   AIDN_EUNSUPPORTED = 2, /* valid request that no kernel of this build serves               */
   AIDN_ECUDA = 3,        /* a CUDA call failed; aidn_sdpa_last_error() carries its message   */
   AIDN_EWORKSPACE = 4,   /* workspace missing or too small                                   */
-  AIDN_ETIMEOUT = 5,     /* a bounded device-side wait expired (reported by aidn_sdpa_poll)  */
+  AIDN_ETIMEOUT = 5,     /* a bounded device-side wait expired (reported by aidn_sdpa_poll,
+                            aidn_qkv_rope_poll)                                             */
   AIDN_ENCCL = 6         /* NCCL missing or an NCCL call failed                              */
 } aidn_status;
 
@@ -275,6 +276,10 @@ typedef struct {
   int64_t max_position;      /* rows of cosine / sine; a position outside them is left unrotated                */
 } aidn_qkv_rope_args;
 AIDN_API int aidn_qkv_rope_cache(const aidn_qkv_rope_args* args, void* cu_stream);
+/* Synchronises `cu_stream` and returns AIDN_ETIMEOUT if an aidn_qkv_rope_cache call of several tokens gave up a bounded wait since the
+ * last report (elements of the row tiles concerned are then NaN or were not stored), AIDN_ECUDA on a CUDA error, else AIDN_OK.  These calls
+ * have no handle: the word is one per CUDA context, and reporting it clears it.  For tests and diagnostics, as aidn_sdpa_poll. */
+AIDN_API int aidn_qkv_rope_poll(void* cu_stream);
 /* rope_interleaved (CUDA/Kernels/CudaAttentionKernels.cs:1023-1050; CudaBackend.RopeInterleaved): rows of head_dim
  * fp32 values, row r at position start_position + r % seq_len, pairs (2i, 2i+1) rotated by (cos, sin)[position][i]. */
 AIDN_API int aidn_rope_interleaved(const float* input, const float* cosine, const float* sine, float* output,

@@ -16,6 +16,8 @@ extern "C" {
  *         loads and every bounded device-side wait gives up after 20 ms instead of 2 s, so that a test can watch
  *         aidn_sdpa_poll report AIDN_ETIMEOUT and the next launch succeed — without any fault on the device.  `buf`
  *         is ignored.
+ *         With a null handle: the calling thread's next aidn_qkv_rope_cache does so, and aidn_qkv_rope_poll reports it
+ *         (mode 0 takes that back).
  * modes 1, 2 and 4 exist only in development builds of the library (compiled with -DAIDN_PREFILL_TRACE=1): value tap,
  *         per-work-item timeline and per-step clock stamps of the prefill kernel, written to `buf`.  The shipped build
  *         ignores them. */

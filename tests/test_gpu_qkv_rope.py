@@ -333,3 +333,70 @@ def test_infinite_activations_and_weights_of_several_tokens():
     got = q.cpu().numpy()
     assert np.isneginf(got[1, 9]) or np.isnan(got[1, 9])     # -inf through the rotation's 0 * x of the pair
     assert np.isfinite(np.delete(got[1:], [8, 9], axis=1)).all()
+
+
+_EXPIRE = '''
+import sys
+import numpy as np, torch
+from aidotnet.tensors_b200 import native as N
+check = sys.argv[1] == "1"
+torch.cuda.set_device(0)
+st = torch.cuda.current_stream().cuda_stream
+heads, kv, D, T, cap = 40, 8, 128, 16, 64
+model, rows = heads * D, (heads + 2 * kv) * D
+g = torch.Generator("cuda").manual_seed(1)
+x = torch.randn((T, model), device="cuda", generator=g)
+w = (torch.randn((rows, model), device="cuda", generator=g) / model ** 0.5).to(torch.bfloat16)
+cos, sin = torch.ones((cap, D // 2), device="cuda"), torch.zeros((cap, D // 2), device="cuda")
+q = torch.full((T, model), 7.0, device="cuda")
+kc, vc = (torch.full((cap, kv * D), 7.0, device="cuda") for _ in range(2))
+def call(tokens=T, weights=w, dtype=N.BF16):
+    N.qkv_rope_cache(input=x.data_ptr(), weights=weights.data_ptr(), bias=None, cosine=cos.data_ptr(), sine=sin.data_ptr(), query=q.data_ptr(),
+                     key_cache=kc.data_ptr(), value_cache=vc.data_ptr(), tokens=tokens, heads=heads, kv_heads=kv, head_dim=D, position=0,
+                     weight_dtype=dtype, cache_capacity=cap, max_position=cap, stream=st)
+def timed_out(f):
+    try:
+        f()
+    except N.AidnError as e:
+        assert e.status == N.ETIMEOUT, (e.status, e.message)
+        return True
+    return False
+arm = lambda: N.load().aidn_sdpa_debug_set(None, None, 3)
+poll = lambda: N.qkv_rope_poll(st)
+assert arm() == 0
+if check:
+    assert timed_out(call)             # by the call itself, which clears the word:
+    assert not timed_out(poll)
+else:
+    call()
+    call(tokens=1)                     # a kernel without such waits, between the failure and its report
+    torch.cuda.synchronize()
+    assert torch.equal(q[1:], torch.full_like(q[1:], 7.0)) and (kc[1:] == 7).all() and (vc[1:] == 7).all()
+    assert timed_out(poll)
+    assert not timed_out(poll)
+assert torch.equal(q[1:], torch.full_like(q[1:], 7.0)) and (kc[1:] == 7).all() and (vc[1:] == 7).all()   # nothing was stored
+assert not timed_out(call) and not timed_out(poll)
+want = x.double() @ w.double().T
+got = torch.cat([q.double(), kc[:T].double(), vc[:T].double()], 1)
+assert (got - want).abs().max() <= 1e-5 * want.abs().max()
+wf = w.float()
+assert not timed_out(lambda: call(tokens=2, weights=wf, dtype=N.F32)) and not timed_out(poll)
+print("expired cleanly")
+'''
+
+
+@pytest.mark.parametrize("launch_check", ["0", "1"])
+def test_several_tokens_bounded_waits_expire_cleanly(launch_check):
+    """Failure detection without a fault: with the test hook the producer withholds its loads and the waits (20 ms) run out.  No row is
+    stored, the failure is reported once - by the poll, or with AIDOTNET_KERNEL_LAUNCH_CHECK by the call itself - and calls after
+    it are correct and succeed."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, PYTHONPATH=root)
+    env.pop("AIDOTNET_KERNEL_LAUNCH_CHECK", None)
+    if launch_check == "1":
+        env["AIDOTNET_KERNEL_LAUNCH_CHECK"] = "1"
+    r = subprocess.run([sys.executable, "-c", _EXPIRE, launch_check], capture_output=True, text=True, timeout=300, env=env, cwd=root)
+    assert r.returncode == 0 and "expired cleanly" in r.stdout, f"stdout:\n{r.stdout}\nstderr:\n{r.stderr[-2000:]}"
