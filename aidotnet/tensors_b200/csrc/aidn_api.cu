@@ -372,6 +372,7 @@ int build_params(aidn_sdpa_t h, const aidn_sdpa_args* a, const aidn_paged_kv* pg
   p.softcap = d.softcap;
   p.status = h->status_dev;
   p.no_tcgen05 = d.path == AIDN_PATH_GENERIC ? 1 : 0;
+  p.expire = h->debug_mode == 3 ? 1 : 0;
   const int64_t D = d.head_dim;
   if (all_zero(a->q_stride)) dense_strides(p.qs, d.num_q_heads, a->seq_q, D);
   else std::memcpy(p.qs, a->q_stride, sizeof(p.qs));

@@ -52,6 +52,7 @@ struct SdpaParams {
   int32_t block_shift;  // log2(block_size) when it is a power of two, else -1
   int32_t num_blocks;   // > 0: entries are range-checked against it
   int32_t no_tcgen05;   // 1: stay on the FP32 units (desc.path == AIDN_PATH_GENERIC); fp32 attention only
+  int32_t expire;       // test hook of the fp32 tcgen05 kernel: nothing is loaded and every bounded wait gives up after 20 ms
 };
 
 template <typename T>

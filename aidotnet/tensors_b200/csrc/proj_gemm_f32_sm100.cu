@@ -217,7 +217,11 @@ __global__ void __launch_bounds__(kThreads, 1) proj_gemm_f32_sm100_kernel(const 
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag && tid == 0 && g.status) atomicOr(g.status, kStatusTimeout);
+  if (*abort_flag) {
+    abort_grace();
+    if (tid == 0 && g.status) atomicOr(g.status, kStatusTimeout);
+    __syncthreads();
+  }
   if (warp == kWorkers / 32) {
     tc_fence_after();
     tmem_dealloc(tmem_base, C::kTmemCols);

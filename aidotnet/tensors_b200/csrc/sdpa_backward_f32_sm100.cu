@@ -53,6 +53,7 @@ constexpr int kTS = 0, kTdP = 64, kTP = 128, kTdS = 224, kTAcc0 = 320, kTAcc1 = 
 
 struct BwdTcParams {
   int32_t splits;
+  int32_t withhold;   // test hook: the loaders load nothing, so that the bounded waits run out
   uint64_t wait_budget_ns;
 };
 
@@ -433,6 +434,13 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
     float *dst0, *dst1 = nullptr;
     if (tp.splits > 1) {   // this CTA's partial gradients, over the images (every product has read them)
       if (n > 0) asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (!alive) {   // the CTAs that add it up must not take it for a result
+#pragma unroll
+        for (int c = 0; c < kCols / 2; ++c) {
+          acc0[c] = pack2(NAN, NAN);
+          if constexpr (KEYS) acc1[c] = pack2(NAN, NAN);
+        }
+      }
       dst0 = reinterpret_cast<float*>(smem_gen) + lrow * kPartPitch + half * kCols;
       dst1 = dst0 + kOwn * kPartPitch;
 #pragma unroll
@@ -490,7 +498,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
       }
     };
     if (n > 0) load(0);
-    for (int j = 0; j < n; ++j) {
+    for (int j = 0; j < n && !tp.withhold; ++j) {
       if (j >= 2) wait(bar_g + 8 * (j & 1), (j - 2) >> 1);   // the gradients of block j - 2 have read the buffer
       if (!alive) break;
       const uint32_t u = u_s + (uint32_t)((j & 1) * 2 * kStrImage);
@@ -569,11 +577,15 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
   __syncwarp();
   ptx::tc_fence_before();
   __syncthreads();
+  if (*abort_flag) {
+    ptx::abort_grace();
+    if (tid == 0 && p.status) atomicOr(p.status, kStatusTimeout);
+    __syncthreads();
+  }
   if (warp == kIssuer) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, 512);
   }
-  if (*abort_flag && tid == 0 && p.status) atomicOr(p.status, kStatusTimeout);
   if (tp.splits > 1) {
     __syncwarp();
     cluster_sync_all();   // every CTA's partial is written
@@ -610,7 +622,8 @@ cudaError_t launch_one(const BwdParams& bp, cudaStream_t stream) {
   const int64_t rows = KEYS ? p.seq_kv : p.seq_q, heads = KEYS ? p.head_count / p.group : p.head_count;
   const int64_t tiles = (rows + kOwn - 1) / kOwn, steps = ((KEYS ? p.seq_q : p.seq_kv) + kStr - 1) / kStr * (KEYS ? p.group : 1);
   BwdTcParams tp;
-  tp.wait_budget_ns = ptx::kWaitBudgetNs;
+  tp.withhold = bp.expire;
+  tp.wait_budget_ns = bp.expire ? 20000000ull : ptx::kWaitBudgetNs;   // 20 ms in the time-out test
   tp.splits = 1;
   while (tp.splits < 8 && tiles * heads * p.batch * tp.splits * 2 <= 148 && tp.splits * 2 <= steps) tp.splits *= 2;
   cudaLaunchAttribute attr;

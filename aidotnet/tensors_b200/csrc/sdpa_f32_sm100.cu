@@ -70,6 +70,7 @@ struct TCfg {
 
 struct F32TcParams {
   int32_t splits, vec_out;
+  int32_t withhold;   // test hook: the loaders load nothing, so that the bounded waits run out
   uint64_t wait_budget_ns;
 };
 
@@ -450,6 +451,10 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
     float* dst;
     if (tp.splits > 1) {   // this CTA's partial, over the images (every product has read them)
       if (n > 0) asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (!alive) {   // the CTAs that merge it must not take it for a result
+#pragma unroll
+        for (int i = 0; i < kCols / 2; ++i) acc[i] = pack2(NAN, NAN);
+      }
       float* part = reinterpret_cast<float*>(smem_gen);
       dst = part + lrow * C::kPartPitch + half * kCols;
 #pragma unroll
@@ -523,7 +528,7 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
         split3::store_split8(image + split3::chunk_at(lt / CPR + (piece * kPiece + e) * kRowsAt, ch & 7), C::kKPlane, reg[e][0], reg[e][1]);
       if (piece == kPieces - 1) publish((is_v ? bar_v : bar_k) + 8 * slot);
     };
-    if (n > 0) {
+    if (n > 0 && !tp.withhold) {
       ulonglong2 even[kPiece][2], odd[kPiece][2];
       load(0, even);
       for (int q = 0; q < n * 2 * kPieces && alive; q += 2) {
@@ -592,11 +597,15 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
   __syncwarp();
   ptx::tc_fence_before();
   __syncthreads();
+  if (*abort_flag) {
+    ptx::abort_grace();
+    if (tid == 0 && p.status) atomicOr(p.status, kStatusTimeout);
+    __syncthreads();
+  }
   if (warp == kIssuer) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, 512);
   }
-  if (*abort_flag && tid == 0 && p.status) atomicOr(p.status, kStatusTimeout);
   if (tp.splits > 1) {
     __syncwarp();
     cluster_sync_all();   // every CTA's partial is written
@@ -704,7 +713,8 @@ cudaError_t launch_f32_sm100(const SdpaParams& p, cudaStream_t stream) {
   F32TcParams tp;
   tp.vec_out = reinterpret_cast<uintptr_t>(p.out) % 16 == 0;
   for (int i = 0; i < 3; ++i) tp.vec_out = tp.vec_out && p.os[i] % 4 == 0;
-  tp.wait_budget_ns = ptx::kWaitBudgetNs;
+  tp.withhold = p.expire;
+  tp.wait_budget_ns = p.expire ? 20000000ull : ptx::kWaitBudgetNs;   // 20 ms in the time-out test
   const int64_t tiles = (p.seq_q + kRows - 1) / kRows * p.head_count * p.batch, blocks = (p.seq_kv + kKeys - 1) / kKeys;
   tp.splits = 1;
   while (tp.splits < 8 && tiles * tp.splits * 2 <= 148 && tp.splits * 2 <= blocks) tp.splits *= 2;

@@ -97,6 +97,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return true;
 }
 
+// For a CTA whose waits gave up, before it releases tensor and shared memory: a bounded chance for what was already issued to complete.
+__device__ __forceinline__ void abort_grace() {
+  const uint64_t t0 = globaltimer_ns();
+  while (globaltimer_ns() - t0 < 2000000ull) {
+  }
+}
+
 // ---- TMA ------------------------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* tm) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tm)) : "memory");

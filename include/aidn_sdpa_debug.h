@@ -12,8 +12,8 @@ extern "C" {
 #endif
 
 /* mode 0: off.
- * mode 3: the TMA producers of the tcgen05 kernels of this handle (prefill, backward, projection GEMM) withhold their
- *         loads and every bounded device-side wait gives up after 20 ms instead of 2 s, so that a test can watch
+ * mode 3: the producers of the tcgen05 kernels of this handle (prefill, backward, projection GEMM, in 16 bits and in fp32)
+ *         withhold their loads and every bounded device-side wait gives up after 20 ms instead of 2 s, so that a test can watch
  *         aidn_sdpa_poll report AIDN_ETIMEOUT and the next launch succeed — without any fault on the device.  `buf`
  *         is ignored.
  *         With a null handle: the calling thread's next aidn_qkv_rope_cache does so, and aidn_qkv_rope_poll reports it

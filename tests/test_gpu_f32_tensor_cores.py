@@ -1,6 +1,6 @@
-"""fp32 attention from three bf16 terms (csrc/sdpa_f32_sm100.cu, sdpa_backward_f32_sm100.cu) where it can go wrong: one row or key
-more or less than a tile, every number of k steps, one to eight CTAs per tile, every mask kind, values that are not finite, and
-the line between these kernels and the register-tiled ones."""
+"""fp32 attention and projections from three bf16 terms (csrc/sdpa_f32_sm100.cu, sdpa_backward_f32_sm100.cu, proj_gemm_f32_sm100.cu) where
+they can go wrong: one row or key more or less than a tile, every number of k steps, one to eight CTAs per tile, every mask kind,
+values that are not finite, waits that run out, and the line between these kernels and the register-tiled ones."""
 import numpy as np
 import pytest
 import torch
@@ -252,3 +252,134 @@ def test_backward_infinite_value_in_v(D, heads):
     assert torch.isneginf(dk[:, :, others]).all() and torch.isnan(dk[:, :, key]).all() and torch.isnan(dq).all()
     want = O.sdpa_backward(qf, kf, vf, gf)[2]
     assert np.abs(dv.cpu().numpy() - want).max() <= 16 * 2.0 ** -24 * np.sqrt(S) * np.abs(want).max()
+
+
+def _times_out(h, launch):
+    """Whether the call runs on a tcgen05 kernel: with the time-out hook those load nothing, and their bounded waits (20 ms) run out,
+    which poll reports.  The same call without the hook then has to succeed."""
+    stream = torch.cuda.current_stream().cuda_stream
+    h.debug_set(None, 3)
+    launch()
+    try:
+        h.poll(stream)
+        expired = False
+    except N.AidnError as e:
+        assert e.status == N.ETIMEOUT
+        expired = True
+    h.debug_set(None, 0)
+    launch()
+    h.poll(stream)
+    return expired
+
+
+# (B, H, Sq, Sk, D, softcap, with log-sum-exp) and whether the call is large enough for the tcgen05 kernel
+ROUTES = [((1, 2, 16, 64, 64, 0.0, False), True), ((1, 2, 16, 63, 64, 0.0, False), False),
+          ((2, 80, 128, 64, 64, 0.0, False), True), ((2, 80, 128, 63, 64, 0.0, False), False),
+          ((1, 2, 16, 129, 128, 0.0, False), True), ((1, 2, 16, 128, 128, 0.0, False), False),
+          ((2, 80, 16, 128, 128, 0.0, False), True), ((2, 80, 16, 127, 128, 0.0, False), False),
+          ((1, 2, 16, 257, 128, 20.0, False), True), ((1, 2, 16, 256, 128, 20.0, False), False),
+          ((2, 80, 32, 128, 128, 20.0, False), True), ((2, 80, 32, 127, 128, 20.0, False), False),
+          ((1, 2, 16, 257, 32, 20.0, False), True), ((1, 2, 16, 256, 32, 20.0, False), False),
+          ((1, 2, 320, 320, 64, 0.0, True), True), ((1, 2, 320, 319, 64, 0.0, True), False), ((1, 2, 319, 320, 64, 0.0, True), False),
+          ((1, 2, 400, 400, 80, 0.0, True), False)]
+
+
+@pytest.mark.parametrize("call,tcgen05", ROUTES)
+@pytest.mark.parametrize("path", [N.PATH_AUTO, N.PATH_GENERIC])
+def test_forward_route_and_bounded_waits(call, tcgen05, path):
+    """Both sides of every line of the rule run where they should, path GENERIC on multiply-adds; and the tcgen05 kernel unwinds when its
+    waits run out: TMEM is given back, clusters part, and the next call on the handle is correct."""
+    B, H, Sq, Sk, D, softcap, want_lse = call
+    (q, qf), (k, kf), (v, vf) = [gen((B, H, S, D), "f32", i + 1, 1.0) for i, S in enumerate([Sq, Sk, Sk])]
+    out, lse = torch.zeros((B, H, Sq, D), device="cuda"), torch.zeros((B, H, Sq), device="cuda")
+    h = N.Handle(device=0, qkv_dtype=N.F32, head_dim=D, num_q_heads=H, num_kv_heads=H, softcap=softcap, emit_lse=want_lse, path=path)
+    launch = lambda: h.launch(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), out=out.data_ptr(), batch=B, seq_q=Sq, seq_kv=Sk,
+                              lse=lse.data_ptr() if want_lse else None, stream=torch.cuda.current_stream().cuda_stream)
+    assert _times_out(h, launch) == (tcgen05 and path == N.PATH_AUTO)
+    h.close()
+    compare(out, O.sdpa(qf, kf, vf, softcap=softcap), "f32", str(call))
+
+
+@pytest.mark.parametrize("shape,tcgen05", [((1, 2, 320, 320, 64), True), ((1, 40, 320, 321, 32), True), ((1, 2, 319, 320, 64), False),
+                                           ((1, 2, 320, 319, 64), False), ((1, 2, 400, 400, 68), False)])
+@pytest.mark.parametrize("path", [N.PATH_AUTO, N.PATH_GENERIC])
+def test_backward_route_and_bounded_waits(shape, tcgen05, path):
+    B, H, Sq, Sk, D = shape
+    (q, qf), (k, kf), (v, vf), (g, gf) = [gen((B, H, S, D), "f32", i + 1, 1.0) for i, S in enumerate([Sq, Sk, Sk, Sq])]
+    out, lse = torch.zeros((B, H, Sq, D), device="cuda"), torch.zeros((B, H, Sq), device="cuda")
+    grads = [torch.zeros_like(x) for x in (q, k, v)]
+    h = N.Handle(device=0, qkv_dtype=N.F32, head_dim=D, num_q_heads=H, num_kv_heads=H, emit_lse=True, path=path)
+    ws = torch.empty(h.backward_workspace_bytes(B, Sq), dtype=torch.uint8, device="cuda")
+    common = dict(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), out=out.data_ptr(), lse=lse.data_ptr(), batch=B, seq_q=Sq, seq_kv=Sk,
+                  stream=torch.cuda.current_stream().cuda_stream)
+    h.launch(**common)
+    launch = lambda: h.backward(dout=g.data_ptr(), dq=grads[0].data_ptr(), dk=grads[1].data_ptr(), dv=grads[2].data_ptr(),
+                                workspace=ws.data_ptr(), workspace_bytes=ws.numel(), **common)
+    assert _times_out(h, launch) == (tcgen05 and path == N.PATH_AUTO)
+    h.close()
+    for x, y, name in zip(grads, O.sdpa_backward(qf, kf, vf, gf)[:3], ("dQ", "dK", "dV")):
+        assert np.abs(x.cpu().numpy() - y).max() <= 16 * 2.0 ** -24 * np.sqrt(max(Sq, Sk, D)) * max(1.0, np.abs(y).max()), name
+
+
+def _layer(x, ws, heads, path=N.PATH_AUTO):
+    B, S, Dm = x.shape
+    out = torch.full((B, S, Dm), float("nan"), device="cuda")
+    h = N.Handle(device=0, qkv_dtype=N.F32, out_dtype=N.F32, head_dim=Dm // heads, num_q_heads=heads, num_kv_heads=heads, path=path)
+    nb = h.mha_workspace_bytes(B, S, N.F32, N.F32)
+    scratch = torch.zeros(nb + 1024, dtype=torch.uint8, device="cuda")
+    launch = lambda: h.mha_forward(input=x.data_ptr(), q_weight=ws[0].data_ptr(), k_weight=ws[1].data_ptr(), v_weight=ws[2].data_ptr(),
+                                   out_weight=ws[3].data_ptr(), out=out.data_ptr(), batch=B, seq=S, input_dtype=N.F32, weight_dtype=N.F32,
+                                   out_dtype=N.F32, workspace=(scratch.data_ptr() + 1023) // 1024 * 1024, workspace_bytes=nb,
+                                   stream=torch.cuda.current_stream().cuda_stream)
+    return h, launch, out
+
+
+@pytest.mark.parametrize("heads,d,tcgen05", [(4, 64, True), (3, 84, False), (5, 52, True), (6, 62, True), (3, 100, True), (7, 54, False), (9, 36, True)])
+@pytest.mark.parametrize("B,S", [(1, 1), (1, 127), (3, 43), (8, 197)])
+def test_projections(heads, d, tcgen05, B, S):
+    """Widths off the tiles of 64 or 128 columns and the K blocks of 64, head sizes that are not multiples of 4, rows on both sides of 128:
+    the layer against float64.  Every matrix adds 2^-24 x sqrt(width) x 4 of its largest element (three terms are exact to 2^-26 of a
+    product; four truncated additions a block), three of them in a row: 1e-5 of the largest output is above that at width 512."""
+    Dm = heads * d
+    x, xf = gen((B, S, Dm), "f32", 1, 1.0)
+    ws, wfs = zip(*[gen((Dm, Dm), "f32", 2 + i, Dm ** -0.5) for i in range(4)])
+    h, launch, out = _layer(x, ws, heads)
+    want = O.mha_forward(xf, *wfs, heads)
+    launch()
+    h.poll(torch.cuda.current_stream().cuda_stream)
+    assert np.abs(out.cpu().numpy() - want).max() <= 1e-5 * np.abs(want).max()
+    if S == 1:   # (one key: the attention itself is too small for a tcgen05 kernel)
+        assert _times_out(h, launch) == tcgen05
+    h.close()
+
+
+@pytest.mark.parametrize("heads,d,S", [(4, 64, 130), (5, 52, 130), (16, 32, 1000)])
+def test_projections_of_values_that_are_not_finite(heads, d, S):
+    """In the output weight, in columns of their own: an infinity gives infinities of the sign of what it meets, NaN gives NaN, a value
+    above the largest bf16 a finite sum, and no other column changes.  A row of NaN in one sequence leaves the others alone."""
+    B, Dm = 2, heads * d
+    x, xf = gen((B, S, Dm), "f32", 1, 1.0)
+    ws, wfs = zip(*[gen((Dm, Dm), "f32", 2 + i, Dm ** -0.5) for i in range(4)])
+    _, launch, attended = _layer(x, [*ws[:3], torch.eye(Dm, device="cuda")], heads)
+    launch()
+    torch.cuda.synchronize()
+    w = ws[3].clone()
+    for c, value in ((0, float("inf")), (Dm // 2 + 1, float("-inf")), (77, float("nan")), (Dm - 1, 3.4e38)):
+        w[c // 2, c] = value
+    _, launch, out = _layer(x, [*ws[:3], w], heads)
+    launch()
+    torch.cuda.synchronize()
+    want = attended.double() @ w.double()
+    for test in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(test(out), test(want.float()))
+    fin = torch.isfinite(want)
+    fin[..., Dm - 1] = False
+    assert (out - want)[fin].abs().max() <= 1e-5 * want[fin].abs().max()
+    assert (out - want)[..., Dm - 1].abs().max() <= 1e-5 * want[..., Dm - 1].abs().max()
+    y = x.clone()
+    y[1, S // 2] = float("nan")
+    _, launch, out = _layer(y, ws, heads)
+    launch()
+    torch.cuda.synchronize()
+    ref = O.mha_forward(xf[:1], *wfs, heads)
+    assert np.abs(out[:1].cpu().numpy() - ref).max() <= 1e-5 * np.abs(ref).max() and torch.isnan(out[1]).all()
