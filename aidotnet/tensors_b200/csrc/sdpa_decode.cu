@@ -939,40 +939,62 @@ bool decode_supported(int dtype, int head_dim) {
 }
 
 // Clusters save the merge kernel and its trip through L2, and cut each sequence by its own length; but CTAs that wait for one
-// another hold their place, so they pay only while all of a launch's CTAs are resident at once.  Measured, us, chunks with a
-// merge kernel / clusters of (n), bf16 unless stated: 32 heads of 64, 1237 keys 9.8 / 6.5 (8), 8192 keys 22 / 19 (8);
-// 32/8 heads of 128, 1000 keys 7.8 / 6.1 (8); B8 8/8 x 1024 13.6 / 9.0 (4), 12.7 (8); B20 4/2 x 700 8.9 / 7.2 (4), 10.4 (8);
-// B12 8/8 x 2000 19.0 / 20.2 (2), B3 32/32 x 900 13.0 / 12.5 (2); B16 32/8 x 2048 27.5 / 26.4 (2); B8 32/32 x 300 15.6 / 12.8 (2);
-// B40 32/8 x 1000 30.7 / 32.0 (2).  Where eight CTAs would walk many keys each, several clusters and the merge kernel: 64/8
-// heads of 128, 16384 keys 35 / 29 (8) / 20.8 (4 x 8); 8/2 30 / 12.7 (8 x 8).  fp32 on the FP32 units needs more CTAs:
-// 32 heads of 64, 1237 keys 13.8 / 11.4 (8), 6000 keys 29.6 / 38.7 (8) / 27.1 (2 x 8); 128 wide 3000 keys 21.6 / 22.1 (4 x 8).
+// another hold their place, so they pay only while all of a launch's CTAs are resident at once, and while a CTA's keys do not last
+// longer than chunks would that keep every SM busy to the end.  Measured with 200 to 16384 keys, and with lengths from 1 / 16 of the keys
+// to all of them; us, chunks with a merge kernel / clusters of (n), bf16 heads of 128 unless stated:
+//   * Clusters of 8 are all resident up to 0.89 of the places (heads of 64, three CTAs an SM: 0.86, not at 0.88), of 4 up to 0.93, of 2 up
+//     to all; then the largest that is.  500 keys: 33 items 7.9 / 7.4 (8), 34 items 8.2 / 10.4 (8) / 7.3 (4); 69 items 14.3 / 8.8 (4),
+//     74 items 14.4 / 13.5 (4) / 9.6 (2); heads of 64, 49 items, 305 keys 6.6 / 8.5 (8).
+//   * Keys of a CTA: 28 items, 16384 keys 55 / 42 (8); 50 items, 8192 keys 48 / 41 (4), with lengths 32 / 36; heads of 64, 56 items,
+//     4096 keys 16.2 / 15.5 (4) at 1024 a CTA, 8192 keys 31 / 34, 3000 keys with lengths 12.4 / 13.2; 103 items, 7254 keys 41 / 33 (4);
+//     48 items, 7733 keys 29 / 21 (8).
+//   * Several clusters of 8 and the merge kernel where one would have more than 400 keys a CTA: 4 items of heads of 64, 4096 keys
+//     8.3 / 8.5 (2 x 8) / 7.9 (8 x 8); 2 items, 16384 keys 30 / 12.7 (8 x 8).
+//   * Two CTAs each, at most one wave: 128 items, 2048 keys 37 / 29, with lengths 23.3 / 22.9; 80 items, 2048 keys 27.6 / 23.8, with
+//     lengths 19.2 / 21.5.  Two waves pay where the second is nearly full: 256 items, 2048 keys 55 / 51, with lengths 36.2 / 37.5;
+//     180 items 44.6 / 49.2, 500 keys 20.4 / 20.4; 149 items, 500 keys 23.2 / 17.6.
+//   * fp32 on the FP32 units is bound by them, not by bytes, and chunks spread better (heads of 64): 4 items, 700 keys 6.9 / 6.6 (8),
+//     2000 keys 8.1 / 11.7 (8) / 7.9 (8 x 8), 8000 keys 13.6 / 12.3 (8 x 8); 32 items, 2000 keys 16.6 / 15.0 (8), 4000 keys 22.5 / 25.4 (8) /
+//     20.2 (2 x 8); 64 items, 8000 keys 53 / 53 (8), 4000 keys 33.6 / 29.2; 74 items are not all resident: 8000 keys 59 / 94 (8); 22 items,
+//     4786 keys 21 / 19 (3 x 8); of four heads: 43 items, 3402 keys 39 / 50 (8), 2 items, 695 keys 10.2 / 11.3, 10 items, 464 keys 10.4 / 9.6.
+//     Few items with 1000 to 1280 keys lose 0.1 to 1.4 us of 7 to 8 on the GPU; the second launch would cost the host of a token more.
+// 1100 shapes drawn from 1 to 300 items and 150 to 16384 keys: 0.83 of the chunks' time for 16-bit tensors, 0.91 for fp32, and more than
+// 8 % above it in 12 of them (clusters without these limits: 0.86, 0.95 and 111, the longest 1.6 times the chunks' time).
 void decode_plan_clusters(const SdpaParams& p, int dtype, int num_sms, DecodePlan* plan) {
-  const bool ring = takes_ring(p, dtype);
+  const bool ring = takes_ring(p, dtype), lengths = p.kv_len != nullptr, wide = p.head_dim == 128;
   if (!ring && (dtype != AIDN_F32 || p.group > 8)) return;
   const int64_t items = (int64_t)p.batch * (p.head_count / p.group), keys = p.seq_kv;
-  const int64_t room = (ring ? (p.head_dim == 128 ? 2 : 3) : 4) * (int64_t)num_sms;   // CTAs that are resident at once
-  const int64_t parts = room / items;
-  int cluster = 1;
-  int64_t clusters = 1;
-  if (parts >= 8) {
-    if (!ring && p.head_dim == 128 && keys > 512) return;
-    cluster = 8;
-    clusters = keys / 8 / (ring ? 256 : 80);
-    if (!ring && clusters >= 5) clusters = 8;   // 4 heads of 64, 4000 keys: 10.2 us with six clusters, 9.0 with eight
-    if (clusters > parts / 8) clusters = parts / 8;
-    if (clusters > plan->nchunks) clusters = plan->nchunks;
-    if (clusters < 1) clusters = 1;
-  } else if (!ring) {
-    return;
-  } else if (parts >= 4) {
-    cluster = 4;
-  } else if (parts == 3) {
-    cluster = keys <= 1024 ? 2 : 1;
-  } else if (parts >= 1) {
-    cluster = keys <= 2048 ? 2 : 1;
+  const int64_t room = (ring ? (wide ? 2 : 3) : 4) * (int64_t)num_sms;   // CTAs that are resident at once
+  int64_t cluster = 1, clusters = 1;
+  if (!ring) {
+    const int64_t eights = (wide ? room : room * 94 / 100) / (8 * items);   // clusters of 8 per item
+    const int64_t little = p.group == 1 ? (lengths ? 768 : 1280) : 480, some = (lengths ? 28 : 80) * items / p.group;
+    if (eights < 1) return;
+    if (wide ? keys <= 512 : (keys <= little || keys <= some || (items >= 60 * p.group && !lengths))) cluster = 8;
+    else if (wide) return;
+    else if (eights >= 8) { if (keys >= 3200) cluster = clusters = 8; }
+    else if (!lengths && eights >= 2 && keys >= 1600 && (eights >= 4 || keys <= 8192)) cluster = 8, clusters = eights;
+  } else {
+    const int64_t eights = room * (wide ? 90 : 87) / 100 / (8 * items), fours = room * 95 / 100 / (4 * items);
+    int64_t most = lengths ? (wide ? 1024 : 700) : (wide || 40 * items >= 3 * room ? 2048 : 1300);   // keys of a CTA
+    if (eights >= 1) {
+      if ((eights >= 8 && keys > 3072) || (eights >= 4 && keys > 3500) || keys > (lengths ? 5600 : 5000)) clusters = eights >= 8 ? 8 : (eights > 4 ? 4 : eights);
+      if (clusters > plan->nchunks) clusters = plan->nchunks;
+      if (clusters > 1 && lengths) most = wide ? 768 : 384;
+      if (keys <= 8 * clusters * most) cluster = 8;
+    } else if (fours >= 1) {
+      if (!lengths) most = 20 * items >= 3 * room ? 4096 : (wide ? 2048 : 1024);   // (three places in five are taken)
+      if (keys <= 4 * most) cluster = 4;
+    } else if (2 * items <= room) {
+      if (keys <= (lengths && 8 * items < 3 * room ? 1024 : 2048)) cluster = 2;
+    } else if (items <= room) {
+      if (4 * items >= 3 * room) { if (keys <= (lengths ? 1024 : 2048)) cluster = 2; }
+      else if (keys <= 512 && (!lengths || 5 * items < 3 * room)) cluster = 2;
+    }
   }
   if (cluster == 1) return;
-  plan->cluster = cluster;
+  if (clusters > plan->nchunks) clusters = plan->nchunks;   // never more workspace
+  plan->cluster = (int)cluster;
   plan->nchunks = (int)clusters;
 }
 

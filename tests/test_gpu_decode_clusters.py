@@ -60,3 +60,23 @@ def test_clusters_keep_non_finite_values(dtype, D, Sk, value):
     assert info["launches"] == (2 if Sk == 5000 else 1) and info1["launches"] == 1
     assert torch.isnan(one[1, 3, 0, 7])
     assert torch.equal(torch.isnan(split), torch.isnan(one))
+
+
+# (B, Hq, Hkv, D, dtype): keys on either side of a line of the plan, and the launches there (one: a cluster; two: a merge kernel)
+LINES = [((33, 4, 1, 128, "bf16"), 3000, 1, 17000, 2), ((34, 2, 1, 128, "bf16"), 4000, 1, 8200, 2), ((50, 1, 1, 64, "bf16"), 4000, 1, 4200, 2),
+         ((100, 1, 1, 128, "f16"), 2048, 1, 2049, 2), ((160, 1, 1, 128, "bf16"), 512, 1, 520, 2), ((8, 1, 1, 64, "f32"), 1280, 1, 1300, 2),
+         ((74, 1, 1, 64, "f32"), 64, 1, 200, 2), ((6, 4, 1, 64, "f32"), 480, 1, 500, 2)]
+
+
+@pytest.mark.parametrize("heads,below,launches_below,above,launches_above", LINES)
+def test_plan_lines(heads, below, launches_below, above, launches_above):
+    """Where clusters stop being faster than chunks with a merge kernel, both sides against float64."""
+    B, Hq, Hkv, D, dtype = heads
+    scale = 1.0 if dtype == "f32" else 0.5
+    for Sk, launches in ((below, launches_below), (above, launches_above)):
+        q, qf = gen((B, Hq, 1, D), dtype, 1, scale)
+        k, kf = gen((B, Hkv, Sk, D), dtype, 2, scale)
+        v, vf = gen((B, Hkv, Sk, D), dtype, 3, scale)
+        out, _, info = run_gpu(q, k, v, dtype=dtype, path=N.PATH_DECODE)
+        assert info["launches"] == launches, (heads, Sk)
+        compare(out, O.sdpa(qf, kf, vf), dtype, f"{heads} {Sk}")
