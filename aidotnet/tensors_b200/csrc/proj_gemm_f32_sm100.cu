@@ -217,12 +217,9 @@ __global__ void __launch_bounds__(kThreads, 1) proj_gemm_f32_sm100_kernel(const 
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag) {
-    abort_grace();
-    if (tid == 0 && g.status) atomicOr(g.status, kStatusTimeout);
-    __syncthreads();
-  }
-  if (warp == kWorkers / 32) {
+  if (*abort_flag && tid == 0 && g.status) atomicOr(g.status, kStatusTimeout);
+  if (warp == kWorkers / 32) {   // (shared memory stays until this warp ends; a barrier for all in a branch of its own costs 0.4 us a launch)
+    if (*abort_flag) abort_grace();
     tc_fence_after();
     tmem_dealloc(tmem_base, C::kTmemCols);
   }
