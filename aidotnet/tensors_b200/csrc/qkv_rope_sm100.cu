@@ -19,8 +19,8 @@
 // distributed shared memory in rank order: no scratch memory, no atomics, the same bits every time.
 //
 // Hq32 / Hkv8 D128 (50 MB of weights, 7.8 us at the copy bandwidth), against one mma.sync pass per eight tokens:
-// 16 tokens 35.5 -> 15.1 us, 2 tokens 19.0 -> 13.9, 64 tokens 133 -> 33; Hq64 / Hkv8 D128 (168 MB) with 16 tokens 255 -> 32.
-// Error of fp32 outputs against 64 bits 2.5e-6 -> 1.3e-7 (3.2e-7 with 64 tokens).  What is left is the latency of set-up, first
+// 16 tokens 35.5 -> 15.5 us, 2 tokens 19.0 -> 14.2, 64 tokens 133 -> 33.4; Hq64 / Hkv8 D128 (168 MB) with 16 tokens 255 -> 33.
+// Error of fp32 outputs against 64 bits 2.5e-6 -> 1.3e-7 (3.2e-7 with 64 tokens, Hq64 2.6e-7 to 4.2e-7).  What is left is the latency of set-up, first
 // bytes and finish (a launch over 3 MB of weights takes 5 us).
 #include <cuda.h>
 
@@ -345,8 +345,8 @@ QkvTcPlan plan_of(int tokens, int tiles, int k_blocks, int num_sms) {
   pl.tmem_cols = 128;
   while (pl.tmem_cols < (2 + kAccs) * pl.tpad) pl.tmem_cols *= 2;
   const int resident = pl.tpad <= 16 ? 3 : (pl.tpad <= 32 ? 2 : 1);   // CTAs per SM, by shared memory
-  // As many CTAs as are resident at once hide one another's latencies (with four splitting warps: 16 tokens, 48 tiles of 64
-  // K blocks 18.0 us with 3 splits, 15.8 with 4, 13.3 with 8); a second wave costs as much as the first (80 tiles of 128: 5 splits = 400 CTAs 30.6 us,
+  // As many CTAs as are resident at once hide one another's latencies (measured with four splitting warps, whose times are not those
+  // above: 16 tokens, 48 tiles of 64 K blocks 18.0 us with 3 splits, 15.8 with 4, 13.3 with 8); a second wave costs as much as the first (80 tiles of 128: 5 splits = 400 CTAs 30.6 us,
   // 6 = 480 CTAs 41), and clusters of three or more do not pack the SMs to the last one (48 tiles with 64 tokens, one CTA per
   // SM: 2 splits 37 us, 3 splits = 144 CTAs 53).
   pl.splits = 1;

@@ -1,6 +1,8 @@
-// fp32 operands on the 16-bit tensor cores: x = t0 + t1 + t2 with bf16 terms (8 significant bits each, round to nearest), exact
-// to 2^-27 of x.  A product of two such operands is the sum of the six products of terms whose weights together are at least
-// 2^-16 of the whole; the ones left out are below 2^-26 of it.  bf16 products are exact in fp32, so what remains is the rounding of
+// fp32 operands on the 16-bit tensor cores: x = t0 + t1 + t2 with bf16 terms (8 significant bits each, round to nearest), which is
+// exact where bf16's exponents reach: of an x below 2^-110 (7.7e-34) the bits under bf16's smallest number, 2^-133, are lost; above the
+// largest bf16 (3.39e38) t0 is an infinity, as for an infinity, and the kernels form such sums again with multiply-adds.  A product of
+// two operands is the sum of the six products of terms whose weights together are at least 2^-16 of the whole; the ones left out are
+// below 2^-26 of it.  bf16 products are exact in fp32, so what remains is the rounding of
 // the accumulation, and for that the leading products t0 * t0 are summed apart from the small ones where it matters.
 #pragma once
 
