@@ -778,7 +778,7 @@ int aidn_paged_kv_append(const void* new_keys, const void* new_values, void* key
 // ---- fused multi-head attention forward ---------------------------------------------------------------------------
 namespace {
 struct MhaPlan {
-  int64_t off_x, off_w, off_q, off_k, off_v, off_o, total;
+  int64_t off_x, off_w, off_q, off_k, off_v, off_o, off_t[2], total;   // off_t: terms of the fp32 weights, Q / K / V and output
 };
 MhaPlan mha_plan(const aidn_sdpa* h, int64_t batch, int64_t seq, int input_dtype, int weight_dtype) {
   const int64_t dm = (int64_t)h->d.num_q_heads * h->d.head_dim;
@@ -792,6 +792,11 @@ MhaPlan mha_plan(const aidn_sdpa* h, int64_t batch, int64_t seq, int input_dtype
   pl.off_k = off; off += act;
   pl.off_v = off; off += act;
   pl.off_o = off; off += act;
+  for (int i = 0; i < 2; ++i) {
+    pl.off_t[i] = off;
+    if (h->d.qkv_dtype == AIDN_F32 && h->d.path != AIDN_PATH_GENERIC && aidn::proj_gemm_f32_sm100_fits(dm, dm))
+      off += align_up(aidn::proj_gemm_f32_sm100_bytes(batch * seq, dm, dm, i == 0 ? 3 : 1, h->num_sms), 1024);
+  }
   pl.total = off;
   return pl;
 }
@@ -880,13 +885,36 @@ int aidn_mha_forward(aidn_sdpa_t h, const aidn_mha_args* a, void* cu_stream) {
   for (int i = 0; i < 3; ++i) g.w[i] = w[i];
   g.c[0] = ws + pl.off_q; g.c[1] = ws + pl.off_k; g.c[2] = ws + pl.off_v;
   g.c_stride[0] = H * S * D; g.c_stride[1] = S * D; g.c_stride[2] = D;    // [B, H, S, d]
-  auto gemm = [&](const char* what) -> int {
+  aidn::ProjGemm go = g;
+  go.a = ws + pl.off_o;
+  go.num_mats = 1;
+  go.w[0] = w[3];
+  go.c[0] = a->out;
+  go.out_f32 = a->out_dtype == AIDN_F32;
+  go.c_stride[0] = S * dm; go.c_stride[1] = D; go.c_stride[2] = dm;
+  bool f32_sm100[2] = {false, false};   // projections of Q, K and V, and of the output
+  if (d.qkv_dtype == AIDN_F32 && d.path != AIDN_PATH_GENERIC) {
+    f32_sm100[0] = aidn::proj_gemm_f32_sm100_supported(g);
+    f32_sm100[1] = aidn::proj_gemm_f32_sm100_supported(go);
+    aidn::ProjGemm split[2];
+    int count = 0;
+    g.image = ws + pl.off_t[0];
+    go.image = ws + pl.off_t[1];
+    if (f32_sm100[0] && pl.off_t[1] > pl.off_t[0]) split[count++] = g;
+    if (f32_sm100[1] && pl.total > pl.off_t[1]) split[count++] = go;
+    if (count > 0) {
+      e = aidn::launch_proj_split_f32(split, count, stream, h->num_sms);
+      if (e != cudaSuccess) return fail_cuda(e, "mha: terms of the weights");
+      ++launches;
+    }
+  }
+  auto gemm = [&](const aidn::ProjGemm& g, bool f32_sm100, const char* what) -> int {
     if (tensor_route) {
       if (!aidn::proj_gemm_sm100_supported(g, &why)) return fail(AIDN_EUNSUPPORTED, "mha: %s", why);
       e = aidn::launch_proj_gemm_sm100(g, stream, h->num_sms, h->status_dev, &why, h->debug_mode == 3);
     } else {
       if (!aidn::proj_gemm_generic_supported(g, &why)) return fail(AIDN_EUNSUPPORTED, "mha: %s", why);
-      if (d.qkv_dtype == AIDN_F32 && d.path != AIDN_PATH_GENERIC && aidn::proj_gemm_f32_sm100_supported(g))
+      if (f32_sm100)
         e = aidn::launch_proj_gemm_f32_sm100(g, stream, h->num_sms, h->status_dev, h->debug_mode == 3);
       else
         e = aidn::launch_proj_gemm_generic(g, d.qkv_dtype, stream);
@@ -895,7 +923,7 @@ int aidn_mha_forward(aidn_sdpa_t h, const aidn_mha_args* a, void* cu_stream) {
     ++launches;
     return AIDN_OK;
   };
-  rc = gemm("mha: QKV projection");
+  rc = gemm(g, f32_sm100[0], "mha: QKV projection");
   if (rc != AIDN_OK) return rc;
 
   aidn_sdpa_args sa;
@@ -910,13 +938,7 @@ int aidn_mha_forward(aidn_sdpa_t h, const aidn_mha_args* a, void* cu_stream) {
   if (rc != AIDN_OK) return rc;
   launches += h->last_launches;
 
-  g.a = ws + pl.off_o;
-  g.num_mats = 1;
-  g.w[0] = w[3];
-  g.c[0] = a->out;
-  g.out_f32 = a->out_dtype == AIDN_F32;
-  g.c_stride[0] = S * dm; g.c_stride[1] = D; g.c_stride[2] = dm;
-  rc = gemm("mha: output projection");
+  rc = gemm(go, f32_sm100[1], "mha: output projection");
   if (rc != AIDN_OK) return rc;
   h->last_launches = launches;
   return post_launch_check(stream, "aidn_mha_forward", h->status_dev);

@@ -237,6 +237,13 @@ __device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr, uint32_t rank) {
   asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(remote) : "memory");
   return v;
 }
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
+  uint32_t remote;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+  return v;
+}
 
 // Host-side launchers (one per kernel family); each returns the CUDA error of its launch.
 cudaError_t launch_generic(const SdpaParams& p, int dtype, cudaStream_t stream);
@@ -359,13 +366,19 @@ struct ProjGemm {
   int32_t head_dim;
   bool out_f32;         // fp32 output, else the input dtype
   bool bf16;            // bf16 inputs, else fp16
+  void* image;          // the terms of w (proj_gemm_f32_sm100 only)
 };
 bool proj_gemm_sm100_supported(const ProjGemm& g, const char** why);
 // expire: test hook - the producer withholds its loads and every bounded wait gives up after 20 ms.
 cudaError_t launch_proj_gemm_sm100(const ProjGemm& g, cudaStream_t stream, int num_sms, int32_t* status,
                                    const char** why, bool expire = false);
-// fp32 operands with 16-byte rows, every one as three bf16 terms on tcgen05 (csrc/proj_gemm_f32_sm100.cu).
+// fp32 operands with 16-byte rows, every one as three bf16 terms on tcgen05 (csrc/proj_gemm_f32_sm100.cu).  launch_proj_split_f32
+// writes the terms of the weights of one or two GEMMs to their `image`, of proj_gemm_f32_sm100_bytes bytes each, for the GEMMs
+// behind it on the stream; where that is 0 (few rows) a GEMM cuts its weights itself.
+bool proj_gemm_f32_sm100_fits(int64_t k, int64_t n);
 bool proj_gemm_f32_sm100_supported(const ProjGemm& g);
+int64_t proj_gemm_f32_sm100_bytes(int64_t rows, int64_t k, int64_t n, int mats, int num_sms);
+cudaError_t launch_proj_split_f32(const ProjGemm* gemms, int count, cudaStream_t stream, int num_sms);
 cudaError_t launch_proj_gemm_f32_sm100(const ProjGemm& g, cudaStream_t stream, int num_sms, int32_t* status, bool expire = false);
 // The same contract in fp32 FFMA arithmetic for any sizes and for a / w of `dtype` (csrc/proj_gemm_generic.cu).
 bool proj_gemm_generic_supported(const ProjGemm& g, const char** why);

@@ -353,6 +353,38 @@ def test_projections(heads, d, tcgen05, B, S):
     h.close()
 
 
+@pytest.mark.parametrize("B,S,heads,d", [(1, 100, 20, 20), (1, 127, 25, 40), (1, 1, 241, 4), (2, 70, 32, 64), (27, 19, 17, 32), (8, 125, 20, 38), (13, 100, 20, 40),
+                                         (4, 100, 32, 64), (7, 100, 8, 109), (5, 77, 16, 48), (8, 250, 41, 20), (8, 250, 11, 40), (3, 100, 137, 8), (12, 50, 20, 54),
+                                         (8, 250, 37, 8)])
+def test_projection_plans(B, S, heads, d):
+    """Every tile width (32 to 160 columns), weights cut in place and by a launch of their own, K over 1, 2, 4 and 8 CTAs of a cluster, widths and
+    K off the tiles: the layer against float64, and the same bits again.  Bound: test_projections' 2^-24 x sqrt(width) x 4 a matrix."""
+    Dm = heads * d
+    x, xf = gen((B, S, Dm), "f32", 1, 1.0)
+    ws, wfs = zip(*[gen((Dm, Dm), "f32", 2 + i, Dm ** -0.5) for i in range(4)])
+    h, launch, out = _layer(x, ws, heads)
+    want = O.mha_forward(xf, *wfs, heads)
+    launch()
+    first = out.clone()
+    out.fill_(float("nan"))
+    launch()
+    h.poll(torch.cuda.current_stream().cuda_stream)
+    assert np.abs(first.cpu().numpy() - want).max() <= 12 * 2.0 ** -24 * Dm ** 0.5 * np.abs(want).max()
+    assert torch.equal(first, out)
+    # a cluster's merge, too, stores nothing that an expired wait left behind, and the next call is whole again
+    out.fill_(7.0)
+    h.debug_set(None, 3)
+    launch()
+    with pytest.raises(N.AidnError):
+        h.poll(torch.cuda.current_stream().cuda_stream)
+    assert (out == 7.0).all()
+    h.debug_set(None, 0)
+    launch()
+    h.poll(torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(first, out)
+    h.close()
+
+
 @pytest.mark.parametrize("heads,d,S", [(4, 64, 130), (5, 52, 130), (16, 32, 1000)])
 def test_projections_of_values_that_are_not_finite(heads, d, S):
     """In the output weight, in columns of their own: an infinity gives infinities of the sign of what it meets, NaN gives NaN, a value
