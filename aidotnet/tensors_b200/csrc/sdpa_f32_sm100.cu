@@ -170,11 +170,6 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int D = p.head_dim;
 
-  const Place at = place_of(p, tp.splits);
-  const int b = at.b, h = at.h, kvh = h / p.group, rank = (int)blockIdx.x % tp.splits, n = at.n;
-  const int64_t row0 = at.row0, kv_limit = at.kv_limit, blk0 = at.blk0;
-  const int64_t kend = visible_end(p, kv_limit, row0 + kRows < p.seq_q ? row0 + kRows - 1 : p.seq_q - 1);
-
   if (tid == 0) {
     *abort_flag = 0;
     for (int i = 0; i < 2; ++i) {
@@ -196,6 +191,12 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_wait();   // the set-up above runs under the end of the launch before
+  pdl_trigger();
+  const Place at = place_of(p, tp.splits);
+  const int b = at.b, h = at.h, kvh = h / p.group, rank = (int)blockIdx.x % tp.splits, n = at.n;
+  const int64_t row0 = at.row0, kv_limit = at.kv_limit, blk0 = at.blk0;
+  const int64_t kend = visible_end(p, kv_limit, row0 + kRows < p.seq_q ? row0 + kRows - 1 : p.seq_q - 1);
   const uint32_t q_s = smem_base, k_s = smem_base + C::kKOff, v_s = smem_base + C::kVOff;
 
   bool alive = true;
@@ -663,20 +664,8 @@ cudaError_t launch_t(const SdpaParams& p, F32TcParams tp, cudaStream_t stream) {
   auto kern = sdpa_f32_sm100_kernel<DP, KS, MODE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TCfg<DP, KS, MODE>::kSmem);
   if (e != cudaSuccess) return e;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)tp.splits;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((p.seq_q + kRows - 1) / kRows * tp.splits), (unsigned)p.head_count, (unsigned)p.batch);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = TCfg<DP, KS, MODE>::kSmem;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = tp.splits > 1 ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, kern, p, tp);
-  if (e != cudaSuccess) cudaGetLastError();   // reported here: the next launch must not find it as its own
-  return e;
+  return launch_dependent_cluster(kern, dim3((unsigned)((p.seq_q + kRows - 1) / kRows * tp.splits), (unsigned)p.head_count, (unsigned)p.batch), kThreads,
+                                  dim3((unsigned)tp.splits), TCfg<DP, KS, MODE>::kSmem, stream, p, tp);
 }
 
 template <int DP, int KS>
