@@ -117,11 +117,11 @@ cudaError_t launch_cast(int kind, const void* src, void* dst, int64_t n, cudaStr
 // per block crossed); here one kernel scatters all rows of K and V with 16-byte copies.  Block bookkeeping (free list,
 // reference counts, copy-on-write) stays with the caller.
 namespace {
-__global__ void __launch_bounds__(256) paged_append_kernel(const uint4* __restrict__ src_k, const uint4* __restrict__ src_v,
-                                                           uint4* __restrict__ pool_k, uint4* __restrict__ pool_v,
-                                                           const int32_t* __restrict__ block_table, int64_t start,
-                                                           int64_t tokens, int block_size, int num_blocks, int row_vecs) {
+__global__ void __launch_bounds__(256) paged_append_kernel(const uint4* src_k, const uint4* src_v, uint4* pool_k, uint4* pool_v,
+                                                           const int32_t* block_table, int64_t start, int64_t tokens, int block_size, int num_blocks, int row_vecs) {
   const int64_t total = tokens * row_vecs;
+  pdl_wait();
+  pdl_trigger();
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t t = idx / row_vecs;
     const int vec = (int)(idx - t * row_vecs);
@@ -129,8 +129,9 @@ __global__ void __launch_bounds__(256) paged_append_kernel(const uint4* __restri
     const int32_t blk = block_table[pos / block_size];
     if (blk < 0 || blk >= num_blocks) continue;   // an entry outside the pool is skipped, not written through
     const int64_t row = (int64_t)blk * block_size + pos % block_size;
-    pool_k[row * row_vecs + vec] = src_k[idx];
-    pool_v[row * row_vecs + vec] = src_v[idx];
+    const uint4 k = src_k[idx], v = src_v[idx];   // both loads before the first store, which might lie over them for all the compiler knows
+    pool_k[row * row_vecs + vec] = k;
+    pool_v[row * row_vecs + vec] = v;
   }
 }
 }  // namespace
@@ -143,10 +144,9 @@ cudaError_t launch_paged_append(const void* src_k, const void* src_v, void* pool
   const int64_t total = tokens * row_vecs;
   const int64_t blocks = (total + 255) / 256;
   const unsigned grid = (unsigned)(blocks < 148 * 16 ? blocks : 148 * 16);
-  paged_append_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint4*>(src_k), static_cast<const uint4*>(src_v),
-                                                static_cast<uint4*>(pool_k), static_cast<uint4*>(pool_v), block_table,
-                                                start, tokens, block_size, num_blocks, row_vecs);
-  return cudaGetLastError();
+  return launch_dependent(paged_append_kernel, grid, 256, 0, stream, static_cast<const uint4*>(src_k), static_cast<const uint4*>(src_v),
+                          static_cast<uint4*>(pool_k), static_cast<uint4*>(pool_v), block_table, start, tokens, block_size, num_blocks,
+                          row_vecs);
 }
 
 }  // namespace aidn

@@ -37,6 +37,8 @@ __global__ void __launch_bounds__(128) bwd_delta_kernel(const BwdParams bp) {
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   const int hl = blockIdx.y, b = blockIdx.z;
+  pdl_wait();
+  pdl_trigger();
   if (row >= p.seq_q) return;
   const int h = p.head_begin + hl;
   const int64_t ob = b * p.os[0] + (int64_t)h * p.os[1] + row * p.os[2];
@@ -69,6 +71,8 @@ __global__ void __launch_bounds__(128) bwd_delta_vec_kernel(const BwdParams bp) 
   const int hl = blockIdx.y, b = blockIdx.z, h = p.head_begin + hl;
   const TO* ob = static_cast<const TO*>(p.out) + b * p.os[0] + (int64_t)h * p.os[1] + d;
   const TO* gb = static_cast<const TO*>(bp.dout) + b * bp.dos[0] + (int64_t)h * bp.dos[1] + d;
+  pdl_wait();
+  pdl_trigger();
   uint4 o[kSteps], g[kSteps];
 #pragma unroll
   for (int s = 0; s < kSteps; ++s) {
@@ -110,9 +114,7 @@ template <typename TO, typename TT>
 cudaError_t launch_delta_vec(const BwdParams& bp, cudaStream_t stream) {
   const int rows = 4 * 4 * 32 * 16 / (bp.p.head_dim * (int)sizeof(TO));   // rows per CTA
   const dim3 grid((unsigned)((bp.p.seq_q + rows - 1) / rows), (unsigned)bp.p.head_count, (unsigned)bp.p.batch);
-  if (bp.p.head_dim == 64) bwd_delta_vec_kernel<TO, TT, 64><<<grid, 128, 0, stream>>>(bp);
-  else bwd_delta_vec_kernel<TO, TT, 128><<<grid, 128, 0, stream>>>(bp);
-  return cudaGetLastError();
+  return launch_dependent(bp.p.head_dim == 64 ? bwd_delta_vec_kernel<TO, TT, 64> : bwd_delta_vec_kernel<TO, TT, 128>, grid, 128, 0, stream, bp);
 }
 
 template <typename T>
@@ -130,8 +132,7 @@ cudaError_t launch_delta(const BwdParams& bp, cudaStream_t stream) {
     return launch_delta_vec<float, T>(bp, stream);
   }
   const dim3 grid((unsigned)((p.seq_q + 3) / 4), (unsigned)p.head_count, (unsigned)p.batch);
-  bwd_delta_kernel<T><<<grid, 128, 0, stream>>>(bp);
-  return cudaGetLastError();
+  return launch_dependent(bwd_delta_kernel<T>, grid, 128, 0, stream, bp);
 }
 
 // Probability and score gradient of (row, key): p = exp(logit - lse), ds = p * (dp - delta).

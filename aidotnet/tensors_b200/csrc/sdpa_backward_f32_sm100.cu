@@ -168,6 +168,9 @@ __device__ __forceinline__ bool all_finite(const uint64_t (&acc)[N]) {   // (or 
 }
 
 // KS: k steps of 16 columns (2: head sizes up to 32).
+// dQ waits for the kernel that formed delta.  dK / dV, which follows on the stream, needs nothing of dQ: it starts when all of dQ's CTAs
+// have begun - by then every launch before dQ is complete - and takes the SMs that dQ leaves idle; it ends only after dQ has, so that
+// what comes next on the stream may rely on both.
 template <int KS, bool KEYS, bool PLAIN>
 __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid_constant__ BwdParams bp, const BwdTcParams tp) {
   const SdpaParams& p = bp.p;
@@ -179,11 +182,6 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int D = p.head_dim;
-
-  const Place at = place_of<KEYS>(p, tp.splits);
-  const int b = at.b, hl0 = at.hl0, h0 = at.h0, kvh = h0 / p.group, kv_heads = p.head_count / p.group, rank = (int)blockIdx.x % tp.splits;
-  const int per_head = at.per_head, s_begin = at.s_begin, n = at.n;
-  const int64_t own0 = at.own0, own_end = at.own_end, kv_limit = at.kv_limit, first = at.first, last = at.last;
 
   if (tid == 0) {
     *abort_flag = 0;
@@ -205,6 +203,12 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  if (!KEYS) pdl_wait();   // (dK / dV: at its end)
+  pdl_trigger();
+  const Place at = place_of<KEYS>(p, tp.splits);
+  const int b = at.b, hl0 = at.hl0, h0 = at.h0, kvh = h0 / p.group, kv_heads = p.head_count / p.group, rank = (int)blockIdx.x % tp.splits;
+  const int per_head = at.per_head, s_begin = at.s_begin, n = at.n;
+  const int64_t own0 = at.own0, own_end = at.own_end, kv_limit = at.kv_limit, first = at.first, last = at.last;
   const uint32_t x_s = smem_base, y_s = smem_base + kYOff, u_s = smem_base + kUOff;   // buffer i: U at u_s + 2 i images, W behind it
 
   const float* kb = static_cast<const float*>(p.k) + b * p.ks[0] + (int64_t)kvh * p.ks[1];
@@ -611,6 +615,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
     __syncwarp();
     cluster_sync_all();   // nobody reads this CTA's shared memory any more
   }
+  if (KEYS) pdl_wait();
 }
 
 template <int KS, bool KEYS, bool PLAIN>
@@ -626,20 +631,8 @@ cudaError_t launch_one(const BwdParams& bp, cudaStream_t stream) {
   tp.wait_budget_ns = bp.expire ? 20000000ull : ptx::kWaitBudgetNs;   // 20 ms in the time-out test
   tp.splits = 1;
   while (tp.splits < 8 && tiles * heads * p.batch * tp.splits * 2 <= 148 && tp.splits * 2 <= steps) tp.splits *= 2;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)tp.splits;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(tiles * tp.splits), (unsigned)heads, (unsigned)p.batch);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem_bytes(PLAIN);
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = tp.splits > 1 ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, kern, bp, tp);
-  if (e != cudaSuccess) cudaGetLastError();   // reported here: the next launch must not find it as its own
-  return e;
+  return launch_dependent_cluster(kern, dim3((unsigned)(tiles * tp.splits), (unsigned)heads, (unsigned)p.batch), kThreads, dim3((unsigned)tp.splits),
+                                  smem_bytes(PLAIN), stream, bp, tp);
 }
 
 template <int KS>

@@ -133,6 +133,9 @@ __device__ __forceinline__ int step_head(const Work& w, int j) { return KEYS ? w
 template <bool KEYS>
 __device__ __forceinline__ int step_tile(const Work& w, int j) { return KEYS ? w.first + j % w.count : j; }
 
+// dQ waits for the kernel that formed delta.  dK / dV, which follows on the stream, needs nothing of dQ: it starts when all of dQ's CTAs
+// have begun - by then every launch before dQ is complete - and takes the SMs that dQ leaves idle; it ends only after dQ has, so that
+// what comes next on the stream may rely on both.
 template <typename T, int HD, bool KEYS, bool MASKED>
 __global__ void __launch_bounds__(kThreads, 1)
     sdpa_backward_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -188,6 +191,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  if (!KEYS) pdl_wait();   // (dK / dV: at its end)
+  pdl_trigger();
 
   // Persistent CTAs: CTA k takes items k, 2G-1-k, 2G+k, ... (G = grid size; the item list is ordered heaviest first, and
   // the snake keeps the sum per CTA even).  Counters that persist across items give every barrier its phase:
@@ -555,6 +560,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
   }
+  if (KEYS) pdl_wait();
 }
 
 bool aligned_bhs(const void* base, const int64_t* stride, int64_t H, int64_t B, int align) {
@@ -611,13 +617,11 @@ cudaError_t launch_t(const BwdParams& bp, cudaStream_t stream, int* launches, co
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess || sms <= 0) { *why = "cannot read the SM count"; return e != cudaSuccess ? e : cudaErrorInvalidValue; }
   sp.total_items = (int)items_q;
-  kq<<<(unsigned)(items_q < sms ? items_q : sms), kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, tdo, sp);
-  e = cudaGetLastError();
+  e = launch_dependent(kq, dim3((unsigned)(items_q < sms ? items_q : sms)), kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo, sp);
   if (e != cudaSuccess) return e;
   sp.total_items = (int)items_kv;
-  kkv<<<(unsigned)(items_kv < sms ? items_kv : sms), kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, tdo, sp);
   *launches += 2;
-  return cudaGetLastError();
+  return launch_dependent(kkv, dim3((unsigned)(items_kv < sms ? items_kv : sms)), kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo, sp);
 }
 
 }  // namespace
