@@ -32,6 +32,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "mask_tile.cuh"
 #include "ffma2.cuh"
 #include "sm100_ptx.cuh"
 #include "tensor_map.hpp"
@@ -46,7 +47,7 @@ constexpr int kThreads = 320;     // producer, issuer, 2 x 4 row warps
 constexpr int kTmemCols = 512;
 constexpr float kLog2e = 1.4426950408889634f;
 
-template <int HD>
+template <int HD, bool TILES>
 struct BCfg {
   static constexpr int kTileBytes = kT * HD * 2;
   static constexpr int kHalfBytes = kT * 128;          // one 64-column block of a tile
@@ -54,7 +55,7 @@ struct BCfg {
   static constexpr int kRing = HD == 128 ? 2 : 4;      // streamed (U, W) pairs in flight
   static constexpr int kRingOff = 2 * kTileBytes;
   static constexpr int kVecOff = kRingOff + kRing * 2 * kTileBytes;   // per-warp lse / delta rows: 8 warps x 2 x 2 x 64 floats
-  static constexpr int kVecBytes = 8 * 2 * 2 * 64 * 4;
+  static constexpr int kVecBytes = TILES ? 8 * masktile::kBytes : 8 * 2 * 2 * 64 * 4;   // or the row warps' mask tiles
   static constexpr int kBarOff = kVecOff + kVecBytes;
   static constexpr int kNumBars = 8 + 2 * kRing;       // xy_full acc_full s_full[2] p_full[2] xy_empty acc_empty ring_full[R] ring_empty[R]
   static constexpr int kMiscOff = kBarOff + kNumBars * 8;
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     sdpa_backward_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                                const BwdSm100Params bp) {
-  using C = BCfg<HD>;
+  using C = BCfg<HD, MASKED && !KEYS>;
   constexpr bool kBf16 = !std::is_same_v<T, __half>;
   const SdpaParams& p = bp.p;
 
@@ -352,7 +353,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t t_s = tmem_base + lane_bits + (uint32_t)(half * 128), t_dp = t_s + 64u;
     const float sl2 = p.scale * kLog2e;
     const uint64_t sl2_2 = pack2(sl2, sl2);
-    float* my_vec = vec_smem + (warp - 2) * (2 * 2 * 64);   // [buffer][-lse*log2e, -delta][64]
+    float* my_vec = vec_smem + (warp - 2) * (2 * 2 * 64);   // KEYS: [buffer][-lse*log2e, -delta][64]
+    const uint32_t my_mask = smem_base + (uint32_t)(C::kVecOff + (warp - 2) * masktile::kBytes);   // dQ with a bias
     uint32_t g = 0, live = 0;
     bool alive = true;
     for (int wave = 0; wave < waves && alive; ++wave) {
@@ -368,13 +370,50 @@ __global__ void __launch_bounds__(kThreads, 1)
         my_nl = (lse == -INFINITY || lse == INFINITY) ? -INFINITY : -lse * kLog2e;
         my_nd = -bp.delta[((int64_t)w.b * p.head_count + (w.h - p.head_begin)) * p.seq_q + my_row];
       }
+      // The explicit mask, a step ahead; lanes take keys.  Rows are queries (dQ): bits of the row's 64 keys, or a bias of the first 32 in
+      // shared memory and of the other 32 in registers.  Rows are keys: the lane's own, bits of 64 queries or a bias of the first 32.
+      const bool add = MASKED && p.mask_kind == AIDN_MASK_ADD_F32;
+      uint32_t keep0 = ~0u, keep1 = ~0u;
+      float bias[MASKED ? 32 : 1];
+      auto mask_of = [&](int j, int c, int& rows, int& keys) {   // streamed rows from c on: offset in the mask, and how much of it there is
+        const int64_t col = (int64_t)step_tile<KEYS>(w, j) * kT + half * 64 + c, own = (int64_t)w.tile * kT + quarter * 32;
+        const int64_t query = KEYS ? col : own, key = KEYS ? own : col;
+        rows = masktile::clamp32(p.seq_q - query);
+        keys = masktile::clamp32(p.seq_kv - key);
+        return (int64_t)w.b * p.mask_stride[0] + (int64_t)(KEYS ? step_head<KEYS>(w, j) : w.h) * p.mask_stride[1] + query * p.mask_stride[2] +
+               key * p.mask_stride[3];
+      };
+      auto bias_rows = [&](int j, int c, float (&x)[32]) {
+        int rows, keys;
+        const int64_t at = mask_of(j, c, rows, keys);
+        masktile::load_rows(static_cast<const float*>(p.mask) + at, p.mask_stride[2], p.mask_stride[3], rows, keys, lane, x);
+      };
+      auto keep_row = [&](int j, int c) {
+        int rows, keys;
+        const int64_t at = mask_of(j, c, rows, keys);
+        if (!KEYS) return masktile::keep_bits_of(p, at, p.mask_stride[2], p.mask_stride[3], rows, keys, lane);
+        return masktile::keep_column_of(p, at, p.mask_stride[2], p.mask_stride[3], rows, keys, lane);
+      };
+      auto request_mask = [&](int j) {
+        if constexpr (MASKED) {
+          if (!add) {
+            keep0 = keep_row(j, 0);
+            keep1 = keep_row(j, 32);
+          } else if constexpr (KEYS) {
+            bias_rows(j, 0, bias);
+          } else {
+            int rows, keys;
+            const int64_t at = mask_of(j, 0, rows, keys);
+            masktile::request(my_mask, static_cast<const float*>(p.mask) + at, p.mask_stride[2], p.mask_stride[3], rows, keys, lane);
+            bias_rows(j, 32, bias);
+          }
+        }
+      };
+      if (MASKED && w.steps > 0) request_mask(0);
       for (int j = 0; j < w.steps; ++j) {
         const int64_t col0 = (int64_t)step_tile<KEYS>(w, j) * kT + half * 64;   // first query (KEYS) or key of this half
         const float* nls = my_vec + (j & 1) * (2 * 64);
         const float* nds = nls + 64;
-        int64_t mask_base = 0;
-        if constexpr (MASKED)
-          mask_base = (int64_t)w.b * p.mask_stride[0] + (int64_t)(KEYS ? step_head<KEYS>(w, j) : w.h) * p.mask_stride[1];
         if constexpr (KEYS) {
           // the streamed queries' -lse*log2(e) and -delta, one private copy per warp (no cross-warp barrier)
           const int h = step_head<KEYS>(w, j);
@@ -417,7 +456,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         // what the loop waits for (17 instructions per element with 64-bit comparisons in every one took a half 1119 per warp).
         // B1 H32 S2048 D128 causal with its forward 241 -> 225 us, the same bits.
         // A masked position is selected, not multiplied: it stays 0 whatever its score or dP is (0 * NaN is NaN).
-        auto block32 = [&](int c0, auto at_edge) {
+        const uint64_t log2e_2 = pack2(kLog2e, kLog2e);
+        auto block32 = [&](int c0, auto at_edge, uint32_t bits, const float* bias) {
           constexpr bool kEdge = decltype(at_edge)::value;
           uint64_t sr[16], dr[16];
           tmem_ld32(t_s + (uint32_t)c0, reinterpret_cast<uint32_t*>(sr));
@@ -426,6 +466,10 @@ __global__ void __launch_bounds__(kThreads, 1)
           uint32_t pk[16], dk[16];
 #pragma unroll
           for (int c4 = 0; c4 < 32; c4 += 4) {
+            float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            if constexpr (MASKED && !KEYS) {
+              if (add) b4 = masktile::row4(my_mask, c4 / 4, lane);
+            }
             ulonglong2 nl4 = make_ulonglong2(pack2(my_nl, my_nl), pack2(my_nl, my_nl)), nd4 = make_ulonglong2(pack2(my_nd, my_nd), pack2(my_nd, my_nd));
             if constexpr (KEYS) {   // 16-byte reads: all lanes read the same words, and the tensor cores need the shared memory
               nl4 = *reinterpret_cast<const ulonglong2*>(nls + c0 + c4);
@@ -436,22 +480,10 @@ __global__ void __launch_bounds__(kThreads, 1)
               const int i = c4 / 2 + e, cc = c0 + 2 * i;
               uint64_t nl = e ? nl4.y : nl4.x;
               bool keep0 = !kEdge || (cc >= lo && cc <= hi), keep1 = !kEdge || (cc + 1 >= lo && cc + 1 <= hi);
-              if constexpr (MASKED) {
-                // additive bias (after the scale) or keep-mask of these (query, key), as finish_logit() applies them
-                float2 add = unpack2(nl);
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                  const int64_t qi = KEYS ? col0 + cc + x : my_row, kj = KEYS ? my_row : col0 + cc + x;
-                  if (qi < p.seq_q && kj < p.seq_kv) {
-                    const int64_t idx = mask_base + qi * p.mask_stride[2] + kj * p.mask_stride[3];
-                    bool& keep = x ? keep1 : keep0;
-                    float& a = x ? add.y : add.x;
-                    if (p.mask_kind == AIDN_MASK_KEEP_U8) keep = keep && static_cast<const uint8_t*>(p.mask)[idx] != 0;
-                    else if (p.mask_kind == AIDN_MASK_KEEP_F32) keep = keep && static_cast<const float*>(p.mask)[idx] != 0.0f;
-                    else a = fmaf(static_cast<const float*>(p.mask)[idx], kLog2e, a);
-                  }
-                }
-                nl = pack2(add.x, add.y);
+              if constexpr (MASKED) {   // additive bias (after the scale) or keep-mask, as finish_logit() applies them
+                if (add) nl = fma2(KEYS ? pack2(bias[2 * i], bias[2 * i + 1]) : (e ? pack2(b4.z, b4.w) : pack2(b4.x, b4.y)), log2e_2, nl);
+                keep0 = keep0 && (bits & (1u << (2 * i))) != 0;
+                keep1 = keep1 && (bits & (2u << (2 * i))) != 0;
               }
               const float2 t = unpack2(fma2(sr[i], sl2_2, nl));
               float p0 = ex2_approx(t.x), p1 = ex2_approx(t.y);
@@ -472,16 +504,39 @@ __global__ void __launch_bounds__(kThreads, 1)
           if constexpr (KEYS) tmem_st16(t_s + (uint32_t)(c0 >> 1), pk);
           tmem_st16(t_dp + (uint32_t)(c0 >> 1), dk);
         };
-        if (edge) {
+        if constexpr (!MASKED) {
+          if (edge) {
 #pragma unroll
-          for (int c0 = 0; c0 < 64; c0 += 32) block32(c0, std::true_type());
+            for (int c0 = 0; c0 < 64; c0 += 32) block32(c0, std::true_type(), ~0u, nullptr);
+          } else {
+#pragma unroll
+            for (int c0 = 0; c0 < 64; c0 += 32) block32(c0, std::false_type(), ~0u, nullptr);
+          }
         } else {
-#pragma unroll
-          for (int c0 = 0; c0 < 64; c0 += 32) block32(c0, std::false_type());
+          float late[KEYS ? 32 : 1];
+          if constexpr (KEYS) {
+            if (add) bias_rows(j, 32, late);
+          } else if (add) {
+            cp_async_wait_f<0>();
+            __syncwarp();   // every lane's copies are there
+          }
+          block32(0, std::true_type(), keep0, bias);
+          if constexpr (!KEYS) {
+            if (add) {
+              __syncwarp();   // the values have been read
+              masktile::put(my_mask, bias, lane);
+              __syncwarp();
+            }
+          }
+          block32(32, std::true_type(), keep1, late);
         }
         tc_wait_st();
         tc_fence_before();
         mbar_arrive(bar_p_full + 8 * half);
+        if constexpr (MASKED) {
+          __syncwarp();
+          if (j + 1 < w.steps) request_mask(j + 1);
+        }
       }
       if (!alive) break;
 
@@ -573,7 +628,6 @@ bool aligned_bhs(const void* base, const int64_t* stride, int64_t H, int64_t B, 
 
 template <typename T, int HD>
 cudaError_t launch_t(const BwdParams& bp, cudaStream_t stream, int* launches, const char** why) {
-  using C = BCfg<HD>;
   const SdpaParams& p = bp.p;
   cudaError_t e = tmap::resolve_encode();
   if (e != cudaSuccess) { *why = "cuTensorMapEncodeTiled is not available from the driver"; return e; }
@@ -606,8 +660,9 @@ cudaError_t launch_t(const BwdParams& bp, cudaStream_t stream, int* launches, co
   const bool masked = p.mask_kind != AIDN_MASK_NONE;
   auto kq = masked ? sdpa_backward_sm100_kernel<T, HD, false, true> : sdpa_backward_sm100_kernel<T, HD, false, false>;
   auto kkv = masked ? sdpa_backward_sm100_kernel<T, HD, true, true> : sdpa_backward_sm100_kernel<T, HD, true, false>;
-  e = cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+  const int smem_kv = BCfg<HD, false>::kSmemBytes, smem_q = masked ? BCfg<HD, true>::kSmemBytes : smem_kv;
+  e = cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_q);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_kv);
   if (e != cudaSuccess) { *why = "cannot raise the dynamic shared memory limit"; return e; }
   const int64_t items_q = (int64_t)sp.q_tiles * p.head_count * p.batch;
   const int64_t items_kv = (int64_t)sp.k_tiles * (p.head_count / p.group) * p.batch;
@@ -617,11 +672,11 @@ cudaError_t launch_t(const BwdParams& bp, cudaStream_t stream, int* launches, co
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess || sms <= 0) { *why = "cannot read the SM count"; return e != cudaSuccess ? e : cudaErrorInvalidValue; }
   sp.total_items = (int)items_q;
-  e = launch_dependent(kq, dim3((unsigned)(items_q < sms ? items_q : sms)), kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo, sp);
+  e = launch_dependent(kq, dim3((unsigned)(items_q < sms ? items_q : sms)), kThreads, smem_q, stream, tq, tk, tv, tdo, sp);
   if (e != cudaSuccess) return e;
   sp.total_items = (int)items_kv;
   *launches += 2;
-  return launch_dependent(kkv, dim3((unsigned)(items_kv < sms ? items_kv : sms)), kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo, sp);
+  return launch_dependent(kkv, dim3((unsigned)(items_kv < sms ? items_kv : sms)), kThreads, smem_kv, stream, tq, tk, tv, tdo, sp);
 }
 
 }  // namespace

@@ -48,6 +48,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "mask_tile.cuh"
 #include "ffma2.cuh"
 #include "sm100_ptx.cuh"
 #include "tensor_map.hpp"
@@ -525,10 +526,59 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
 
       float m = -INFINITY, l = 0.f;
 
+      // The explicit mask, a sub-tile ahead: bits of the row's 64 keys, or a bias of its first 32 in the staging buffer and of the other
+      // 32 - by the lanes' keys - in registers (a bias takes the layout without epilogue warps).
+      // Bytes of aligned rows: the row's own, four 16-byte loads (1 x 25 heads of 432, D 64, causal: 23 us, by lanes' keys 35).
+      const bool add = MASKED && !EPI && p.mask_kind == AIDN_MASK_ADD_F32;
+      uint32_t keep0 = 0, keep1 = 0;
+      float held[!MASKED ? 1 : (EPI ? 16 : 32)];   // the bias in registers, or the row's 64 bytes
+      const int64_t mask_row = (int64_t)ti.t * kBM + quarter * 32;
+      const int mask_rows = masktile::clamp32(p.seq_q - mask_row);
+      const uint8_t* byte_row = static_cast<const uint8_t*>(p.mask);   // of this thread, at the item's first key
+      bool bytes = false;
+      if (MASKED && p.mask_kind == AIDN_MASK_KEEP_U8 && p.mask_stride[3] == 1 && p.mask_stride[2] != 0 && p.seq_kv % 16 == 0) {
+        byte_row += (int64_t)b * p.mask_stride[0] + (int64_t)ti.h * p.mask_stride[1] + (qrow < p.seq_q ? qrow : p.seq_q - 1) * p.mask_stride[2] +
+                    (int64_t)it.k0 * kBS;
+        bytes = __all_sync(0xffffffffu, (reinterpret_cast<uintptr_t>(byte_row) & 15) == 0);
+      }
+      const bool keep = MASKED && !bytes && (p.mask_kind == AIDN_MASK_KEEP_U8 || p.mask_kind == AIDN_MASK_KEEP_F32);
+      const int64_t mask_at = MASKED ? (int64_t)b * p.mask_stride[0] + (int64_t)ti.h * p.mask_stride[1] + mask_row * p.mask_stride[2] : 0;
+      auto request_keep = [&](int u) {
+        const int64_t key = (int64_t)(it.k0 + u) * kBS, ms2 = p.mask_stride[2], ms3 = p.mask_stride[3];
+        keep0 = masktile::keep_bits_of(p, mask_at + key * ms3, ms2, ms3, mask_rows, masktile::clamp32(p.seq_kv - key), lane);
+        keep1 = masktile::keep_bits_of(p, mask_at + (key + 32) * ms3, ms2, ms3, mask_rows, masktile::clamp32(p.seq_kv - key - 32), lane);
+      };
+      auto request_bias = [&](int u) {
+        if constexpr (MASKED && !EPI) {
+          const int64_t key = (int64_t)(it.k0 + u) * kBS, ms2 = p.mask_stride[2], ms3 = p.mask_stride[3];
+          const float* src = static_cast<const float*>(p.mask) + mask_at + key * ms3;
+          masktile::request(my_stage, src, ms2, ms3, mask_rows, masktile::clamp32(p.seq_kv - key), lane);
+          masktile::load_rows(src + 32 * ms3, ms2, ms3, mask_rows, masktile::clamp32(p.seq_kv - key - 32), lane, held);
+        }
+      };
+      if (MASKED && ti.n > 0) {
+        if (keep) request_keep(0);
+        if (add) {
+          if (stores_in_flight && lane == 0) bulk_wait_read0();   // the staging buffer may still be read by a store
+          __syncwarp();
+          request_bias(0);
+        }
+      }
+
       for (int u = 0; u < ti.n; ++u) {
         const uint32_t buf = (uint32_t)(u & 1);
         const uint32_t t_sb = t_s + buf * kBS;
         const uint32_t bar_off = 8u * (uint32_t)(2 * i) + 8u * buf;
+        if constexpr (MASKED) {
+          if (bytes) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+              if ((int64_t)(it.k0 + u) * kBS + 16 * q < p.seq_kv) v = *reinterpret_cast<const float4*>(byte_row + u * kBS + 16 * q);
+              held[4 * q] = v.x; held[4 * q + 1] = v.y; held[4 * q + 2] = v.z; held[4 * q + 3] = v.w;
+            }
+          }
+        }
         bool ok = mbar_wait(bar_s_full + bar_off, (s_par >> buf) & 1u, abort_flag, wait_ns);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) { alive = false; break; }
@@ -546,69 +596,42 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
         const int64_t col0 = (int64_t)(it.k0 + u) * kBS;
         if constexpr (MASKED) {
           // scale -> softcap -> bias -> keep-mask, the order of the reference (CpuEngine.cs:27807-27816, 29218-29239)
-          const float inv_cap = p.softcap > 0.f ? 1.f / p.softcap : 0.f;
-          const int64_t mrow = qrow < p.seq_q ? qrow : p.seq_q - 1;   // rows past the end read a valid row
-          const int64_t mbase = (int64_t)b * p.mask_stride[0] + (int64_t)ti.h * p.mask_stride[1] + mrow * p.mask_stride[2];
-          const int64_t ms3 = p.mask_stride[3];
-          const bool full_tile = col0 + kBS <= p.seq_kv;
-          const int kind = p.mask_kind;
-          if (kind == AIDN_MASK_NONE) {
+          if (p.softcap > 0.f) {
+            const float inv_cap = 1.f / p.softcap;
 #pragma unroll
-            for (int c = 0; c < kBS; ++c) {
-              float val = s[c] * p.scale;
-              if (p.softcap > 0.f) val = p.softcap * tanh_approx(val * inv_cap);
-              s[c] = val;
-            }
-          } else if (kind == AIDN_MASK_KEEP_U8) {
-            const uint8_t* mp = static_cast<const uint8_t*>(p.mask) + mbase + col0 * ms3;
-            const bool vec = ms3 == 1 && full_tile && ((reinterpret_cast<uintptr_t>(mp) & 15) == 0);
+            for (int c = 0; c < kBS; ++c) s[c] = p.softcap * tanh_approx(s[c] * p.scale * inv_cap);
+          } else if (!add) {
 #pragma unroll
-            for (int c0 = 0; c0 < kBS; c0 += 16) {
-              uint32_t w[4];
-              if (vec) {
-                const uint4 u4 = *reinterpret_cast<const uint4*>(mp + c0);
-                w[0] = u4.x; w[1] = u4.y; w[2] = u4.z; w[3] = u4.w;
-              } else {
+            for (int c = 0; c < kBS; ++c) s[c] *= p.scale;
+          }
+          if (keep) {
 #pragma unroll
-                for (int q4 = 0; q4 < 4; ++q4) {
-                  w[q4] = 0;
+            for (int c = 0; c < kBS; ++c)
+              if (!((c < 32 ? keep0 : keep1) & (1u << (c & 31)))) s[c] = -INFINITY;
+          } else if (bytes) {
 #pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    const int c = c0 + q4 * 4 + e;
-                    const uint32_t byte = (col0 + c < p.seq_kv) ? mp[(int64_t)c * ms3] : 0u;
-                    w[q4] |= (byte != 0 ? 1u : 0u) << (8 * e);
-                  }
+            for (int c = 0; c < kBS; ++c)
+              if (((__float_as_uint(held[c >> 2]) >> (8 * (c & 3))) & 0xffu) == 0u) s[c] = -INFINITY;
+          }
+          if constexpr (!EPI) {
+            if (add) {
+              const float f = p.softcap > 0.f ? 1.f : p.scale;
+              auto add_tile = [&](int c0) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                  const float4 v = masktile::row4(my_stage, c, lane);
+                  float* x = s + c0 + 4 * c;
+                  x[0] = fmaf(x[0], f, v.x); x[1] = fmaf(x[1], f, v.y); x[2] = fmaf(x[2], f, v.z); x[3] = fmaf(x[3], f, v.w);
                 }
-              }
-#pragma unroll
-              for (int c = 0; c < 16; ++c) {
-                float val = s[c0 + c] * p.scale;
-                if (p.softcap > 0.f) val = p.softcap * tanh_approx(val * inv_cap);
-                if (((w[c >> 2] >> (8 * (c & 3))) & 0xffu) == 0u) val = -INFINITY;
-                s[c0 + c] = val;
-              }
-            }
-          } else {
-            const float* mp = static_cast<const float*>(p.mask) + mbase + col0 * ms3;
-            const bool vec = ms3 == 1 && full_tile && ((reinterpret_cast<uintptr_t>(mp) & 15) == 0);
-#pragma unroll
-            for (int c0 = 0; c0 < kBS; c0 += 4) {
-              float mv[4];
-              if (vec) {
-                const float4 u4 = *reinterpret_cast<const float4*>(mp + c0);
-                mv[0] = u4.x; mv[1] = u4.y; mv[2] = u4.z; mv[3] = u4.w;
-              } else {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) mv[e] = (col0 + c0 + e < p.seq_kv) ? mp[(int64_t)(c0 + e) * ms3] : 0.f;
-              }
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                float val = s[c0 + e] * p.scale;
-                if (p.softcap > 0.f) val = p.softcap * tanh_approx(val * inv_cap);
-                if (kind == AIDN_MASK_ADD_F32) val += mv[e];
-                else if (mv[e] == 0.0f) val = -INFINITY;
-                s[c0 + e] = val;
-              }
+                __syncwarp();   // the values have been read
+              };
+              cp_async_wait_f<0>();
+              __syncwarp();   // every lane's copies are there
+              add_tile(0);
+              masktile::put(my_stage, held, lane);
+              __syncwarp();
+              add_tile(32);
+              if (u + 1 < ti.n) request_bias(u + 1);
             }
           }
         }
@@ -713,6 +736,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_p_full + bar_off);   // one arrival per warp: 128 arrivals on one word serialise
+        if (keep && u + 1 < ti.n) request_keep(u + 1);
         STEP_STAMP(u, 4);
         s_par ^= 1u << buf;
       }
@@ -1435,7 +1459,7 @@ bool prefill_sm100_supported(const SdpaParams& p, int dtype, const char** why) {
 template <typename T, int HD, bool MASKED>
 cudaError_t launch_t(const SdpaParams& p, cudaStream_t stream, int32_t* sched, int num_sms, float* debug,
                      int debug_mode, PrefillMapCache* cache, int splits, const char** why) {
-  const bool epi = (p.group % 2 == 0) || !p.causal;
+  const bool epi = ((p.group % 2 == 0) || !p.causal) && p.mask_kind != AIDN_MASK_ADD_F32;   // (a bias goes through the softmax warps' staging buffers)
   if (epi) return launch_e<T, HD, MASKED, true>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
   return launch_e<T, HD, MASKED, false>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
 }
