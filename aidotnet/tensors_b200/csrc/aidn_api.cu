@@ -149,6 +149,25 @@ int64_t decode_ws_bytes(const aidn_sdpa* h, int64_t batch, int64_t seq_kv, int* 
   return align_up(batch * h->head_count * nchunks * (h->d.head_dim + 2) * (int64_t)sizeof(float), 256);
 }
 
+// What a decode can use: equal shares of all keys, for sequences with lengths, may take more than it needs.
+int64_t decode_ws_most(const aidn_sdpa* h, int64_t batch, int64_t seq_kv) {
+  aidn::DecodePlan chunks = {0, 0, 1, 0};
+  const int64_t need = decode_ws_bytes(h, batch, seq_kv, &chunks.chunk, &chunks.nchunks);
+  if (need == 0 || h->d.decode_chunk > 0 || batch > 0x7fffffff) return need;
+  aidn::SdpaParams p;
+  std::memset(&p, 0, sizeof(p));
+  p.batch = (int32_t)batch;
+  p.seq_q = 1;
+  p.seq_kv = seq_kv;
+  p.head_dim = h->d.head_dim;
+  p.group = h->group;
+  p.head_count = h->head_count;
+  p.ks[2] = 1;   // (any layout: the one that takes the most)
+  int ctas = 0;
+  const int64_t stream = align_up(aidn::decode_stream_bytes(p, h->d.qkv_dtype, h->num_sms, chunks, &ctas), 256);
+  return need > stream ? need : stream;
+}
+
 // Workspace of the split tcgen05 prefill for these sizes, 0 when it would not be split.
 int64_t prefill_split_need(const aidn_sdpa* h, int64_t batch, int64_t seq_q, int64_t seq_kv) {
   aidn::SdpaParams p;
@@ -283,7 +302,7 @@ int64_t aidn_sdpa_workspace_bytes(aidn_sdpa_t h, int64_t batch, int64_t seq_q, i
   // a workspace too, only slower)
   int64_t need = 0;
   if (seq_q == 1 && h->d.path != AIDN_PATH_PREFILL_SM100 && aidn::decode_supported(h->d.qkv_dtype, h->d.head_dim))
-    need = decode_ws_bytes(h, batch, seq_kv, nullptr, nullptr);
+    need = decode_ws_most(h, batch, seq_kv);
   else if (h->d.path != AIDN_PATH_DECODE && h->d.qkv_dtype != AIDN_F32 && (h->d.head_dim == 64 || h->d.head_dim == 128) &&
            batch <= 65535)
     need = prefill_split_need(h, batch, seq_q, seq_kv);
@@ -468,8 +487,13 @@ int launch_common(aidn_sdpa_t h, const aidn_sdpa_args* a, const aidn_paged_kv* p
                     (long long)need, (long long)h->scratch_bytes);
       }
     }
-    aidn::DecodePlan plan = {chunk, nchunks, 1};
-    if (d.decode_chunk == 0 && nchunks > 1) aidn::decode_plan_clusters(p, d.qkv_dtype, h->num_sms, &plan);
+    aidn::DecodePlan plan = {chunk, nchunks, 1, 0};
+    if (d.decode_chunk == 0 && nchunks > 1) {
+      int ctas = 0;
+      const int64_t stream_need = p.kv_len ? aidn::decode_stream_bytes(p, d.qkv_dtype, h->num_sms, plan, &ctas) : 0;
+      if (stream_need > 0 && (ws == a->workspace ? a->workspace_bytes : h->scratch_bytes) >= stream_need) plan.stream_ctas = ctas;   // with less: as without
+      else aidn::decode_plan_clusters(p, d.qkv_dtype, h->num_sms, &plan);
+    }
     e = aidn::launch_decode(p, d.qkv_dtype, plan, ws, stream, &launches);
   } else if (path == AIDN_PATH_PREFILL_SM100) {
     // Keys of few items are split when the caller's workspace holds the partial results; without one they are not.  The

@@ -257,7 +257,11 @@ cudaError_t launch_f32_sm100(const SdpaParams& p, cudaStream_t stream);
 // `cluster` CTAs per (sequence, KV head), which share the sequence's keys evenly.  nchunks > 1 takes the workspace.
 struct DecodePlan {
   int chunk, nchunks, cluster;
+  int stream_ctas;   // > 0: that many CTAs, whose warps share all keys evenly (decode_stream_bytes of workspace)
 };
+// The workspace of such a launch and its CTAs for sequences with lengths that would otherwise be cut into `chunks` (or clusters); 0
+// where that is the better way.  Of p only the sizes are looked at.
+int64_t decode_stream_bytes(const SdpaParams& p, int dtype, int num_sms, const DecodePlan& chunks, int* ctas);
 // Turns a plan of several chunks into one with clusters where that is faster; never one that needs more workspace.
 void decode_plan_clusters(const SdpaParams& p, int dtype, int num_sms, DecodePlan* plan);
 cudaError_t launch_decode(const SdpaParams& p, int dtype, const DecodePlan& plan, float* workspace, cudaStream_t stream, int* launches);

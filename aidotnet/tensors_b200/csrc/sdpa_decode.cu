@@ -405,131 +405,38 @@ struct RingCfg {
 };
 
 
-template <typename T, int D, bool NH16, bool PAGED, bool HEAD_FAST>
-__global__ void __launch_bounds__(kDecWarps * 32, 2)
-    sdpa_decode_gqa_ring_kernel(const SdpaParams p, const int chunk, const int nchunks, float* __restrict__ ws,
-                                const int merge, const int cluster) {
-  static_assert(sizeof(T) == 2 && (D == 64 || D == 128), "16-bit inputs, head_dim 64 or 128");
+// A warp's query heads of one KV head and what it has summed up for them.
+template <typename T, int D, bool NH16>
+struct RingWarp {
+  static constexpr int KI = D / 32, VX = D / 64, MT = D / 16, HN = NH16 ? 2 : 1;
   using R = RingCfg<D>;
-  constexpr int KI = D / 32, VX = D / 64, MT = D / 16;
-  constexpr int HN = NH16 ? 2 : 1;
-  constexpr int ROWS = NH16 ? 16 : 8;
-  constexpr int NG = kDecWarps;
-  constexpr int kStep = 16;
-
-  extern __shared__ __align__(128) uint8_t ring_smem[];
-  const uint32_t smem0 = ptx::smem_u32(ring_smem);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, c = lane & 3;
-  const int b = blockIdx.z;
-  const int kvh = p.head_begin / p.group + (HEAD_FAST ? (int)blockIdx.x : (int)blockIdx.y);
-  const int h0 = kvh * p.group;
-  const int nheads = p.group;
-  const int cidx = HEAD_FAST ? blockIdx.y : blockIdx.x;
-
-  pdl_wait();      // nothing above touches memory that an earlier kernel writes
-  pdl_trigger();   // the merge may be set up while this kernel runs
-  const int64_t L = decode_len(p, b);
-  int64_t start, end;
-  split_range(L, chunk, nchunks * cluster, cidx, merge, start, end);
-  const int Hc = p.head_count;
-
-  if (start >= L && merge < kMergeCluster) {
-    if (merge == kMergeDirect && cidx == 0) {
-      for (int idx = tid; idx < nheads * D; idx += kDecWarps * 32) {
-        const int hh = idx / D, d = idx - hh * D;
-        store_out<T>(p.out, b * p.os[0] + (int64_t)(h0 + hh) * p.os[1] + d, 0.f, p.out_f32);
-        if (p.lse && d == 0) p.lse[((int64_t)b * p.num_q_heads + h0 + hh) * p.seq_q] = -INFINITY;
-      }
-    }
-    return;
-  }
-
-  const uint32_t my_ring = smem0 + warp * R::kWarpBytes;
-  const T* kbase = static_cast<const T*>(p.k) + (PAGED ? 0 : b * p.ks[0]) + (int64_t)kvh * p.ks[1];
-  const T* vbase = static_cast<const T*>(p.v) + (PAGED ? 0 : b * p.vs[0]) + (int64_t)kvh * p.vs[1];
-  bool bad_block = false;
-
-  constexpr int CH = D / 8;          // 16-byte chunks per row
-  constexpr int RPL = 16 * CH / 32;  // rows each lane copies per step (of K, and of V)
-  const int my_ch = lane % CH, my_r0 = lane / CH;
-  // Raw block-table entry of key kb + lane % 16 (paged), read a step before the copies that need it are issued.
-  auto entry_of = [&](int64_t kb) -> int32_t {
-    if constexpr (PAGED) {
-      const int64_t key = kb + (lane & 15);
-      return key < end ? kv_block_read(p, b, key) : 0;
-    } else {
-      return 0;
-    }
-  };
-  // Issues the copies of the step at kb into `stage` and commits them as one group.  Returns the step's row mask
-  // (bit i: key kb + i is inside the chunk and its row inside the pool); the other rows are zero-filled.
-  auto issue = [&](int stage, int64_t kb, int32_t entry) -> uint32_t {
-    const int64_t key = kb + (lane & 15);
-    int64_t row = -1;
-    if (key < end) {
-      if constexpr (PAGED) row = kv_row_from(p, key, entry, bad_block);
-      else row = key;
-    }
-    const uint32_t base = my_ring + stage * R::kStageBytes;
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int ri = my_r0 + (32 / CH) * r;
-      const int64_t rr = __shfl_sync(0xffffffffu, row, ri);
-      const bool valid = rr >= 0;
-      const int64_t ro = valid ? rr : 0;
-      cp_async16(base + ri * R::kRowBytes + ((my_ch ^ ((ri & 1) << 2)) << 4), kbase + ro * p.ks[2] + my_ch * 8, valid);
-      cp_async16(base + R::kKBytes + ri * R::kRowBytes + ((my_ch ^ (((ri >> 1) & 3) << 1)) << 4),
-                 vbase + ro * p.vs[2] + my_ch * 8, valid);
-    }
-    cp_async_commit();
-    return __ballot_sync(0xffffffffu, row >= 0) & 0xffffu;
-  };
-
-  // Q in fragment order
-  uint32_t qa[KI][4], qb[KI][4];
-#pragma unroll
-  for (int i = 0; i < KI; ++i) {
-    uint4 u = make_uint4(0, 0, 0, 0), w = make_uint4(0, 0, 0, 0);
-    if (g < nheads)
-      u = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.q) + b * p.qs[0] + (int64_t)(h0 + g) * p.qs[1] + (i * 4 + c) * 8);
-    if (NH16 && g + 8 < nheads)
-      w = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.q) + b * p.qs[0] + (int64_t)(h0 + g + 8) * p.qs[1] + (i * 4 + c) * 8);
-    qa[i][0] = u.x; qa[i][1] = u.y; qa[i][2] = u.z; qa[i][3] = u.w;
-    qb[i][0] = w.x; qb[i][1] = w.y; qb[i][2] = w.z; qb[i][3] = w.w;
-  }
-
+  uint32_t qa[KI][4], qb[KI][4];   // Q in fragment order
   float acc[MT][HN][4];
-#pragma unroll
-  for (int j = 0; j < MT; ++j)
-#pragma unroll
-    for (int hn = 0; hn < HN; ++hn) acc[j][hn][0] = acc[j][hn][1] = acc[j][hn][2] = acc[j][hn][3] = 0.f;
-  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+  float m0, m1, l0, l1;
 
-  // prologue: fill the ring (a group is committed per stage even when it is empty, so that wait_group counts steps)
-  const int64_t kb0 = start + warp * kStep;
-  constexpr int64_t kStride = NG * kStep;
-  uint32_t row_mask[kRingStages];
+  __device__ __forceinline__ void begin(const SdpaParams& p, int b, int h0, int nheads, int g, int c) {
 #pragma unroll
-  for (int s = 0; s < kRingStages; ++s) {
-    const int64_t kbs = kb0 + s * kStride;
-    row_mask[s] = 0;
-    if (kbs < end) row_mask[s] = issue(s, kbs, entry_of(kbs));
-    else cp_async_commit();
+    for (int i = 0; i < KI; ++i) {
+      uint4 u = make_uint4(0, 0, 0, 0), w = make_uint4(0, 0, 0, 0);
+      if (g < nheads)
+        u = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.q) + b * p.qs[0] + (int64_t)(h0 + g) * p.qs[1] + (i * 4 + c) * 8);
+      if (NH16 && g + 8 < nheads)
+        w = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.q) + b * p.qs[0] + (int64_t)(h0 + g + 8) * p.qs[1] + (i * 4 + c) * 8);
+      qa[i][0] = u.x; qa[i][1] = u.y; qa[i][2] = u.z; qa[i][3] = u.w;
+      qb[i][0] = w.x; qb[i][1] = w.y; qb[i][2] = w.z; qb[i][3] = w.w;
+    }
+#pragma unroll
+    for (int j = 0; j < MT; ++j)
+#pragma unroll
+      for (int hn = 0; hn < HN; ++hn) acc[j][hn][0] = acc[j][hn][1] = acc[j][hn][2] = acc[j][hn][3] = 0.f;
+    m0 = m1 = -INFINITY;
+    l0 = l1 = 0.f;
   }
-  int32_t ent_next = entry_of(kb0 + kRingStages * kStride);
 
-  int step = 0;
-  for (int64_t kb = kb0; kb < end; kb += kStride, ++step) {
-    const int stage = step % kRingStages;
-    cp_async_wait<kRingStages - 1>();   // this step's group has landed (later steps may still be in flight)
-    __syncwarp();                       // ... for every lane's copies
-    const uint32_t base = my_ring + stage * R::kStageBytes;
-    uint32_t rows_ok = 0;
-#pragma unroll
-    for (int s = 0; s < kRingStages; ++s)
-      if (s == stage) rows_ok = row_mask[s];
-
+  // The 16 keys from kb on, in the stage at `base`; bit i of rows_ok: key kb + i counts.  `refill` is called when the stage has been read.
+  template <typename Refill>
+  __device__ __forceinline__ void step(const SdpaParams& p, uint32_t base, uint32_t rows_ok, int b, int h0, int nheads, int64_t kb, int64_t L, int g,
+                                       int c, Refill refill) {
     // ---- S = Q K^T ------------------------------------------------------------------------------------
     float sacc[2][4];
 #pragma unroll
@@ -558,17 +465,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2)
                      : "r"(base + R::kKBytes + vr * R::kRowBytes + (((g + 8 * x) ^ (c << 1)) << 4)));
       }
     __syncwarp();   // every lane has read the stage: refill it with the step kRingStages ahead
-    {
-      const int64_t kb_new = kb + kRingStages * kStride;
-      const int32_t ent_new = ent_next;
-      ent_next = entry_of(kb_new + kStride);
-      uint32_t mask_new = 0;
-      if (kb_new < end) mask_new = issue(stage, kb_new, ent_new);
-      else cp_async_commit();
-#pragma unroll
-      for (int s = 0; s < kRingStages; ++s)
-        if (s == stage) row_mask[s] = mask_new;
-    }
+    refill();
 
     // ---- online softmax over the step's 16 keys ---------------------------------------------------------
     float pr[2][4];
@@ -649,6 +546,138 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2)
     }
   }
 
+  // The row sums, which are in four lanes' parts.
+  __device__ __forceinline__ void gather_sums() {
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+  }
+};
+
+template <typename T, int D, bool NH16, bool PAGED, bool HEAD_FAST>
+__global__ void __launch_bounds__(kDecWarps * 32, 2)
+    sdpa_decode_gqa_ring_kernel(const SdpaParams p, const int chunk, const int nchunks, float* __restrict__ ws,
+                                const int merge, const int cluster) {
+  static_assert(sizeof(T) == 2 && (D == 64 || D == 128), "16-bit inputs, head_dim 64 or 128");
+  using R = RingCfg<D>;
+  constexpr int MT = D / 16, HN = NH16 ? 2 : 1;
+  constexpr int ROWS = NH16 ? 16 : 8;
+  constexpr int NG = kDecWarps;
+  constexpr int kStep = 16;
+
+  extern __shared__ __align__(128) uint8_t ring_smem[];
+  const uint32_t smem0 = ptx::smem_u32(ring_smem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, c = lane & 3;
+  const int b = blockIdx.z;
+  const int kvh = p.head_begin / p.group + (HEAD_FAST ? (int)blockIdx.x : (int)blockIdx.y);
+  const int h0 = kvh * p.group;
+  const int nheads = p.group;
+  const int cidx = HEAD_FAST ? blockIdx.y : blockIdx.x;
+
+  pdl_wait();      // nothing above touches memory that an earlier kernel writes
+  pdl_trigger();   // the merge may be set up while this kernel runs
+  const int64_t L = decode_len(p, b);
+  int64_t start, end;
+  split_range(L, chunk, nchunks * cluster, cidx, merge, start, end);
+  const int Hc = p.head_count;
+
+  if (start >= L && merge < kMergeCluster) {
+    if (merge == kMergeDirect && cidx == 0) {
+      for (int idx = tid; idx < nheads * D; idx += kDecWarps * 32) {
+        const int hh = idx / D, d = idx - hh * D;
+        store_out<T>(p.out, b * p.os[0] + (int64_t)(h0 + hh) * p.os[1] + d, 0.f, p.out_f32);
+        if (p.lse && d == 0) p.lse[((int64_t)b * p.num_q_heads + h0 + hh) * p.seq_q] = -INFINITY;
+      }
+    }
+    return;
+  }
+
+  const uint32_t my_ring = smem0 + warp * R::kWarpBytes;
+  const T* kbase = static_cast<const T*>(p.k) + (PAGED ? 0 : b * p.ks[0]) + (int64_t)kvh * p.ks[1];
+  const T* vbase = static_cast<const T*>(p.v) + (PAGED ? 0 : b * p.vs[0]) + (int64_t)kvh * p.vs[1];
+  bool bad_block = false;
+
+  constexpr int CH = D / 8;          // 16-byte chunks per row
+  constexpr int RPL = 16 * CH / 32;  // rows each lane copies per step (of K, and of V)
+  const int my_ch = lane % CH, my_r0 = lane / CH;
+  // Raw block-table entry of key kb + lane % 16 (paged), read a step before the copies that need it are issued.
+  auto entry_of = [&](int64_t kb) -> int32_t {
+    if constexpr (PAGED) {
+      const int64_t key = kb + (lane & 15);
+      return key < end ? kv_block_read(p, b, key) : 0;
+    } else {
+      return 0;
+    }
+  };
+  // Issues the copies of the step at kb into `stage` and commits them as one group.  Returns the step's row mask
+  // (bit i: key kb + i is inside the chunk and its row inside the pool); the other rows are zero-filled.
+  auto issue = [&](int stage, int64_t kb, int32_t entry) -> uint32_t {
+    const int64_t key = kb + (lane & 15);
+    int64_t row = -1;
+    if (key < end) {
+      if constexpr (PAGED) row = kv_row_from(p, key, entry, bad_block);
+      else row = key;
+    }
+    const uint32_t base = my_ring + stage * R::kStageBytes;
+#pragma unroll
+    for (int r = 0; r < RPL; ++r) {
+      const int ri = my_r0 + (32 / CH) * r;
+      const int64_t rr = __shfl_sync(0xffffffffu, row, ri);
+      const bool valid = rr >= 0;
+      const int64_t ro = valid ? rr : 0;
+      cp_async16(base + ri * R::kRowBytes + ((my_ch ^ ((ri & 1) << 2)) << 4), kbase + ro * p.ks[2] + my_ch * 8, valid);
+      cp_async16(base + R::kKBytes + ri * R::kRowBytes + ((my_ch ^ (((ri >> 1) & 3) << 1)) << 4),
+                 vbase + ro * p.vs[2] + my_ch * 8, valid);
+    }
+    cp_async_commit();
+    return __ballot_sync(0xffffffffu, row >= 0) & 0xffffu;
+  };
+
+  RingWarp<T, D, NH16> rw;
+  rw.begin(p, b, h0, nheads, g, c);
+
+  // prologue: fill the ring (a group is committed per stage even when it is empty, so that wait_group counts steps)
+  const int64_t kb0 = start + warp * kStep;
+  constexpr int64_t kStride = NG * kStep;
+  uint32_t row_mask[kRingStages];
+  int32_t first_entries[kRingStages];   // read together: one latency
+#pragma unroll
+  for (int s = 0; s < kRingStages; ++s) first_entries[s] = entry_of(kb0 + s * kStride);
+#pragma unroll
+  for (int s = 0; s < kRingStages; ++s) {
+    const int64_t kbs = kb0 + s * kStride;
+    row_mask[s] = 0;
+    if (kbs < end) row_mask[s] = issue(s, kbs, first_entries[s]);
+    else cp_async_commit();
+  }
+  int32_t ent_next = entry_of(kb0 + kRingStages * kStride);
+
+  int step = 0;
+  for (int64_t kb = kb0; kb < end; kb += kStride, ++step) {
+    const int stage = step % kRingStages;
+    cp_async_wait<kRingStages - 1>();   // this step's group has landed (later steps may still be in flight)
+    __syncwarp();                       // ... for every lane's copies
+    const uint32_t base = my_ring + stage * R::kStageBytes;
+    uint32_t rows_ok = 0;
+#pragma unroll
+    for (int s = 0; s < kRingStages; ++s)
+      if (s == stage) rows_ok = row_mask[s];
+
+    rw.step(p, base, rows_ok, b, h0, nheads, kb, L, g, c, [&] {
+        const int64_t kb_new = kb + kRingStages * kStride;
+        const int32_t ent_new = ent_next;
+        ent_next = entry_of(kb_new + kStride);
+        uint32_t mask_new = 0;
+        if (kb_new < end) mask_new = issue(stage, kb_new, ent_new);
+        else cp_async_commit();
+#pragma unroll
+        for (int s = 0; s < kRingStages; ++s)
+          if (s == stage) row_mask[s] = mask_new;
+    });
+  }
+
   report_bad_block(p, bad_block);
   cp_async_wait<0>();
   __syncwarp();
@@ -658,16 +687,13 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2)
   float* sm_l = sm_m + ROWS;
   constexpr int kWarpFloats = R::kWarpBytes / 4;
   // ---- merge the warps of the CTA ---------------------------------------------------------------------------
-  l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-  l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-  l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-  l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+  rw.gather_sums();
   if (c == 0) {
-    sm_m[g] = m0;
-    sm_l[g] = l0;
+    sm_m[g] = rw.m0;
+    sm_l[g] = rw.l0;
     if (NH16) {
-      sm_m[g + 8] = m1;
-      sm_l[g + 8] = l1;
+      sm_m[g + 8] = rw.m1;
+      sm_l[g + 8] = rw.l1;
     }
   }
 #pragma unroll
@@ -677,8 +703,8 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2)
     for (int hn = 0; hn < HN; ++hn)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        sm_acc[(8 * hn + 2 * c + e) * D + d_lo] = acc[m][hn][e];
-        sm_acc[(8 * hn + 2 * c + e) * D + d_hi] = acc[m][hn][2 + e];
+        sm_acc[(8 * hn + 2 * c + e) * D + d_lo] = rw.acc[m][hn][e];
+        sm_acc[(8 * hn + 2 * c + e) * D + d_hi] = rw.acc[m][hn][2 + e];
       }
   }
   __syncthreads();
@@ -726,18 +752,221 @@ __global__ void __launch_bounds__(kDecWarps * 32, 2)
   if (merge >= kMergeCluster) merge_cluster<T, D, ROWS>(p, b, h0, nheads, cidx % cluster, cluster, ptx::smem_u32(part), ws, cidx / cluster, nchunks);
 }
 
+// ---- sequences of unequal lengths: equal shares of all keys --------------------------------------------------------
+// The keys of a launch are one row of 16-key steps, sequence after sequence, which is cut into equal shares; neighbouring warps take the
+// KV heads of one share, so that what lies together in a pool is read together, and all of them are resident at once.  A warp streams
+// its share through its ring without a pause at the ends of sequences, of which it writes a partial each: share j's partial of
+// sequence b is slot j + b (both only ever grow by one along the row), so that a sequence's slots are neighbours and the merge finds
+// them from the lengths alone.
+// Cut by sequence and head, the CTA of the longest sequence ran on alone, and every CTA spent 5 us on its way to its first keys
+// and on its merge (16 sequences of 128 to 2048 keys, Hq32 / Hkv8 D128, 71 MB: 26.9 us in clusters of two, 27.3 in chunks of 256).
+struct StreamPlan {
+  int total, per;   // steps of a KV head, and of a share
+};
+constexpr int kStreamLeast = 4;   // steps of a share at least
+__device__ __forceinline__ int stream_steps(const SdpaParams& p, int b) { return (int)((decode_len(p, b) + 15) / 16); }
+__device__ __forceinline__ StreamPlan stream_plan(int total, int shares) {
+  StreamPlan s;
+  s.total = total;
+  s.per = (total + shares - 1) / shares;
+  if (s.per < kStreamLeast) s.per = kStreamLeast;
+  return s;
+}
+
+template <typename T, int D, bool NH16, bool PAGED>
+__global__ void __launch_bounds__(kDecWarps * 32, 2) sdpa_decode_stream_kernel(const SdpaParams p, float* __restrict__ ws, const int kv_heads, const int shares) {
+  using R = RingCfg<D>;
+  constexpr int MT = D / 16, HN = NH16 ? 2 : 1;
+  extern __shared__ __align__(128) uint8_t ring_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+  const int w = (int)blockIdx.x * kDecWarps + warp, share = w / kv_heads, kvh = w - share * kv_heads;
+  const int nheads = p.group, h0 = p.head_begin + kvh * p.group;
+  const uint32_t my_ring = ptx::smem_u32(ring_smem) + warp * R::kWarpBytes;
+  pdl_wait();
+  pdl_trigger();
+
+  int all = 0;
+  for (int b0 = 0; b0 < p.batch; b0 += 32) all += __reduce_add_sync(0xffffffffu, b0 + lane < p.batch ? stream_steps(p, b0 + lane) : 0);
+  const StreamPlan plan = stream_plan(all, shares);
+  const int x0 = share * plan.per, x1 = x0 + plan.per < plan.total ? x0 + plan.per : plan.total;
+  if (share >= shares || x0 >= x1) return;
+
+  // A place on the row of steps.
+  struct Cursor {
+    int b, s, steps;   // sequence, step, steps of the sequence
+    int64_t L;
+  };
+  auto at_sequence = [&](Cursor& k, int b) {
+    k.b = b;
+    k.L = decode_len(p, b);
+    k.steps = (int)((k.L + 15) / 16);
+  };
+  auto advance = [&](Cursor& k) {   // (only where there is a next step)
+    if (++k.s < k.steps) return;
+    k.s = 0;
+    do at_sequence(k, k.b + 1);
+    while (k.steps == 0);
+  };
+  Cursor cur;
+  {
+    int before = 0, found = -1, found_before = 0;
+    for (int b0 = 0; b0 < p.batch && found < 0; b0 += 32) {
+      const int mine = b0 + lane < p.batch ? stream_steps(p, b0 + lane) : 0;
+      int upto = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += y;
+      }
+      const uint32_t past = __ballot_sync(0xffffffffu, x0 < before + upto);
+      if (past) {
+        const int at = __ffs(past) - 1;
+        found = b0 + at;
+        found_before = before + __shfl_sync(0xffffffffu, upto - mine, at);
+      }
+      before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    at_sequence(cur, found);
+    cur.s = x0 - found_before;
+  }
+
+  bool bad_block = false;
+  constexpr int CH = D / 8, RPL = 16 * CH / 32;   // 16-byte chunks per row; rows that a lane copies per step
+  const int my_ch = lane % CH, my_r0 = lane / CH;
+  const T* head_k = static_cast<const T*>(p.k) + (int64_t)(h0 / p.group) * p.ks[1];
+  const T* head_v = static_cast<const T*>(p.v) + (int64_t)(h0 / p.group) * p.vs[1];
+  auto entry_of = [&](const Cursor& k) -> int32_t {
+    if constexpr (PAGED) {
+      const int64_t key = (int64_t)k.s * 16 + (lane & 15);
+      return key < k.L ? kv_block_read(p, k.b, key) : 0;
+    } else {
+      return 0;
+    }
+  };
+  auto issue = [&](int stage, const Cursor& k, int32_t entry) -> uint32_t {
+    const int64_t key = (int64_t)k.s * 16 + (lane & 15);
+    int64_t row = -1;
+    if (key < k.L) {
+      if constexpr (PAGED) row = kv_row_from(p, key, entry, bad_block);
+      else row = key;
+    }
+    const T* kbase = head_k + (PAGED ? 0 : k.b * p.ks[0]);
+    const T* vbase = head_v + (PAGED ? 0 : k.b * p.vs[0]);
+    const uint32_t base = my_ring + stage * R::kStageBytes;
+#pragma unroll
+    for (int r = 0; r < RPL; ++r) {
+      const int ri = my_r0 + (32 / CH) * r;
+      const int64_t rr = __shfl_sync(0xffffffffu, row, ri);
+      const bool valid = rr >= 0;
+      const int64_t ro = valid ? rr : 0;
+      cp_async16(base + ri * R::kRowBytes + ((my_ch ^ ((ri & 1) << 2)) << 4), kbase + ro * p.ks[2] + my_ch * 8, valid);
+      cp_async16(base + R::kKBytes + ri * R::kRowBytes + ((my_ch ^ (((ri >> 1) & 3) << 1)) << 4), vbase + ro * p.vs[2] + my_ch * 8, valid);
+    }
+    return __ballot_sync(0xffffffffu, row >= 0) & 0xffffu;
+  };
+
+  // The ring runs ahead of the products by its stages, across the ends of sequences.  A group is committed even where there is no
+  // step, so that wait_group counts steps; the entries of the first steps are read together, later ones a step before they are needed.
+  uint32_t row_mask[kRingStages];
+  Cursor ahead = cur;
+  int x_ahead = x0 + kRingStages;
+  int32_t entry = 0;
+  {
+    Cursor k[kRingStages];
+    int32_t e[kRingStages];
+#pragma unroll
+    for (int s = 0; s < kRingStages; ++s) {
+      k[s] = ahead;
+      e[s] = x0 + s < x1 ? entry_of(ahead) : 0;
+      if (x0 + s + 1 < x1) advance(ahead);
+    }
+    if (x_ahead < x1) entry = entry_of(ahead);
+#pragma unroll
+    for (int s = 0; s < kRingStages; ++s) {
+      row_mask[s] = x0 + s < x1 ? issue(s, k[s], e[s]) : 0;
+      cp_async_commit();
+    }
+  }
+  auto feed = [&](int stage) -> uint32_t {
+    uint32_t mask = 0;
+    if (x_ahead < x1) {
+      const Cursor now = ahead;
+      const int32_t e = entry;
+      if (++x_ahead < x1) {
+        advance(ahead);
+        entry = entry_of(ahead);
+      }
+      mask = issue(stage, now, e);
+    }
+    cp_async_commit();
+    return mask;
+  };
+
+  RingWarp<T, D, NH16> rw;
+  rw.begin(p, cur.b, h0, nheads, g, c);
+  for (int x = x0; x < x1; ++x) {
+    const int stage = (x - x0) % kRingStages;
+    cp_async_wait<kRingStages - 1>();
+    __syncwarp();
+    uint32_t rows_ok = 0;
+#pragma unroll
+    for (int s = 0; s < kRingStages; ++s)
+      if (s == stage) rows_ok = row_mask[s];
+    rw.step(p, my_ring + stage * R::kStageBytes, rows_ok, cur.b, h0, nheads, (int64_t)cur.s * 16, cur.L, g, c, [&] {
+      const uint32_t mask = feed(stage);
+#pragma unroll
+      for (int s = 0; s < kRingStages; ++s)
+        if (s == stage) row_mask[s] = mask;
+    });
+    const bool last = x + 1 == x1;
+    if (last || cur.s + 1 == cur.steps) {   // the end of the sequence, or of the share
+      rw.gather_sums();
+      const int64_t slot = ((int64_t)(share + cur.b) * kv_heads + kvh) * nheads;
+      float* ml = ws + (int64_t)(shares + p.batch) * kv_heads * nheads * D;
+      if (c == 0) {
+        if (g < nheads) *reinterpret_cast<float2*>(ml + (slot + g) * 2) = make_float2(rw.m0, rw.l0);
+        if (NH16 && g + 8 < nheads) *reinterpret_cast<float2*>(ml + (slot + g + 8) * 2) = make_float2(rw.m1, rw.l1);
+      }
+      // a thread's columns of a head are neighbours: d = 8 g + m and, from the second half of the fragments, 64 + 8 g + m (D 128) or 8 g + 4 + m
+#pragma unroll
+      for (int hn = 0; hn < HN; ++hn)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int hh = 8 * hn + 2 * c + e;
+          if (hh >= nheads) continue;
+          float* dst = ws + (slot + hh) * D + g * 8;
+#pragma unroll
+          for (int m = 0; m < MT; m += 4) {
+            *reinterpret_cast<float4*>(dst + m) = make_float4(rw.acc[m][hn][e], rw.acc[m + 1][hn][e], rw.acc[m + 2][hn][e], rw.acc[m + 3][hn][e]);
+            *reinterpret_cast<float4*>(dst + (D == 128 ? 64 : 4) + m) =
+                make_float4(rw.acc[m][hn][2 + e], rw.acc[m + 1][hn][2 + e], rw.acc[m + 2][hn][2 + e], rw.acc[m + 3][hn][2 + e]);
+          }
+        }
+      if (!last) {
+        advance(cur);
+        rw.begin(p, cur.b, h0, nheads, g, c);
+      }
+    } else {
+      advance(cur);
+    }
+  }
+  report_bad_block(p, bad_block);
+}
+
 // Merges the splits of one (sequence, head): the weight of every split is formed once, in parallel, and the columns are
 // summed by 16-byte vectors over groups of splits.  Bound by latency - a few KB per CTA - so nothing in it is a serial
 // chain over the splits except the last sum of 128 / (D / 4) partial columns.
 constexpr int kMaxCombine = 1024;   // split weights held in shared memory; more splits are taken in rounds
 
-template <typename T>
+// STREAM: the slots of sdpa_decode_stream_kernel; `nchunks` is then its number of shares.
+template <typename T, bool STREAM>
 __global__ void __launch_bounds__(128)
     sdpa_decode_combine_kernel(const SdpaParams p, const int chunk, const int nchunks, const float* ws) {
   __shared__ float weight[kMaxCombine];
   __shared__ float red[8];
   __shared__ float4 cols[128];
-  pdl_wait();   // the partial results of the kernel before this one
+  // The lengths come from a launch before the kernel that this one waits for, which has begun only after that one: they can be read now.
+  if constexpr (!STREAM) pdl_wait();   // the partial results of the kernel before this one
   const int b = blockIdx.y;
   const int hl = blockIdx.x;
   const int h = p.head_begin + hl;
@@ -745,39 +974,81 @@ __global__ void __launch_bounds__(128)
   const int Hc = p.head_count;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t L = decode_len(p, b);
-  int nvalid = (int)((L + chunk - 1) / chunk);
-  if (nvalid > nchunks) nvalid = nchunks;
-  const int64_t slot0 = ((int64_t)b * Hc + hl) * nchunks;
-  const float2* ml = reinterpret_cast<const float2*>(ws + (int64_t)p.batch * Hc * nchunks * D) + slot0;
+  int nvalid;
+  int64_t slot0;
+  const int hop = STREAM ? p.head_count : 1;   // partials from one of the head to its next
+  if constexpr (STREAM) {
+    __shared__ int sums[8];
+    int before = 0, all = 0;
+    for (int i = tid; i < p.batch; i += 128) {
+      const int n = stream_steps(p, i);
+      all += n;
+      if (i < b) before += n;
+    }
+    all = __reduce_add_sync(0xffffffffu, all);
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) {
+      sums[warp] = all;
+      sums[4 + warp] = before;
+    }
+    __syncthreads();
+    const StreamPlan plan = stream_plan(sums[0] + sums[1] + sums[2] + sums[3], nchunks);
+    const int first = sums[4] + sums[5] + sums[6] + sums[7], steps = stream_steps(p, b);
+    nvalid = steps > 0 ? (first + steps - 1) / plan.per - first / plan.per + 1 : 0;
+    slot0 = (int64_t)(first / plan.per + b) * Hc + hl;
+    pdl_wait();
+  } else {
+    nvalid = (int)((L + chunk - 1) / chunk);
+    if (nvalid > nchunks) nvalid = nchunks;
+    slot0 = ((int64_t)b * Hc + hl) * nchunks;
+  }
+  const float2* ml = reinterpret_cast<const float2*>(ws + (STREAM ? (int64_t)(nchunks + p.batch) * Hc : (int64_t)p.batch * Hc * nchunks) * D) + slot0;
 
+  const int vecs = D / 4, groups = 128 / vecs;      // D = 64, 128, 256: 8, 4, 2 groups of splits
+  const int grp = tid / vecs, d4 = tid - grp * vecs;
+  const float4* rows = reinterpret_cast<const float4*>(ws + slot0 * D) + d4;
+  float4 early[4];   // STREAM: the thread's first columns, requested with the maxima
+  if constexpr (STREAM) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      early[i] = grp + i * groups < nvalid ? rows[(int64_t)(grp + i * groups) * hop * vecs] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   float M = -INFINITY;
-  for (int c = tid; c < nvalid; c += 128) M = fmaxf(M, ml[c].x);
+  for (int c = tid; c < nvalid; c += 128) M = fmaxf(M, ml[(int64_t)c * hop].x);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
   if (lane == 0) red[warp] = M;
   __syncthreads();
   M = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
 
-  const int vecs = D / 4, groups = 128 / vecs;      // D = 64, 128, 256: 8, 4, 2 groups of splits
-  const int grp = tid / vecs, d4 = tid - grp * vecs;
-  const float4* rows = reinterpret_cast<const float4*>(ws + slot0 * D) + d4;
   float lsum = 0.f;
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int c0 = 0; c0 < nvalid; c0 += kMaxCombine) {
     const int n = min(kMaxCombine, nvalid - c0);
     if (c0 > 0) __syncthreads();
     for (int c = tid; c < n; c += 128) {
-      const float2 v = ml[c0 + c];
+      const float2 v = ml[(int64_t)(c0 + c) * hop];
       const float w = v.x == -INFINITY ? -1.f : softmax_exp<T>(v.x - M);   // -1: a split that saw no key
       weight[c] = w;
       if (v.x != -INFINITY) lsum = fmaf(w, v.y, lsum);
     }
     __syncthreads();
+    int c = grp;
+    if constexpr (STREAM) {
+      if (c0 == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i, c += groups) {
+          const float w = c < n ? weight[c] : -1.f;
+          if (w < 0.f) continue;
+          a.x = fmaf(w, early[i].x, a.x); a.y = fmaf(w, early[i].y, a.y); a.z = fmaf(w, early[i].z, a.z); a.w = fmaf(w, early[i].w, a.w);
+        }
+      }
+    }
 #pragma unroll 4
-    for (int c = grp; c < n; c += groups) {
+    for (; c < n; c += groups) {
       const float w = weight[c];
       if (w < 0.f) continue;   // its columns are undefined; a weight that underflows to 0 still carries their NaN and Inf
-      const float4 x = rows[(int64_t)(c0 + c) * vecs];
+      const float4 x = rows[(int64_t)(c0 + c) * hop * vecs];
       a.x = fmaf(w, x.x, a.x); a.y = fmaf(w, x.y, a.y); a.z = fmaf(w, x.z, a.z); a.w = fmaf(w, x.w, a.w);
     }
   }
@@ -846,11 +1117,33 @@ cudaError_t launch_partial_g(const SdpaParams& p, const DecodePlan& plan, float*
   return launch_partial<T, D, 8>(p, plan, ws, merge, stream);
 }
 
+constexpr int stream_ctas(int head_dim, int num_sms) { return (head_dim == 128 ? 2 : 3) * num_sms; }   // resident at once
+
+template <typename T, int D, bool NH16>
+cudaError_t launch_stream(const SdpaParams& p, const DecodePlan& plan, float* ws, cudaStream_t stream) {
+  auto kern = p.block_table ? sdpa_decode_stream_kernel<T, D, NH16, true> : sdpa_decode_stream_kernel<T, D, NH16, false>;
+  constexpr int smem = RingCfg<D>::kSmemBytes;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  const int kv_heads = p.head_count / p.group, shares = plan.stream_ctas * kDecWarps / kv_heads;
+  e = launch_dependent(kern, dim3((unsigned)plan.stream_ctas), kDecWarps * 32, smem, stream, p, ws, kv_heads, shares);
+  if (e != cudaSuccess) return e;
+  return launch_dependent(sdpa_decode_combine_kernel<T, true>, dim3((unsigned)p.head_count, (unsigned)p.batch), 128, 0, stream, p, 0, shares,
+                          static_cast<const float*>(ws));
+}
+
 template <typename T>
 cudaError_t launch_decode_t(const SdpaParams& p, const DecodePlan& plan, float* ws, cudaStream_t stream, int* launches) {
   const int nchunks = plan.nchunks;
   const int merge = plan.cluster > 1 ? (nchunks == 1 ? kMergeCluster : kMergeBoth) : (nchunks == 1 ? kMergeDirect : kMergeWorkspace);
   cudaError_t e;
+  if constexpr (sizeof(T) == 2) {
+    if (plan.stream_ctas > 0) {
+      *launches = 2;
+      if (p.head_dim == 64) return p.group <= 8 ? launch_stream<T, 64, false>(p, plan, ws, stream) : launch_stream<T, 64, true>(p, plan, ws, stream);
+      return p.group <= 8 ? launch_stream<T, 128, false>(p, plan, ws, stream) : launch_stream<T, 128, true>(p, plan, ws, stream);
+    }
+  }
   switch (p.head_dim) {
     case 64: e = launch_partial_g<T, 64>(p, plan, ws, merge, stream); break;
     case 128: e = launch_partial_g<T, 128>(p, plan, ws, merge, stream); break;
@@ -867,7 +1160,7 @@ cudaError_t launch_decode_t(const SdpaParams& p, const DecodePlan& plan, float* 
   dim3 grid((unsigned)p.head_count, (unsigned)p.batch);
   *launches = 2;
   // chunk 1: with clusters every slot is written (m = -inf where there was no key)
-  return launch_dependent(sdpa_decode_combine_kernel<T>, grid, 128, 0, stream, p, plan.cluster > 1 ? 1 : plan.chunk, nchunks, static_cast<const float*>(ws));
+  return launch_dependent(sdpa_decode_combine_kernel<T, false>, grid, 128, 0, stream, p, plan.cluster > 1 ? 1 : plan.chunk, nchunks, static_cast<const float*>(ws));
 }
 
 
@@ -996,6 +1289,35 @@ void decode_plan_clusters(const SdpaParams& p, int dtype, int num_sms, DecodePla
   if (clusters > plan->nchunks) clusters = plan->nchunks;   // never more workspace
   plan->cluster = (int)cluster;
   plan->nchunks = (int)clusters;
+}
+
+// Equal shares of all keys pay where the plan without them has no clusters, two waves of them, or CTAs with so many keys that the longest
+// sequence's run on alone.  Below 48 items, and with less than that to a CTA, the second launch and the way to the first keys (10 us)
+// weigh more.  Lengths from 1 / 8 or 1 / 16 of the keys to all of them, us before -> after; items are (sequence, KV head) pairs:
+//   pays       128 items, 2048 keys, D 128 26.9 -> 21.5; 72 items, 1584 keys 16.3 -> 14.5; 182 items, 750 keys 19.6 -> 16.8; 228 items, 1117
+//              keys 28.6 -> 24.9; 266 items, 353 keys 16.9 -> 13.8; 222 items, 4234 keys 59 -> 51; 512 items, 4096 keys 115 -> 106;
+//              heads of 64: 60 items, 3549 keys 15.6 -> 14.6; 405 items, 483 keys 13.7 -> 12.5; 128 items, 2048 keys 18.5 -> 15.9
+//   does not   96 items, 618 keys 10.2 -> 11.2; 110 items, 241 keys 7.2 -> 11.0; 54 items, 1395 keys 16.1 -> 17.9; 24 items, 5170 keys 15.3 ->
+//              16.9; 20 items, 8626 keys 21.5 -> 23.1; heads of 64: 190 items, 814 keys 11.0 -> 15.4; 84 items, 2711 keys 15.9 -> 19.4
+// Sequences that are all as long as the tensor lose a little (128 items of 2048 keys 29.6 -> 31.7): the host does not see the lengths.
+int64_t decode_stream_bytes(const SdpaParams& p, int dtype, int num_sms, const DecodePlan& chunks, int* ctas) {
+  *ctas = 0;
+  if (!takes_ring(p, dtype) || chunks.nchunks <= 1) return 0;
+  const int kv_heads = p.head_count / p.group, n = stream_ctas(p.head_dim, num_sms);
+  const int64_t items = (int64_t)p.batch * kv_heads, steps = (p.seq_kv + 15) / 16;
+  if (items < 48 || items * steps > 0x3fffffff || p.batch > 256 || kv_heads > n * kDecWarps) return 0;
+  // Long launches stream at the memory's rate either way, and chunks read larger pieces: of 400 MB, or with the heads of a token side by
+  // side of 1.2 GB, on (2048 items of 4096 keys 382 -> 405 us; in a pool 512 items of 4096 keys, 1.07 GB, 115 -> 106).
+  if (items * p.seq_kv * p.head_dim * 4 > (p.block_table || p.ks[1] < p.ks[2] ? 1200000000 : 400000000)) return 0;
+  SdpaParams q = p;
+  const int32_t some_lengths = 0;
+  q.kv_len = &some_lengths;   // (only whether there are any)
+  DecodePlan plan = chunks;
+  decode_plan_clusters(q, dtype, num_sms, &plan);
+  const int64_t parts = (int64_t)plan.cluster * plan.nchunks;
+  if (plan.cluster > 1 && items * parts <= n && p.seq_kv / parts * p.head_dim < 100000) return 0;
+  *ctas = n;
+  return ((int64_t)(n * kDecWarps / kv_heads) + p.batch) * kv_heads * p.group * (p.head_dim + 2) * (int64_t)sizeof(float);
 }
 
 cudaError_t launch_decode(const SdpaParams& p, int dtype, const DecodePlan& plan, float* workspace, cudaStream_t stream, int* launches) {
