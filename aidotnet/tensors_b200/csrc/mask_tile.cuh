@@ -83,6 +83,19 @@ __device__ __forceinline__ void request(uint32_t tile, const float* src, int64_t
   cp_async_commit_f();
 }
 
+// The same for rows that are keys: the lane's key is the tile's row, the mask's row the tile's column.
+__device__ __forceinline__ void request_columns(uint32_t tile, const float* src, int64_t row_stride, int64_t key_stride, int rows, int keys, int lane) {
+  const float* p = src + lane * key_stride;
+  const bool in = lane < keys;
+#pragma unroll
+  for (int r = 0; r < 32; ++r) {
+    const bool ok = in && r < rows;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(tile + at(lane, r)), "l"(ok ? p : src), "r"(ok ? 4u : 0u) : "memory");
+    p += row_stride;
+  }
+  cp_async_commit_f();
+}
+
 // ... and out of registers (load_rows).
 __device__ __forceinline__ void put(uint32_t tile, const float (&x)[32], int lane) {
 #pragma unroll

@@ -10,6 +10,7 @@
 //               terms of P and dS into it, and the gradients of the block before added up in registers
 //   warps 8-11  the blocks from global memory through registers into swizzled images of their terms, two buffers
 //   warps 12-13 UMMA issuers (one elected lane each) of the scores and of the gradients; the first one owns TMEM
+//   warps 14-15 a bias: asynchronous copies into the row warps' tiles (by the row warps themselves they were half of a block's 6000 cycles)
 // The scores of block j + 1 are formed while the row threads work on block j.  The gradient accumulators start afresh with every
 // block, so that the tensor cores, which truncate when they accumulate, never add more than four times into one cell.
 // An infinity times a term that is 0 is not a number, a value above the largest bf16 rounds to an infinity, and a block is multiplied
@@ -20,6 +21,7 @@
 // shared memory: every gradient is summed in a fixed order (deterministic, no atomics).
 #include "common.cuh"
 #include "ffma2.cuh"
+#include "mask_tile.cuh"
 #include "sm100_ptx.cuh"
 #include "split3.cuh"
 
@@ -41,7 +43,7 @@ constexpr int kStrImage = split3::kTerms * kStrPlane;             // U or W of o
 constexpr int kYOff = split3::kTerms * kOwnPlane, kUOff = 2 * kYOff;
 constexpr int kRowOff = kUOff + 4 * kStrImage;                    // -lse and -delta of streamed query rows: [2 buffers][2][64]
 constexpr int kMaskOff = kRowOff + 2 * 2 * kStr * 4;
-constexpr int kBars = 8;                                          // full[2], g_full[2], s_full, s_empty, p_ready, xy_full
+constexpr int kBars = 10;                                         // full[2], g_full[2], s_full, s_empty, p_ready, xy_full, mask_full, mask_empty
 constexpr int bar_off(bool plain) { return kMaskOff + (plain ? 0 : kWorkers * 32 * 4); }
 constexpr int smem_bytes(bool plain) { return bar_off(plain) + 8 * kBars + 8 + 1024; }
 static_assert(smem_bytes(false) <= 227 * 1024, "shared memory");
@@ -177,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t bar_full = smem_base + bar_off(PLAIN), bar_g = bar_full + 16, bar_s = bar_g + 16, bar_se = bar_s + 8, bar_p = bar_se + 8, bar_xy = bar_p + 8;
+  const uint32_t bar_full = smem_base + bar_off(PLAIN), bar_g = bar_full + 16, bar_s = bar_g + 16, bar_se = bar_s + 8, bar_p = bar_se + 8, bar_xy = bar_p + 8, bar_mf = bar_xy + 8, bar_me = bar_mf + 8;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem_gen + bar_off(PLAIN) + 8 * kBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -193,6 +195,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
     mbar_init(bar_s, 1);
     mbar_init(bar_se, kWorkers / 32);
     mbar_init(bar_p, kWorkers / 32);
+    mbar_init(bar_mf, 2);
+    mbar_init(bar_me, kWorkers / 32);
     ptx::fence_mbar_init();
   }
   if (warp == kIssuer) {
@@ -225,6 +229,15 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
     const int s = s_begin + j, g = KEYS ? s / per_head : 0;
     return Block{g, first + (int64_t)(s - g * per_head) * kStr};
   };
+  // Where the mask of own rows 32 * quarter .. and rows 32 * half .. of block j lies, and how much of it there is.
+  const bool add = !PLAIN && p.mask_kind == AIDN_MASK_ADD_F32;
+  auto mask_at = [&](int j, int quarter, int half, int& rows, int& keys) {
+    const Block bk = block_of(j);
+    const int64_t o0 = own0 + quarter * 32, s0 = bk.base + half * kHalf, key = KEYS ? o0 : s0, query = KEYS ? s0 : o0;
+    rows = masktile::clamp32(p.seq_q - query);
+    keys = masktile::clamp32(kv_limit - key);
+    return b * p.mask_stride[0] + (h0 + bk.g) * p.mask_stride[1] + query * p.mask_stride[2] + key * p.mask_stride[3];
+  };
   bool alive = true;
   auto wait = [&](uint32_t bar, int phase) {   // by whole warps
     alive = alive && mbar_wait(bar, (uint32_t)(phase & 1), abort_flag, tp.wait_budget_ns);
@@ -240,40 +253,15 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
     const float* xb = KEYS ? kb : qb;
     const float* yb = KEYS ? vb : gb;
     const int64_t xstr = KEYS ? p.ks[2] : p.qs[2], ystr = KEYS ? p.vs[2] : bp.dos[2];
-    float* mask_s = PLAIN ? nullptr : reinterpret_cast<float*>(smem_gen + kMaskOff) + warp * 32 * 32;
-    // The mask of the warp's 32 own rows and its 32 rows of block j: lanes take keys, so that it is read in whole lines, and the
-    // lane that owns a row finds its values in shared memory (16-byte chunk c of row r at c ^ r: eight
-    // rows read theirs without a conflict).
-    auto mask_at = [](int r, int k) { return r * 32 + (((k >> 2) ^ (r & 7)) << 2) + (k & 3); };
-    auto fetch_mask_tile = [&](int j) {
-      const Block bk = block_of(j);
-      const int64_t o0 = own0 + quarter * 32, s0 = bk.base + half * kHalf;
-      const int64_t key = (KEYS ? o0 : s0) + lane, q0 = KEYS ? s0 : o0;
-      const int64_t at0 = b * p.mask_stride[0] + (h0 + bk.g) * p.mask_stride[1] + q0 * p.mask_stride[2] + key * p.mask_stride[3];
-      const int64_t from64 = p.causal ? key - p.causal_offset - q0 : 0;   // rows before it do not see the key
-      const int64_t count64 = key < kv_limit ? p.seq_q - q0 : 0;
-      const int from = from64 < 0 ? 0 : (from64 > 32 ? 32 : (int)from64), count = count64 > 32 ? 32 : (int)count64;
-      if (p.mask_kind == AIDN_MASK_KEEP_U8) {
-#pragma unroll
-        for (int i0 = 0; i0 < 32; i0 += 16) {
-          uint32_t x[16];
-#pragma unroll
-          for (int e = 0; e < 16; ++e)
-            x[e] = i0 + e >= from && i0 + e < count ? static_cast<const uint8_t*>(p.mask)[at0 + (i0 + e) * p.mask_stride[2]] : 0;
-#pragma unroll
-          for (int e = 0; e < 16; ++e) mask_s[KEYS ? mask_at(lane, i0 + e) : mask_at(i0 + e, lane)] = x[e] ? 1.f : 0.f;
-        }
-      } else {
-#pragma unroll 8
-        for (int i = 0; i < 32; ++i) {
-          const bool ok = i >= from && i < count;
-          const int at = KEYS ? mask_at(lane, i) : mask_at(i, lane);
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;"
-                       ::"r"(smem_u32(mask_s + at)), "l"(static_cast<const float*>(p.mask) + (ok ? at0 + i * p.mask_stride[2] : 0)), "r"(ok ? 4u : 0u)
-                       : "memory");
-        }
-      }
-      cp_async_commit_f();
+    // The mask of the warp's 32 own rows and its 32 rows of block j: a bias in its tile, a keep-mask as bits of the thread's row, one block
+    // ahead; lanes take keys, so that either is read in whole lines.
+    const uint32_t mask_s = smem_base + (uint32_t)(kMaskOff + warp * masktile::kBytes);
+    uint32_t keep = ~0u;
+    auto fetch_keep = [&](int j) {
+      int rows, keys;
+      const int64_t at0 = mask_at(j, quarter, half, rows, keys);
+      keep = KEYS ? masktile::keep_column_of(p, at0, p.mask_stride[2], p.mask_stride[3], rows, keys, lane)
+                  : masktile::keep_bits_of(p, at0, p.mask_stride[2], p.mask_stride[3], rows, keys, lane);
     };
 
     uint64_t acc0[kCols / 2], acc1[KEYS ? kCols / 2 : 1];
@@ -283,20 +271,31 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
       if constexpr (KEYS) acc1[c] = 0;
     }
     if (n > 0) {
-      if constexpr (!PLAIN) fetch_mask_tile(0);
-#pragma unroll 2
-      for (int idx = tid; idx < kOwn * CPR; idx += kWorkers) {
-        const int r = idx / CPR, c = idx % CPR, d = c * 8;
-        const bool lo = own0 + r < own_end && d < D, hi = own0 + r < own_end && d + 4 < D;
-        const float* xr = xb + (own0 + r) * xstr + d;
-        const float* yr = yb + (own0 + r) * ystr + d;
-        const ulonglong2 xa = split3::load4(xr, lo), xc = split3::load4(xr + 4, hi), ya = split3::load4(yr, lo), yc = split3::load4(yr + 4, hi);
-        split3::store_split8(x_s + split3::chunk_at(r, c), kOwnPlane, xa, xc);
-        split3::store_split8(y_s + split3::chunk_at(r, c), kOwnPlane, ya, yc);
+      {
+        constexpr int kPer = kOwn * CPR / kWorkers;
+        ulonglong2 xv[kPer][2], yv[kPer][2];   // all requested before the first is cut: one latency
+#pragma unroll
+        for (int e = 0; e < kPer; ++e) {
+          const int idx = tid + e * kWorkers, r = idx / CPR, d = idx % CPR * 8;
+          const bool lo = own0 + r < own_end && d < D, hi = own0 + r < own_end && d + 4 < D;
+          const float* xr = xb + (own0 + r) * xstr + d;
+          const float* yr = yb + (own0 + r) * ystr + d;
+          xv[e][0] = split3::load4(xr, lo);
+          xv[e][1] = split3::load4(xr + 4, hi);
+          yv[e][0] = split3::load4(yr, lo);
+          yv[e][1] = split3::load4(yr + 4, hi);
+        }
+#pragma unroll
+        for (int e = 0; e < kPer; ++e) {
+          const int idx = tid + e * kWorkers;
+          split3::store_split8(x_s + split3::chunk_at(idx / CPR, idx % CPR), kOwnPlane, xv[e][0], xv[e][1]);
+          split3::store_split8(y_s + split3::chunk_at(idx / CPR, idx % CPR), kOwnPlane, yv[e][0], yv[e][1]);
+        }
       }
       ptx::fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_xy);
+      if (!PLAIN && !add) fetch_keep(0);
       float nl_own = -INFINITY, nd_own = 0.f;   // -lse (-inf where no key is visible, which makes every P 0) and -delta
       if (!KEYS && own < p.seq_q) {
         const float lse = p.lse[((int64_t)b * p.num_q_heads + h0) * p.seq_q + own];
@@ -359,18 +358,22 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
         const int lo = from < 0 ? 0 : (from > kHalf ? kHalf : (int)from), hi = to < 0 ? 0 : (to > kHalf ? kHalf : (int)to);
         const bool whole = !__any_sync(0xffffffffu, lo > 0 || hi < kHalf);
         if constexpr (!PLAIN) {   // the finished logits
-          cp_async_wait_f<0>();   // every lane's copies of the mask are there
-          __syncwarp();
+          if (add) {
+            wait(bar_mf, j);
+            if (!alive) break;
 #pragma unroll
-          for (int k = 0; k < kHalf / 2; k += 2) {
-            const ulonglong2 mk = *reinterpret_cast<const ulonglong2*>(mask_s + mask_at(lane, 2 * k));
-            if (p.mask_kind == AIDN_MASK_ADD_F32) {
-              pr[k] = fma2(pr[k], scale2, mk.x);
-              pr[k + 1] = fma2(pr[k + 1], scale2, mk.y);
-            } else {
-              const float2 x = unpack2(mul2(pr[k], scale2)), y = unpack2(mul2(pr[k + 1], scale2)), u = unpack2(mk.x), v = unpack2(mk.y);
-              pr[k] = pack2(u.x == 0.f ? -INFINITY : x.x, u.y == 0.f ? -INFINITY : x.y);
-              pr[k + 1] = pack2(v.x == 0.f ? -INFINITY : y.x, v.y == 0.f ? -INFINITY : y.y);
+            for (int k = 0; k < kHalf / 2; k += 2) {
+              const float4 m4 = masktile::row4(mask_s, k / 2, lane);
+              pr[k] = fma2(pr[k], scale2, pack2(m4.x, m4.y));
+              pr[k + 1] = fma2(pr[k + 1], scale2, pack2(m4.z, m4.w));
+            }
+            __syncwarp();   // the values have been read
+            if (lane == 0) mbar_arrive(bar_me);
+          } else {
+#pragma unroll
+            for (int k = 0; k < kHalf / 2; ++k) {
+              const float2 x = unpack2(mul2(pr[k], scale2));
+              pr[k] = pack2(keep & (1u << (2 * k)) ? x.x : -INFINITY, keep & (2u << (2 * k)) ? x.y : -INFINITY);
             }
           }
         }
@@ -406,10 +409,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
           }
         }
         if constexpr (!PLAIN) {
-          if (j + 1 < n) {
-            __syncwarp();   // the values have been read
-            fetch_mask_tile(j + 1);
-          }
+          if (!add && j + 1 < n) fetch_keep(j + 1);
         }
         if (j > 0) add_block(j - 1);   // the terms of P and dS of block j - 1 have been read, and so have its gradients
         if (!alive) break;
@@ -573,6 +573,24 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
         }
         if (leader) ptx::tc_commit(bar_g + 8 * (j & 1));
       }
+    } else if (add) {   // half of every row warp's tiles each
+      const int half = warp - kIssuer - 2;
+      for (int j = 0; j < n; ++j) {
+        if (j > 0) wait(bar_me, j - 1);
+        if (!alive) break;
+#pragma unroll 1
+        for (int quarter = 0; quarter < 4; ++quarter) {
+          int rows, keys;
+          const int64_t at0 = mask_at(j, quarter, half, rows, keys);
+          const uint32_t tile = smem_base + (uint32_t)(kMaskOff + (half * 4 + quarter) * masktile::kBytes);
+          const float* src = static_cast<const float*>(p.mask) + at0;
+          if (KEYS) masktile::request_columns(tile, src, p.mask_stride[2], p.mask_stride[3], rows, keys, lane);
+          else masktile::request(tile, src, p.mask_stride[2], p.mask_stride[3], rows, keys, lane);
+        }
+        cp_async_wait_f<0>();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_mf);
+      }
     }
   }
 
@@ -596,20 +614,32 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
     if (warp < kWorkers / 32 && !*abort_flag) {
       const int64_t out_rows = KEYS ? p.seq_kv : p.seq_q;
       const int64_t base = KEYS ? ((int64_t)b * kv_heads + blockIdx.y) * out_rows : ((int64_t)b * p.head_count + hl0) * out_rows;
-      const int d4s = D / 4, items = kOwn * d4s * (KEYS ? 2 : 1);
-      for (int idx = rank * kWorkers + tid; idx < items; idx += tp.splits * kWorkers) {
-        const int which = idx / (kOwn * d4s), at = idx - which * kOwn * d4s, r = at / d4s, d = (at - r * d4s) * 4;
-        if (own0 + r >= out_rows) continue;
-        const uint32_t src = smem_base + (uint32_t)(((which * kOwn + r) * kPartPitch + d) * 4);
-        float y[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
+      // Four vectors of every CTA in flight, and nothing divided (one at a time, the sums of two CTAs took 8000 cycles).
+      constexpr int kVecs = KS * 4, kItems = kOwn * kVecs * (KEYS ? 2 : 1);   // (of a row; those past head_dim are not stored)
+      const int hop = tp.splits * kWorkers;
+      for (int idx0 = rank * kWorkers + tid; idx0 < kItems; idx0 += 4 * hop) {
+        float4 y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
         for (int i = 0; i < tp.splits; ++i) {
-          const float2 a = ld_cluster_f2(src, (uint32_t)i), c = ld_cluster_f2(src + 8, (uint32_t)i);
-          y[0] += a.x; y[1] += a.y; y[2] += c.x; y[3] += c.y;
+          float4 u[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int idx = idx0 + e * hop < kItems ? idx0 + e * hop : idx0;
+            u[e] = ld_cluster_f4(smem_base + (uint32_t)((idx / kVecs * kPartPitch + idx % kVecs * 4) * 4), (uint32_t)i);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) y[e].x += u[e].x, y[e].y += u[e].y, y[e].z += u[e].z, y[e].w += u[e].w;
         }
-        const float f = which ? 1.f : p.scale;
-        float* out = (which ? bp.dv : (KEYS ? bp.dk : bp.dq)) + (base + own0 + r) * D + d;
-        *reinterpret_cast<float4*>(out) = make_float4(y[0] * f, y[1] * f, y[2] * f, y[3] * f);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int idx = idx0 + e * hop, which = idx / (kOwn * kVecs), r = idx / kVecs % kOwn, d = idx % kVecs * 4;
+          if (idx >= kItems || own0 + r >= out_rows || d >= D) continue;
+          const float f = which ? 1.f : p.scale;
+          float* out = (which ? bp.dv : (KEYS ? bp.dk : bp.dq)) + (base + own0 + r) * D + d;
+          *reinterpret_cast<float4*>(out) = make_float4(y[e].x * f, y[e].y * f, y[e].z * f, y[e].w * f);
+        }
       }
     }
     __syncwarp();

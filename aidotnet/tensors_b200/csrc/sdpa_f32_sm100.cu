@@ -7,6 +7,7 @@
 //               of P back into TMEM over the scores, P V of the block before out of TMEM and added to the output in registers
 //   warps 8-11  K and V from global memory through registers into swizzled images of their terms
 //   warps 12-13 UMMA issuers (one elected lane each) of the scores and of P V; the first one owns TMEM
+//   warps 14-15 a bias: asynchronous copies into the row warps' tiles
 // S(j + 1) and P(j - 1) V are formed while the softmax of block j runs.  TMEM: two score buffers (leading products, small ones;
 // P over them) and one pair of output accumulators that start afresh with every block, so that the tensor cores, which
 // truncate when they accumulate, never add more than head_dim / 16 or four times into one cell.
@@ -22,6 +23,7 @@
 // Launches with few tiles cut the keys over the CTAs of a cluster, which merge through distributed shared memory.
 #include "common.cuh"
 #include "ffma2.cuh"
+#include "mask_tile.cuh"
 #include "sm100_ptx.cuh"
 #include "split3.cuh"
 
@@ -36,7 +38,6 @@ using ptx::tmem_ld16;
 using ptx::tmem_ld32;
 
 constexpr int kRows = 128, kKeys = 64, kHalf = 32;
-constexpr int kMaskPitch = 33;   // floats per row of a warp's mask tile
 constexpr int kIssuer = 12;   // warp
 constexpr int kWorkers = 256, kLoaders = 128, kThreads = 512;   // row threads, loading threads, and a warpgroup with the issuer
 
@@ -55,10 +56,10 @@ struct TCfg {
   static constexpr int kImage = split3::kTerms * kKPlane;
   static constexpr int kKOff = split3::kTerms * kQPlane, kVOff = kKOff + kBufs * kImage;
   static constexpr int kMaskOff = kVOff + kBufs * kImage;
-  static constexpr int kXOff = kMaskOff + (PLAIN ? 0 : kWorkers * kMaskPitch * 4);
-  static constexpr int kXBufs = DP == 128 && !PLAIN ? 1 : 2;   // row maxima: [2][2 halves][128], or one set in the mask tiles' padding
-  static constexpr int kBarOff = kXOff + (kXBufs == 2 ? 2 * 2 * kRows * 4 : 0);
-  static constexpr int kNumBars = 1 /*q*/ + 2 /*k_full*/ + 2 /*v_full*/ + 2 /*s_full*/ + 1 /*p_ready*/ + 2 /*o_full*/ + 4 /*pair*/;
+  static constexpr int kXOff = kMaskOff + (PLAIN ? 0 : kWorkers / 32 * masktile::kBytes);
+  static constexpr int kXBufs = DP == 128 && !PLAIN ? 1 : 2;   // row maxima: sets of [2 halves][128]
+  static constexpr int kBarOff = kXOff + kXBufs * 2 * kRows * 4;
+  static constexpr int kNumBars = 1 /*q*/ + 2 /*k_full*/ + 2 /*v_full*/ + 2 /*s_full*/ + 1 /*p_ready*/ + 2 /*o_full*/ + 4 /*pair*/ + 2 /*mask*/;
   static constexpr int kSmem = kBarOff + 8 * kNumBars + 8 + 1024;
   static_assert(kSmem <= 227 * 1024, "shared memory");
   static constexpr int kPartPitch = kOut + 4;               // floats per row of a CTA's partial output, over the images
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t bar_q = smem_base + C::kBarOff, bar_k = bar_q + 8, bar_v = bar_k + 16, bar_s = bar_v + 16, bar_p = bar_s + 16, bar_o = bar_p + 8,
-                 bar_pair = bar_o + 16;
+                 bar_pair = bar_o + 16, bar_mf = bar_pair + 32, bar_me = bar_mf + 8;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem_gen + C::kBarOff + 8 * C::kNumBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -181,6 +182,8 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
     mbar_init(bar_q, kWorkers / 32);
     mbar_init(bar_p, kWorkers / 32);
     for (int i = 0; i < 4; ++i) mbar_init(bar_pair + 8 * i, 2);
+    mbar_init(bar_mf, 2);
+    mbar_init(bar_me, kWorkers / 32);
     ptx::fence_mbar_init();
   }
   if (warp == kIssuer) {
@@ -211,6 +214,14 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
     if (lane == 0) mbar_arrive(bar);
   };
   constexpr int CPR = DP / 8;   // chunks of eight columns per row
+  // Where the mask of rows 32 * quarter .. and keys 32 * half .. of block j lies, and how much of it there is.
+  const bool add = !PLAIN && p.mask_kind == AIDN_MASK_ADD_F32;
+  auto mask_at = [&](int j, int quarter, int half, int& rows, int& keys) {
+    const int64_t key = (blk0 + j) * kKeys + half * kHalf, r0 = row0 + quarter * 32;
+    rows = masktile::clamp32(p.seq_q - r0);
+    keys = masktile::clamp32(kv_limit - key);
+    return b * p.mask_stride[0] + h * p.mask_stride[1] + r0 * p.mask_stride[2] + key * p.mask_stride[3];
+  };
   if (warp < kWorkers / 32) {
     ptx::setmaxnreg_inc<C::kRegRows>();
     const int quarter = warp & 3, half = warp >> 2, lrow = quarter * 32 + lane;
@@ -224,48 +235,15 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
       if (lane == 0) mbar_arrive(bar_pair + 8 * quarter);
       wait(bar_pair + 8 * quarter, pair_phase++);
     };
-    float* mask_s = PLAIN ? nullptr : reinterpret_cast<float*>(smem_gen + C::kMaskOff) + warp * 32 * kMaskPitch;
-    const bool masked = !PLAIN && p.mask_kind != AIDN_MASK_NONE;
-    const bool keep_bytes = !PLAIN && p.mask_kind == AIDN_MASK_KEEP_U8, add = !PLAIN && p.mask_kind == AIDN_MASK_ADD_F32;
-    // The mask of the warp's 32 rows and its 32 keys of block j: a lane takes a key, so that rows are read in whole lines.  Bytes
-    // become one word of bits per row; floats go through shared memory, where the lane that owns a row finds its values
-    // (rows of 33: no bank conflicts either way).
+    const bool masked = !PLAIN && p.mask_kind != AIDN_MASK_NONE, keeps = masked && !add;
+    // The mask of the warp's 32 rows and its 32 keys of block j: a bias in its tile, a keep-mask as bits of the thread's row, one block
+    // ahead; lanes take keys, so that either is read in whole lines.
+    const uint32_t mask_s = smem_base + (uint32_t)(C::kMaskOff + warp * masktile::kBytes);
     uint32_t keep_next = 0;
-    auto fetch_mask_tile = [&](int j) {
-      const int64_t key = (blk0 + j) * kKeys + half * kHalf + lane;
-      const int64_t r0 = row0 + quarter * 32;
-      const int64_t at0 = b * p.mask_stride[0] + h * p.mask_stride[1] + r0 * p.mask_stride[2] + key * p.mask_stride[3];
-      const int64_t first64 = p.causal ? key - p.causal_offset - r0 : 0;          // rows before it do not see the key
-      const int64_t count64 = key < kv_limit ? p.seq_q - r0 : 0;
-      const int first = first64 < 0 ? 0 : (first64 > 32 ? 32 : (int)first64), count = count64 > 32 ? 32 : (int)count64;
-      if (keep_bytes) {
-        const uint8_t* src = static_cast<const uint8_t*>(p.mask) + at0;
-        if (p.mask_stride[2] == 0) {   // one row of bytes for all (what is not visible does not count)
-          keep_next = __ballot_sync(0xffffffffu, first < 32 && count > 0 && *src != 0);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; i += 16) {
-            uint32_t x[16];
-#pragma unroll
-            for (int r = 0; r < 16; ++r) x[r] = i + r >= first && i + r < count ? src[(i + r) * p.mask_stride[2]] : 0;
-#pragma unroll
-            for (int r = 0; r < 16; ++r) {
-              const uint32_t w = __ballot_sync(0xffffffffu, x[r] != 0);
-              if (i + r == lane) keep_next = w;
-            }
-          }
-        }
-      } else {
-        const float* src = static_cast<const float*>(p.mask);
-        const uint32_t dst = smem_u32(mask_s);
-#pragma unroll 8
-        for (int r = 0; r < 32; ++r) {
-          const bool ok = r >= first && r < count;
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;"
-                       ::"r"(dst + (uint32_t)((r * kMaskPitch + lane) * 4)), "l"(src + (ok ? at0 + r * p.mask_stride[2] : 0)), "r"(ok ? 4u : 0u) : "memory");
-        }
-        cp_async_commit_f();
-      }
+    auto fetch_keep = [&](int j) {
+      int rows, keys;
+      const int64_t at0 = mask_at(j, quarter, half, rows, keys);
+      keep_next = masktile::keep_bits_of(p, at0, p.mask_stride[2], p.mask_stride[3], rows, keys, lane);
     };
     // p = 2^((s - m) c): s is the raw score and c = scale log2(e), or the finished logit and log2(e) with a bias or a softcap
     const bool raw = MODE != kSoftcap && !add;
@@ -277,20 +255,28 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
     for (int i = 0; i < kCols / 2; ++i) acc[i] = 0;
     float m = -INFINITY, l = 0.f;
     if (n > 0) {
-      if (masked) fetch_mask_tile(0);
+      if (keeps) fetch_keep(0);
       const float* qb = static_cast<const float*>(p.q) + b * p.qs[0] + h * p.qs[1];
-#pragma unroll 4
-      for (int idx = tid; idx < kRows * CPR; idx += kWorkers) {
-        const int r = idx / CPR, ch = idx % CPR, d = ch * 8;
-        const float* src = qb + (row0 + r) * p.qs[2] + d;
-        const bool ok = row0 + r < p.seq_q;
-        split3::store_split8(q_s + (uint32_t)((ch >> 3) * kRows * 128) + split3::chunk_at(r, ch & 7), C::kQPlane, split3::load4(src, ok && d < D),
-                             split3::load4(src + 4, ok && d + 4 < D));
+      {
+        constexpr int kPer = kRows * CPR / kWorkers;
+        ulonglong2 v[kPer][2];   // all requested before the first is cut: one latency
+#pragma unroll
+        for (int e = 0; e < kPer; ++e) {
+          const int idx = tid + e * kWorkers, r = idx / CPR, d = idx % CPR * 8;
+          const float* src = qb + (row0 + r) * p.qs[2] + d;
+          const bool ok = row0 + r < p.seq_q;
+          v[e][0] = split3::load4(src, ok && d < D);
+          v[e][1] = split3::load4(src + 4, ok && d + 4 < D);
+        }
+#pragma unroll
+        for (int e = 0; e < kPer; ++e) {
+          const int idx = tid + e * kWorkers, r = idx / CPR, ch = idx % CPR;
+          split3::store_split8(q_s + (uint32_t)((ch >> 3) * kRows * 128) + split3::chunk_at(r, ch & 7), C::kQPlane, v[e][0], v[e][1]);
+        }
       }
       publish(bar_q);
       auto x_of = [&](int j, int h) -> float& {   // what half h of the row exchanges at block j
-        if (C::kXBufs == 2) return reinterpret_cast<float*>(smem_gen + C::kXOff)[((j & 1) * 2 + h) * kRows + lrow];
-        return reinterpret_cast<float*>(smem_gen + C::kMaskOff)[((h * 4 + quarter) * 32 + lane) * kMaskPitch + 32];
+        return reinterpret_cast<float*>(smem_gen + C::kXOff)[((C::kXBufs == 2 ? j & 1 : 0) * 2 + h) * kRows + lrow];
       };
       auto add_block = [&](int i) {   // P V of block i onto the output
         wait(bar_o + 8 * (i & 1), i >> 1);
@@ -333,12 +319,7 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
           }
         }
         uint32_t keep = seen < kHalf ? (1u << seen) - 1u : 0xffffffffu;
-        const float* mine = PLAIN ? nullptr : mask_s + lane * kMaskPitch;   // the row's values
         if constexpr (!PLAIN) {
-          if (masked && !keep_bytes) {   // every lane's copies are there
-            cp_async_wait_f<0>();
-            __syncwarp();
-          }
           if constexpr (MODE == kSoftcap) {
 #pragma unroll
             for (int k = 0; k < kHalf / 2; ++k) {
@@ -347,18 +328,19 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
             }
           }
           if (add) {
+            wait(bar_mf, j);
+            if (!alive) break;
 #pragma unroll
-            for (int k = 0; k < kHalf / 2; ++k) {
-              const uint64_t bias = pack2(mine[2 * k], mine[2 * k + 1]);
-              s[k] = MODE == kSoftcap ? add2(s[k], bias) : fma2(s[k], scale2, bias);
+            for (int k = 0; k < kHalf / 2; k += 2) {
+              const float4 m4 = masktile::row4(mask_s, k / 2, lane);
+              const uint64_t b0 = pack2(m4.x, m4.y), b1 = pack2(m4.z, m4.w);
+              s[k] = MODE == kSoftcap ? add2(s[k], b0) : fma2(s[k], scale2, b0);
+              s[k + 1] = MODE == kSoftcap ? add2(s[k + 1], b1) : fma2(s[k + 1], scale2, b1);
             }
-          } else if (keep_bytes) {
+            __syncwarp();   // the values have been read
+            if (lane == 0) mbar_arrive(bar_me);
+          } else if (keeps) {
             keep &= keep_next;
-          } else if (masked) {
-            uint32_t w = 0;
-#pragma unroll
-            for (int k = 0; k < kHalf; ++k) w |= mine[k] != 0.f ? 1u << k : 0u;
-            keep &= w;
           }
           if (__any_sync(0xffffffffu, keep != 0xffffffffu)) {
 #pragma unroll
@@ -416,10 +398,7 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
           sums = add2(sums, s[k]);
         }
         l = fmaf(l, corr, sum2(sums));
-        if (masked && j + 1 < n) {
-          __syncwarp();   // the values have been read
-          fetch_mask_tile(j + 1);
-        }
+        if (keeps && j + 1 < n) fetch_keep(j + 1);
         if (j > 0) {
           add_block(j - 1);
           if (!alive) break;
@@ -590,6 +569,22 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
         for (int t = 0; t < split3::kSmall; ++t) product(tmem_base + C::kTmemO + C::kOut, split3::small_a(t), split3::small_b(t), t == 0);
         if (leader) ptx::tc_commit(bar_o + 8 * (j & 1));
       }
+    } else if (add) {   // half of every row warp's tiles each
+      const int half = warp - kIssuer - 2;
+      for (int j = 0; j < n; ++j) {
+        if (j > 0) wait(bar_me, j - 1);
+        if (!alive) break;
+#pragma unroll 1
+        for (int quarter = 0; quarter < 4; ++quarter) {
+          int rows, keys;
+          const int64_t at0 = mask_at(j, quarter, half, rows, keys);
+          masktile::request(smem_base + (uint32_t)(C::kMaskOff + (half * 4 + quarter) * masktile::kBytes), static_cast<const float*>(p.mask) + at0,
+                            p.mask_stride[2], p.mask_stride[3], rows, keys, lane);
+        }
+        cp_async_wait_f<0>();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_mf);
+      }
     }
   }
 
@@ -618,17 +613,16 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
         const int64_t row = row0 + r;
         if (row >= p.seq_q) continue;
         float ms[8], ls[8], M = -INFINITY, lsum = 0.f;
-        float2 o[8][2];
+        float4 o[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           ms[i] = -INFINITY;
           ls[i] = 0.f;
-          o[i][0] = o[i][1] = make_float2(0.f, 0.f);
+          o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
           if (i < tp.splits) {
             ms[i] = ld_cluster_f32(pm + (uint32_t)(r * 4), (uint32_t)i);
             ls[i] = ld_cluster_f32(pl + (uint32_t)(r * 4), (uint32_t)i);
-            o[i][0] = ld_cluster_f2(part + (uint32_t)((r * C::kPartPitch + d) * 4), (uint32_t)i);
-            o[i][1] = ld_cluster_f2(part + (uint32_t)((r * C::kPartPitch + d + 2) * 4), (uint32_t)i);
+            o[i] = ld_cluster_f4(part + (uint32_t)((r * C::kPartPitch + d) * 4), (uint32_t)i);
           }
         }
 #pragma unroll
@@ -640,8 +634,7 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
           if (i >= tp.splits) continue;
           const float w = expf(ms[i] - M_use);
           lsum = fmaf(w, ls[i], lsum);
-          y[0] = fmaf(w, o[i][0].x, y[0]); y[1] = fmaf(w, o[i][0].y, y[1]);
-          y[2] = fmaf(w, o[i][1].x, y[2]); y[3] = fmaf(w, o[i][1].y, y[3]);
+          y[0] = fmaf(w, o[i].x, y[0]); y[1] = fmaf(w, o[i].y, y[1]); y[2] = fmaf(w, o[i].z, y[2]); y[3] = fmaf(w, o[i].w, y[3]);
         }
         const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
         float* out = static_cast<float*>(p.out) + b * p.os[0] + h * p.os[1] + row * p.os[2] + d;
