@@ -294,18 +294,19 @@ class CudaBackend:
             raise ValueError("heads must be a positive multiple of kvHeads")
         if seqLen <= 0:
             raise ValueError("seqLen must be positive")
-        if q.Size < heads * headDim or k.Size < seqLen * kvHeads * headDim or v.Size < seqLen * kvHeads * headDim:
+        cached = seqLen * kvHeads * headDim
+        if q.tensor.numel() < heads * headDim or k.tensor.numel() < cached or v.tensor.numel() < cached:
             raise ValueError("FlashDecode buffers are smaller than the requested dimensions.")
         out = self.AllocateBuffer(heads * headDim)
         chunk = 0
         if splits > 0:
             chunk = max(8, (math.ceil(seqLen / min(splits, seqLen)) + 7) // 8 * 8)
-        key = dict(qkv_dtype=_DTYPE[q.dtype], out_dtype=N.F32, head_dim=headDim, num_q_heads=heads,
-                   num_kv_heads=kvHeads, causal=False)
-        hkey = frozenset(key.items()) | {("chunk", chunk)}
+        dtype = _DTYPE[q.tensor.dtype]
+        hkey = (dtype, headDim, heads, kvHeads, chunk)   # (a decode step of one sequence waits for this code, not for the GPU)
         h = self._handles.get(hkey)
         if h is None:
-            h = N.Handle(device=self.device, path=self._path, decode_chunk=chunk or self._decode_chunk, **key)
+            h = N.Handle(device=self.device, path=self._path, decode_chunk=chunk or self._decode_chunk, qkv_dtype=dtype,
+                         out_dtype=N.F32, head_dim=headDim, num_q_heads=heads, num_kv_heads=kvHeads, causal=False)
             self._handles[hkey] = h
         stride = (0, headDim, kvHeads * headDim)  # (B, H, S) element strides of the [S, Hkv, D] cache
         self._run(h, query=q, key=k, value=v, output=out, batch=1, seqQ=1, seqK=seqLen, scale=float(scale),
@@ -505,10 +506,10 @@ class CudaBackend:
         bias, interleaved RoPE on Q and K, Q written to ``query`` and the K / V rows to row ``position`` of the dense
         caches [cacheCapacity, heads, 64] (``CudaBackend.cs:8389-8439``).  One kernel, no scratch buffers; the weights
         may be bf16 and the caches 16-bit (``GpuBuffer.dtype``), which is what the decode kernel then reads."""
-        for name, buf in (("input", input), ("packedWeights", packedWeights), ("bias", bias), ("cosine", cosine),
-                          ("sine", sine), ("query", query), ("keyCache", keyCache), ("valueCache", valueCache)):
-            if buf is None:
-                raise ValueError(f"{name} must not be null")          # ArgumentNullException
+        buffers = (input, packedWeights, bias, cosine, sine, query, keyCache, valueCache)
+        if None in buffers:
+            names = ("input", "packedWeights", "bias", "cosine", "sine", "query", "keyCache", "valueCache")
+            raise ValueError(f"{names[buffers.index(None)]} must not be null")          # ArgumentNullException
         if heads <= 0:
             raise ValueError("heads must be > 0")
         if cacheCapacity <= 0:
@@ -518,16 +519,16 @@ class CudaBackend:
         dimension = 64
         model = heads * dimension
         projection = 3 * model
-        if (input.Size < model or packedWeights.Size < projection * model or bias.Size < projection or
-                cosine.Size < cacheCapacity * (dimension // 2) or sine.Size < cacheCapacity * (dimension // 2) or
-                query.Size < model or keyCache.Size < cacheCapacity * model or valueCache.Size < cacheCapacity * model):
+        x, w, b, c, s, q, k, v = [buf.tensor for buf in buffers]
+        cached, rotations = cacheCapacity * model, cacheCapacity * (dimension // 2)
+        if (x.numel() < model or w.numel() < projection * model or b.numel() < projection or c.numel() < rotations or
+                s.numel() < rotations or q.numel() < model or k.numel() < cached or v.numel() < cached):
             raise ValueError("QKV/RoPE/cache buffers are smaller than the requested canonical extents.")
-        N.qkv_rope_cache(input=input.Handle, weights=packedWeights.Handle, bias=bias.Handle, cosine=cosine.Handle,
-                         sine=sine.Handle, query=query.Handle, key_cache=keyCache.Handle, value_cache=valueCache.Handle,
-                         tokens=1, heads=heads, kv_heads=heads, head_dim=dimension, position=position,
-                         weight_dtype=_DTYPE[packedWeights.dtype], query_dtype=_DTYPE[query.dtype],
-                         cache_dtype=_DTYPE[keyCache.dtype], cache_capacity=cacheCapacity, max_position=cacheCapacity,
-                         stream=self._raw_stream)
+        N.qkv_rope_cache(input=x.data_ptr(), weights=w.data_ptr(), bias=b.data_ptr(), cosine=c.data_ptr(), sine=s.data_ptr(),
+                         query=q.data_ptr(), key_cache=k.data_ptr(), value_cache=v.data_ptr(), tokens=1, heads=heads,
+                         kv_heads=heads, head_dim=dimension, position=position, weight_dtype=_DTYPE[w.dtype],
+                         query_dtype=_DTYPE[q.dtype], cache_dtype=_DTYPE[k.dtype], cache_capacity=cacheCapacity,
+                         max_position=cacheCapacity, stream=self._raw_stream)
         self.launch_count += 1
 
     def RopeInterleaved(self, input: GpuBuffer, cos: GpuBuffer, sin: GpuBuffer, output: GpuBuffer, rows: int,

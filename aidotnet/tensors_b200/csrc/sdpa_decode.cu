@@ -1094,8 +1094,10 @@ cudaError_t launch_gqa(const SdpaParams& p, const DecodePlan& plan, float* ws, i
   auto kern = head_fast ? (p.block_table ? sdpa_decode_gqa_ring_kernel<T, D, NH16, true, true> : sdpa_decode_gqa_ring_kernel<T, D, NH16, false, true>)
                         : (p.block_table ? sdpa_decode_gqa_ring_kernel<T, D, NH16, true, false> : sdpa_decode_gqa_ring_kernel<T, D, NH16, false, false>);
   constexpr int smem = RingCfg<D>::kSmemBytes;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
+  if (smem > 48 * 1024) {   // (below, a launch needs no leave for it)
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
   return launch_dependent_cluster(kern, grid, kDecWarps * 32, shape, smem, stream, p, plan.chunk, plan.nchunks, ws, merge, plan.cluster);
 }
 
