@@ -672,11 +672,20 @@ cudaError_t launch_t(const BwdParams& bp, cudaStream_t stream, int* launches, co
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess || sms <= 0) { *why = "cannot read the SM count"; return e != cudaSuccess ? e : cudaErrorInvalidValue; }
   sp.total_items = (int)items_q;
-  e = launch_dependent(kq, dim3((unsigned)(items_q < sms ? items_q : sms)), kThreads, smem_q, stream, tq, tk, tv, tdo, sp);
-  if (e != cudaSuccess) return e;
-  sp.total_items = (int)items_kv;
   *launches += 2;
-  return launch_dependent(kkv, dim3((unsigned)(items_kv < sms ? items_kv : sms)), kThreads, smem_kv, stream, tq, tk, tv, tdo, sp);
+  const unsigned grid_q = (unsigned)(items_q < sms ? items_q : sms), grid_kv = (unsigned)(items_kv < sms ? items_kv : sms);
+  BwdSm100Params sk = sp;
+  sk.total_items = (int)items_kv;
+  // (long launches gain nothing by it, and dK / dV beside dQ would share the L2 cache: B2 H19 S7521 D64 causal 1254 -> 1277 us)
+  if (items_q * sp.k_tiles <= (int64_t)sms * 256) {
+    e = launch_dependent(kq, dim3(grid_q), kThreads, smem_q, stream, tq, tk, tv, tdo, sp);
+    return e != cudaSuccess ? e : launch_dependent(kkv, dim3(grid_kv), kThreads, smem_kv, stream, tq, tk, tv, tdo, sk);
+  }
+  kq<<<grid_q, kThreads, smem_q, stream>>>(tq, tk, tv, tdo, sp);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  kkv<<<grid_kv, kThreads, smem_kv, stream>>>(tq, tk, tv, tdo, sk);
+  return cudaGetLastError();
 }
 
 }  // namespace

@@ -360,9 +360,12 @@ __device__ __forceinline__ void store_o_tile(const SdpaParams& p, const CUtensor
   }
 }
 
-// MASKED: the softmax warps also apply softcap, an additive bias or a keep-mask read from global memory (one row
-// per thread); the plain variant carries none of that code.
-template <typename T, int HD, bool MASKED, bool EPI>
+// What the softmax warps do to a score besides scaling it: nothing, a softcap, or a bias or keep-mask read from global memory (and perhaps a
+// softcap).  Each carries none of the others' code: behind the masks' branches and registers the softcap alone took 512 -> 640 us
+// on a long prefill.
+enum PrefillMode { kPlain, kCapped, kMasked };
+
+template <typename T, int HD, PrefillMode MODE, bool EPI>
 __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
     sdpa_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -370,6 +373,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
   using C = Cfg<HD>;
   using R = Roles<EPI>;
   constexpr bool kBf16 = !std::is_same_v<T, __half>;
+  constexpr bool MASKED = MODE == kMasked, kScaled = MODE != kPlain;
   const SdpaParams& p = pp.p;
 
   extern __shared__ uint8_t smem_raw[];
@@ -457,8 +461,8 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
 
   // Plain: scores stay raw and the scale is folded into the exponent (one FMA).  Masked: scores are scaled first
   // (softcap and bias act on scaled logits), so the exponent only needs log2(e).
-  const float sl2 = MASKED ? kLog2e : p.scale * kLog2e;
-  const float lse_scale = MASKED ? 1.f : p.scale;
+  const float sl2 = kScaled ? kLog2e : p.scale * kLog2e;
+  const float lse_scale = kScaled ? 1.f : p.scale;
 
   if (warp < kSoftmaxWarps) {
     // =================================== softmax / epilogue ===================================
@@ -594,12 +598,17 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
         float* s = reinterpret_cast<float*>(sr);
 
         const int64_t col0 = (int64_t)(it.k0 + u) * kBS;
+        if constexpr (MODE == kCapped) {
+          const float f = p.scale / p.softcap;
+#pragma unroll
+          for (int c = 0; c < kBS; ++c) s[c] = p.softcap * tanh_approx(s[c] * f);
+        }
         if constexpr (MASKED) {
           // scale -> softcap -> bias -> keep-mask, the order of the reference (CpuEngine.cs:27807-27816, 29218-29239)
           if (p.softcap > 0.f) {
-            const float inv_cap = 1.f / p.softcap;
+            const float f = p.scale / p.softcap;
 #pragma unroll
-            for (int c = 0; c < kBS; ++c) s[c] = p.softcap * tanh_approx(s[c] * p.scale * inv_cap);
+            for (int c = 0; c < kBS; ++c) s[c] = p.softcap * tanh_approx(s[c] * f);
           } else if (!add) {
 #pragma unroll
             for (int c = 0; c < kBS; ++c) s[c] *= p.scale;
@@ -701,7 +710,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
         // Packed multiply-adds and additions take half of their instructions and give the same bits: B4 H32 S2048 D128 causal
         // 190.4 -> 187.3 us, B6 H16 S997 D64 40.7 -> 39.8.  The unmasked D 128 kernel with epilogue warps has no registers for
         // the pairs (416 bytes of spill reads; the layer of B4 S2048 and 32 heads 1190 -> 1199) and keeps single ones.
-        constexpr bool kPacked = !EPI || MASKED || HD == 64;
+        constexpr bool kPacked = !EPI || kScaled || HD == 64;
         float ls0 = 0.f, ls1 = 0.f, ls2 = 0.f, ls3 = 0.f;
         uint64_t ls01 = 0, ls23 = 0;
         const uint64_t mul_2 = pack2(mul, mul), neg_2 = pack2(neg_ms, neg_ms);
@@ -831,6 +840,12 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
     }
   } else {
     setmaxnreg_dec<R::kOtherRegs>();
+    if (warp == kProducerWarp) {
+      // The set-up above runs under the end of the launch before.  Every other warp touches memory only behind an item that this one
+      // has published (in their code, even ahead of the barrier, the wait costs the softmax loop registers).
+      pdl_wait();
+      pdl_trigger();
+    }
   }
 
   // ---- K / V loads: one 64-key sub-tile into ring position t (waits until the position's slot is free) ----
@@ -901,10 +916,6 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
     // ==================================== TMA producer + scheduler ====================================
     // warp-uniform like the UMMA issuer: one elected lane issues the TMA loads and barrier operations
     {
-      // The set-up above runs under the end of the launch before.  Every other warp touches memory only behind an item that this one
-      // has published (in their code, even ahead of the barrier, the wait costs the softmax loop registers).
-      pdl_wait();
-      pdl_trigger();
       const bool leader = elect_one();
       bool alive = true;
       uint32_t t_load = 0;          // K/V sub-tiles of earlier items (ring position)
@@ -1323,7 +1334,7 @@ bool aligned_bhs(const void* base, const int64_t* stride, int64_t H, int64_t B, 
   return true;
 }
 
-template <typename T, int HD, bool MASKED, bool EPI>
+template <typename T, int HD, PrefillMode MODE, bool EPI>
 cudaError_t launch_e(const SdpaParams& p, cudaStream_t stream, int32_t* sched, int num_sms, float* debug,
                      int debug_mode, PrefillMapCache* cache, int splits, const char** why) {
   using C = Cfg<HD>;
@@ -1414,8 +1425,8 @@ cudaError_t launch_e(const SdpaParams& p, cudaStream_t stream, int32_t* sched, i
   const int64_t total = (int64_t)pp.ranks * pp.items_per_rank * splits;
   if (total <= 0 || total > 0x3fffffff) { *why = "work item count out of range"; return cudaErrorInvalidValue; }
   pp.total_items = (int)total;
-  auto kern = sdpa_prefill_sm100_kernel<T, HD, MASKED, EPI>;
-  constexpr int inst = (EPI ? 8 : 0) + (bf16 ? 0 : 4) + (HD == 128 ? 2 : 0) + (MASKED ? 1 : 0);
+  auto kern = sdpa_prefill_sm100_kernel<T, HD, MODE, EPI>;
+  constexpr int inst = 8 * MODE + (EPI ? 4 : 0) + (bf16 ? 0 : 2) + (HD == 128 ? 1 : 0);
   if (!mc->attr_set[inst]) {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) { *why = "cannot raise the dynamic shared memory limit"; return e; }
@@ -1423,7 +1434,12 @@ cudaError_t launch_e(const SdpaParams& p, cudaStream_t stream, int32_t* sched, i
   }
   const unsigned grid = (unsigned)(total < num_sms ? total : num_sms);
   // Set up under the end of the launch before: six sequences of 166 to 997 keys, H16 D64 39.2 -> 38.0 us, Hq10 / Hkv5 255 x 255 D128 14.4 -> 13.4.
-  return launch_dependent(kern, grid, Roles<EPI>::kThreads, C::kSmemBytes, stream, *tq, *tk, *tv, *to, pm, pp);
+  // Not launches of half a millisecond and more, where that gains nothing and the CTAs would start wherever an SM comes free
+  // (B2 H19 S7521 D64 causal 395.6 -> 398.5).
+  if (total * ((p.seq_kv + kBS - 1) / kBS) <= (int64_t)num_sms * 512)
+    return launch_dependent(kern, grid, Roles<EPI>::kThreads, C::kSmemBytes, stream, *tq, *tk, *tv, *to, pm, pp);
+  kern<<<grid, Roles<EPI>::kThreads, C::kSmemBytes, stream>>>(*tq, *tk, *tv, *to, pm, pp);
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -1456,20 +1472,20 @@ bool prefill_sm100_supported(const SdpaParams& p, int dtype, const char** why) {
 }
 
 // The epilogue warpgroup pays when both tiles of an item end together: head pairs, or row pairs without a causal mask.
-template <typename T, int HD, bool MASKED>
+template <typename T, int HD, PrefillMode MODE>
 cudaError_t launch_t(const SdpaParams& p, cudaStream_t stream, int32_t* sched, int num_sms, float* debug,
                      int debug_mode, PrefillMapCache* cache, int splits, const char** why) {
   const bool epi = ((p.group % 2 == 0) || !p.causal) && p.mask_kind != AIDN_MASK_ADD_F32;   // (a bias goes through the softmax warps' staging buffers)
-  if (epi) return launch_e<T, HD, MASKED, true>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
-  return launch_e<T, HD, MASKED, false>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  if (epi) return launch_e<T, HD, MODE, true>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  return launch_e<T, HD, MODE, false>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
 }
 
 template <typename T, int HD>
 cudaError_t launch_m(const SdpaParams& p, cudaStream_t stream, int32_t* sched, int num_sms, float* debug, int debug_mode,
                      PrefillMapCache* cache, int splits, const char** why) {
-  if (p.mask_kind != AIDN_MASK_NONE || p.softcap > 0.f)
-    return launch_t<T, HD, true>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
-  return launch_t<T, HD, false>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  if (p.mask_kind != AIDN_MASK_NONE) return launch_t<T, HD, kMasked>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  if (p.softcap > 0.f) return launch_t<T, HD, kCapped>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  return launch_t<T, HD, kPlain>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
 }
 
 namespace {
