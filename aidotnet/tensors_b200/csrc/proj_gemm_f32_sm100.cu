@@ -483,7 +483,8 @@ TilePlan tile_plan(int64_t rows, int64_t k, int64_t n, int mats, int num_sms) {
 
 }  // namespace
 
-// Whole layers, the attention unchanged: 64 rows x 3072 and 1024 x 1024 211 -> 138 and 336 -> 181 us.  Error of a whole layer against
+// Whole layers, the attention unchanged, multiply-adds against these kernels' first form: 64 rows x 3072 and 1024 x 1024
+// 211 -> 138 and 336 -> 181 us (the latter 125 with the fp32 attention on the tensor cores, 101 with the kernels above).  Error of a whole layer against
 // 64 bits 7.2e-7 -> 4.0e-7 at K = 768, 5.4e-7 -> 3.8e-7 at 512; below K = 256 the truncation of four additions weighs more than the
 // rounding of K (2.5e-7 -> 3.4e-7 at 64) and the times are equal: there the multiply-adds stay.
 bool proj_gemm_f32_sm100_fits(int64_t k, int64_t n) { return k >= 256 && k % 4 == 0 && n % 4 == 0 && n * 3 + 160 <= 0x7fffffff; }

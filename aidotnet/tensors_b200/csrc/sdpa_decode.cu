@@ -4,10 +4,12 @@
 // kv head, and forms an un-normalised partial (max, sum, acc[D]).  The partials of a (batch, head) are merged by
 // log-sum-exp: among the CTAs of a cluster through distributed shared memory where few enough CTAs run at once, by a
 // second kernel through a workspace otherwise (decode_plan_clusters).  Only keys below kv_len[b] (and the causal limit) are touched, so padding costs no
-// bandwidth.  Two partial kernels:
+// bandwidth.  Three partial kernels:
 //   * sdpa_decode_gqa_ring_kernel - fp16 / bf16, head_dim 64 or 128, up to 16 query heads per kv head (plain
 //     multi-head attention included): K/V go through a per-warp cp.async shared-memory ring and both products run
 //     on mma.sync with the heads as the M / N dimension.  This is the kernel the benchmark's decode step uses.
+//   * sdpa_decode_stream_kernel   - the same ring over equal shares of the keys of all sequences together, for launches with
+//     lengths (decode_stream_bytes): the shares follow from the lengths on the device.
 //   * sdpa_decode_partial_kernel  - everything else (fp32 inputs, head_dim 256, more than 16 heads per kv head):
 //     16-byte streaming loads straight into registers and FFMA arithmetic.
 //

@@ -174,7 +174,8 @@ typedef struct {
 AIDN_API int aidn_sdpa_create(const aidn_sdpa_desc* desc, aidn_sdpa_t* out);
 /* Bytes of caller workspace for a launch of this shape; < 0 on error.  A decode launch needs them (or the handle's scratch);
  * a tcgen05 prefill with fewer work items than SMs uses them for the partial results of its split keys, and runs unsplit
- * when the workspace is NULL or smaller.  Launches that overlap on the GPU must not share a workspace, and a launch that
+ * when the workspace is NULL or smaller.  For a decode this may be more than a launch needs
+ * at least: one with kv_len uses all of it to cut the keys of all sequences into equal shares, and cuts by sequence with less.  Launches that overlap on the GPU must not share a workspace, and a launch that
  * was captured into a graph uses the same one at every replay. */
 AIDN_API int64_t aidn_sdpa_workspace_bytes(aidn_sdpa_t h, int64_t batch, int64_t seq_q, int64_t seq_kv);
 /* Enqueues the attention forward on `cu_stream` (a CUstream / cudaStream_t).  No allocation, no synchronisation; safe
@@ -290,7 +291,8 @@ AIDN_API int aidn_rope_interleaved(const float* input, const float* cosine, cons
  * IEngine.MultiHeadAttentionForward (src/AiDotNet.Tensors/Engines/IEngine.cs:4201-4208; CPU
  * CpuEngine.MultiHeadAttention.cs:68-338, GPU composition DirectGpuTensorEngine.MissingKernels.cs:5793-5870):
  *   out = softmax((X Wq)(X Wk)^T / sqrt(d) [keep-mask]) (X Wv) Wout,   X [batch, seq, heads*d], each W [heads*d, heads*d]
- * row-major and applied as x * W.  Three launches on the stream: one GEMM for the Q, K and V projections that writes
+ * row-major and applied as x * W.  Three launches on the stream (fp32 on the tensor cores with many rows: a
+ * fourth in front of them cuts the weights into their terms): one GEMM for the Q, K and V projections that writes
  * [B, H, S, d] directly, the attention kernel of the handle, one GEMM for the output projection reading the attention
  * output as [B, S, H*d].  Two routes, chosen from the handle:
  *   - 16-bit qkv_dtype, head_dim 64 or 128, heads*head_dim a multiple of 128: tcgen05 GEMMs and the tcgen05 attention
