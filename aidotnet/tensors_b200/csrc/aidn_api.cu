@@ -803,12 +803,15 @@ int aidn_paged_kv_append(const void* new_keys, const void* new_values, void* key
 namespace {
 struct MhaPlan {
   int64_t off_x, off_w, off_q, off_k, off_v, off_o, off_t[2], total;   // off_t: terms of the fp32 weights, Q / K / V and output
+  aidn::ProjPlanF32 f32_plan[2];
 };
-MhaPlan mha_plan(const aidn_sdpa* h, int64_t batch, int64_t seq, int input_dtype, int weight_dtype) {
+// `images`: with the terms of the fp32 weights in the workspace, where that is faster.
+MhaPlan mha_plan(const aidn_sdpa* h, int64_t batch, int64_t seq, int input_dtype, int weight_dtype, bool images) {
   const int64_t dm = (int64_t)h->d.num_q_heads * h->d.head_dim;
   const int64_t esz = (int64_t)elem_size(h->d.qkv_dtype);
   const int64_t act = align_up(batch * seq * dm * esz, 1024), wgt = align_up(dm * dm * esz, 1024);
   MhaPlan pl;
+  std::memset(&pl, 0, sizeof(pl));
   int64_t off = 0;
   pl.off_x = off; off += input_dtype != h->d.qkv_dtype ? act : 0;
   pl.off_w = off; off += weight_dtype != h->d.qkv_dtype ? 4 * wgt : 0;
@@ -818,8 +821,10 @@ MhaPlan mha_plan(const aidn_sdpa* h, int64_t batch, int64_t seq, int input_dtype
   pl.off_o = off; off += act;
   for (int i = 0; i < 2; ++i) {
     pl.off_t[i] = off;
-    if (h->d.qkv_dtype == AIDN_F32 && h->d.path != AIDN_PATH_GENERIC && aidn::proj_gemm_f32_sm100_fits(dm, dm))
-      off += align_up(aidn::proj_gemm_f32_sm100_bytes(batch * seq, dm, dm, i == 0 ? 3 : 1, h->num_sms), 1024);
+    if (h->d.qkv_dtype != AIDN_F32 || h->d.path == AIDN_PATH_GENERIC || !aidn::proj_gemm_f32_sm100_fits(dm, dm)) continue;
+    const int mats = i == 0 ? 3 : 1;
+    pl.f32_plan[i] = aidn::proj_gemm_f32_sm100_plan(batch * seq, dm, dm, mats, h->num_sms, images, i == 1 && !pl.f32_plan[0].cut_w);
+    off += align_up(aidn::proj_gemm_f32_sm100_bytes(pl.f32_plan[i], dm, dm, mats), 1024);
   }
   pl.total = off;
   return pl;
@@ -846,7 +851,7 @@ int64_t aidn_mha_workspace_bytes(aidn_sdpa_t h, int64_t batch, int64_t seq, int3
     return -1;
   }
   if (mha_check_handle(h) != AIDN_OK) return -1;
-  return mha_plan(h, batch, seq, input_dtype, weight_dtype).total;
+  return mha_plan(h, batch, seq, input_dtype, weight_dtype, true).total;
 }
 
 int aidn_mha_forward(aidn_sdpa_t h, const aidn_mha_args* a, void* cu_stream) {
@@ -862,7 +867,9 @@ int aidn_mha_forward(aidn_sdpa_t h, const aidn_mha_args* a, void* cu_stream) {
   if (!dtype_ok(a->input_dtype) || !dtype_ok(a->weight_dtype) || !dtype_ok(a->out_dtype))
     return fail(AIDN_EINVAL, "mha: input, weight and output dtypes must be fp32 or the handle's qkv_dtype");
   if (d.mask_kind != AIDN_MASK_NONE && !a->mask) return fail(AIDN_EINVAL, "mha: mask_kind set but mask pointer is null");
-  const MhaPlan pl = mha_plan(h, a->batch, a->seq, a->input_dtype, a->weight_dtype);
+  MhaPlan pl = mha_plan(h, a->batch, a->seq, a->input_dtype, a->weight_dtype, true);
+  if (a->workspace && a->workspace_bytes < pl.total)   // no room for the images: the GEMMs cut the weights themselves
+    pl = mha_plan(h, a->batch, a->seq, a->input_dtype, a->weight_dtype, false);
   if (!a->workspace || a->workspace_bytes < pl.total)
     return fail(AIDN_EWORKSPACE, "mha: workspace of %lld bytes, need %lld", (long long)(a->workspace ? a->workspace_bytes : 0),
                 (long long)pl.total);
@@ -923,11 +930,13 @@ int aidn_mha_forward(aidn_sdpa_t h, const aidn_mha_args* a, void* cu_stream) {
     aidn::ProjGemm split[2];
     int count = 0;
     g.image = ws + pl.off_t[0];
+    g.f32_plan = pl.f32_plan[0];
     go.image = ws + pl.off_t[1];
+    go.f32_plan = pl.f32_plan[1];
     if (f32_sm100[0] && pl.off_t[1] > pl.off_t[0]) split[count++] = g;
     if (f32_sm100[1] && pl.total > pl.off_t[1]) split[count++] = go;
     if (count > 0) {
-      e = aidn::launch_proj_split_f32(split, count, stream, h->num_sms);
+      e = aidn::launch_proj_split_f32(split, count, stream);
       if (e != cudaSuccess) return fail_cuda(e, "mha: terms of the weights");
       ++launches;
     }
@@ -939,7 +948,7 @@ int aidn_mha_forward(aidn_sdpa_t h, const aidn_mha_args* a, void* cu_stream) {
     } else {
       if (!aidn::proj_gemm_generic_supported(g, &why)) return fail(AIDN_EUNSUPPORTED, "mha: %s", why);
       if (f32_sm100)
-        e = aidn::launch_proj_gemm_f32_sm100(g, stream, h->num_sms, h->status_dev, h->debug_mode == 3);
+        e = aidn::launch_proj_gemm_f32_sm100(g, stream, h->status_dev, h->debug_mode == 3);
       else
         e = aidn::launch_proj_gemm_generic(g, d.qkv_dtype, stream);
     }

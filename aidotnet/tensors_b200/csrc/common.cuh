@@ -357,6 +357,13 @@ cudaError_t launch_prefill_sm100(const SdpaParams& p, int dtype, cudaStream_t st
                                  float* debug, int debug_mode, PrefillMapCache* cache, int splits, float* workspace,
                                  const char** why);
 
+// How proj_gemm_f32_sm100 does one GEMM: columns of a tile, CTAs of a cluster that share its K, and whether they cut W into its terms
+// themselves or copy them in from an image.
+struct ProjPlanF32 {
+  int32_t width, splits;
+  bool cut_w;
+};
+
 // Projection GEMM of the fused multi-head-attention forward (csrc/proj_gemm_sm100.cu):
 // c[i][b, s, n] = sum_k a[b, s, k] * w[i][k, n] for up to three weight matrices that share a; column n lands at
 // c[i] + b*c_stride[0] + (n / head_dim)*c_stride[1] + s*c_stride[2] + n % head_dim.
@@ -370,7 +377,8 @@ struct ProjGemm {
   int32_t head_dim;
   bool out_f32;         // fp32 output, else the input dtype
   bool bf16;            // bf16 inputs, else fp16
-  void* image;          // the terms of w (proj_gemm_f32_sm100 only)
+  void* image;          // the terms of w, in tiles of f32_plan (proj_gemm_f32_sm100 only)
+  ProjPlanF32 f32_plan; // the same for the launch that writes the image and the one that reads it
 };
 bool proj_gemm_sm100_supported(const ProjGemm& g, const char** why);
 // expire: test hook - the producer withholds its loads and every bounded wait gives up after 20 ms.
@@ -378,12 +386,13 @@ cudaError_t launch_proj_gemm_sm100(const ProjGemm& g, cudaStream_t stream, int n
                                    const char** why, bool expire = false);
 // fp32 operands with 16-byte rows, every one as three bf16 terms on tcgen05 (csrc/proj_gemm_f32_sm100.cu).  launch_proj_split_f32
 // writes the terms of the weights of one or two GEMMs to their `image`, of proj_gemm_f32_sm100_bytes bytes each, for the GEMMs
-// behind it on the stream; where that is 0 (few rows) a GEMM cuts its weights itself.
+// behind it on the stream; where that is 0 (few rows, or a plan made without `images`) a GEMM cuts its weights itself.
 bool proj_gemm_f32_sm100_fits(int64_t k, int64_t n);
 bool proj_gemm_f32_sm100_supported(const ProjGemm& g);
-int64_t proj_gemm_f32_sm100_bytes(int64_t rows, int64_t k, int64_t n, int mats, int num_sms);
-cudaError_t launch_proj_split_f32(const ProjGemm* gemms, int count, cudaStream_t stream, int num_sms);
-cudaError_t launch_proj_gemm_f32_sm100(const ProjGemm& g, cudaStream_t stream, int num_sms, int32_t* status, bool expire = false);
+ProjPlanF32 proj_gemm_f32_sm100_plan(int64_t rows, int64_t k, int64_t n, int mats, int num_sms, bool images, bool launched);
+int64_t proj_gemm_f32_sm100_bytes(const ProjPlanF32& plan, int64_t k, int64_t n, int mats);
+cudaError_t launch_proj_split_f32(const ProjGemm* gemms, int count, cudaStream_t stream);
+cudaError_t launch_proj_gemm_f32_sm100(const ProjGemm& g, cudaStream_t stream, int32_t* status, bool expire = false);
 // The same contract in fp32 FFMA arithmetic for any sizes and for a / w of `dtype` (csrc/proj_gemm_generic.cu).
 bool proj_gemm_generic_supported(const ProjGemm& g, const char** why);
 cudaError_t launch_proj_gemm_generic(const ProjGemm& g, int dtype, cudaStream_t stream);

@@ -450,10 +450,7 @@ cudaError_t launch_t(F32GemmParams& f, int splits, cudaStream_t stream) {
   return launch_dependent_cluster(kern, dim3((unsigned)ctas), kThreads, dim3((unsigned)splits), FCfg<BN>::kSmem, stream, f);
 }
 
-struct TilePlan {
-  int width, splits;
-  bool cut_w;
-};
+}  // namespace
 
 // Columns of a tile, CTAs that share its K, and whether they cut W themselves: what has the shortest time by waves of CTAs, in cycles.
 // A block of K takes 1190 at 32 and 2330 at 160 columns, with W cut in place 1950 and 3300 at 64 and 128; the rest 7600 at 48 and 10000
@@ -461,10 +458,10 @@ struct TilePlan {
 // read again).  Clusters only where all of a launch's CTAs are resident at once.  Layers, in us, before -> with these rules:
 //   rows x width  16 x 512 35 -> 25, 100 x 1024 57 -> 48, 256 x 2048 118 -> 92, 384 x 3072 268 -> 245, 1024 x 1024 125 -> 102,
 //   2048 x 3072 1416 -> 1242; 1576 x 512 (143 tiles of 144 and of 48 columns) 83 -> 57
-// (The launch serves both GEMMs of a layer, so that it costs the output's projection nothing where that of Q, K and V has one.)
-TilePlan tile_plan(int64_t rows, int64_t k, int64_t n, int mats, int num_sms) {
-  const int64_t cols = n * mats, launch = mats == 1 && !tile_plan(rows, k, n, 3, num_sms).cut_w ? 0 : 5000;
-  TilePlan best = {0, 0, false};
+// (`launched`: the launch for the terms is there for another GEMM of the layer already, and costs this one nothing.)
+ProjPlanF32 proj_gemm_f32_sm100_plan(int64_t rows, int64_t k, int64_t n, int mats, int num_sms, bool images, bool launched) {
+  const int64_t cols = n * mats, launch = launched ? 0 : 5000;
+  ProjPlanF32 best = {0, 0, false};
   int64_t best_cost = 0;
   const int64_t blocks = (k + kBK - 1) / kBK;
   auto consider = [&](int bn, bool cut, int64_t block, int64_t once) {
@@ -477,11 +474,10 @@ TilePlan tile_plan(int64_t rows, int64_t k, int64_t n, int mats, int num_sms) {
   };
   consider(64, true, 1950, 0);
   consider(128, true, 3300, 0);
-  for (int bn : {32, 48, 64, 96, 128, 144, 160}) consider(bn, false, bn <= 96 ? 900 + 9 * bn : 1050 + 8 * bn, launch + cols * k / 220);
+  if (images)
+    for (int bn : {32, 48, 64, 96, 128, 144, 160}) consider(bn, false, bn <= 96 ? 900 + 9 * bn : 1050 + 8 * bn, launch + cols * k / 220);
   return best;
 }
-
-}  // namespace
 
 // Whole layers, the attention unchanged, multiply-adds against these kernels' first form: 64 rows x 3072 and 1024 x 1024
 // 211 -> 138 and 336 -> 181 us (the latter 125 with the fp32 attention on the tensor cores, 101 with the kernels above).  Error of a whole layer against
@@ -495,13 +491,12 @@ bool proj_gemm_f32_sm100_supported(const ProjGemm& g) {
   return ok;
 }
 
-int64_t proj_gemm_f32_sm100_bytes(int64_t rows, int64_t k, int64_t n, int mats, int num_sms) {
-  const TilePlan plan = tile_plan(rows, k, n, mats, num_sms);
+int64_t proj_gemm_f32_sm100_bytes(const ProjPlanF32& plan, int64_t k, int64_t n, int mats) {
   if (plan.cut_w) return 0;
   return (n * mats + plan.width - 1) / plan.width * plan.width * ((k + kBK - 1) / kBK) * 128 * split3::kTerms;
 }
 
-cudaError_t launch_proj_split_f32(const ProjGemm* gemms, int count, cudaStream_t stream, int num_sms) {
+cudaError_t launch_proj_split_f32(const ProjGemm* gemms, int count, cudaStream_t stream) {
   SplitParams p = {};
   int64_t units = 0;
   for (int i = 0; i < count; ++i) {
@@ -512,7 +507,7 @@ cudaError_t launch_proj_split_f32(const ProjGemm* gemms, int count, cudaStream_t
     s.k = (int)g.k;
     s.n = (int)g.n;
     s.cols = (int)(g.n * g.num_mats);
-    s.bn = tile_plan(g.batch * g.seq, g.k, g.n, g.num_mats, num_sms).width;
+    s.bn = g.f32_plan.width;
     s.col_tiles = (s.cols + s.bn - 1) / s.bn;
     s.k_blocks = (int)((g.k + kBK - 1) / kBK);
     s.col_units = s.col_tiles * (s.bn / 16);
@@ -524,7 +519,7 @@ cudaError_t launch_proj_split_f32(const ProjGemm* gemms, int count, cudaStream_t
   return launch_dependent(proj_split_f32_kernel, dim3((unsigned)units), 128, 0, stream, p);
 }
 
-cudaError_t launch_proj_gemm_f32_sm100(const ProjGemm& p, cudaStream_t stream, int num_sms, int32_t* status, bool expire) {
+cudaError_t launch_proj_gemm_f32_sm100(const ProjGemm& p, cudaStream_t stream, int32_t* status, bool expire) {
   F32GemmParams f;
   f.a = static_cast<const float*>(p.a);
   f.image = static_cast<const uint8_t*>(p.image);
@@ -546,7 +541,7 @@ cudaError_t launch_proj_gemm_f32_sm100(const ProjGemm& p, cudaStream_t stream, i
   f.status = status;
   f.withhold = expire ? 1 : 0;
   f.wait_budget_ns = expire ? 20000000ull : kWaitBudgetNs;   // 20 ms in the time-out test
-  const TilePlan plan = tile_plan(f.rows, f.k, f.n, p.num_mats, num_sms);
+  const ProjPlanF32& plan = p.f32_plan;
   if (plan.cut_w) return plan.width == 64 ? launch_t<64, true>(f, plan.splits, stream) : launch_t<128, true>(f, plan.splits, stream);
   switch (plan.width) {
     case 32: return launch_t<32>(f, plan.splits, stream);

@@ -321,7 +321,9 @@ typedef struct {
   int32_t weight_dtype;     /* AIDN_F32 or desc.qkv_dtype                                                        */
   int32_t out_dtype;        /* AIDN_F32 or desc.qkv_dtype                                                        */
   int32_t reserved;
-  void* workspace;          /* device scratch of at least aidn_mha_workspace_bytes(), 256-byte aligned           */
+  void* workspace;          /* device scratch of aidn_mha_workspace_bytes(), 256-byte aligned; for an fp32 handle that
+                               includes room for the terms of the weights (6 bytes a weight): with less, down to the activations (and
+                               operands in 16 bits) alone, every projection cuts its weights itself, only slower              */
   int64_t workspace_bytes;
 } aidn_mha_args;
 AIDN_API int64_t aidn_mha_workspace_bytes(aidn_sdpa_t h, int64_t batch, int64_t seq, int32_t input_dtype,

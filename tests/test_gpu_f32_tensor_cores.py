@@ -321,11 +321,11 @@ def test_backward_route_and_bounded_waits(shape, tcgen05, path):
         assert np.abs(x.cpu().numpy() - y).max() <= 16 * 2.0 ** -24 * np.sqrt(max(Sq, Sk, D)) * max(1.0, np.abs(y).max()), name
 
 
-def _layer(x, ws, heads, path=N.PATH_AUTO):
+def _layer(x, ws, heads, path=N.PATH_AUTO, workspace=None):
     B, S, Dm = x.shape
     out = torch.full((B, S, Dm), float("nan"), device="cuda")
     h = N.Handle(device=0, qkv_dtype=N.F32, out_dtype=N.F32, head_dim=Dm // heads, num_q_heads=heads, num_kv_heads=heads, path=path)
-    nb = h.mha_workspace_bytes(B, S, N.F32, N.F32)
+    nb = h.mha_workspace_bytes(B, S, N.F32, N.F32) if workspace is None else workspace
     scratch = torch.zeros(nb + 1024, dtype=torch.uint8, device="cuda")
     launch = lambda: h.mha_forward(input=x.data_ptr(), q_weight=ws[0].data_ptr(), k_weight=ws[1].data_ptr(), v_weight=ws[2].data_ptr(),
                                    out_weight=ws[3].data_ptr(), out=out.data_ptr(), batch=B, seq=S, input_dtype=N.F32, weight_dtype=N.F32,
@@ -382,6 +382,32 @@ def test_projection_plans(B, S, heads, d):
     launch()
     h.poll(torch.cuda.current_stream().cuda_stream)
     assert torch.equal(first, out)
+    h.close()
+
+
+@pytest.mark.parametrize("B,S,heads,d", [(8, 197, 16, 32), (13, 100, 20, 40), (8, 250, 11, 40)])
+def test_projections_without_room_for_the_images(B, S, heads, d):
+    """The weights' terms are an offer: a workspace of the activations alone (Q, K, V and the attention's output), or one byte short of
+    what is asked for, gives the same layer with the weights cut in place; less is refused.  Bound: test_projection_plans'."""
+    Dm = heads * d
+    x, xf = gen((B, S, Dm), "f32", 1, 1.0)
+    ws, wfs = zip(*[gen((Dm, Dm), "f32", 2 + i, Dm ** -0.5) for i in range(4)])
+    want = O.mha_forward(xf, *wfs, heads)
+    with N.Handle(device=0, qkv_dtype=N.F32, out_dtype=N.F32, head_dim=d, num_q_heads=heads, num_kv_heads=heads) as h:
+        asked = h.mha_workspace_bytes(B, S, N.F32, N.F32)
+    least = 4 * ((B * S * Dm * 4 + 1023) // 1024 * 1024)
+    assert asked > least
+    for nbytes, launches in ((asked, 4), (asked - 1, 3), (least, 3)):
+        h, launch, out = _layer(x, ws, heads, workspace=nbytes)
+        launch()
+        h.poll(torch.cuda.current_stream().cuda_stream)
+        assert h.last_launch_count == launches
+        assert np.abs(out.cpu().numpy() - want).max() <= 12 * 2.0 ** -24 * Dm ** 0.5 * np.abs(want).max()
+        h.close()
+    h, launch, out = _layer(x, ws, heads, workspace=least - 1)
+    with pytest.raises(N.AidnError) as error:
+        launch()
+    assert error.value.status == N.EWORKSPACE
     h.close()
 
 
