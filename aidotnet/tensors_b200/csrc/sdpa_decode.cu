@@ -395,6 +395,11 @@ __global__ void __launch_bounds__(kDecWarps * 32)
 // bank-conflict free.  After the loop a warp reuses its own ring for the partials it hands to the merge.
 // NH16: more than 8 query heads per KV head (rows 8..15 of the tile are live).
 constexpr int kRingStages = 3;
+// CTAs of the ring kernels that an SM holds: by shared memory, and the compiler is held to it in registers.  (Left at two, heads of 64 took 168 to 186
+// of them for more than eight query heads, so that a third of the equal shares were a second wave: 245 items of up to 3521 keys and nine
+// heads 73 us, with three 46.)
+template <int D>
+constexpr int kRingCtas = D == 128 ? 2 : 3;
 
 template <int D>
 struct RingCfg {
@@ -558,7 +563,7 @@ struct RingWarp {
 };
 
 template <typename T, int D, bool NH16, bool PAGED, bool HEAD_FAST>
-__global__ void __launch_bounds__(kDecWarps * 32, 2)
+__global__ void __launch_bounds__(kDecWarps * 32, kRingCtas<D>)
     sdpa_decode_gqa_ring_kernel(const SdpaParams p, const int chunk, const int nchunks, float* __restrict__ ws,
                                 const int merge, const int cluster) {
   static_assert(sizeof(T) == 2 && (D == 64 || D == 128), "16-bit inputs, head_dim 64 or 128");
@@ -776,7 +781,7 @@ __device__ __forceinline__ StreamPlan stream_plan(int total, int shares) {
 }
 
 template <typename T, int D, bool NH16, bool PAGED>
-__global__ void __launch_bounds__(kDecWarps * 32, 2) sdpa_decode_stream_kernel(const SdpaParams p, float* __restrict__ ws, const int kv_heads, const int shares) {
+__global__ void __launch_bounds__(kDecWarps * 32, kRingCtas<D>) sdpa_decode_stream_kernel(const SdpaParams p, float* __restrict__ ws, const int kv_heads, const int shares) {
   using R = RingCfg<D>;
   constexpr int MT = D / 16, HN = NH16 ? 2 : 1;
   extern __shared__ __align__(128) uint8_t ring_smem[];
@@ -1121,7 +1126,7 @@ cudaError_t launch_partial_g(const SdpaParams& p, const DecodePlan& plan, float*
   return launch_partial<T, D, 8>(p, plan, ws, merge, stream);
 }
 
-constexpr int stream_ctas(int head_dim, int num_sms) { return (head_dim == 128 ? 2 : 3) * num_sms; }   // resident at once
+constexpr int stream_ctas(int head_dim, int num_sms) { return (head_dim == 128 ? kRingCtas<128> : kRingCtas<64>) * num_sms; }   // resident at once
 
 template <typename T, int D, bool NH16>
 cudaError_t launch_stream(const SdpaParams& p, const DecodePlan& plan, float* ws, cudaStream_t stream) {
@@ -1261,7 +1266,7 @@ void decode_plan_clusters(const SdpaParams& p, int dtype, int num_sms, DecodePla
   const bool ring = takes_ring(p, dtype), lengths = p.kv_len != nullptr, wide = p.head_dim == 128;
   if (!ring && (dtype != AIDN_F32 || p.group > 8)) return;
   const int64_t items = (int64_t)p.batch * (p.head_count / p.group), keys = p.seq_kv;
-  const int64_t room = (ring ? (wide ? 2 : 3) : 4) * (int64_t)num_sms;   // CTAs that are resident at once
+  const int64_t room = (ring ? (wide ? kRingCtas<128> : kRingCtas<64>) : 4) * (int64_t)num_sms;   // CTAs that are resident at once
   int64_t cluster = 1, clusters = 1;
   if (!ring) {
     const int64_t eights = (wide ? room : room * 94 / 100) / (8 * items);   // clusters of 8 per item
