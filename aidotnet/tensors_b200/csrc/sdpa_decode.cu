@@ -68,8 +68,7 @@ __device__ __forceinline__ void unpack16<__half>(const uint4& u, float* f) {
 }
 
 // Visible key count of a decode query of batch entry b: padding limit, then the causal limit of query 0.
-__device__ __forceinline__ int64_t decode_len(const SdpaParams& p, int b) {
-  int64_t L = kv_limit_of(p, b);
+__device__ __forceinline__ int64_t causal_len(const SdpaParams& p, int64_t L) {
   if (p.causal) {
     int64_t c = p.causal_offset + 1;
     if (c < 0) c = 0;
@@ -77,6 +76,7 @@ __device__ __forceinline__ int64_t decode_len(const SdpaParams& p, int b) {
   }
   return L;
 }
+__device__ __forceinline__ int64_t decode_len(const SdpaParams& p, int b) { return causal_len(p, kv_limit_of(p, b)); }
 
 // What a CTA does with the merged partial of its keys.
 enum DecodeMerge : int {
@@ -772,6 +772,11 @@ struct StreamPlan {
 };
 constexpr int kStreamLeast = 4;   // steps of a share at least
 __device__ __forceinline__ int stream_steps(const SdpaParams& p, int b) { return (int)((decode_len(p, b) + 15) / 16); }
+// The same for the merge, which reads the lengths ahead of its wait (sdpa_decode_stream_kernel triggers behind its own); there are lengths.
+__device__ __forceinline__ int stream_steps_early(const SdpaParams& p, int b) {
+  const int64_t n = ld_l2(p.kv_len + b);
+  return (int)((causal_len(p, n < 0 ? 0 : (n < p.seq_kv ? n : p.seq_kv)) + 15) / 16);
+}
 __device__ __forceinline__ StreamPlan stream_plan(int total, int shares) {
   StreamPlan s;
   s.total = total;
@@ -790,7 +795,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, kRingCtas<D>) sdpa_decode_stre
   const int nheads = p.group, h0 = p.head_begin + kvh * p.group;
   const uint32_t my_ring = ptx::smem_u32(ring_smem) + warp * R::kWarpBytes;
   pdl_wait();
-  pdl_trigger();
+  pdl_trigger();   // the merge finds its slots while this kernel runs
 
   int all = 0;
   for (int b0 = 0; b0 < p.batch; b0 += 32) all += __reduce_add_sync(0xffffffffu, b0 + lane < p.batch ? stream_steps(p, b0 + lane) : 0);
@@ -965,15 +970,13 @@ __global__ void __launch_bounds__(kDecWarps * 32, kRingCtas<D>) sdpa_decode_stre
 // chain over the splits except the last sum of 128 / (D / 4) partial columns.
 constexpr int kMaxCombine = 1024;   // split weights held in shared memory; more splits are taken in rounds
 
-// STREAM: the slots of sdpa_decode_stream_kernel; `nchunks` is then its number of shares.
-template <typename T, bool STREAM>
+template <typename T>
 __global__ void __launch_bounds__(128)
     sdpa_decode_combine_kernel(const SdpaParams p, const int chunk, const int nchunks, const float* ws) {
   __shared__ float weight[kMaxCombine];
   __shared__ float red[8];
   __shared__ float4 cols[128];
-  // The lengths come from a launch before the kernel that this one waits for, which has begun only after that one: they can be read now.
-  if constexpr (!STREAM) pdl_wait();   // the partial results of the kernel before this one
+  pdl_wait();   // the partial results of the kernel before this one
   const int b = blockIdx.y;
   const int hl = blockIdx.x;
   const int h = p.head_begin + hl;
@@ -981,81 +984,39 @@ __global__ void __launch_bounds__(128)
   const int Hc = p.head_count;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t L = decode_len(p, b);
-  int nvalid;
-  int64_t slot0;
-  const int hop = STREAM ? p.head_count : 1;   // partials from one of the head to its next
-  if constexpr (STREAM) {
-    __shared__ int sums[8];
-    int before = 0, all = 0;
-    for (int i = tid; i < p.batch; i += 128) {
-      const int n = stream_steps(p, i);
-      all += n;
-      if (i < b) before += n;
-    }
-    all = __reduce_add_sync(0xffffffffu, all);
-    before = __reduce_add_sync(0xffffffffu, before);
-    if (lane == 0) {
-      sums[warp] = all;
-      sums[4 + warp] = before;
-    }
-    __syncthreads();
-    const StreamPlan plan = stream_plan(sums[0] + sums[1] + sums[2] + sums[3], nchunks);
-    const int first = sums[4] + sums[5] + sums[6] + sums[7], steps = stream_steps(p, b);
-    nvalid = steps > 0 ? (first + steps - 1) / plan.per - first / plan.per + 1 : 0;
-    slot0 = (int64_t)(first / plan.per + b) * Hc + hl;
-    pdl_wait();
-  } else {
-    nvalid = (int)((L + chunk - 1) / chunk);
-    if (nvalid > nchunks) nvalid = nchunks;
-    slot0 = ((int64_t)b * Hc + hl) * nchunks;
-  }
-  const float2* ml = reinterpret_cast<const float2*>(ws + (STREAM ? (int64_t)(nchunks + p.batch) * Hc : (int64_t)p.batch * Hc * nchunks) * D) + slot0;
+  int nvalid = (int)((L + chunk - 1) / chunk);
+  if (nvalid > nchunks) nvalid = nchunks;
+  const int64_t slot0 = ((int64_t)b * Hc + hl) * nchunks;
+  const float2* ml = reinterpret_cast<const float2*>(ws + (int64_t)p.batch * Hc * nchunks * D) + slot0;
 
-  const int vecs = D / 4, groups = 128 / vecs;      // D = 64, 128, 256: 8, 4, 2 groups of splits
-  const int grp = tid / vecs, d4 = tid - grp * vecs;
-  const float4* rows = reinterpret_cast<const float4*>(ws + slot0 * D) + d4;
-  float4 early[4];   // STREAM: the thread's first columns, requested with the maxima
-  if constexpr (STREAM) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      early[i] = grp + i * groups < nvalid ? rows[(int64_t)(grp + i * groups) * hop * vecs] : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
   float M = -INFINITY;
-  for (int c = tid; c < nvalid; c += 128) M = fmaxf(M, ml[(int64_t)c * hop].x);
+  for (int c = tid; c < nvalid; c += 128) M = fmaxf(M, ml[c].x);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
   if (lane == 0) red[warp] = M;
   __syncthreads();
   M = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
 
+  const int vecs = D / 4, groups = 128 / vecs;      // D = 64, 128, 256: 8, 4, 2 groups of splits
+  const int grp = tid / vecs, d4 = tid - grp * vecs;
+  const float4* rows = reinterpret_cast<const float4*>(ws + slot0 * D) + d4;
   float lsum = 0.f;
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int c0 = 0; c0 < nvalid; c0 += kMaxCombine) {
     const int n = min(kMaxCombine, nvalid - c0);
     if (c0 > 0) __syncthreads();
     for (int c = tid; c < n; c += 128) {
-      const float2 v = ml[(int64_t)(c0 + c) * hop];
+      const float2 v = ml[c0 + c];
       const float w = v.x == -INFINITY ? -1.f : softmax_exp<T>(v.x - M);   // -1: a split that saw no key
       weight[c] = w;
       if (v.x != -INFINITY) lsum = fmaf(w, v.y, lsum);
     }
     __syncthreads();
-    int c = grp;
-    if constexpr (STREAM) {
-      if (c0 == 0) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i, c += groups) {
-          const float w = c < n ? weight[c] : -1.f;
-          if (w < 0.f) continue;
-          a.x = fmaf(w, early[i].x, a.x); a.y = fmaf(w, early[i].y, a.y); a.z = fmaf(w, early[i].z, a.z); a.w = fmaf(w, early[i].w, a.w);
-        }
-      }
-    }
 #pragma unroll 4
-    for (; c < n; c += groups) {
+    for (int c = grp; c < n; c += groups) {
       const float w = weight[c];
       if (w < 0.f) continue;   // its columns are undefined; a weight that underflows to 0 still carries their NaN and Inf
-      const float4 x = rows[(int64_t)(c0 + c) * hop * vecs];
+      const float4 x = rows[(int64_t)(c0 + c) * vecs];
       a.x = fmaf(w, x.x, a.x); a.y = fmaf(w, x.y, a.y); a.z = fmaf(w, x.z, a.z); a.w = fmaf(w, x.w, a.w);
     }
   }
@@ -1079,6 +1040,105 @@ __global__ void __launch_bounds__(128)
   }
   if (p.lse && tid == 0)
     p.lse[((int64_t)b * p.num_q_heads + h) * p.seq_q] = lsum > 0.f ? M + logf(lsum) : -INFINITY;
+}
+
+// The same for the slots of sdpa_decode_stream_kernel, which are found from the lengths alone, before the launch in front has ended.  W warps per
+// (sequence, head), each with every W-th row (heads of 64: two rows at a time) and eight passes in flight, a lane with four columns.  With
+// CTAs of a head each, whose threads met three times, it took 3 to 9 us behind its launch, and sequences of equal lengths were faster by
+// chunks; us, equal lengths / from 1 / 16 of the keys, chunks or clusters -> that -> this:
+//   D 128: 128 items, 2048 keys 27.9 -> 29.6 -> 28.4 / 22.1 -> 20.0 -> 18.9, in a pool 28.5 -> 30.8 -> 29.8 / 26.5 -> 20.9 -> 20.2; 65 items, 3729 keys
+//          24.9 -> 27.2 -> 25.2 / 20.1 -> 20.4 -> 18.3; 512 items, 500 keys 35.6 -> 29.3 -> 28.2 / 25.1 -> 20.5 -> 19.6
+//   D 64:  406 items, 885 keys 23.2 -> 24.8 -> 23.7 / 17.5 -> 17.7 -> 16.6; 368 items, 336 keys 14.4 -> 17.3 -> 13.8 / 11.8 -> 14.1 -> 11.0;
+//          402 items of eight heads, 1712 keys 42.8 -> 44.2 -> 37.9 / 29.1 -> 31.1 -> 24.5
+template <typename T, int D, int W>
+__global__ void __launch_bounds__(128) sdpa_decode_stream_merge_kernel(const SdpaParams p, const int shares, const float* ws) {
+  constexpr int kLanes = D / 4, kRows = 32 / kLanes, kHop = W * kRows, kFlight = 8;   // lanes of a row, rows of a warp's pass, rows to its next
+  __shared__ float4 cols[W][W > 1 ? kLanes : 1];
+  __shared__ float sums[W];
+  static_assert(W == 1 || W == 4, "a head per warp, or per CTA");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, b = blockIdx.y, Hc = p.head_count;
+  const int hl = W == 1 ? (int)blockIdx.x * 4 + warp : (int)blockIdx.x;
+  __shared__ int all_of[4], before_of[4], steps_of_b;
+  int before = 0, all = 0;
+  for (int i = threadIdx.x; i < p.batch; i += 128) {   // (every thread of all CTAs reads the same few lines of L2: once each)
+    const int n = stream_steps_early(p, i);
+    all += n;
+    if (i < b) before += n;
+    if (i == b) steps_of_b = n;
+  }
+  all = __reduce_add_sync(0xffffffffu, all);
+  before = __reduce_add_sync(0xffffffffu, before);
+  if (lane == 0) {
+    all_of[warp] = all;
+    before_of[warp] = before;
+  }
+  __syncthreads();
+  before = before_of[0] + before_of[1] + before_of[2] + before_of[3];
+  const StreamPlan plan = stream_plan(all_of[0] + all_of[1] + all_of[2] + all_of[3], shares);
+  const int steps = steps_of_b, first = before / plan.per;
+  const int n = steps > 0 && hl < Hc ? (before + steps - 1) / plan.per - first + 1 : 0;
+  const int64_t slot0 = (int64_t)(first + b) * Hc + hl;
+  const float2* ml = reinterpret_cast<const float2*>(ws + (int64_t)(shares + p.batch) * Hc * D) + slot0;
+  const float4* rows = reinterpret_cast<const float4*>(ws + slot0 * D) + lane % kLanes;
+  const int c0 = (W == 1 ? 0 : warp * kRows) + lane / kLanes;
+  pdl_wait();   // the partial results
+  pdl_trigger();
+
+  float4 x[kFlight];
+  float2 v[kFlight];
+  auto request = [&](int c) {
+#pragma unroll
+    for (int i = 0; i < kFlight; ++i) {
+      const int at = c + i * kHop;
+      x[i] = at < n ? rows[(int64_t)at * Hc * kLanes] : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[i] = at < n ? ml[(int64_t)at * Hc] : make_float2(-INFINITY, 0.f);
+    }
+  };
+  request(c0);
+  float M = -INFINITY;
+  for (int c = lane; c < n; c += 32) M = fmaxf(M, ml[(int64_t)c * Hc].x);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+  float l = 0.f;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int c = c0; c < n; c += kFlight * kHop) {
+    if (c > c0) request(c);
+#pragma unroll
+    for (int i = 0; i < kFlight; ++i) {
+      if (v[i].x == -INFINITY) continue;   // saw no key: its columns are undefined; a weight that underflows to 0 still carries NaN and Inf
+      const float w = softmax_exp<T>(v[i].x - M);
+      l = fmaf(w, v[i].y, l);
+      a.x = fmaf(w, x[i].x, a.x); a.y = fmaf(w, x[i].y, a.y); a.z = fmaf(w, x[i].z, a.z); a.w = fmaf(w, x[i].w, a.w);
+    }
+  }
+  if constexpr (kRows == 2) {
+    l += __shfl_xor_sync(0xffffffffu, l, 16);
+    a.x += __shfl_xor_sync(0xffffffffu, a.x, 16);
+    a.y += __shfl_xor_sync(0xffffffffu, a.y, 16);
+    a.z += __shfl_xor_sync(0xffffffffu, a.z, 16);
+    a.w += __shfl_xor_sync(0xffffffffu, a.w, 16);
+  }
+  if constexpr (W > 1) {
+    if (lane < kLanes) cols[warp][lane] = a;
+    if (lane == 0) sums[warp] = l;
+    __syncthreads();
+    if (warp > 0) return;
+#pragma unroll
+    for (int i = 1; i < W; ++i) {
+      const float4 y = cols[i][lane % kLanes];
+      a.x += y.x; a.y += y.y; a.z += y.z; a.w += y.w;
+      l += sums[i];
+    }
+  }
+  if (hl >= Hc || lane >= kLanes) return;
+  const int h = p.head_begin + hl;
+  const float inv = l > 0.f ? 1.f / l : 0.f;
+  const int64_t at = b * p.os[0] + (int64_t)h * p.os[1] + lane * 4;
+  store_out<T>(p.out, at, a.x * inv, p.out_f32);
+  store_out<T>(p.out, at + 1, a.y * inv, p.out_f32);
+  store_out<T>(p.out, at + 2, a.z * inv, p.out_f32);
+  store_out<T>(p.out, at + 3, a.w * inv, p.out_f32);
+  if (p.lse && lane == 0) p.lse[((int64_t)b * p.num_q_heads + h) * p.seq_q] = l > 0.f ? M + logf(l) : -INFINITY;
 }
 
 template <typename T, int D, int GT>
@@ -1137,8 +1197,11 @@ cudaError_t launch_stream(const SdpaParams& p, const DecodePlan& plan, float* ws
   const int kv_heads = p.head_count / p.group, shares = plan.stream_ctas * kDecWarps / kv_heads;
   e = launch_dependent(kern, dim3((unsigned)plan.stream_ctas), kDecWarps * 32, smem, stream, p, ws, kv_heads, shares);
   if (e != cudaSuccess) return e;
-  return launch_dependent(sdpa_decode_combine_kernel<T, true>, dim3((unsigned)p.head_count, (unsigned)p.batch), 128, 0, stream, p, 0, shares,
-                          static_cast<const float*>(ws));
+  // A CTA per output row while these are few (us at 128 / 65 items above with a warp each: 29.0 / 25.2 for 28.4 / 25.2; D 64, 406 rows 23.7 for 23.9).
+  const unsigned heads = (unsigned)p.head_count, batch = (unsigned)p.batch;
+  if ((int64_t)heads * batch <= (D == 128 ? 1024 : 256))
+    return launch_dependent(sdpa_decode_stream_merge_kernel<T, D, 4>, dim3(heads, batch), 128, 0, stream, p, shares, static_cast<const float*>(ws));
+  return launch_dependent(sdpa_decode_stream_merge_kernel<T, D, 1>, dim3((heads + 3) / 4, batch), 128, 0, stream, p, shares, static_cast<const float*>(ws));
 }
 
 template <typename T>
@@ -1169,7 +1232,7 @@ cudaError_t launch_decode_t(const SdpaParams& p, const DecodePlan& plan, float* 
   dim3 grid((unsigned)p.head_count, (unsigned)p.batch);
   *launches = 2;
   // chunk 1: with clusters every slot is written (m = -inf where there was no key)
-  return launch_dependent(sdpa_decode_combine_kernel<T, false>, grid, 128, 0, stream, p, plan.cluster > 1 ? 1 : plan.chunk, nchunks, static_cast<const float*>(ws));
+  return launch_dependent(sdpa_decode_combine_kernel<T>, grid, 128, 0, stream, p, plan.cluster > 1 ? 1 : plan.chunk, nchunks, static_cast<const float*>(ws));
 }
 
 
@@ -1308,7 +1371,9 @@ void decode_plan_clusters(const SdpaParams& p, int dtype, int num_sms, DecodePla
 //              heads of 64: 60 items, 3549 keys 15.6 -> 14.6; 405 items, 483 keys 13.7 -> 12.5; 128 items, 2048 keys 18.5 -> 15.9
 //   does not   96 items, 618 keys 10.2 -> 11.2; 110 items, 241 keys 7.2 -> 11.0; 54 items, 1395 keys 16.1 -> 17.9; 24 items, 5170 keys 15.3 ->
 //              16.9; 20 items, 8626 keys 21.5 -> 23.1; heads of 64: 190 items, 814 keys 11.0 -> 15.4; 84 items, 2711 keys 15.9 -> 19.4
-// Sequences that are all as long as the tensor lose a little (128 items of 2048 keys 29.6 -> 31.7): the host does not see the lengths.
+// (these with a merge that took 1 to 7 us longer, sdpa_decode_stream_merge_kernel).  The host does not see the lengths: sequences that are all as
+// long as the tensor take 0.82 of the time before in pools and 0.94 otherwise (137 shapes), and up to 1.06 where one wave of clusters of two had
+// been (144 items of 1795 keys 27.3 -> 28.9, 128 of 2048 in a pool 28.5 -> 29.9).
 int64_t decode_stream_bytes(const SdpaParams& p, int dtype, int num_sms, const DecodePlan& chunks, int* ctas) {
   *ctas = 0;
   if (!takes_ring(p, dtype) || chunks.nchunks <= 1) return 0;

@@ -29,8 +29,10 @@ def _lens(kind, B, Sk):
     return lens.astype(np.int32)
 
 
-# (B, Hq, Hkv, Sk, D, dtype): one and several query heads a KV head, above eight of them, KV heads that do not divide the warps
-SHAPES = [(70, 4, 4, 353, 128, "bf16"), (40, 24, 3, 1500, 64, "f16"), (33, 20, 10, 700, 128, "f16"), (24, 48, 4, 3000, 64, "bf16"), (100, 24, 2, 800, 128, "bf16")]
+# (B, Hq, Hkv, Sk, D, dtype): one and several query heads a KV head, above eight of them, KV heads that do not divide the warps; output rows for
+# a merge of a CTA each and of a warp each (heads off the four of a CTA), with "one" more partials than are in flight at once
+SHAPES = [(70, 4, 4, 353, 128, "bf16"), (40, 24, 3, 1500, 64, "f16"), (33, 20, 10, 700, 128, "f16"), (24, 48, 4, 3000, 64, "bf16"), (100, 24, 2, 800, 128, "bf16"),
+          (229, 1, 1, 700, 64, "bf16"), (45, 30, 10, 600, 64, "f16"), (62, 18, 9, 512, 128, "bf16")]
 
 
 @pytest.mark.parametrize("shape", SHAPES)
