@@ -562,8 +562,9 @@ struct RingWarp {
   }
 };
 
-template <typename T, int D, bool NH16, bool PAGED, bool HEAD_FAST>
-__global__ void __launch_bounds__(kDecWarps * 32, kRingCtas<D>)
+// CTAS: that the compiler leaves registers for.
+template <typename T, int D, bool NH16, bool PAGED, bool HEAD_FAST, int CTAS>
+__global__ void __launch_bounds__(kDecWarps * 32, CTAS)
     sdpa_decode_gqa_ring_kernel(const SdpaParams p, const int chunk, const int nchunks, float* __restrict__ ws,
                                 const int merge, const int cluster) {
   static_assert(sizeof(T) == 2 && (D == 64 || D == 128), "16-bit inputs, head_dim 64 or 128");
@@ -1152,20 +1153,31 @@ cudaError_t launch_partial(const SdpaParams& p, const DecodePlan& plan, float* w
   return launch_dependent_cluster(kern, grid, kDecWarps * 32, shape, 0, stream, p, plan.chunk, plan.nchunks, ws, merge, plan.cluster);
 }
 
-template <typename T, int D, bool NH16>
-cudaError_t launch_gqa(const SdpaParams& p, const DecodePlan& plan, float* ws, int merge, cudaStream_t stream) {
+template <typename T, int D, bool NH16, int CTAS>
+cudaError_t launch_gqa_ctas(const SdpaParams& p, const DecodePlan& plan, float* ws, int merge, cudaStream_t stream) {
   const unsigned kvheads = (unsigned)(p.head_count / p.group), parts = (unsigned)(plan.nchunks * plan.cluster);
   const bool head_fast = p.ks[1] < p.ks[2] && parts <= 65535;
   const dim3 grid = head_fast ? dim3(kvheads, parts, (unsigned)p.batch) : dim3(parts, kvheads, (unsigned)p.batch);
   const dim3 shape = head_fast ? dim3(1, (unsigned)plan.cluster) : dim3((unsigned)plan.cluster);
-  auto kern = head_fast ? (p.block_table ? sdpa_decode_gqa_ring_kernel<T, D, NH16, true, true> : sdpa_decode_gqa_ring_kernel<T, D, NH16, false, true>)
-                        : (p.block_table ? sdpa_decode_gqa_ring_kernel<T, D, NH16, true, false> : sdpa_decode_gqa_ring_kernel<T, D, NH16, false, false>);
+  auto kern = head_fast ? (p.block_table ? sdpa_decode_gqa_ring_kernel<T, D, NH16, true, true, CTAS> : sdpa_decode_gqa_ring_kernel<T, D, NH16, false, true, CTAS>)
+                        : (p.block_table ? sdpa_decode_gqa_ring_kernel<T, D, NH16, true, false, CTAS> : sdpa_decode_gqa_ring_kernel<T, D, NH16, false, false, CTAS>);
   constexpr int smem = RingCfg<D>::kSmemBytes;
   if (smem > 48 * 1024) {   // (below, a launch needs no leave for it)
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
   }
   return launch_dependent_cluster(kern, grid, kDecWarps * 32, shape, smem, stream, p, plan.chunk, plan.nchunks, ws, merge, plan.cluster);
+}
+
+// Heads of 64 with more than eight query heads in a pool: three CTAs an SM take nine registers from each, 0.6 to 1.2 us where two an SM are all
+// there is (113 items of 508 keys, 16 heads 13.1 -> 14.3), and save a second wave where there are more (100 items of 500 keys, 9 heads 16.1 -> 9.4).
+template <typename T, int D, bool NH16>
+cudaError_t launch_gqa(const SdpaParams& p, const DecodePlan& plan, float* ws, int merge, cudaStream_t stream) {
+  if constexpr (NH16 && D == 64) {
+    const int64_t ctas = (int64_t)(p.head_count / p.group) * p.batch * plan.nchunks * plan.cluster;
+    if (ctas <= 2 * 148) return launch_gqa_ctas<T, D, NH16, 2>(p, plan, ws, merge, stream);
+  }
+  return launch_gqa_ctas<T, D, NH16, kRingCtas<D>>(p, plan, ws, merge, stream);
 }
 
 // 16-bit inputs with up to 16 query heads per KV head (plain multi-head attention included: the padding rows of the MMA

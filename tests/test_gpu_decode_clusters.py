@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 # (B, Hq, Hkv, Sk, D, dtype, launches)
 CASES = [(1, 4, 4, 1237, 64, "bf16", 1), (3, 8, 2, 700, 128, "f16", 1), (1, 16, 1, 600, 128, "bf16", 1), (20, 4, 2, 500, 128, "bf16", 1),
          (16, 8, 8, 300, 128, "bf16", 1), (40, 12, 4, 200, 64, "f16", 1), (2, 4, 2, 4400, 128, "bf16", 2), (1, 8, 8, 9000, 64, "bf16", 2),
-         (2, 4, 4, 500, 64, "f32", 1), (1, 6, 2, 400, 128, "f32", 1), (1, 4, 4, 4000, 64, "f32", 2)]
+         (2, 4, 4, 500, 64, "f32", 1), (1, 6, 2, 400, 128, "f32", 1), (1, 4, 4, 4000, 64, "f32", 2),
+         (9, 48, 4, 600, 64, "bf16", 1), (12, 36, 4, 500, 64, "f16", 1)]   # more than eight heads: up to two CTAs an SM, and three
 
 
 @pytest.mark.parametrize("case", CASES)
