@@ -614,31 +614,43 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
     if (warp < kWorkers / 32 && !*abort_flag) {
       const int64_t out_rows = KEYS ? p.seq_kv : p.seq_q;
       const int64_t base = KEYS ? ((int64_t)b * kv_heads + blockIdx.y) * out_rows : ((int64_t)b * p.head_count + hl0) * out_rows;
-      // Four vectors of every CTA in flight, and nothing divided (one at a time, the sums of two CTAs took 8000 cycles).
+      // Eight vectors in flight, and nothing divided (one at a time, the sums of two CTAs took 8000 cycles): four of a thread's own from two CTAs, or
+      // where it has fewer one from all (four whatever it has, the missing ones read again, took B2 H1 S512 D64 causal 34 -> 38 us; this 28).
+      // All numbers here are powers of two: four times their distance divides the vectors, or there are fewer.
       constexpr int kVecs = KS * 4, kItems = kOwn * kVecs * (KEYS ? 2 : 1);   // (of a row; those past head_dim are not stored)
       const int hop = tp.splits * kWorkers;
-      for (int idx0 = rank * kWorkers + tid; idx0 < kItems; idx0 += 4 * hop) {
-        float4 y[4];
+      auto at = [&](int idx) { return smem_base + (uint32_t)((idx / kVecs * kPartPitch + idx % kVecs * 4) * 4); };
+      auto put = [&](int idx, const float4& y) {
+        const int which = idx / (kOwn * kVecs), r = idx / kVecs % kOwn, d = idx % kVecs * 4;
+        if (own0 + r >= out_rows || d >= D) return;
+        const float f = which ? 1.f : p.scale;
+        float* out = (which ? bp.dv : (KEYS ? bp.dk : bp.dq)) + (base + own0 + r) * D + d;
+        *reinterpret_cast<float4*>(out) = make_float4(y.x * f, y.y * f, y.z * f, y.w * f);
+      };
+      if (kItems >= 4 * hop) {
+        for (int idx = rank * kWorkers + tid; idx < kItems; idx += 4 * hop) {
+          float4 y[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int e = 0; e < 4; ++e) y[e] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 2
-        for (int i = 0; i < tp.splits; ++i) {
-          float4 u[4];
+          for (int i = 0; i < tp.splits; ++i) {
+            float4 u[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int idx = idx0 + e * hop < kItems ? idx0 + e * hop : idx0;
-            u[e] = ld_cluster_f4(smem_base + (uint32_t)((idx / kVecs * kPartPitch + idx % kVecs * 4) * 4), (uint32_t)i);
+            for (int e = 0; e < 4; ++e) u[e] = ld_cluster_f4(at(idx + e * hop), (uint32_t)i);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[e].x += u[e].x, y[e].y += u[e].y, y[e].z += u[e].z, y[e].w += u[e].w;
           }
 #pragma unroll
-          for (int e = 0; e < 4; ++e) y[e].x += u[e].x, y[e].y += u[e].y, y[e].z += u[e].z, y[e].w += u[e].w;
+          for (int e = 0; e < 4; ++e) put(idx + e * hop, y[e]);
         }
+      } else {
+        for (int idx = rank * kWorkers + tid; idx < kItems; idx += hop) {
+          float4 u[8], y = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int idx = idx0 + e * hop, which = idx / (kOwn * kVecs), r = idx / kVecs % kOwn, d = idx % kVecs * 4;
-          if (idx >= kItems || own0 + r >= out_rows || d >= D) continue;
-          const float f = which ? 1.f : p.scale;
-          float* out = (which ? bp.dv : (KEYS ? bp.dk : bp.dq)) + (base + own0 + r) * D + d;
-          *reinterpret_cast<float4*>(out) = make_float4(y[e].x * f, y[e].y * f, y[e].z * f, y[e].w * f);
+          for (int i = 0; i < 8; ++i) u[i] = i < tp.splits ? ld_cluster_f4(at(idx), (uint32_t)i) : y;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) y.x += u[i].x, y.y += u[i].y, y.z += u[i].z, y.w += u[i].w;
+          put(idx, y);
         }
       }
     }
