@@ -676,14 +676,24 @@ cudaError_t launch_t(const BwdParams& bp, cudaStream_t stream, int* launches, co
   const unsigned grid_q = (unsigned)(items_q < sms ? items_q : sms), grid_kv = (unsigned)(items_kv < sms ? items_kv : sms);
   BwdSm100Params sk = sp;
   sk.total_items = (int)items_kv;
-  // (long launches gain nothing by it, and dK / dV beside dQ would share the L2 cache: B2 H19 S7521 D64 causal 1254 -> 1277 us)
-  if (items_q * sp.k_tiles <= (int64_t)sms * 256) {
+  // Long launches gain nothing by it, and dK / dV beside dQ would share the L2 cache (B2 H19 S7521 D64 causal 1254 -> 1277 us).
+  const bool shorter = items_q * sp.k_tiles <= (int64_t)sms * 256;
+  // dK / dV beside dQ.  In its last wave dQ leaves `spare` SMs to the first of dK / dV's CTAs; items of one length gain by that only if those are
+  // the ones with an item more than the others (by the snake the first where the whole waves are even in number).  Where they are not, heads
+  // of 64 only share the memory: 182 items of each, B1 H7 S3264, 143.6 -> 146.8 us (one after the other, with a dependent dQ, 142.9), 640 and 160, B2 Hq64 / Hkv16 S587, 112.0 -> 113.4
+  // (110.1); where they are: 312, B3 H8 S1574, 119 -> 103, 448 and 112, B2 Hq32 / Hkv8 S824, 91 -> 82.  One wave (S1020 35.0 -> 33.8), items of unequal length (S2018
+  // causal 98 -> 94) and heads of 128 (252 items, B4 H9 S850, 80.6 -> 79.9) gain either way.
+  const int64_t waves_q = (items_q + sms - 1) / sms, waves_kv = (items_kv + sms - 1) / sms;
+  const int64_t spare = waves_q * sms - items_q, more = items_kv - (waves_kv - 1) * sms;
+  const bool beside = shorter && (HD == 128 || p.causal || waves_q == 1 || (waves_kv % 2 == 1 && more <= spare));
+  if (shorter) {
     e = launch_dependent(kq, dim3(grid_q), kThreads, smem_q, stream, tq, tk, tv, tdo, sp);
-    return e != cudaSuccess ? e : launch_dependent(kkv, dim3(grid_kv), kThreads, smem_kv, stream, tq, tk, tv, tdo, sk);
+  } else {
+    kq<<<grid_q, kThreads, smem_q, stream>>>(tq, tk, tv, tdo, sp);
+    e = cudaGetLastError();
   }
-  kq<<<grid_q, kThreads, smem_q, stream>>>(tq, tk, tv, tdo, sp);
-  e = cudaGetLastError();
   if (e != cudaSuccess) return e;
+  if (beside) return launch_dependent(kkv, dim3(grid_kv), kThreads, smem_kv, stream, tq, tk, tv, tdo, sk);
   kkv<<<grid_kv, kThreads, smem_kv, stream>>>(tq, tk, tv, tdo, sk);
   return cudaGetLastError();
 }

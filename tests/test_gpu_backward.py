@@ -284,3 +284,17 @@ def test_backward_bounded_waits_expire_cleanly():
     _check(dk, rk, "bf16", "dK after a timed-out backward")
     _check(dv, rv, "bf16", "dV after a timed-out backward")
     h.close()
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,D", [(16, 5, 5, 64), (12, 13, 13, 64), (16, 20, 5, 64), (16, 5, 5, 128)])
+def test_waves_of_items(B, Hq, Hkv, D):
+    """More items than SMs, two of 129 rows to a sequence and head: dK / dV behind dQ (its CTAs with two items are the last), beside it (the first), in one wave
+    beside several of dQ, and heads of 128."""
+    S = 129
+    q, qf = gen((B, Hq, S, D), "bf16", 1)
+    k, kf = gen((B, Hkv, S, D), "bf16", 2)
+    v, vf = gen((B, Hkv, S, D), "bf16", 3)
+    g, gf = gen((B, Hq, S, D), "f32", 4, scale=1.0)
+    got = _fwd_bwd(q, k, v, g, dtype="bf16")
+    for x, y, name in zip(got, O.sdpa_backward(qf, kf, vf, gf), ("dQ", "dK", "dV")):
+        _check(x, y, "bf16", f"{name} {(B, Hq, Hkv, D)}")
