@@ -354,7 +354,7 @@ struct alignas(64) PrefillMapCache {
     int32_t batch, kv_batch, num_q_heads, num_kv_heads, head_dim, kv_box, out_f32, splits, dtype;
   } key;
   bool valid;
-  bool attr_set[24];            // by instantiation: 8 * (plain, softcap, mask) + (epilogue warpgroup ? 4 : 0) + (fp16 ? 2 : 0) + (head_dim 128 ? 1 : 0)
+  bool attr_set[40];            // by instantiation: 8 * (PrefillMode) + (epilogue warpgroup ? 4 : 0) + (fp16 ? 2 : 0) + (head_dim 128 ? 1 : 0)
 };
 bool prefill_sm100_supported(const SdpaParams& p, int dtype, const char** why);
 // How many parts the keys of every work item should be cut into (1: none), and the workspace (16-byte aligned) that this

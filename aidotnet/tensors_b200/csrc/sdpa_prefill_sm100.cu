@@ -360,10 +360,12 @@ __device__ __forceinline__ void store_o_tile(const SdpaParams& p, const CUtensor
   }
 }
 
-// What the softmax warps do to a score besides scaling it: nothing, a softcap, or a bias or keep-mask read from global memory (and perhaps a
+// What the softmax warps do to a score besides scaling it: nothing, a softcap, or a keep-mask or bias read from global memory (and perhaps a
 // softcap).  Each carries none of the others' code: behind the masks' branches and registers the softcap alone took 512 -> 640 us
-// on a long prefill.
-enum PrefillMode { kPlain, kCapped, kMasked };
+// on a long prefill, and a bias beside the other masks of its kind 90 -> 99 (3 x 4 heads of 1788 x 1792, D 128, causal).
+// kKeep: bytes, and one row of floats for all queries, as bits.  kBias and kKeepFloats: floats through the softmax warps' staging buffers, so
+// in the layout without epilogue warps.
+enum PrefillMode { kPlain, kCapped, kKeep, kBias, kKeepFloats };
 
 template <typename T, int HD, PrefillMode MODE, bool EPI>
 __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
@@ -373,7 +375,8 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
   using C = Cfg<HD>;
   using R = Roles<EPI>;
   constexpr bool kBf16 = !std::is_same_v<T, __half>;
-  constexpr bool MASKED = MODE == kMasked, kScaled = MODE != kPlain;
+  constexpr bool MASKED = MODE >= kKeep, kTiles = MODE == kBias || MODE == kKeepFloats, kScaled = MODE != kPlain;
+  static_assert(!(kTiles && EPI), "the staging buffers are the epilogue warps'");
   const SdpaParams& p = pp.p;
 
   extern __shared__ uint8_t smem_raw[];
@@ -530,30 +533,31 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
 
       float m = -INFINITY, l = 0.f;
 
-      // The explicit mask, a sub-tile ahead: bits of the row's 64 keys, or a bias of its first 32 in the staging buffer and of the other
-      // 32 - by the lanes' keys - in registers (a bias takes the layout without epilogue warps).
-      // Bytes of aligned rows: the row's own, four 16-byte loads (1 x 25 heads of 432, D 64, causal: 23 us, by lanes' keys 35).
-      const bool add = MASKED && !EPI && p.mask_kind == AIDN_MASK_ADD_F32;
+      // The explicit mask, a sub-tile ahead: bits of the row's 64 keys, or floats of its first 32 in the staging buffer and of the other
+      // 32 - by the lanes' keys - in registers.
+      // Bytes: the row's own, by loads of 16 or of 4 as it is aligned, or bits where it is less than that.  us, by the row's single bytes (16-byte rows:
+      // vectors) -> bits of 64 rows -> this: 25 heads of 432, D 64, causal - -> 35 -> 23; 7 x 2 of 1016, D 64 47.4 -> 54.8 -> 26.3; 2 x 12 of 120,
+      // D 128, causal 15.6 -> 17.7 -> 11.3.
       uint32_t keep0 = 0, keep1 = 0;
-      float held[!MASKED ? 1 : (EPI ? 16 : 32)];   // the bias in registers, or the row's 64 bytes
+      float held[!MASKED ? 1 : (kTiles ? 32 : 16)];   // floats of the mask, or the row's 64 bytes
       const int64_t mask_row = (int64_t)ti.t * kBM + quarter * 32;
       const int mask_rows = masktile::clamp32(p.seq_q - mask_row);
       const uint8_t* byte_row = static_cast<const uint8_t*>(p.mask);   // of this thread, at the item's first key
-      bool bytes = false;
-      if (MASKED && p.mask_kind == AIDN_MASK_KEEP_U8 && p.mask_stride[3] == 1 && p.mask_stride[2] != 0 && p.seq_kv % 16 == 0) {
+      uint32_t off = 15;   // where its ends are off 16 bytes
+      if (MODE == kKeep && p.mask_kind == AIDN_MASK_KEEP_U8 && p.mask_stride[3] == 1 && p.mask_stride[2] != 0) {
         byte_row += (int64_t)b * p.mask_stride[0] + (int64_t)ti.h * p.mask_stride[1] + (qrow < p.seq_q ? qrow : p.seq_q - 1) * p.mask_stride[2] +
                     (int64_t)it.k0 * kBS;
-        bytes = __all_sync(0xffffffffu, (reinterpret_cast<uintptr_t>(byte_row) & 15) == 0);
+        off = __reduce_or_sync(0xffffffffu, ((uint32_t)reinterpret_cast<uintptr_t>(byte_row) | (uint32_t)p.seq_kv) & 15u);
       }
-      const bool keep = MASKED && !bytes && (p.mask_kind == AIDN_MASK_KEEP_U8 || p.mask_kind == AIDN_MASK_KEEP_F32);
+      const bool bytes = MODE == kKeep && (off & 3) == 0, keep = MODE == kKeep && !bytes;
       const int64_t mask_at = MASKED ? (int64_t)b * p.mask_stride[0] + (int64_t)ti.h * p.mask_stride[1] + mask_row * p.mask_stride[2] : 0;
       auto request_keep = [&](int u) {
         const int64_t key = (int64_t)(it.k0 + u) * kBS, ms2 = p.mask_stride[2], ms3 = p.mask_stride[3];
         keep0 = masktile::keep_bits_of(p, mask_at + key * ms3, ms2, ms3, mask_rows, masktile::clamp32(p.seq_kv - key), lane);
         keep1 = masktile::keep_bits_of(p, mask_at + (key + 32) * ms3, ms2, ms3, mask_rows, masktile::clamp32(p.seq_kv - key - 32), lane);
       };
-      auto request_bias = [&](int u) {
-        if constexpr (MASKED && !EPI) {
+      auto request_tile = [&](int u) {
+        if constexpr (kTiles) {
           const int64_t key = (int64_t)(it.k0 + u) * kBS, ms2 = p.mask_stride[2], ms3 = p.mask_stride[3];
           const float* src = static_cast<const float*>(p.mask) + mask_at + key * ms3;
           masktile::request(my_stage, src, ms2, ms3, mask_rows, masktile::clamp32(p.seq_kv - key), lane);
@@ -562,10 +566,10 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
       };
       if (MASKED && ti.n > 0) {
         if (keep) request_keep(0);
-        if (add) {
+        if (kTiles) {
           if (stores_in_flight && lane == 0) bulk_wait_read0();   // the staging buffer may still be read by a store
           __syncwarp();
-          request_bias(0);
+          request_tile(0);
         }
       }
 
@@ -573,13 +577,20 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
         const uint32_t buf = (uint32_t)(u & 1);
         const uint32_t t_sb = t_s + buf * kBS;
         const uint32_t bar_off = 8u * (uint32_t)(2 * i) + 8u * buf;
-        if constexpr (MASKED) {
+        if constexpr (MODE == kKeep) {
           if (bytes) {
+            const int64_t left = p.seq_kv - (int64_t)(it.k0 + u) * kBS;
+            const uint8_t* src = byte_row + u * kBS;
+            if (off == 0) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-              if ((int64_t)(it.k0 + u) * kBS + 16 * q < p.seq_kv) v = *reinterpret_cast<const float4*>(byte_row + u * kBS + 16 * q);
-              held[4 * q] = v.x; held[4 * q + 1] = v.y; held[4 * q + 2] = v.z; held[4 * q + 3] = v.w;
+              for (int q = 0; q < 16; q += 4) {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (4 * q < left) v = *reinterpret_cast<const float4*>(src + 4 * q);
+                held[q] = v.x; held[q + 1] = v.y; held[q + 2] = v.z; held[q + 3] = v.w;
+              }
+            } else {
+#pragma unroll
+              for (int q = 0; q < 16; ++q) held[q] = 4 * q < left ? *reinterpret_cast<const float*>(src + 4 * q) : 0.f;
             }
           }
         }
@@ -609,7 +620,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
             const float f = p.scale / p.softcap;
 #pragma unroll
             for (int c = 0; c < kBS; ++c) s[c] = p.softcap * tanh_approx(s[c] * f);
-          } else if (!add) {
+          } else if (MODE != kBias) {
 #pragma unroll
             for (int c = 0; c < kBS; ++c) s[c] *= p.scale;
           }
@@ -622,26 +633,29 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
             for (int c = 0; c < kBS; ++c)
               if (((__float_as_uint(held[c >> 2]) >> (8 * (c & 3))) & 0xffu) == 0u) s[c] = -INFINITY;
           }
-          if constexpr (!EPI) {
-            if (add) {
-              const float f = p.softcap > 0.f ? 1.f : p.scale;
-              auto add_tile = [&](int c0) {
+          if constexpr (kTiles) {
+            const float f = p.softcap > 0.f ? 1.f : p.scale;
+            auto take_tile = [&](int c0) {
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                  const float4 v = masktile::row4(my_stage, c, lane);
-                  float* x = s + c0 + 4 * c;
+              for (int c = 0; c < 8; ++c) {
+                const float4 v = masktile::row4(my_stage, c, lane);
+                float* x = s + c0 + 4 * c;
+                if constexpr (MODE == kBias) {
                   x[0] = fmaf(x[0], f, v.x); x[1] = fmaf(x[1], f, v.y); x[2] = fmaf(x[2], f, v.z); x[3] = fmaf(x[3], f, v.w);
+                } else {
+                  x[0] = v.x == 0.f ? -INFINITY : x[0]; x[1] = v.y == 0.f ? -INFINITY : x[1];
+                  x[2] = v.z == 0.f ? -INFINITY : x[2]; x[3] = v.w == 0.f ? -INFINITY : x[3];
                 }
-                __syncwarp();   // the values have been read
-              };
-              cp_async_wait_f<0>();
-              __syncwarp();   // every lane's copies are there
-              add_tile(0);
-              masktile::put(my_stage, held, lane);
-              __syncwarp();
-              add_tile(32);
-              if (u + 1 < ti.n) request_bias(u + 1);
-            }
+              }
+              __syncwarp();   // the values have been read
+            };
+            cp_async_wait_f<0>();
+            __syncwarp();   // every lane's copies are there
+            take_tile(0);
+            masktile::put(my_stage, held, lane);
+            __syncwarp();
+            take_tile(32);
+            if (u + 1 < ti.n) request_tile(u + 1);
           }
         }
         if (col0 + kBS - 1 > kmax_row) {
@@ -1475,15 +1489,21 @@ bool prefill_sm100_supported(const SdpaParams& p, int dtype, const char** why) {
 template <typename T, int HD, PrefillMode MODE>
 cudaError_t launch_t(const SdpaParams& p, cudaStream_t stream, int32_t* sched, int num_sms, float* debug,
                      int debug_mode, PrefillMapCache* cache, int splits, const char** why) {
-  const bool epi = ((p.group % 2 == 0) || !p.causal) && p.mask_kind != AIDN_MASK_ADD_F32;   // (a bias goes through the softmax warps' staging buffers)
-  if (epi) return launch_e<T, HD, MODE, true>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  if constexpr (MODE < kBias) {
+    if (p.group % 2 == 0 || !p.causal) return launch_e<T, HD, MODE, true>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  }
   return launch_e<T, HD, MODE, false>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
 }
 
 template <typename T, int HD>
 cudaError_t launch_m(const SdpaParams& p, cudaStream_t stream, int32_t* sched, int num_sms, float* debug, int debug_mode,
                      PrefillMapCache* cache, int splits, const char** why) {
-  if (p.mask_kind != AIDN_MASK_NONE) return launch_t<T, HD, kMasked>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  if (p.mask_kind == AIDN_MASK_ADD_F32) return launch_t<T, HD, kBias>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  // Keep-masks of floats, us, by threads' own rows -> bits of 64 rows -> tiles: 6 x 4 heads of 832, D 64, causal 60.5 -> 70.1 -> 43.8; 7 x 2 of 1016, D 64
+  // 47.6 -> 54.1 -> 38.7; 4 x 9 of 1402 x 1408, D 128 255 -> 232 -> 157.  One row of them is a pair of ballots.
+  if (p.mask_kind == AIDN_MASK_KEEP_F32 && p.mask_stride[2] != 0)
+    return launch_t<T, HD, kKeepFloats>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
+  if (p.mask_kind != AIDN_MASK_NONE) return launch_t<T, HD, kKeep>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
   if (p.softcap > 0.f) return launch_t<T, HD, kCapped>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
   return launch_t<T, HD, kPlain>(p, stream, sched, num_sms, debug, debug_mode, cache, splits, why);
 }

@@ -12,8 +12,9 @@ from tests.test_gpu_backward import _check, _fwd_bwd
 
 pytestmark = pytest.mark.gpu
 
-# (B, Hq, Hkv, Sq, Sk, D): keys in whole tiles of 64, in whole 16-byte rows, and neither; rows up to one past a tile
-SHAPES = [(2, 2, 2, 128, 192, 64), (1, 4, 2, 129, 208, 128), (2, 3, 1, 33, 97, 64), (1, 2, 1, 257, 450, 128), (3, 2, 2, 31, 523, 64)]
+# (B, Hq, Hkv, Sq, Sk, D): keys in whole tiles of 64, in whole 16-byte rows, neither, and in whole 4-byte rows; rows up to one past a tile
+SHAPES = [(2, 2, 2, 128, 192, 64), (1, 4, 2, 129, 208, 128), (2, 3, 1, 33, 97, 64), (1, 2, 1, 257, 450, 128), (3, 2, 2, 31, 523, 64), (2, 2, 2, 70, 100, 64),
+          (1, 3, 3, 129, 120, 128)]
 KINDS = ["bytes", "floats", "bias"]
 LAYOUTS = ["dense", "offset", "one_row", "one_key", "transposed"]
 
