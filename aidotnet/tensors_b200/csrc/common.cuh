@@ -183,8 +183,18 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // The one exception: what launches before its predecessor have written, a kernel may read ahead of its own wait if every CTA of
 // the predecessor triggers behind the predecessor's wait.  Those launches have then ended, and their writes are in the L2 cache; the wait
-// made them visible to the predecessor alone, though, so an older copy might still be in an L1: it is read past that (ld_l2).  What the
-// predecessor reads or writes itself stays behind the wait, and the kernel must not end without one: the next launch relies on both.
+// made them visible to the predecessor alone, though, so an older copy might still be in an L1.  Either the kernel reads past that (ld_l2),
+// or the predecessor triggers by pdl_hand_over and every thread of the kernel begins with pdl_take_over, whose fences carry on what the wait has
+// given.  What the predecessor writes, and writes that it might read, stay behind the wait, and the kernel must not end without one: the next launch
+// relies on both.
+__device__ __forceinline__ void pdl_hand_over() {
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  pdl_trigger();
+}
+__device__ __forceinline__ void pdl_take_over() {
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  asm volatile("fence.proxy.async.global;" ::: "memory");   // TMA loads too
+}
 __device__ __forceinline__ int32_t ld_l2(const int32_t* ptr) {
   int32_t r;
   asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(r) : "l"(ptr) : "memory");

@@ -171,8 +171,8 @@ __device__ __forceinline__ bool all_finite(const uint64_t (&acc)[N]) {   // (or 
 
 // KS: k steps of 16 columns (2: head sizes up to 32).
 // dQ waits for the kernel that formed delta.  dK / dV, which follows on the stream, needs nothing of dQ: it starts when all of dQ's CTAs
-// have begun - by then every launch before dQ is complete - and takes the SMs that dQ leaves idle; it ends only after dQ has, so that
-// what comes next on the stream may rely on both.
+// have begun - by then every launch before dQ is complete, and what it reads of theirs dQ hands over - and takes the SMs that dQ leaves idle; it
+// ends only after dQ has, so that what comes next on the stream may rely on both.
 template <int KS, bool KEYS, bool PLAIN>
 __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid_constant__ BwdParams bp, const BwdTcParams tp) {
   const SdpaParams& p = bp.p;
@@ -207,8 +207,13 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
-  if (!KEYS) pdl_wait();   // (dK / dV: at its end)
-  pdl_trigger();
+  if (!KEYS) {
+    pdl_wait();
+    if (warp == kIssuer + 1) pdl_hand_over();   // (a warp that has to wait first; it speaks for the CTA)
+  } else {   // waits at its end
+    pdl_take_over();
+    pdl_trigger();
+  }
   const Place at = place_of<KEYS>(p, tp.splits);
   const int b = at.b, hl0 = at.hl0, h0 = at.h0, kvh = h0 / p.group, kv_heads = p.head_count / p.group, rank = (int)blockIdx.x % tp.splits;
   const int per_head = at.per_head, s_begin = at.s_begin, n = at.n;

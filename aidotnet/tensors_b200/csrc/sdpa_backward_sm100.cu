@@ -135,8 +135,8 @@ template <bool KEYS>
 __device__ __forceinline__ int step_tile(const Work& w, int j) { return KEYS ? w.first + j % w.count : j; }
 
 // dQ waits for the kernel that formed delta.  dK / dV, which follows on the stream, needs nothing of dQ: it starts when all of dQ's CTAs
-// have begun - by then every launch before dQ is complete - and takes the SMs that dQ leaves idle; it ends only after dQ has, so that
-// what comes next on the stream may rely on both.
+// have begun - by then every launch before dQ is complete, and what it reads of theirs dQ hands over - and takes the SMs that dQ leaves idle; it
+// ends only after dQ has, so that what comes next on the stream may rely on both.
 template <typename T, int HD, bool KEYS, bool MASKED>
 __global__ void __launch_bounds__(kThreads, 1)
     sdpa_backward_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -192,8 +192,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
-  if (!KEYS) pdl_wait();   // (dK / dV: at its end)
-  pdl_trigger();
+  if (!KEYS) {
+    pdl_wait();
+    if (warp == 2) pdl_hand_over();   // (a warp that has to wait first; it speaks for the CTA)
+  } else {   // waits at its end
+    pdl_take_over();
+    pdl_trigger();
+  }
 
   // Persistent CTAs: CTA k takes items k, 2G-1-k, 2G+k, ... (G = grid size; the item list is ordered heaviest first, and
   // the snake keeps the sum per CTA even).  Counters that persist across items give every barrier its phase:
