@@ -210,13 +210,13 @@ __device__ __forceinline__ uint4 ld_stream16(const void* ptr) {
   return r;
 }
 
-// Launched as thread-block clusters of `cluster` CTAs (1 x 1 x 1: none).
+// Launched as thread-block clusters of `cluster` CTAs (1 x 1 x 1: none), behind the whole of the launch before or as a dependent of it.
 template <typename... P, typename... A>
-inline cudaError_t launch_dependent_cluster(void (*kern)(P...), dim3 grid, unsigned threads, dim3 cluster, size_t smem,
-                                            cudaStream_t stream, A... args) {
+inline cudaError_t launch_cluster(bool dependent, void (*kern)(P...), dim3 grid, unsigned threads, dim3 cluster, size_t smem,
+                                  cudaStream_t stream, A... args) {
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].val.programmaticStreamSerializationAllowed = dependent ? 1 : 0;
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = cluster.x;
   attr[1].val.clusterDim.y = cluster.y;
@@ -231,6 +231,12 @@ inline cudaError_t launch_dependent_cluster(void (*kern)(P...), dim3 grid, unsig
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
   if (e != cudaSuccess) cudaGetLastError();   // reported here: the next launch must not find it as its own
   return e;
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent_cluster(void (*kern)(P...), dim3 grid, unsigned threads, dim3 cluster, size_t smem,
+                                            cudaStream_t stream, A... args) {
+  return launch_cluster(true, kern, grid, threads, cluster, smem, stream, args...);
 }
 
 template <typename... P, typename... A>

@@ -665,6 +665,18 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_sm100_kernel(const __grid
   if (KEYS) pdl_wait();
 }
 
+// dK / dV laid over K or V, which a CTA has read by the time it stores its own rows: not beside dQ, whose CTAs still read them.
+bool gradients_over_keys(const BwdParams& bp) {
+  const SdpaParams& p = bp.p;
+  const int64_t heads = p.num_kv_heads, count = (int64_t)p.batch * (p.head_count / p.group) * p.seq_kv * p.head_dim;
+  auto over = [&](const float* grad, const void* in, const int64_t* stride) {
+    const uintptr_t g = reinterpret_cast<uintptr_t>(grad), i = reinterpret_cast<uintptr_t>(in);
+    const int64_t last = (p.batch - 1) * stride[0] + (heads - 1) * stride[1] + (p.seq_kv - 1) * stride[2] + p.head_dim;
+    return g < i + (uintptr_t)last * sizeof(float) && i < g + (uintptr_t)count * sizeof(float);
+  };
+  return over(bp.dk, p.k, p.ks) || over(bp.dk, p.v, p.vs) || over(bp.dv, p.k, p.ks) || over(bp.dv, p.v, p.vs);
+}
+
 template <int KS, bool KEYS, bool PLAIN>
 cudaError_t launch_one(const BwdParams& bp, cudaStream_t stream) {
   const SdpaParams& p = bp.p;
@@ -678,8 +690,8 @@ cudaError_t launch_one(const BwdParams& bp, cudaStream_t stream) {
   tp.wait_budget_ns = bp.expire ? 20000000ull : ptx::kWaitBudgetNs;   // 20 ms in the time-out test
   tp.splits = 1;
   while (tp.splits < 8 && tiles * heads * p.batch * tp.splits * 2 <= 148 && tp.splits * 2 <= steps) tp.splits *= 2;
-  return launch_dependent_cluster(kern, dim3((unsigned)(tiles * tp.splits), (unsigned)heads, (unsigned)p.batch), kThreads, dim3((unsigned)tp.splits),
-                                  smem_bytes(PLAIN), stream, bp, tp);
+  return launch_cluster(!KEYS || !gradients_over_keys(bp), kern, dim3((unsigned)(tiles * tp.splits), (unsigned)heads, (unsigned)p.batch), kThreads,
+                        dim3((unsigned)tp.splits), smem_bytes(PLAIN), stream, bp, tp);
 }
 
 template <int KS>

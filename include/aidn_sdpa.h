@@ -237,7 +237,9 @@ AIDN_API int aidn_paged_kv_append(const void* new_keys, const void* new_values, 
  * launch's argument block with fwd.out = O and fwd.lse = the statistics, both read here; masks, bias, causal offset,
  * kv_len, grouped-query heads and paged K/V mean what they mean forward (no gradient is produced for a bias).  dO has
  * O's dtype; the gradients are dense fp32: dq [B, Hc, Sq, D], dk / dv [B, Hc / group, Sk, D], Hc = the heads of the
- * handle's shard.  fwd.workspace must hold aidn_sdpa_backward_workspace_bytes().  Logit softcap is not supported. */
+ * handle's shard.  fwd.workspace must hold aidn_sdpa_backward_workspace_bytes().  Logit softcap is not supported.  dq, dk and dv must overlap
+ * neither one another nor what the call reads: dK / dV may be formed while dQ is.  (fp32 gradients laid element by element over K and V are
+ * noticed, and formed behind dQ.) */
 typedef struct {
   aidn_sdpa_args fwd;
   const aidn_paged_kv* paged; /* NULL for contiguous K / V                                                     */

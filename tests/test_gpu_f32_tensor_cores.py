@@ -441,3 +441,26 @@ def test_projections_of_values_that_are_not_finite(heads, d, S):
     torch.cuda.synchronize()
     ref = O.mha_forward(xf[:1], *wfs, heads)
     assert np.abs(out[:1].cpu().numpy() - ref).max() <= 1e-5 * np.abs(ref).max() and torch.isnan(out[1]).all()
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk", [(1, 2, 2, 512, 640), (2, 6, 2, 350, 400), (2, 8, 8, 130, 700)])
+@pytest.mark.parametrize("swapped", [False, True])
+def test_backward_gradients_over_keys(B, Hq, Hkv, Sq, Sk, swapped):
+    """dK and dV in the place of K and V, or of V and K: the same bits as in buffers of their own, dQ too."""
+    D = 64
+    q, k, v, g = (gen((B, H, S, D), "f32", i, 1.0)[0] for i, (H, S) in enumerate(((Hq, Sq), (Hkv, Sk), (Hkv, Sk), (Hq, Sq))))
+    out, lse = torch.empty(B, Hq, Sq, D, device="cuda"), torch.empty(B, Hq, Sq, device="cuda")
+    with N.Handle(device=0, qkv_dtype=N.F32, out_dtype=N.F32, head_dim=D, num_q_heads=Hq, num_kv_heads=Hkv, emit_lse=True) as h:
+        stream = torch.cuda.current_stream().cuda_stream
+        ws = torch.empty(h.backward_workspace_bytes(B, Sq), dtype=torch.uint8, device="cuda")
+        dq = [torch.empty_like(q) for _ in range(2)]
+        dk, dv = torch.empty_like(k), torch.empty_like(v)
+        k2, v2 = k.clone(), v.clone()
+        common = dict(q=q.data_ptr(), out=out.data_ptr(), lse=lse.data_ptr(), batch=B, seq_q=Sq, seq_kv=Sk, stream=stream)
+        h.launch(k=k.data_ptr(), v=v.data_ptr(), **common)
+        for dq_, k_, v_, dk_, dv_ in ((dq[0], k, v, dk, dv), (dq[1], k2, v2, *((v2, k2) if swapped else (k2, v2)))):
+            h.backward(k=k_.data_ptr(), v=v_.data_ptr(), dout=g.data_ptr(), dq=dq_.data_ptr(), dk=dk_.data_ptr(), dv=dv_.data_ptr(), workspace=ws.data_ptr(),
+                       workspace_bytes=ws.numel(), **common)
+        h.poll(stream)
+    assert torch.equal(dq[0], dq[1])
+    assert torch.equal(dk, v2 if swapped else k2) and torch.equal(dv, k2 if swapped else v2)
