@@ -134,16 +134,17 @@ __global__ void __launch_bounds__(kThreads, 1)
     tmem_alloc(smem_u32(tmem_ptr_smem), C::kTmemCols);
     tmem_relinquish();
   }
+  // The set-up above runs under the end of the launch before; the other warps touch memory only behind this one's loads, and their waits, which
+  // are bounded, begin behind its own.
+  if (warp == 0) pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
   if (warp == 0) {
     // ============================================ TMA producer ============================================
-    // The set-up above runs under the end of the launch before; the other warps touch memory only behind this one's loads.  Not in
-    // launches of several waves: their CTAs would start wherever an SM comes free, and the tiles in flight share less in L2 (layer of
-    // B4 S2048 and 32 heads of 128: 1172 -> 1184 us).
-    pdl_wait();
+    // Dependents only of launches of one wave: where there are several, their CTAs would start wherever an SM comes free, and the tiles in
+    // flight share less in L2 (layer of B4 S2048 and 32 heads of 128: 1172 -> 1184 us).
     if (gp.total_tiles <= (int)gridDim.x) pdl_trigger();
     const bool leader = elect_one();
     uint32_t kb_total = 0;   // K blocks loaded so far (ring position)

@@ -445,6 +445,9 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
     tmem_alloc(smem_u32(tmem_ptr_smem), kTmemCols);
     tmem_relinquish();
   }
+  // The set-up above runs under the end of the launch before.  Of the other warps none touches memory ahead of an item that the producer has
+  // published, but their waits are bounded: they begin behind its own (by every warp, it costs the softmax loop registers).
+  if (warp == kProducerWarp) pdl_wait();
   if (warp == 1 && by_length(p)) {
     pdl_wait();
     length_order(p, lane, order);
@@ -854,12 +857,7 @@ __global__ void __launch_bounds__(Roles<EPI>::kThreads, 1)
     }
   } else {
     setmaxnreg_dec<R::kOtherRegs>();
-    if (warp == kProducerWarp) {
-      // The set-up above runs under the end of the launch before.  Every other warp touches memory only behind an item that this one
-      // has published (in their code, even ahead of the barrier, the wait costs the softmax loop registers).
-      pdl_wait();
-      pdl_trigger();
-    }
+    if (warp == kProducerWarp) pdl_trigger();
   }
 
   // ---- K / V loads: one 64-key sub-tile into ring position t (waits until the position's slot is free) ----

@@ -1,6 +1,11 @@
 """Launches that are set up under the end of the one before (csrc/common.cuh, launch_dependent), back to back on one stream: what a launch reads was
 written by the one in front of it, and what it writes is read by that one.  Every result is the same bits as with a synchronisation
 behind every call."""
+import ctypes
+import os
+import shutil
+import subprocess
+
 import numpy as np
 import pytest
 import torch
@@ -143,4 +148,62 @@ def test_layers_of_different_weights(B, S, heads, d):
              for w, x, y in zip(weights, acts, acts[1:])]
     _same_bits(steps, lambda: acts[1:])
     h.poll(stream)
+    h.close()
+
+
+@pytest.fixture(scope="module")
+def early_trigger(tmp_path_factory):
+    """(milliseconds, stream): enqueues a launch of one thread that lets dependent ones begin and then takes that long."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("no nvcc")
+    lib = str(tmp_path_factory.mktemp("cuda") / "early_trigger.so")
+    src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "cuda", "early_trigger.cu")
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC", "-o", lib, src], check=True, capture_output=True)
+    call = ctypes.CDLL(lib).early_trigger
+    call.argtypes = [ctypes.c_int, ctypes.c_void_p]
+
+    def enqueue(ms, stream):
+        assert call(ms, stream) == 0
+    return enqueue
+
+
+@pytest.mark.parametrize("kind", ["prefill", "layer", "fp32", "backward"])
+def test_bounded_waits_count_their_own_time(kind, early_trigger):
+    """A launch that is set up beside one of 2.4 s, above the 2 s that any wait may take: none of its waits runs out."""
+    stream = torch.cuda.current_stream().cuda_stream
+    B, H, S, D = 1, 4, 300, 64
+    dtype = N.F32 if kind == "fp32" else N.BF16
+    q, k, v, g = (gen((B, H, S, D), "f32" if kind == "fp32" else "bf16", i)[0] for i in range(4))
+    weights = [gen((H * D, H * D), "bf16", 10 + i, (H * D) ** -0.5)[0] for i in range(4)]
+    out, lse = torch.empty(B, H, S, D, device="cuda"), torch.empty(B, H, S, device="cuda")
+    grads = [torch.empty(B, H, S, D, device="cuda") for _ in range(3)]
+    h = N.Handle(device=0, qkv_dtype=dtype, out_dtype=N.BF16 if kind == "layer" else N.F32, head_dim=D, num_q_heads=H, num_kv_heads=H, emit_lse=kind == "backward")
+    ws = torch.empty(1 << 24, dtype=torch.uint8, device="cuda")
+    assert ws.data_ptr() % 256 == 0
+    common = dict(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), out=out.data_ptr(), batch=B, seq_q=S, seq_kv=S, stream=stream,
+                  lse=lse.data_ptr() if kind == "backward" else None)
+    if kind == "layer":
+        run = lambda: h.mha_forward(input=q.data_ptr(), q_weight=weights[0].data_ptr(), k_weight=weights[1].data_ptr(), v_weight=weights[2].data_ptr(),
+                                    out_weight=weights[3].data_ptr(), out=out.data_ptr(), batch=B, seq=S, input_dtype=N.BF16, weight_dtype=N.BF16, out_dtype=N.F32,
+                                    workspace=ws.data_ptr(), workspace_bytes=ws.numel(), stream=stream)
+    elif kind == "backward":
+        h.launch(**common)
+        g = g.float()
+        run = lambda: h.backward(dout=g.data_ptr(), dq=grads[0].data_ptr(), dk=grads[1].data_ptr(), dv=grads[2].data_ptr(), workspace=ws.data_ptr(),
+                                 workspace_bytes=ws.numel(), **common)
+    else:
+        run = lambda: h.launch(**common)
+    results = grads if kind == "backward" else [out]
+    run()
+    h.poll(stream)
+    want = [t.clone() for t in results]
+    for t in results:
+        t.fill_(float("nan"))
+    torch.cuda.synchronize()
+    early_trigger(2400, stream)
+    run()
+    h.poll(stream)
+    for got, ref in zip(results, want):
+        assert torch.equal(got, ref)
     h.close()
