@@ -105,3 +105,22 @@ def test_line_of_equal_shares(batch, kv_heads, keys, dim, shares):
     chunks = -(-keys // chunk)
     plain = -(-(items * chunks * (dim + 2) * 4) // 256) * 256 if chunks > 1 else 0
     assert need == (max(plain, even) if shares else plain)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_weights_are_not_rounded_to_16_bits(shape):
+    """Against 64 bits.  Operands of 16 bits are exact, weights of two 16-bit terms are off by 2^-18 of themselves at most, exponentials and sums in fp32 by less
+    than that again each: 2^-16 of the largest value.  Weights of one term, whose number that are rounded depends on how the keys are shared, miss it."""
+    B, Hq, Hkv, Sk, D, dtype = shape
+    q, qf = gen((B, Hq, 1, D), dtype, 1)
+    k, kf = gen((B, Hkv, Sk, D), dtype, 2)
+    v, vf = gen((B, Hkv, Sk, D), dtype, 3)
+    lens = np.maximum(_lens("ragged", B, Sk), 1)
+    out, _, info = run_gpu(q, k, v, dtype=dtype, path=N.PATH_DECODE, kv_len=torch.from_numpy(lens).cuda())
+    assert info["launches"] == 2
+    for b in range(B):
+        n, g = lens[b], Hq // Hkv
+        s = np.einsum("hgd,hkd->hgk", qf[b, :, 0].reshape(Hkv, g, D).astype(np.float64), kf[b, :, :n].astype(np.float64)) / np.sqrt(D)
+        w = np.exp(s - s.max(-1, keepdims=True))
+        want = np.einsum("hgk,hkd->hgd", w / w.sum(-1, keepdims=True), vf[b, :, :n].astype(np.float64)).reshape(Hq, D)
+        assert np.abs(out[b, :, 0].cpu().numpy() - want).max() <= 2.0 ** -16 * np.abs(vf).max(), b
