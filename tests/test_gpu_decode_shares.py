@@ -124,3 +124,8 @@ def test_weights_are_not_rounded_to_16_bits(shape):
         w = np.exp(s - s.max(-1, keepdims=True))
         want = np.einsum("hgk,hkd->hgd", w / w.sum(-1, keepdims=True), vf[b, :, :n].astype(np.float64)).reshape(Hq, D)
         assert np.abs(out[b, :, 0].cpu().numpy() - want).max() <= 2.0 ** -16 * np.abs(vf).max(), b
+
+
+@pytest.mark.parametrize("batch,kv_heads,keys,dim,shares", [(87, 2, 128, 128, False), (216, 1, 239, 128, True), (209, 2, 166, 64, False), (168, 2, 274, 64, True)])
+def test_line_of_few_steps(batch, kv_heads, keys, dim, shares):
+    test_line_of_equal_shares(batch, kv_heads, keys, dim, shares)
