@@ -99,3 +99,23 @@ def test_masks_with_softcap_and_lengths(shape, kind):
     h.close()
     ref = O.sdpa(qf, kf, vf, mask=m, mask_kind=mask_kind, softcap=20.0, kv_len=lens)
     compare(out, ref[0] if isinstance(ref, tuple) else ref, "bf16", f"{shape} {kind}")
+
+
+@pytest.mark.parametrize("shape", [(1, 3, 3, 129, 120, 64), (2, 2, 1, 300, 333, 32), (2, 2, 2, 200, 450, 128)])
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("layout", LAYOUTS)
+@pytest.mark.parametrize("softcap", [0.0, 20.0])
+def test_masks_fp32(shape, kind, layout, softcap):
+    """fp32 calls: floats through the row warps' tiles, one row of them and bytes as bits, whole tiles of rows and the last ones."""
+    B, Hq, Hkv, Sq, Sk, D = shape
+    (q, qf), (k, kf), (v, vf) = (gen((B, H, S, D), "f32", i, 1.0) for i, (H, S) in enumerate(((Hq, Sq), (Hkv, Sk), (Hkv, Sk))))
+    dev, m = _mask(shape, kind, layout, 7)
+    mask_kind = {"bytes": N.MASK_KEEP_U8, "floats": N.MASK_KEEP_F32, "bias": N.MASK_ADD_F32}[kind]
+    out = torch.full((B, Hq, Sq, D), float("nan"), device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    with N.Handle(device=0, qkv_dtype=N.F32, out_dtype=N.F32, head_dim=D, num_q_heads=Hq, num_kv_heads=Hkv, mask_kind=mask_kind, softcap=softcap) as h:
+        h.launch(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), out=out.data_ptr(), batch=B, seq_q=Sq, seq_kv=Sk, stream=stream, mask=dev.data_ptr(),
+                 mask_stride=_strides(dev, (B, Hq, Sq, Sk)))
+        h.poll(stream)
+    ref = O.sdpa(qf, kf, vf, mask=m, mask_kind=mask_kind, softcap=softcap)
+    compare(out, ref[0] if isinstance(ref, tuple) else ref, "f32", f"{shape} {kind} {layout} {softcap}")
