@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kThreads, 1) sdpa_f32_sm100_kernel(const __gri
     auto fetch_keep = [&](int j) {
       int rows, keys;
       const int64_t at0 = mask_at(j, quarter, half, rows, keys);
-      keep_next = masktile::keep_bits_of(p, at0, p.mask_stride[2], p.mask_stride[3], rows, keys, lane);
+      keep_next = masktile::keep_bits_of<true>(p, at0, p.mask_stride[2], p.mask_stride[3], rows, keys, lane);
     };
     // p = 2^((s - m) c): s is the raw score and c = scale log2(e), or the finished logit and log2(e) with a bias or a softcap
     const bool raw = MODE != kSoftcap && !add;
