@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       // shared memory and of the other 32 in registers.  Rows are keys: the lane's own, bits of 64 queries or a bias of the first 32.
       const bool add = MASKED && p.mask_kind == AIDN_MASK_ADD_F32;
       uint32_t keep0 = ~0u, keep1 = ~0u;
-      float bias[MASKED ? 32 : 1];
+      float bias[MASKED ? 32 : 1];   // (with `late` below more than dK / dV has registers for: 112 bytes of stack, 200 stored and 208 read, which the loads' latency hides)
       auto mask_of = [&](int j, int c, int& rows, int& keys) {   // streamed rows from c on: offset in the mask, and how much of it there is
         const int64_t col = (int64_t)step_tile<KEYS>(w, j) * kT + half * 64 + c, own = (int64_t)w.tile * kT + quarter * 32;
         const int64_t query = KEYS ? col : own, key = KEYS ? own : col;
@@ -687,10 +687,11 @@ cudaError_t launch_t(const BwdParams& bp, cudaStream_t stream, int* launches, co
   // the ones with an item more than the others (by the snake the first where the whole waves are even in number).  Where they are not, heads
   // of 64 only share the memory: 182 items of each, B1 H7 S3264, 143.6 -> 146.8 us (one after the other, with a dependent dQ, 142.9), 640 and 160, B2 Hq64 / Hkv16 S587, 112.0 -> 113.4
   // (110.1); where they are: 312, B3 H8 S1574, 119 -> 103, 448 and 112, B2 Hq32 / Hkv8 S824, 91 -> 82.  One wave (S1020 35.0 -> 33.8), items of unequal length (S2018
-  // causal 98 -> 94) and heads of 128 (252 items, B4 H9 S850, 80.6 -> 79.9) gain either way.
+  // causal 98 -> 94), heads of 128 (252 items, B4 H9 S850, 80.6 -> 79.9) and masks, whose loads are waited for (B8 H13 1139 x 97 with a bias 114.4 -> 104.9, B3 H15 S1146
+  // with a keep-mask 349 -> 333), gain either way.
   const int64_t waves_q = (items_q + sms - 1) / sms, waves_kv = (items_kv + sms - 1) / sms;
   const int64_t spare = waves_q * sms - items_q, more = items_kv - (waves_kv - 1) * sms;
-  const bool beside = shorter && (HD == 128 || p.causal || waves_q == 1 || (waves_kv % 2 == 1 && more <= spare));
+  const bool beside = shorter && (HD == 128 || p.causal || masked || waves_q == 1 || (waves_kv % 2 == 1 && more <= spare));
   if (shorter) {
     e = launch_dependent(kq, dim3(grid_q), kThreads, smem_q, stream, tq, tk, tv, tdo, sp);
   } else {
