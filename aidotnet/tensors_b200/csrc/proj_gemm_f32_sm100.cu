@@ -456,8 +456,9 @@ cudaError_t launch_t(F32GemmParams& f, int splits, cudaStream_t stream) {
 // A block of K takes 1190 at 32 and 2330 at 160 columns, with W cut in place 1950 and 3300 at 64 and 128; the rest 7600 at 48 and 10000
 // at 144 columns, the merge of a cluster 7000 to 12000, a launch for the terms of W 5000 and an element 1 / 220 (they are written and
 // read again).  Clusters only where all of a launch's CTAs are resident at once.  Layers, in us, before -> with these rules:
-//   rows x width  16 x 512 35 -> 25, 100 x 1024 57 -> 48, 256 x 2048 118 -> 92, 384 x 3072 268 -> 245, 1024 x 1024 125 -> 102,
-//   2048 x 3072 1416 -> 1242; 1576 x 512 (143 tiles of 144 and of 48 columns) 83 -> 57
+//   rows x width  16 x 512 35 -> 25, 100 x 1024 57 -> 46, 256 x 2048 123 -> 93, 384 x 3072 256 -> 215, 1024 x 1024 127 -> 101,
+//   2048 x 3072 1294 -> 1124; 1576 x 512 (143 tiles of 144 and of 48 columns) 83 -> 57
+// (The instantiations that cut W have 96 registers a thread and keep 24 and 40 bytes of stack at 64 and 128 columns.)
 // (`launched`: the launch for the terms is there for another GEMM of the layer already, and costs this one nothing.)
 ProjPlanF32 proj_gemm_f32_sm100_plan(int64_t rows, int64_t k, int64_t n, int mats, int num_sms, bool images, bool launched) {
   const int64_t cols = n * mats, launch = launched ? 0 : 5000;

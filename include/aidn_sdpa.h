@@ -175,7 +175,8 @@ AIDN_API int aidn_sdpa_create(const aidn_sdpa_desc* desc, aidn_sdpa_t* out);
 /* Bytes of caller workspace for a launch of this shape; < 0 on error.  A decode launch needs them (or the handle's scratch);
  * a tcgen05 prefill with fewer work items than SMs uses them for the partial results of its split keys, and runs unsplit
  * when the workspace is NULL or smaller.  For a decode this may be more than a launch needs
- * at least: one with kv_len uses all of it to cut the keys of all sequences into equal shares, and cuts by sequence with less.  Launches that overlap on the GPU must not share a workspace, and a launch that
+ * at least: one with kv_len uses all of it to cut the keys of all sequences into equal shares, and cuts by sequence with less.  (In equal shares
+ * the cuts fall by all lengths together, so that the last bits of a sequence's result depend on the other lengths of its batch.)  Launches that overlap on the GPU must not share a workspace, and a launch that
  * was captured into a graph uses the same one at every replay. */
 AIDN_API int64_t aidn_sdpa_workspace_bytes(aidn_sdpa_t h, int64_t batch, int64_t seq_q, int64_t seq_kv);
 /* Enqueues the attention forward on `cu_stream` (a CUstream / cudaStream_t).  No allocation, no synchronisation; safe
