@@ -428,9 +428,7 @@ __device__ __forceinline__ uint32_t pack_rest(float a, float b, uint32_t packed)
 }
 
 // A warp's query heads of one KV head and what it has summed up for them.
-// TWO_TERMS: the weights go into their product as two 16-bit terms.  The fewer partials the keys are cut into, the fewer weights are 1 without rounding (each
-// partial's largest): equal shares with one term were 0.7 to 4 % further from 64 bits than chunks in every one of 24 calls.
-template <typename T, int D, bool NH16, bool TWO_TERMS>
+template <typename T, int D, bool NH16>
 struct RingWarp {
   static constexpr int KI = D / 32, VX = D / 64, MT = D / 16, HN = NH16 ? 2 : 1;
   using R = RingCfg<D>;
@@ -458,9 +456,10 @@ struct RingWarp {
   }
 
   // The 16 keys from kb on, in the stage at `base`; bit i of rows_ok: key kb + i counts.  `refill` is called when the stage has been read.
+  // two_terms: the weights go into their product as two 16-bit terms (sdpa_decode_stream_kernel).
   template <typename Refill>
   __device__ __forceinline__ void step(const SdpaParams& p, uint32_t base, uint32_t rows_ok, int b, int h0, int nheads, int64_t kb, int64_t L, int g,
-                                       int c, Refill refill) {
+                                       int c, bool two_terms, Refill refill) {
     // ---- S = Q K^T ------------------------------------------------------------------------------------
     float sacc[2][4];
 #pragma unroll
@@ -555,7 +554,7 @@ struct RingWarp {
     const uint32_t pb0 = pack_pair<T>(pr[0][0], pr[0][1]), pb1 = pack_pair<T>(pr[1][0], pr[1][1]);
     const uint32_t pc0 = pack_pair<T>(pr[0][2], pr[0][3]), pc1 = pack_pair<T>(pr[1][2], pr[1][3]);
     uint32_t rb0 = 0, rb1 = 0, rc0 = 0, rc1 = 0;
-    if (TWO_TERMS) {
+    if (two_terms) {
       rb0 = pack_rest<T>(pr[0][0], pr[0][1], pb0);
       rb1 = pack_rest<T>(pr[1][0], pr[1][1], pb1);
       rc0 = pack_rest<T>(pr[0][2], pr[0][3], pc0);
@@ -574,7 +573,7 @@ struct RingWarp {
       const uint32_t a3 = __byte_perm(vw[2][xh][wh], vw[3][xh][wh], sel);
       mma16816<T>(acc[m][0], a0, a1, a2, a3, pb0, pb1);
       if (NH16) mma16816<T>(acc[m][HN - 1], a0, a1, a2, a3, pc0, pc1);
-      if (TWO_TERMS) {
+      if (two_terms) {
         mma16816<T>(acc[m][0], a0, a1, a2, a3, rb0, rb1);
         if (NH16) mma16816<T>(acc[m][HN - 1], a0, a1, a2, a3, rc0, rc1);
       }
@@ -671,7 +670,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, CTAS)
     return __ballot_sync(0xffffffffu, row >= 0) & 0xffffu;
   };
 
-  RingWarp<T, D, NH16, false> rw;
+  RingWarp<T, D, NH16> rw;
   rw.begin(p, b, h0, nheads, g, c);
 
   // prologue: fill the ring (a group is committed per stage even when it is empty, so that wait_group counts steps)
@@ -706,7 +705,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, CTAS)
     for (int s = 0; s < kRingStages; ++s)
       if (s == stage) rows_ok = row_mask[s];
 
-    rw.step(p, base, rows_ok, b, h0, nheads, kb, L, g, c, [&] {
+    rw.step(p, base, rows_ok, b, h0, nheads, kb, L, g, c, false, [&] {
         const int64_t kb_new = kb + kRingStages * kStride;
         const int32_t ent_new = ent_next;
         ent_next = entry_of(kb_new + kStride);
@@ -948,7 +947,11 @@ __global__ void __launch_bounds__(kDecWarps * 32, kRingCtas<D>) sdpa_decode_stre
     return mask;
   };
 
-  RingWarp<T, D, NH16, true> rw;
+  // A weight is 1 without rounding where its key is the largest of a partial, and shares have fewer partials than chunks: with weights of one term, outputs
+  // are 0.7 to 4 % further from 64 bits than by chunks.  16-bit outputs therefore get two (16 sequences of up to 2048 keys with their projection
+  // 2.44e-3 -> 1.94e-3, by chunks 2.42e-3; the time is the same).  fp32 outputs, which would move by what the rounding is, 1.5e-3, keep the values they have.
+  const bool two_terms = !p.out_f32;
+  RingWarp<T, D, NH16> rw;
   rw.begin(p, cur.b, h0, nheads, g, c);
   for (int x = x0; x < x1; ++x) {
     const int stage = (x - x0) % kRingStages;
@@ -958,7 +961,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, kRingCtas<D>) sdpa_decode_stre
 #pragma unroll
     for (int s = 0; s < kRingStages; ++s)
       if (s == stage) rows_ok = row_mask[s];
-    rw.step(p, my_ring + stage * R::kStageBytes, rows_ok, cur.b, h0, nheads, (int64_t)cur.s * 16, cur.L, g, c, [&] {
+    rw.step(p, my_ring + stage * R::kStageBytes, rows_ok, cur.b, h0, nheads, (int64_t)cur.s * 16, cur.L, g, c, two_terms, [&] {
       const uint32_t mask = feed(stage);
 #pragma unroll
       for (int s = 0; s < kRingStages; ++s)
