@@ -1428,9 +1428,9 @@ int64_t decode_stream_bytes(const SdpaParams& p, int dtype, int num_sms, const D
   const int kv_heads = p.head_count / p.group, n = stream_ctas(p.head_dim, num_sms);
   const int64_t items = (int64_t)p.batch * kv_heads, steps = (p.seq_kv + 15) / 16;
   if (items < 48 || items * steps > 0x3fffffff || p.batch > 256 || kv_heads > n * kDecWarps) return 0;
-  // Less than 2.5 steps to a warp, 3 with heads of 64: 174 items of up to 128 keys, D 128, 9.6 -> 11.0 us, 255 of 134 in a pool, with its projection, 22.7 -> 24.4; heads of
-  // 64: 418 items of 166 keys 10.6 -> 11.3, 225 of 143 22.7 -> 25.5.  Above that 216 items of 239 keys, D 128, 28.1 -> 26.7, 336 of 274, D 64, 34.9 -> 33.6.
-  if (items * steps * 2 < (int64_t)n * kDecWarps * (p.head_dim == 64 ? 6 : 5)) return 0;
+  // Less than 2.5 steps to a warp, 3.3 with heads of 64: 174 items of up to 128 keys, D 128, 9.6 -> 11.4 us, 255 of 134 in a pool, with its projection, 22.7 -> 25.4; heads of
+  // 64: 418 items of 166 keys 10.6 -> 14.0, 402 of 218 10.4 -> 11.5, 225 of 143 22.8 -> 27.2.  Above that 216 items of 239 keys, D 128, 28.1 -> 26.7, 336 of 274, D 64, 34.9 -> 33.6.
+  if (items * steps * 6 < (int64_t)n * kDecWarps * (p.head_dim == 64 ? 20 : 15)) return 0;
   // Long launches stream at the memory's rate either way, and chunks read larger pieces: of 400 MB, or with the heads of a token side by
   // side of 1.2 GB, on (2048 items of 4096 keys 382 -> 405 us; in a pool 512 items of 4096 keys, 1.07 GB, 115 -> 106).
   if (items * p.seq_kv * p.head_dim * 4 > (p.block_table || p.ks[1] < p.ks[2] ? 1200000000 : 400000000)) return 0;
