@@ -1442,6 +1442,9 @@ int64_t decode_stream_bytes(const SdpaParams& p, int dtype, int num_sms, const D
   decode_plan_clusters(q, dtype, num_sms, &plan);
   const int64_t parts = (int64_t)plan.cluster * plan.nchunks;
   if (plan.cluster > 1 && items * parts <= n && p.seq_kv / parts * p.head_dim < 100000) return 0;
+  // A fifth more CTAs than are resident at once, in clusters of two, few keys and heads of 64: the rest finds places soon enough (224 to 264 items of up to 450 to 512 keys
+  // 9.8 to 11.4 us, in shares 12.0; in a pool 12.2 and 15.2).
+  if (plan.cluster == 2 && p.head_dim == 64 && p.seq_kv <= 512 && items * parts * 5 <= (int64_t)n * 6) return 0;
   *ctas = n;
   return ((int64_t)(n * kDecWarps / kv_heads) + p.batch) * kv_heads * p.group * (p.head_dim + 2) * (int64_t)sizeof(float);
 }

@@ -130,6 +130,6 @@ def test_weights_of_two_terms(shape):
     assert got <= 1.1 ** 2 * own, (got / own) ** 0.5
 
 
-@pytest.mark.parametrize("batch,kv_heads,keys,dim,shares", [(87, 2, 128, 128, False), (216, 1, 239, 128, True), (209, 2, 166, 64, False), (201, 2, 218, 64, False), (168, 2, 274, 64, True)])
+@pytest.mark.parametrize("batch,kv_heads,keys,dim,shares", [(87, 2, 128, 128, False), (216, 1, 239, 128, True), (209, 2, 166, 64, False), (201, 2, 218, 64, False), (168, 2, 274, 64, True), (126, 2, 450, 64, False), (134, 2, 450, 64, True)])
 def test_line_of_few_steps(batch, kv_heads, keys, dim, shares):
     test_line_of_equal_shares(batch, kv_heads, keys, dim, shares)
